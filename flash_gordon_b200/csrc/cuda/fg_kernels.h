@@ -172,9 +172,12 @@ typedef struct fgk_nucleus_launch {
     fg_sampler_config config0;
     uint32_t config_count;
     const float *uniforms;
-    float *scratch;          /* ctas rows of scratch_stride floats */
+    float *scratch;          /* ctas / team rows of scratch_stride floats */
     uint64_t scratch_stride;
-    uint32_t ctas;           /* persistent CTAs, one scratch row each */
+    void *seen;              /* with a history: per CTA seen_stride pairs of 8 bytes */
+    uint64_t seen_stride;
+    uint32_t ctas;           /* persistent CTAs, a multiple of `team` */
+    uint32_t team;           /* CTAs that share a row: 1, 2, 4 or 8 */
     const uint32_t *history_global;
     uint64_t history_stride_words;
     const void *history_meta;
@@ -182,7 +185,9 @@ typedef struct fgk_nucleus_launch {
     fgk_select_output out;
 } fgk_nucleus_launch;
 
-int fgk_nucleus_prepare(void);
+/* most_teams[i]: how many teams of 2^i CTAs the current device runs at a time (0: none) */
+#define FGK_NUCLEUS_TEAM_SIZES 4
+int fgk_nucleus_prepare(uint32_t most_teams[FGK_NUCLEUS_TEAM_SIZES]);
 int fgk_launch_nucleus_select(const fgk_nucleus_launch *launch, void *stream);
 /* the history pass (fills history_global / history_meta) */
 int fgk_launch_history_build(const fgk_stream_launch *launch, void *stream);

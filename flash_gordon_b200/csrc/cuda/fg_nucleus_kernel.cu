@@ -3,28 +3,39 @@
 // finite logit.  The reference caps candidates at 64; this is the documented
 // generalisation for rows whose nucleus spans tens of thousands of tokens.
 //
-// The vocabulary is never sorted.  A persistent CTA per SM streams a row from HBM once
-// (penalties applied on the way) into its own scratch row, which stays in L2, and then
-// narrows down two positions of the (value descending, id ascending) order by MSB-first
-// radix descent over the 32-bit monotone value key, 12 + 12 + 8 bits: first the element
-// where the cumulative raw-softmax mass reaches top_p, then the element the draw lands
-// on under the tempered weights.  Each level is one pass over the scratch row that
-// builds a bucketed histogram of counts and masses in shared memory, followed by a
-// block-wide prefix sum from the top bucket down.  Equal values are resolved on the
-// id with the same descent (counts only).
+// The vocabulary is never sorted.  A row belongs to a team of one, two, four or eight CTAs (a
+// thread-block cluster), each of which takes a range of its columns.
 //
-// Masses are exp(s - max) in fp64, accumulated as 2^-40 fixed point in 64-bit
-// integers: integer addition is associative, so the result does not depend on the
-// order threads arrive in, and the 1e-12 grid is far below one element's weight.
-// The reference adds doubles left to right; the two agree unless the top-p bound or
-// the draw falls within ~1e-11 (relative) of an edge of the CDF.
+// The short way.  One pass over the logits counts the values into 16,384 narrow buckets in
+// shared memory.  A bucket holds the number of its members and the first two moments of
+// their distances from its middle, which give its raw and its tempered softmax mass alike
+// (a short series); prefix sums over the buckets' masses tell in which bucket the
+// cumulative mass reaches top_p and, to within a bucket or two, where the draw lands.  A
+// second pass (from L2) gathers the members of those buckets, a few hundred, which are
+// ordered exactly: the element at which top_p is reached, then the element drawn.
+//
+// The long way, for rows the short one cannot take (heavy ties, extreme temperatures): the
+// team's first CTA works on the penalised row in its scratch memory, histogram pass by
+// histogram pass, down to an MSB-first radix descent over the 32-bit monotone value key and,
+// among equal values, over the id.
+//
+// Masses are exp(s - max) as 2^-40 fixed point in 64-bit integers: integer addition is
+// associative, so the result does not depend on the order threads arrive in, and the 1e-12
+// grid is far below one element's weight.  The reference adds doubles left to right; the two
+// agree unless the top-p bound or the draw falls within ~1e-11 (relative) of an edge of the
+// CDF.
+#include <cooperative_groups.h>
+
+#include <cstddef>
+
 #include "fg_block_select.cuh"
 #include "fg_kernels.h"
 
 namespace fgk {
 
 
-constexpr int kNucleusThreads = 1024;
+constexpr int kNucleusThreads = 512;  // two CTAs to an SM: one streams while the other scans and sorts
+constexpr int kNucleusWarps = kNucleusThreads / 32;
 constexpr int kBuckets = 4096;
 // per bucket: two masses (raw and tempered weights) and a count
 constexpr size_t kNucleusHistogramBytes = kBuckets * (2 * sizeof(unsigned long long) + sizeof(uint32_t));
@@ -38,8 +49,11 @@ struct NucleusParams {
     SamplerConfig config0;
     uint32_t config_count;
     const float *uniforms;
-    float *scratch;            // gridDim.x rows of scratch_stride floats
+    uint32_t team;             // CTAs that share a row (the cluster size): 1, 2, 4 or 8
+    float *scratch;            // gridDim.x / team rows of scratch_stride floats, used on the long way
     uint64_t scratch_stride;
+    float2 *seen;              // per CTA seen_stride (penalised value, id) pairs
+    uint64_t seen_stride;
     // history structures built by history_build_kernel, one per (row, split)
     const uint32_t *history_global;
     uint64_t history_stride_words;
@@ -53,11 +67,11 @@ struct NucleusShared {
     unsigned long long *other_mass;   // kBuckets entries: the tempered masses while `mass` holds the raw ones
     uint32_t *count;                  // kBuckets entries
     double table[64];                 // 2^(j/64)
-    unsigned long long scan_mass[32];
-    uint32_t scan_count[32];
+    unsigned long long scan_mass[kNucleusWarps];
+    uint32_t scan_count[kNucleusWarps];
     unsigned long long total_mass;
-    float reduce_max[32];
-    uint32_t reduce_count[32];
+    float reduce_max[kNucleusWarps];
+    float zero;
     // result of a scan
     uint32_t hit_bucket;
     unsigned long long hit_mass_before;
@@ -335,15 +349,26 @@ __device__ void descend(NucleusShared &sh, const float *values, uint32_t vocab, 
 // paid), a prefix sum finds the bucket in which the target is reached, a second pass
 // gathers that bucket's members — a few hundred — and they are ordered exactly.
 
-constexpr uint32_t kListCap = 2048;
+constexpr uint32_t kListCap = 1024;    // members of a bucket the long way takes
+constexpr uint32_t kOrderCap = 2048;   // entries order_members takes
+
+// Entries to be ordered and the memory that takes.
+struct OrderWork {
+    float *value;
+    uint32_t *id;
+    float *sorted_value;
+    uint32_t *sorted_id;
+    unsigned long long *weight;  // of the sorted entries, then their running sum
+};
 
 struct NucleusList {
     float value[kListCap];
     uint32_t id[kListCap];
     float sorted_value[kListCap];
     uint32_t sorted_id[kListCap];
-    unsigned long long weight[kListCap];  // of the sorted entries, then their running sum
+    unsigned long long weight[kListCap];
     uint32_t count;
+    __device__ __forceinline__ OrderWork work() { return {value, id, sorted_value, sorted_id, weight}; }
 };
 
 // (fp32 arithmetic: the bucket edges need not be exact, only the same in every pass and
@@ -421,6 +446,7 @@ __device__ unsigned long long find_crossing_up(NucleusShared &sh, TargetOf targe
 
 struct Position {
     uint32_t key, id;            // the element found
+    float value;
     unsigned long long mass;     // cumulative weight up to and including it
     uint32_t rank;               // its 1-based position in the order
     unsigned long long total;    // weight of everything inside
@@ -431,12 +457,166 @@ struct Position {
 // first element of the (value descending, id ascending) order at which the running
 // weight reaches target_of(total) (strict: exceeds it); if it never does, the last
 // element inside.  All threads call.
-// The members of one value bucket (restricted to `inside`), ordered exactly, and among them the
-// first at which the running weight -- `before` plus the weights exp((v - top) * inv_t) of the
-// members so far -- reaches `target` (strict: exceeds it); the last member when none does or
-// when `clipped`.  ok = false: the bucket is empty or holds more than the list takes.  With
-// `also_inv_t` != 0 the weights exp((v - top) * also_inv_t) of the members up to and including
-// the one found are summed into *also_sum.  All threads call.
+// The first `members` entries of the list, those of them that lie `inside`, ordered exactly, and
+// among them the first at which the running weight -- `before` plus the weights
+// exp((v - top) * inv_t) of the members so far -- reaches `target` (strict: exceeds it); the last
+// one when none does or when `clipped`.  ok = false: there is no member inside.  With
+// `also_sum` the weights exp((v - top) * also_inv_t) of the members up to and including the
+// one found are summed into it.  All threads call.
+__device__ __forceinline__ Position order_members(NucleusShared &sh, const OrderWork &list, uint32_t members, double inv_t, float top,
+                                  const Nucleus inside, unsigned long long before, uint32_t rank_before,
+                                  unsigned long long target, bool strict, bool clipped, double also_inv_t,
+                                  unsigned long long *also_sum) {
+    const uint32_t tid = threadIdx.x;
+    Position found;
+    found.ok = false;
+    found.total = 0;
+    const uint32_t listed = members;
+    // order them by their (value, ~id) keys
+    unsigned long long *key = list.weight;
+    if (members <= 256u) {
+        // an entry's rank is the number of larger keys; several threads count for one entry, each
+        // over a part of the list
+        uint32_t *rank = list.sorted_id;
+        for (uint32_t a = tid; a < members; a += kNucleusThreads) {
+            key[a] = select_key(list.value[a], list.id[a]);
+            rank[a] = 0;
+        }
+        __syncthreads();
+        const uint32_t parts = members <= 64u ? 8u : members <= 128u ? 4u : 2u;
+        const uint32_t abreast = kNucleusThreads / parts, length = (members + parts - 1u) / parts;
+        const uint32_t from = tid / abreast * length, to = min(members, from + length), a = tid % abreast;
+        const unsigned long long mine = a < members ? key[a] : 0ull;
+        if (a < members) {
+            uint32_t larger = 0;
+#pragma unroll 4
+            for (uint32_t b = from; b < to; b++) larger += key[b] > mine ? 1u : 0u;
+            atomicAdd(&rank[a], larger);
+        }
+        __syncthreads();
+        const uint32_t place = a < members ? rank[a] : 0u;
+        __syncthreads();
+        if (a < members && tid < abreast) key[place] = mine;
+        __syncthreads();
+    } else {
+        // a bitonic network, the largest first; zeros fill up to a power of two
+        uint32_t size = 512u;
+        while (size < members) size *= 2u;
+        for (uint32_t a = tid; a < size; a += kNucleusThreads)
+            key[a] = a < members ? select_key(list.value[a], list.id[a]) : 0ull;
+        for (uint32_t run = 2; run <= size; run <<= 1) {
+            for (uint32_t stride = run >> 1; stride > 0; stride >>= 1) {
+                __syncthreads();
+                for (uint32_t pair = tid; pair < size / 2; pair += kNucleusThreads) {
+                    const uint32_t low = ((pair & ~(stride - 1)) << 1) | (pair & (stride - 1)), high = low | stride;
+                    const unsigned long long x = key[low], y = key[high];
+                    if ((x < y) == ((low & run) == 0)) {
+                        key[low] = y;
+                        key[high] = x;
+                    }
+                }
+            }
+        }
+        __syncthreads();
+    }
+    constexpr int kOwned = kOrderCap / kNucleusThreads;
+#pragma unroll
+    for (int h = 0; h < kOwned; h++) {
+        const uint32_t a = h * kNucleusThreads + tid;
+        if (a >= members) continue;
+        const unsigned long long mine = key[a];
+        const float value = key_to_float((uint32_t)(mine >> 32));  // (-0.0 comes back as +0.0: see below)
+        list.sorted_value[a] = value;
+        list.sorted_id[a] = ~(uint32_t)mine;
+        list.weight[a] = exp_fixed(((double)value - (double)top) * inv_t, sh.table);
+    }
+    __syncthreads();
+    // (what is not inside the nucleus comes last in the order)
+    uint32_t held = 0;
+    for (uint32_t a = 0; a < members; a += kNucleusThreads) {
+        const uint32_t at = a + tid;
+        held += __syncthreads_count(at < members && inside.holds(float_key(list.sorted_value[at]), list.sorted_id[at]));
+    }
+    members = held;
+    if (members == 0) return found;
+    // running sum: a few entries per thread, then the usual scan
+    {
+        const uint32_t lane = tid & 31u, warp = tid >> 5;
+        unsigned long long sums[kOwned], own = 0;
+#pragma unroll
+        for (int h = 0; h < kOwned; h++) {
+            const uint32_t a = kOwned * tid + h;
+            own += a < members ? list.weight[a] : 0ull;
+            sums[h] = own;
+        }
+        unsigned long long incl = own;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const unsigned long long up = __shfl_up_sync(kFullMask, incl, d);
+            if (lane >= (uint32_t)d) incl += up;
+        }
+        if (lane == 31) sh.scan_mass[warp] = incl;
+        __syncthreads();
+        unsigned long long prior = before + incl - own;
+#pragma unroll
+        for (uint32_t w = 0; w < (uint32_t)kNucleusWarps; w++) {
+            const unsigned long long sum = sh.scan_mass[w];
+            prior += w < warp ? sum : 0ull;
+        }
+#pragma unroll
+        for (int h = 0; h < kOwned; h++) {
+            const uint32_t a = kOwned * tid + h;
+            if (a < members) list.weight[a] = prior + sums[h];
+        }
+        if (tid == 0) sh.hit_bucket = kPaddingId;
+        __syncthreads();
+    }
+    // the first entry whose running sum reaches the target (exactly one thread sees the step)
+    for (uint32_t a = tid; a < members; a += kNucleusThreads) {
+        const unsigned long long here = list.weight[a];
+        const unsigned long long prev = a ? list.weight[a - 1] : before;
+        const bool was = strict ? prev > target : prev >= target;
+        const bool now = strict ? here > target : here >= target;
+        if (!clipped && !was && now) sh.hit_bucket = a;
+    }
+    __syncthreads();
+    uint32_t at = sh.hit_bucket;
+    if (clipped || at == kPaddingId) at = members - 1;
+    found.key = float_key(list.sorted_value[at]);
+    found.id = list.sorted_id[at];
+    found.value = list.sorted_value[at];
+    if (found.value == 0.0f) {  // the zero's own sign, from the unsorted entry
+        if (tid == 0) sh.zero = 0.0f;
+        __syncthreads();
+        for (uint32_t a = tid; a < listed; a += kNucleusThreads)
+            if (list.id[a] == found.id) sh.zero = list.value[a];
+        __syncthreads();
+        found.value = sh.zero;
+    }
+    found.mass = list.weight[at];
+    found.rank = rank_before + at + 1;
+    found.ok = true;
+    __syncthreads();
+    if (also_sum != nullptr) {
+        // the other weight of the members up to the one found (order does not matter: integers)
+        unsigned long long part = 0;
+        for (uint32_t a = tid; a <= at; a += kNucleusThreads)
+            part += exp_fixed(((double)list.sorted_value[a] - (double)top) * also_inv_t, sh.table);
+        const uint32_t lane = tid & 31u, warp = tid >> 5;
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) part += __shfl_xor_sync(kFullMask, part, d);
+        if (lane == 0) sh.scan_mass[warp] = part;
+        __syncthreads();
+        unsigned long long sum = 0;
+        for (int w = 0; w < kNucleusThreads / 32; w++) sum += sh.scan_mass[w];
+        *also_sum = sum;
+        __syncthreads();
+    }
+    return found;
+}
+
+// The members of one value bucket (restricted to `inside`) gathered from the scratch row, then
+// order_members.  ok = false: the bucket is empty or holds more than the list takes.
 __device__ Position resolve_bucket(NucleusShared &sh, NucleusList &list, const float *values, uint32_t vocab,
                                    double inv_t, float top, const Nucleus inside, uint32_t bucket,
                                    uint32_t members, unsigned long long before, uint32_t rank_before,
@@ -463,71 +643,8 @@ __device__ Position resolve_bucket(NucleusShared &sh, NucleusList &list, const f
     __syncthreads();
     members = min(list.count, kListCap);  // (inside may hold fewer of the bucket than the histogram counted)
     if (members == 0) return found;
-    // order them: rank by counting, (value descending, id ascending); -0.0 and +0.0 tie
-    for (uint32_t a = tid; a < members; a += kNucleusThreads) {
-        const float v = list.value[a];
-        const uint32_t id = list.id[a];
-        uint32_t rank = 0;
-        for (uint32_t b = 0; b < members; b++) rank += precedes(list.value[b], list.id[b], v, id) ? 1u : 0u;
-        list.sorted_value[rank] = v;
-        list.sorted_id[rank] = id;
-        list.weight[rank] = exp_fixed(((double)v - (double)top) * inv_t, sh.table);
-    }
-    __syncthreads();
-    // running sum over at most 2048 entries: two per thread, then the usual scan
-    {
-        const uint32_t lane = tid & 31u, warp = tid >> 5;
-        const uint32_t a0 = 2 * tid, a1 = 2 * tid + 1;
-        const unsigned long long w0 = a0 < members ? list.weight[a0] : 0;
-        const unsigned long long w1 = a1 < members ? list.weight[a1] : 0;
-        unsigned long long incl = w0 + w1;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const unsigned long long up = __shfl_up_sync(kFullMask, incl, d);
-            if (lane >= (uint32_t)d) incl += up;
-        }
-        if (lane == 31) sh.scan_mass[warp] = incl;
-        __syncthreads();
-        unsigned long long prior = incl - (w0 + w1);
-        for (uint32_t w = 0; w < warp; w++) prior += sh.scan_mass[w];
-        if (a0 < members) list.weight[a0] = before + prior + w0;
-        if (a1 < members) list.weight[a1] = before + prior + w0 + w1;
-        if (tid == 0) sh.hit_bucket = kPaddingId;
-        __syncthreads();
-    }
-    // the first entry whose running sum reaches the target (exactly one thread sees the step)
-    for (uint32_t a = tid; a < members; a += kNucleusThreads) {
-        const unsigned long long here = list.weight[a];
-        const unsigned long long prev = a ? list.weight[a - 1] : before;
-        const bool was = strict ? prev > target : prev >= target;
-        const bool now = strict ? here > target : here >= target;
-        if (!clipped && !was && now) sh.hit_bucket = a;
-    }
-    __syncthreads();
-    uint32_t at = sh.hit_bucket;
-    if (clipped || at == kPaddingId) at = members - 1;
-    found.key = float_key(list.sorted_value[at]);
-    found.id = list.sorted_id[at];
-    found.mass = list.weight[at];
-    found.rank = rank_before + at + 1;
-    found.ok = true;
-    __syncthreads();
-    if (also_sum != nullptr) {
-        // the other weight of the members up to the one found (order does not matter: integers)
-        unsigned long long part = 0;
-        for (uint32_t a = tid; a <= at; a += kNucleusThreads)
-            part += exp_fixed(((double)list.sorted_value[a] - (double)top) * also_inv_t, sh.table);
-        const uint32_t lane = tid & 31u, warp = tid >> 5;
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) part += __shfl_xor_sync(kFullMask, part, d);
-        if (lane == 0) sh.scan_mass[warp] = part;
-        __syncthreads();
-        unsigned long long sum = 0;
-        for (int w = 0; w < kNucleusThreads / 32; w++) sum += sh.scan_mass[w];
-        *also_sum = sum;
-        __syncthreads();
-    }
-    return found;
+    return order_members(sh, list.work(), members, inv_t, top, inside, before, rank_before, target, strict, clipped,
+                         also_inv_t, also_sum);
 }
 
 // After a crossing search: the bucket it stopped in, or -- when the total never reaches the
@@ -674,257 +791,113 @@ __device__ bool fill_both(NucleusShared &sh, const float *values, uint32_t vocab
     return fits;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kNucleusThreads, 1) nucleus_select_kernel(const NucleusParams p) {
-    extern __shared__ __align__(16) unsigned char histogram_memory[];
-    __shared__ NucleusShared sh;
+// The long way, by one CTA over the whole penalised row in scratch memory (see the top of the
+// file).  All threads call.
+__device__ __noinline__ void sample_the_long_way(NucleusShared &sh, NucleusList &list, const float *values,
+                                                 uint32_t vocab, const SamplerConfig cfg, float uniform,
+                                                 uint32_t row, const SelectOutput &out) {
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    if (tid == 0) {
-        sh.mass = reinterpret_cast<unsigned long long *>(histogram_memory);
-        sh.other_mass = sh.mass + kBuckets;
-        sh.count = reinterpret_cast<uint32_t *>(histogram_memory + 2 * kBuckets * sizeof(unsigned long long));
-    }
-    if (tid < 64) sh.table[tid] = exp2((double)tid / 64.0);
-    float *values = p.scratch + (size_t)blockIdx.x * p.scratch_stride;
-    NucleusList &list = *reinterpret_cast<NucleusList *>(histogram_memory + kNucleusHistogramBytes);
+    float best = -INFINITY;
+    walk_row(values, vocab, [&](float v, uint32_t) {
+        if (!is_nonfinite(v)) best = fmaxf(best, v);
+    });
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) best = fmaxf(best, __shfl_xor_sync(kFullMask, best, d));
+    if (lane == 0) sh.reduce_max[warp] = best;
     __syncthreads();
-
-    for (uint32_t row = blockIdx.x; row < p.rows; row += gridDim.x) {
-        const SamplerConfig cfg = p.config_count > 1 ? p.configs[row] : p.config0;
-        if (cfg.temperature == 0.0f || cfg.top_k != 0) continue;  // the streaming kernel's rows
-
-        // ---- pass 1: HBM -> penalised fp32 row in scratch, maximum on the way ----
-        const T *columns = static_cast<const T *>(p.logits) + (size_t)row * p.row_stride;
-        const Repetition repetition = make_repetition(cfg.repetition_penalty);
-        const float flat_offset = penalty_offset(1u, cfg.presence_penalty, cfg.frequency_penalty);
-        float best = __uint_as_float(0xff800000u);
-        uint32_t finite = 0, bad_history = 0;
-        for (uint32_t split = 0; split < p.splits; split++) {
-            const uint32_t lo = split * p.split_len;
-            const uint32_t n = min(p.split_len, p.vocab - lo);
-            uint32_t flags = 0;
-            HistoryView history = make_history_view(nullptr, 0, 0, false);
-            if (p.history_meta != nullptr) {
-                const size_t unit = (size_t)row * p.splits + split;
-                const uint2 meta = reinterpret_cast<const uint2 *>(p.history_meta)[unit];
-                flags = meta.x;
-                if (meta.y) bad_history = meta.y;
-                history = make_history_view(
-                    const_cast<uint32_t *>(p.history_global) + unit * p.history_stride_words,
-                    p.bitmap_words, p.count_capacity, p.dense_wide != 0);
-            }
-            // one column: penalise if seen, store, fold into the maximum
-            auto take = [&](float v, uint32_t c, uint32_t word) {
-                if ((word >> (c & 31u)) & 1u) {
-                    float offset = flat_offset;
-                    if (flags & 2u)
-                        offset = penalty_offset(history.count(c >> 5, word, c & 31u),
-                                                cfg.presence_penalty, cfg.frequency_penalty);
-                    v = penalise_with_offset(v, offset, repetition);
-                }
-                if (!is_nonfinite(v)) {
-                    best = fmaxf(best, v);
-                    finite++;
-                }
-                return v;
-            };
-            const T *source = columns + lo;
-            uint32_t done = 0;
-            if ((reinterpret_cast<uintptr_t>(source) & 15u) == 0 && (lo & 3u) == 0) {
-                // four columns per thread and trip (one vector load, one bitmap word, one
-                // 128-bit store), two trips in flight
-                const uint32_t quads = n / 4u;
-                float4 *out = reinterpret_cast<float4 *>(values + lo);
-                auto load4 = [&](uint32_t q) {
-                    float4 v;
-                    if (sizeof(T) == 2) {
-                        const uint2 raw = reinterpret_cast<const uint2 *>(source)[q];
-                        v = make_float4(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u),
-                                        __uint_as_float(raw.y << 16), __uint_as_float(raw.y & 0xffff0000u));
-                    } else {
-                        v = reinterpret_cast<const float4 *>(source)[q];
-                    }
-                    return v;
-                };
-                // What the history says about the four columns of a quad (they share a bitmap word).
-                // The loads go out in two waves that wait for nothing but each other -- the word and
-                // the running count of ids before it, then the four occurrence counts -- instead of
-                // a chain of two loads per seen column.
-                struct Seen {
-                    uint32_t nibble;    // bit j: column 4q + j has been seen
-                    uint32_t times[4];  // how often (with a frequency penalty)
-                };
-                auto look_up = [&](uint32_t q) {
-                    Seen seen;
-                    seen.nibble = 0;
-                    seen.times[0] = seen.times[1] = seen.times[2] = seen.times[3] = 1u;
-                    if (!(flags & 1u)) return seen;
-                    const uint32_t c = q * 4u;
-                    const uint32_t word = history.bitmap[c >> 5];
-                    seen.nibble = (word >> (c & 31u)) & 15u;
-                    if ((flags & 2u) && seen.nibble != 0) {
-                        const uint32_t before = history.running[c >> 5] + __popc(word & ((1u << (c & 31u)) - 1u));
-                        uint32_t at[4];
-                        at[0] = before;
-                        at[1] = at[0] + (seen.nibble & 1u);
-                        at[2] = at[1] + ((seen.nibble >> 1) & 1u);
-                        at[3] = at[2] + ((seen.nibble >> 2) & 1u);
-#pragma unroll
-                        for (int j = 0; j < 4; j++) {
-                            const uint32_t slot = min(at[j], history.capacity - 1u);
-                            seen.times[j] = history.wide ? static_cast<const uint32_t *>(history.dense)[slot]
-                                                         : static_cast<const uint16_t *>(history.dense)[slot];
-                        }
-                    }
-                    return seen;
-                };
-                auto settle = [&](float v, uint32_t j, const Seen &seen) {
-                    if ((seen.nibble >> j) & 1u) {
-                        float offset = flat_offset;
-                        if (flags & 2u) offset = penalty_offset(seen.times[j], cfg.presence_penalty, cfg.frequency_penalty);
-                        v = penalise_with_offset(v, offset, repetition);
-                    }
-                    if (!is_nonfinite(v)) {
-                        best = fmaxf(best, v);
-                        finite++;
-                    }
-                    return v;
-                };
-                auto take4 = [&](float4 v, uint32_t q, const Seen &seen) {
-                    v.x = settle(v.x, 0u, seen);
-                    v.y = settle(v.y, 1u, seen);
-                    v.z = settle(v.z, 2u, seen);
-                    v.w = settle(v.w, 3u, seen);
-                    out[q] = v;
-                };
-                uint32_t q = tid;
-                for (; q + kNucleusThreads < quads; q += 2 * kNucleusThreads) {
-                    const float4 a = load4(q), b = load4(q + kNucleusThreads);
-                    const Seen seen_a = look_up(q), seen_b = look_up(q + kNucleusThreads);
-                    take4(a, q, seen_a);
-                    take4(b, q + kNucleusThreads, seen_b);
-                }
-                if (q < quads) take4(load4(q), q, look_up(q));
-                done = quads * 4u;
-            }
-            for (uint32_t c = done + tid; c < n; c += kNucleusThreads) {
-                float v;
-                if (sizeof(T) == 2) v = bf16_bits_to_float(reinterpret_cast<const uint16_t *>(source)[c]);
-                else v = reinterpret_cast<const float *>(source)[c];
-                const uint32_t word = (flags & 1u) ? history.bitmap[c >> 5] : 0u;
-                values[lo + c] = take(v, c, word);
-            }
-        }
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) {
-            best = fmaxf(best, __shfl_xor_sync(kFullMask, best, d));
-            finite += __shfl_xor_sync(kFullMask, finite, d);
-        }
-        if (lane == 0) {
-            sh.reduce_max[warp] = best;
-            sh.reduce_count[warp] = finite;
-        }
-        __syncthreads();  // also makes the scratch row visible to the whole CTA
-        best = sh.reduce_max[0];
-        finite = sh.reduce_count[0];
-        for (int w = 1; w < kNucleusThreads / 32; w++) {
-            best = fmaxf(best, sh.reduce_max[w]);
-            finite += sh.reduce_count[w];
+    for (int w = 0; w < kNucleusThreads / 32; w++) best = fmaxf(best, sh.reduce_max[w]);
+    if (best == -INFINITY) {  // src/sampler.c:97 "sampler received no finite candidates"
+        if (tid == 0) {
+            report_row(out, row, kErrFormat, kPaddingId, 0.0f);
+            if (out.dbg_count) out.dbg_count[row] = 0;
         }
         __syncthreads();
-        if (bad_history || finite == 0) {
-            // src/output.c:610-612 / src/sampler.c:97 "sampler received no finite candidates"
+        return;
+    }
+    // ---- top-p on the un-tempered softmax: where does the mass reach top_p? ----
+    Nucleus all;
+    all.everything = true;
+    all.key = 0;
+    all.id = 0;
+    const double top_p = (double)cfg.top_p;
+    // cumulative / sum >= top_p  <=>  cumulative >= top_p * sum
+    auto mass_target = [top_p](unsigned long long total) {
+        const unsigned long long t = (unsigned long long)ceil(top_p * (double)total);
+        return t > total ? total : t;
+    };
+    Nucleus nucleus;
+    nucleus.everything = false;
+    unsigned long long raw_sum, mass_at_cut;
+    uint32_t size;
+    const double inv_t = 1.0 / (double)cfg.temperature;
+    float u = uniform;
+    if (is_nonfinite(u) || u < 0.0f) u = 0.0f;
+    if (u >= 1.0f) u = __uint_as_float(0x3f7fffffu);
+    const double draw_at = (double)u;
+    // first element whose cumulative weight exceeds draw = u * sum
+    auto draw_target = [draw_at](unsigned long long total) {
+        return (unsigned long long)floor(draw_at * (double)total);
+    };
+    uint32_t picked_id = kPaddingId;
+    unsigned long long weight_sum = 0;
+
+    // ---- the usual way: one pass fills both histograms, each phase then looks into one bucket ----
+    bool done = false;
+    {
+        const bool filled = fill_both(sh, values, vocab, inv_t, best);
+        const unsigned long long cut_target = find_crossing_up(sh, mass_target, false);
+        raw_sum = sh.total_mass;
+        const bool cut_clipped = settle_crossing(sh);
+        const uint32_t cut_bucket = sh.hit_bucket;
+        const unsigned long long cut_before = sh.hit_mass_before;
+        const uint32_t cut_rank_before = sh.hit_count_before;
+        const uint32_t cut_members = sh.count[cut_bucket];
+        __syncthreads();
+        unsigned long long tempered_inside = 0;  // tempered weight of the bucket's members inside the nucleus
+        const Position cut = resolve_bucket(sh, list, values, vocab, 1.0, best, all, cut_bucket, cut_members,
+                                            cut_before, cut_rank_before, cut_target, false, cut_clipped, inv_t,
+                                            &tempered_inside);
+        if (filled && cut.ok) {
+            nucleus.key = cut.key;
+            nucleus.id = cut.id;
+            mass_at_cut = cut.mass;
+            size = cut.rank;
+            // the tempered masses of the nucleus: whole buckets above the cut's, that bucket as
+            // far as the nucleus reaches into it, nothing below
             if (tid == 0) {
-                report_row(p.out, row, bad_history ? bad_history : kErrFormat, kPaddingId, 0.0f);
-                if (p.out.dbg_count) p.out.dbg_count[row] = 0;
+                unsigned long long *raw = sh.mass;
+                sh.mass = sh.other_mass;
+                sh.other_mass = raw;
             }
-            continue;
-        }
-
-        // ---- top-p on the un-tempered softmax: where does the mass reach top_p? ----
-        Nucleus all;
-        all.everything = true;
-        all.key = 0;
-        all.id = 0;
-        const double top_p = (double)cfg.top_p;
-        // cumulative / sum >= top_p  <=>  cumulative >= top_p * sum
-        auto mass_target = [top_p](unsigned long long total) {
-            const unsigned long long t = (unsigned long long)ceil(top_p * (double)total);
-            return t > total ? total : t;
-        };
-        Nucleus nucleus;
-        nucleus.everything = false;
-        unsigned long long raw_sum, mass_at_cut;
-        uint32_t size;
-        const double inv_t = 1.0 / (double)cfg.temperature;
-        float u = p.uniforms[row];
-        if (is_nonfinite(u) || u < 0.0f) u = 0.0f;
-        if (u >= 1.0f) u = __uint_as_float(0x3f7fffffu);
-        const double draw_at = (double)u;
-        // first element whose cumulative weight exceeds draw = u * sum
-        auto draw_target = [draw_at](unsigned long long total) {
-            return (unsigned long long)floor(draw_at * (double)total);
-        };
-        uint32_t picked_id = kPaddingId;
-        unsigned long long weight_sum = 0;
-
-        // ---- the usual way: one pass fills both histograms, each phase then looks into one bucket ----
-        bool done = false;
-        {
-            const bool filled = fill_both(sh, values, p.vocab, inv_t, best);
-            const unsigned long long cut_target = find_crossing_up(sh, mass_target, false);
-            raw_sum = sh.total_mass;
-            const bool cut_clipped = settle_crossing(sh);
-            const uint32_t cut_bucket = sh.hit_bucket;
-            const unsigned long long cut_before = sh.hit_mass_before;
-            const uint32_t cut_rank_before = sh.hit_count_before;
-            const uint32_t cut_members = sh.count[cut_bucket];
             __syncthreads();
-            unsigned long long tempered_inside = 0;  // tempered weight of the bucket's members inside the nucleus
-            const Position cut = resolve_bucket(sh, list, values, p.vocab, 1.0, best, all, cut_bucket, cut_members,
-                                                cut_before, cut_rank_before, cut_target, false, cut_clipped, inv_t,
-                                                &tempered_inside);
-            if (filled && cut.ok) {
-                nucleus.key = cut.key;
-                nucleus.id = cut.id;
-                mass_at_cut = cut.mass;
-                size = cut.rank;
-                // the tempered masses of the nucleus: whole buckets above the cut's, that bucket as
-                // far as the nucleus reaches into it, nothing below
-                if (tid == 0) {
-                    unsigned long long *raw = sh.mass;
-                    sh.mass = sh.other_mass;
-                    sh.other_mass = raw;
-                }
-                __syncthreads();
-                for (uint32_t b = tid; b < kBuckets; b += kNucleusThreads) {
-                    if (b > cut_bucket) {
-                        sh.mass[b] = 0;
-                        sh.count[b] = 0;
-                    } else if (b == cut_bucket) {
-                        sh.mass[b] = tempered_inside;
-                    }
-                }
-                __syncthreads();
-                const unsigned long long pick_target = find_crossing_up(sh, draw_target, true);
-                weight_sum = sh.total_mass;
-                const bool pick_clipped = settle_crossing(sh);
-                const uint32_t pick_bucket = sh.hit_bucket;
-                const unsigned long long pick_before = sh.hit_mass_before;
-                const uint32_t pick_members = sh.count[pick_bucket];
-                __syncthreads();
-                const Position pick = resolve_bucket(sh, list, values, p.vocab, inv_t, best, nucleus, pick_bucket,
-                                                     pick_members, pick_before, 0u, pick_target, true, pick_clipped,
-                                                     0.0, nullptr);
-                if (pick.ok) {
-                    picked_id = pick.id;
-                    done = true;
+            for (uint32_t b = tid; b < kBuckets; b += kNucleusThreads) {
+                if (b > cut_bucket) {
+                    sh.mass[b] = 0;
+                    sh.count[b] = 0;
+                } else if (b == cut_bucket) {
+                    sh.mass[b] = tempered_inside;
                 }
             }
+            __syncthreads();
+            const unsigned long long pick_target = find_crossing_up(sh, draw_target, true);
+            weight_sum = sh.total_mass;
+            const bool pick_clipped = settle_crossing(sh);
+            const uint32_t pick_bucket = sh.hit_bucket;
+            const unsigned long long pick_before = sh.hit_mass_before;
+            const uint32_t pick_members = sh.count[pick_bucket];
+            __syncthreads();
+            const Position pick = resolve_bucket(sh, list, values, vocab, inv_t, best, nucleus, pick_bucket,
+                                                 pick_members, pick_before, 0u, pick_target, true, pick_clipped,
+                                                 0.0, nullptr);
+            if (pick.ok) {
+                picked_id = pick.id;
+                done = true;
+            }
         }
-        if (!done) {
+    }
+    if (!done) {
         // ---- a bucket too crowded to order in shared memory: phase by phase, with the exact descent ----
-        const Position cut = locate(sh, list, values, p.vocab, 1.0, best, all, mass_target, false);
+        const Position cut = locate(sh, list, values, vocab, 1.0, best, all, mass_target, false);
         if (cut.ok) {
             nucleus.key = cut.key;
             nucleus.id = cut.id;
@@ -934,7 +907,7 @@ __global__ void __launch_bounds__(kNucleusThreads, 1) nucleus_select_kernel(cons
         } else {
             // a bucket too crowded to order in shared memory: the generic radix descent
             unsigned long long partial = 0;
-            for (uint32_t i = tid; i < p.vocab; i += kNucleusThreads) {
+            for (uint32_t i = tid; i < vocab; i += kNucleusThreads) {
                 const float v = values[i];
                 if (!is_nonfinite(v)) partial += exp_fixed((double)v - (double)best, sh.table);
             }
@@ -945,18 +918,18 @@ __global__ void __launch_bounds__(kNucleusThreads, 1) nucleus_select_kernel(cons
             raw_sum = 0;
             for (int w = 0; w < kNucleusThreads / 32; w++) raw_sum += sh.scan_mass[w];
             __syncthreads();
-            descend(sh, values, p.vocab, 1.0, (double)best, all, mass_target(raw_sum), false, &nucleus.key,
+            descend(sh, values, vocab, 1.0, (double)best, all, mass_target(raw_sum), false, &nucleus.key,
                     &nucleus.id, &mass_at_cut, &size);
         }
 
         // ---- temperature weights of the nucleus, then the draw ----
-        const Position pick = locate(sh, list, values, p.vocab, inv_t, best, nucleus, draw_target, true);
+        const Position pick = locate(sh, list, values, vocab, inv_t, best, nucleus, draw_target, true);
         if (pick.ok) {
             picked_id = pick.id;
             weight_sum = pick.total;
         } else {
             unsigned long long partial = 0;
-            for (uint32_t i = tid; i < p.vocab; i += kNucleusThreads) {
+            for (uint32_t i = tid; i < vocab; i += kNucleusThreads) {
                 const float v = values[i];
                 if (is_nonfinite(v)) continue;
                 if (nucleus.holds(float_key(v), i))
@@ -971,19 +944,1278 @@ __global__ void __launch_bounds__(kNucleusThreads, 1) nucleus_select_kernel(cons
             __syncthreads();
             uint32_t picked_key, picked_rank;
             unsigned long long picked_mass;
-            descend(sh, values, p.vocab, inv_t, (double)best, nucleus, draw_target(weight_sum), true,
+            descend(sh, values, vocab, inv_t, (double)best, nucleus, draw_target(weight_sum), true,
                     &picked_key, &picked_id, &picked_mass, &picked_rank);
         }
+    }
+    if (tid == 0) {
+        if (weight_sum == 0 || raw_sum == 0 || picked_id >= vocab) {
+            report_row(out, row, kErrFormat, kPaddingId, 0.0f);
+        } else {
+            report_row(out, row, kOk, picked_id, values[picked_id]);
         }
-        if (tid == 0) {
-            if (weight_sum == 0 || raw_sum == 0 || picked_id >= p.vocab) {
-                report_row(p.out, row, kErrFormat, kPaddingId, 0.0f);
-            } else {
-                report_row(p.out, row, kOk, picked_id, values[picked_id]);
+        if (out.dbg_count) out.dbg_count[row] = size;  // nucleus size; the list itself is not dumped
+    }
+    __syncthreads();
+}
+
+// ================================================================== the short way
+//
+// What bounds it: instruction issue and latency.  The first pass is about twenty instructions and
+// two shared-memory adds per logit; masses are not summed per logit, exp() and fp64 appear once
+// per bucket.  A row's other steps (scanning the buckets, ordering the candidates) are chains of
+// latencies of 20 us, so two CTAs share an SM, one streaming while the other scans and sorts; for
+// few rows a row is spread over several CTAs instead.  A CTA per row and SM that added two fp64 weights
+// per logit to five shared-memory sums took, per call: 512 rows of 151,936 fp32 logits, histories
+// of 32,768 tokens 772 us (now 546), without history 600 (238); 32 rows bf16 410-560 (63).
+// With histories the largest part is the seen columns' gather (amend_seen).
+//
+// A value's place: buckets 1/1024 wide over the top four units of the row's window, 1/256 wide over
+// the next eight, 1/32 over the next 64 (all half as wide for temperatures below 0.36), with
+// their middles on the grid of multiples of the width, so that neither the bucket nor the
+// distance f from its middle depends on a subtraction that rounds: n = rint(v * 1024) by adding
+// and subtracting 1.5 * 2^23, f = v * 1024 - n in [-1/2, 1/2], both exact in fp32.  With
+// w = width * f the members' weights relative to the middle's add up to
+//     sum exp(w) = N + c M1 + c^2/2 M2 + c^3/6 M3 + ...,   c = width (times 1/T: tempered)
+// M3 is not kept: f^3 is replaced by the nearest multiple of f (0.15 f over a bucket), which
+// leaves 0.019 c^3/6 (root mean square) of a member's weight: 3e-12 raw and 2.4e-11 at T = 0.5 in
+// the narrow buckets, at most 6e-12 of the largest weight in the wider ones (they begin 3.5
+// units below the sampled maximum, where a weight is e^-3.5 of it at most, e^-7 at T = 0.5),
+// against 6.7e-11 for weights rounded to 2^-32 of themselves.
+//
+// A bucket is two 32-bit words that are added to, once each, per member:
+//     first    sum of f in units of 2^-22 (the bits of f * 2^22 + 1.5 * 2^23: the constant's
+//              share, N times its bits, is taken off afterwards, modulo 2^32)
+//     second   low 22 bits: sum of f^2 in units of 2^-14; high 10 bits: N times an odd number
+//              (what the bits of the constant leave there), so N modulo 1024
+// Neither can overflow up to 1023 members.  A row whose counts do not add up to the number of
+// values counted had a bucket with more (a wrap loses 1024 and nothing can make up for it): it
+// goes the long way.  Rows of raw bf16 logits have at most eight significant bits, f is 0 above
+// 1/8, and many members share a value: they trade precision they have no use for against twelve
+// bits of count.
+//
+// Slots are xor-swizzled inside their group of 32: bf16 values lie a power of two apart and
+// would meet in a few banks otherwise.
+
+constexpr uint32_t kFineSlots = 4096, kMiddleSlots = 2048, kCoarseSlots = 2048;
+constexpr uint32_t kSlots = kFineSlots + kMiddleSlots + kCoarseSlots;
+constexpr uint32_t kGroups = kSlots / 32;      // the slots a warp looks at side by side
+constexpr uint32_t kPlaces = kGroups + 1;      // place 0: the values above the window
+constexpr float kFineScale = 1024.0f, kMiddleScale = 256.0f, kCoarseScale = 32.0f;
+constexpr int kFineSpan = 12301;               // from 32 times the topmost coarse middle to the topmost fine one
+constexpr float kMagic = 12582912.0f;          // 1.5 * 2^23: adding it rounds to a whole number
+constexpr uint32_t kMagicBits = 0x4b400000u;
+constexpr uint32_t kMostTeam = 8;              // CTAs that may share a row
+constexpr uint32_t kOverCap = 768;             // values above the window that are kept one by one
+constexpr uint32_t kCutCap = 1024, kPickCap = kOrderCap;  // members of the cut's bucket and the draw's
+constexpr float kWindowMargin = 0.5f;          // how far the window reaches above the sample's maximum
+constexpr float kWindowLimit = 3900.0f;        // |v| * 1024 must stay below 2^22
+constexpr int kSamples = 4;                    // logits a thread looks at to place the window
+// Temperatures the short way takes: below, c^3 / T^3 would cost more precision than the rounding
+// it replaces (buckets half as wide take it down to half of the first); above, values under the window would
+// still weigh something.
+constexpr float kWideColdest = 0.36f, kShortColdest = 0.18f, kShortHottest = 2.6f;
+
+constexpr uint32_t inverse_mod(uint32_t a, uint32_t modulus) {  // a odd, modulus a power of two
+    uint32_t x = 1;
+    for (int i = 0; i < 5; i++) x *= 2 - a * x;
+    return x & (modulus - 1);
+}
+
+// How a bucket's words are packed: rows of raw bf16 logits, all others.
+template <bool kRawBf16>
+struct Packing {
+    static constexpr int kCountShift = kRawBf16 ? 20 : 22;
+    static constexpr uint32_t kCountMask = (1u << (32 - kCountShift)) - 1u;
+    static constexpr float kFirstUnit = kRawBf16 ? 1048576.0f : 4194304.0f;  // 2^20, 2^22
+    static constexpr float kSecondUnit = kRawBf16 ? 2048.0f : 16384.0f;      // 2^11, 2^14
+    static constexpr float kSecondMagic = kRawBf16 ? 13631488.0f : kMagic;   // bits 0x4b500000: an odd count field
+    static constexpr uint32_t kField = (kRawBf16 ? 0x4b500000u : kMagicBits) >> kCountShift;
+    static_assert(kField & 1u, "the count can be read back");
+    static constexpr uint32_t kInverse = inverse_mod(kField, kCountMask + 1u);
+
+    static __device__ __forceinline__ uint32_t count(uint32_t second) {
+        return ((second >> kCountShift) * kInverse) & kCountMask;
+    }
+    static __device__ __forceinline__ int sum_f(uint32_t first, uint32_t n) { return (int)(first - n * kMagicBits); }
+    static __device__ __forceinline__ uint32_t sum_ff(uint32_t second) { return second & ((1u << kCountShift) - 1u); }
+};
+
+// The window of a row: which values have a bucket, and which.
+struct Window {
+    float sharp;                          // 1, or 2 for buckets half as wide
+    float top, first_edge, second_edge;   // narrow buckets: [first_edge, top], middle: [second_edge, first_edge),
+    float bottom;                         // wide: [bottom, second_edge)
+    int coarse_top;                       // the middle of the topmost wide bucket, in widths
+    bool usable;
+
+    __device__ __forceinline__ explicit Window(float reference, float sharp_) : sharp(sharp_) {
+        usable = fabsf(reference) * sharp < kWindowLimit;
+        const float at = usable ? reference * sharp : 0.0f, unit = 1.0f / sharp;  // (sharp: a power of two)
+        coarse_top = __float2int_rn(((at + kWindowMargin) * kFineScale - (float)kFineSpan) * 0.03125f);
+        top = (float)(32 * coarse_top + kFineSpan) * (1.0f / kFineScale) * unit;
+        first_edge = ((float)(8 * coarse_top + 2051) + 0.5f) * (1.0f / kMiddleScale) * unit;
+        second_edge = ((float)coarse_top + 0.5f) * (1.0f / kCoarseScale) * unit;
+        bottom = (float)(coarse_top - (int)(kCoarseSlots - 1)) * (1.0f / kCoarseScale) * unit;
+    }
+    // the bucket of a value in [bottom, top], and its distance from the middle in widths
+    __device__ __forceinline__ uint32_t slot(float v, float &f) const {
+        float scale = kCoarseScale * sharp;
+        uint32_t base = kMagicBits + kFineSlots + kMiddleSlots + (uint32_t)coarse_top;
+        if (v >= second_edge) {
+            scale = kMiddleScale * sharp;
+            base = kMagicBits + kFineSlots + (uint32_t)(8 * coarse_top + 2051);
+        }
+        if (v >= first_edge) {
+            scale = kFineScale * sharp;
+            base = kMagicBits + (uint32_t)(32 * coarse_top + kFineSpan);
+        }
+        const float shifted = __fmaf_rn(v, scale, kMagic);
+        f = __fmaf_rn(v, scale, -__fsub_rn(shifted, kMagic));
+        return base - __float_as_uint(shifted);
+    }
+    // a slot's middle in widths, and the width
+    __device__ __forceinline__ int middle_of(uint32_t slot, float &width) const {
+        if (slot < kFineSlots) {
+            width = 1.0f / (kFineScale * sharp);
+            return 32 * coarse_top + kFineSpan - (int)slot;
+        }
+        if (slot < kFineSlots + kMiddleSlots) {
+            width = 1.0f / (kMiddleScale * sharp);
+            return 8 * coarse_top + 2051 - (int)(slot - kFineSlots);
+        }
+        width = 1.0f / (kCoarseScale * sharp);
+        return coarse_top - (int)(slot - kFineSlots - kMiddleSlots);
+    }
+    __device__ __forceinline__ double middle(uint32_t slot) const {
+        float width;
+        const int n = middle_of(slot, width);
+        return (double)n * (double)width;
+    }
+    // the largest and the smallest value in the slot (half-way between two middles the even one takes it)
+    __device__ __forceinline__ float highest(uint32_t at) const {
+        float width, f;
+        const int n = middle_of(at, width);
+        const float edge = fminf(((float)n + 0.5f) * width, top);
+        return slot(edge, f) == at ? edge : key_to_float(float_key(edge) - 1u);
+    }
+    __device__ __forceinline__ float lowest(uint32_t at) const {
+        float width, f;
+        const int n = middle_of(at, width);
+        const float edge = fmaxf(((float)n - 0.5f) * width, bottom);
+        return slot(edge, f) == at ? edge : key_to_float(float_key(edge) + 1u);
+    }
+};
+
+__device__ __forceinline__ uint32_t swizzled(uint32_t slot) { return slot ^ ((slot >> 5) & 31u); }
+
+// What one CTA knows about its columns after the first pass.
+struct Share {
+    float best;          // largest finite value
+    uint32_t finite;     // how many are finite
+    uint32_t crowded;    // a bucket had more members than its words take
+};
+
+enum Verdict : uint32_t { kDone, kLongWay };
+
+// What the team's first CTA has found out: in which buckets the answer lies.
+struct Plan {
+    uint32_t verdict;
+    uint32_t cut;                 // 0: above the window, else 1 + slot
+    uint32_t pick_first, pick_last;  // the draw lands in one of these, numbered the same way
+    unsigned long long cut_target, cut_before, cut_tempered_before;
+    uint32_t cut_rank_before, cut_members;
+    unsigned long long pick_before;
+    uint32_t pick_members;
+};
+
+// Result of looking for a crossing among the 32 slots of a group.
+struct SlotHit {
+    uint32_t slot, count, count_before;
+    unsigned long long raw_before, tempered_before, tempered;
+};
+
+struct ShortShared {
+    Share share;
+    Plan plan;
+    uint32_t over_count, cut_count, pick_count;   // the first CTA's lists
+    int lost, below, above;                       // this CTA: not finite, under the window, over it
+    uint32_t counted;                             // sum of the buckets' counts
+    uint32_t seen_count;                          // seen columns of this CTA
+    uint32_t top_slot;                            // the first bucket that holds anything
+    uint32_t cut_place, pick_place[2];
+    float sample_max[kNucleusWarps];
+    unsigned long long scan_raw[kNucleusWarps], scan_tempered[kNucleusWarps];
+    uint32_t scan_count[kNucleusWarps];
+};
+
+// Dynamic shared memory of the kernel: two CTAs' worth fit an SM.  The long way's memory lies over
+// all but the last two parts; the ordering works where the buckets were; the queues of visit_seen
+// lie over what is only filled after it (`lists` to `edges`).
+struct ShortMemory {
+    uint32_t first[kSlots], second[kSlots];
+    struct {
+        float cut_value[kCutCap];
+        uint32_t cut_id[kCutCap];
+        float pick_value[kPickCap];
+        uint32_t pick_id[kPickCap];
+    } lists;                                             // the first CTA's
+    unsigned long long raw[kPlaces], tempered[kPlaces];  // masses per place, then their running sums
+    uint32_t count[kPlaces];
+    double edges[2][kGroups];         // raw, tempered: the weight of a group's first middle, times 2^40
+    double lanes[2][3][32];           // the weights of the 32 slots relative to it, by kind of bucket
+    float over_value[kOverCap];
+    uint32_t over_id[kOverCap];
+    ShortShared state;
+    NucleusShared scan;               // what the ordering and the long way share
+};
+
+// All of it is reached through this, so that functions of their own know it is shared memory.
+__device__ __forceinline__ ShortMemory &short_memory() {
+    extern __shared__ __align__(16) unsigned char nucleus_memory[];
+    return *reinterpret_cast<ShortMemory *>(nucleus_memory);
+}
+
+// The CTAs that share a row.  With one CTA a team's barrier is the block's.
+struct Team {
+    uint32_t size, rank;
+    __device__ __forceinline__ void sync() const {
+        if (size == 1) {
+            __syncthreads();
+        } else {
+            asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+        }
+    }
+    // the same variable in another CTA's shared memory
+    template <class V>
+    __device__ __forceinline__ V *at(V *mine, uint32_t other) const {
+        return size == 1 ? mine : cooperative_groups::this_cluster().map_shared_rank(mine, other);
+    }
+};
+
+// Hands out the rows without a top-k cut in turn.  Every warp walks by itself and comes to the
+// same rows: with per-row configs it looks at 32 of them at a time.
+struct RowWalk {
+    uint32_t base, mask, turn;
+    __device__ __forceinline__ explicit RowWalk(uint32_t team) : base(0), mask(0), turn(team) {}
+    __device__ __forceinline__ bool next(const NucleusParams &p, uint32_t teams, uint32_t &row) {
+        if (p.config_count <= 1) {
+            row = turn;
+            turn += teams;
+            return row < p.rows;
+        }
+        for (;;) {
+            while (mask == 0) {
+                if (base >= p.rows) return false;
+                const uint32_t mine = base + lane_id();
+                bool ours = false;
+                if (mine < p.rows) ours = p.configs[mine].temperature != 0.0f && p.configs[mine].top_k == 0;
+                mask = __ballot_sync(kFullMask, ours);
+                base += 32;
             }
-            if (p.out.dbg_count) p.out.dbg_count[row] = size;  // nucleus size; the list itself is not dumped
+            const uint32_t lowest = (uint32_t)__ffs(mask) - 1u;
+            mask &= mask - 1;
+            if (turn == 0) {
+                turn = teams - 1;
+                row = base - 32 + lowest;
+                return true;
+            }
+            turn--;
+        }
+    }
+};
+
+template <typename T>
+struct Vector;
+template <>
+struct Vector<float> {
+    static constexpr int kPer = 4;
+    static __device__ __forceinline__ float one(const float *p) { return __ldg(p); }
+    static __device__ __forceinline__ void unpack(const uint4 &raw, float (&v)[4]) {
+        v[0] = __uint_as_float(raw.x);
+        v[1] = __uint_as_float(raw.y);
+        v[2] = __uint_as_float(raw.z);
+        v[3] = __uint_as_float(raw.w);
+    }
+};
+template <>
+struct Vector<uint16_t> {  // bf16 bit patterns
+    static constexpr int kPer = 8;
+    static __device__ __forceinline__ float one(const uint16_t *p) { return bf16_bits_to_float(__ldg(p)); }
+    static __device__ __forceinline__ void unpack(const uint4 &raw, float (&v)[8]) {
+        v[0] = __uint_as_float(raw.x << 16);
+        v[1] = __uint_as_float(raw.x & 0xffff0000u);
+        v[2] = __uint_as_float(raw.y << 16);
+        v[3] = __uint_as_float(raw.y & 0xffff0000u);
+        v[4] = __uint_as_float(raw.z << 16);
+        v[5] = __uint_as_float(raw.z & 0xffff0000u);
+        v[6] = __uint_as_float(raw.w << 16);
+        v[7] = __uint_as_float(raw.w & 0xffff0000u);
+    }
+};
+
+// Walks n logits from `source` on: vectors(v, column) for 128-bit vectors, one(v, column) for the
+// ragged ends and for what lies before the first 16-byte boundary.  The next two vectors of a
+// thread are on their way while it looks at two.
+template <typename T, class Vectors, class One>
+__device__ __forceinline__ void walk_logits(const T *source, uint32_t n, Vectors vectors, One one) {
+    constexpr int kPer = Vector<T>::kPer;
+    const uint32_t tid = threadIdx.x;
+    const uint32_t off = (uint32_t)(reinterpret_cast<uintptr_t>(source) & 15u);
+    const uint32_t head = min(n, (off ? 16u - off : 0u) / (uint32_t)sizeof(T));
+    const uint32_t count = (n - head) / kPer;
+    const T *body = source + head;
+    if (tid < head) one(Vector<T>::one(source + tid), tid);
+    const uint32_t rest = head + count * kPer + tid;
+    if (rest < n) one(Vector<T>::one(source + rest), rest);
+    uint4 a = make_uint4(0, 0, 0, 0), b = a;
+    uint32_t i = tid;
+    if (i < count) a = load_stream_128(body + (size_t)i * kPer);
+    if (i + kNucleusThreads < count) b = load_stream_128(body + (size_t)(i + kNucleusThreads) * kPer);
+    for (; i < count; i += 2 * kNucleusThreads) {
+        const uint4 now_a = a, now_b = b;
+        const uint32_t next = i + 2 * kNucleusThreads;
+        if (next < count) a = load_stream_128(body + (size_t)next * kPer);
+        if (next + kNucleusThreads < count) b = load_stream_128(body + (size_t)(next + kNucleusThreads) * kPer);
+        float v[kPer];
+        Vector<T>::unpack(now_a, v);
+        vectors(v, head + i * kPer);
+        if (i + kNucleusThreads < count) {
+            Vector<T>::unpack(now_b, v);
+            vectors(v, head + (i + kNucleusThreads) * kPer);
+        }
+    }
+}
+
+// v[j] for a j that is not known at compile time, without an array in memory
+template <int kPer>
+__device__ __forceinline__ float pick_element(const float (&v)[kPer], int j) {
+    float x = v[0];
+#pragma unroll
+    for (int i = 1; i < kPer; i++) x = i == j ? v[i] : x;
+    return x;
+}
+
+// What a pass over one CTA's columns finds out beside the buckets.
+struct Findings {
+    float best;                     // largest finite value
+    int lost, below, above;         // not finite, under the window, over it
+};
+
+// Which of a row's columns its history has seen, where that is asked of single columns.
+struct SeenBits {
+    const uint32_t *bitmap;         // the row's first history structure; null: no penalties
+    uint64_t stride;                // words between its splits
+    uint32_t split_len;
+    __device__ __forceinline__ bool test(uint32_t column) const {
+        if (bitmap == nullptr) return false;
+        const uint32_t split = column / split_len, local = column - split * split_len;
+        return (bitmap[split * stride + (local >> 5)] >> (local & 31u)) & 1u;
+    }
+};
+
+// The first pass over one CTA's columns: counts into the buckets, values above the window onto
+// the first CTA's list.
+template <class P>
+struct Counter {
+    const Window window;
+    const Team team;
+    Findings found;
+
+    __device__ __forceinline__ Counter(const Window &w, const Team &team_) : window(w), team(team_) {
+        found.best = -INFINITY;
+        found.lost = found.below = found.above = 0;
+    }
+    // a value inside the window
+    __device__ __forceinline__ void count(float v) {
+        ShortMemory &m = short_memory();
+        float f;
+        const uint32_t at = swizzled(window.slot(v, f));
+        atomicAdd(&m.first[at], __float_as_uint(__fmaf_rn(f, P::kFirstUnit, kMagic)));
+        atomicAdd(&m.second[at], __float_as_uint(__fmaf_rn(__fmul_rn(f, f), P::kSecondUnit, P::kSecondMagic)));
+    }
+    // A vector's values: as a rule all of them lie inside the window, which its largest (NaN if
+    // one is) and its smallest tell.
+    template <int kPer>
+    __device__ __forceinline__ void take_vector(const float (&v)[kPer], uint32_t column, const SeenBits &skip) {
+        float high = v[0], low = v[0];
+#pragma unroll
+        for (int j = 1; j < kPer; j++) {
+            asm("max.NaN.f32 %0, %0, %1;" : "+f"(high) : "f"(v[j]));
+            low = fminf(low, v[j]);
+        }
+        if (high <= window.top && low >= window.bottom) {
+            found.best = fmaxf(found.best, high);
+#pragma unroll
+            for (int j = 0; j < kPer; j++) count(v[j]);
+        } else {
+#pragma unroll 1
+            for (int j = 0; j < kPer; j++) take(pick_element(v, j), column + j, skip);
+        }
+    }
+    // `skip`: values above the window that are not listed (a seen id's raw logit)
+    __device__ __forceinline__ void take(float v, uint32_t column, const SeenBits &skip) {
+        if (v >= window.bottom && v <= window.top) {
+            found.best = fmaxf(found.best, v);
+            count(v);
+        } else if (is_nonfinite(v)) {
+            found.lost++;
+        } else {
+            if (v > window.top) {
+                ShortMemory &m = short_memory();
+                found.above++;
+                if (skip.test(column)) return;
+                found.best = fmaxf(found.best, v);
+                const uint32_t slot = atomicAdd(team.at(&m.state.over_count, 0), 1u);
+                if (slot < kOverCap) {
+                    team.at(m.over_value, 0)[slot] = v;
+                    team.at(m.over_id, 0)[slot] = column;
+                }
+            } else {
+                found.best = fmaxf(found.best, v);
+                found.below++;
+            }
+        }
+    }
+    // takes a counted value back (sums modulo 2^32: nothing of it stays)
+    __device__ __forceinline__ void uncount(float v) {
+        ShortMemory &m = short_memory();
+        float f;
+        const uint32_t at = swizzled(window.slot(v, f));
+        atomicAdd(&m.first[at], 0u - __float_as_uint(__fmaf_rn(f, P::kFirstUnit, kMagic)));
+        atomicAdd(&m.second[at], 0u - __float_as_uint(__fmaf_rn(__fmul_rn(f, f), P::kSecondUnit, P::kSecondMagic)));
+    }
+    __device__ __forceinline__ void take_back(float v) {
+        if (v >= window.bottom && v <= window.top) {
+            uncount(v);
+        } else if (is_nonfinite(v)) {
+            found.lost--;
+        } else if (v > window.top) {
+            found.above--;
+        } else {
+            found.below--;
+        }
+    }
+};
+
+template <typename T, class P>
+__device__ __noinline__ Findings count_logits(const T *columns, uint32_t lo, uint32_t n, const Window window,
+                                              const Team team, const SeenBits seen) {
+    Counter<P> counter(window, team);
+    walk_logits<T>(
+        columns + lo, n,
+        [&](const float (&v)[Vector<T>::kPer], uint32_t c) { counter.take_vector(v, lo + c, seen); },
+        [&](float v, uint32_t c) { counter.take(v, lo + c, seen); });
+    return counter.found;
+}
+
+// Every column in [lo, lo + n) the row's history has seen: visit(column, raw, penalised, slot),
+// slots numbered from 0 (state.seen_count says how many; zeroed by the caller).  A warp takes
+// 32 words of the bitmap at a time and lists the columns whose bits are up, so that the lanes
+// share them evenly however they lie.  All threads call; the lists' memory holds the queues.
+template <typename T, class Visit>
+__device__ __forceinline__ void visit_seen(const NucleusParams &p, uint32_t row, const SamplerConfig &cfg, uint32_t lo,
+                                           uint32_t n, Visit visit) {
+    ShortMemory &m = short_memory();
+    const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+    constexpr uint32_t kWarps = kNucleusWarps;
+    static_assert(offsetof(ShortMemory, lanes) - offsetof(ShortMemory, lists) >= kWarps * 1024 * sizeof(uint16_t),
+                  "a queue of 1024 columns per warp");
+    if (n == 0) return;  // (a CTA without columns does not begin at a multiple of 64)
+    uint16_t *queue = reinterpret_cast<uint16_t *>(&m.lists) + warp * 1024u;
+    const T *columns = static_cast<const T *>(p.logits) + (size_t)row * p.row_stride;
+    const Repetition repetition = make_repetition(cfg.repetition_penalty);
+    const float flat_offset = penalty_offset(1u, cfg.presence_penalty, cfg.frequency_penalty);
+    for (uint32_t split = lo / p.split_len; split < p.splits && split * p.split_len < lo + n; split++) {
+        const uint32_t split_lo = split * p.split_len;
+        const uint32_t from = max(lo, split_lo), to = min(lo + n, min(split_lo + p.split_len, p.vocab));
+        const size_t unit = (size_t)row * p.splits + split;
+        const uint32_t flags = reinterpret_cast<const uint2 *>(p.history_meta)[unit].x;
+        if (!(flags & 1u)) continue;
+        const HistoryView history = make_history_view(
+            const_cast<uint32_t *>(p.history_global) + unit * p.history_stride_words, p.bitmap_words,
+            p.count_capacity, p.dense_wide != 0);
+        // (`from` is a multiple of 64 columns, and so is where a split begins)
+        const uint32_t word_end = (to - split_lo + 31u) / 32u;
+        uint32_t word = (from - split_lo) / 32u + warp * 32u + lane;
+        uint32_t bits = word < word_end ? history.bitmap[word] : 0u;
+        uint32_t next_rank = flags & 2u ? history.running[min(word - lane, word_end - 1u)] : 0u;
+        for (uint32_t base = (from - split_lo) / 32u + warp * 32u; base < word_end; base += kWarps * 32u) {
+            const uint32_t ahead = word + kWarps * 32u;
+            const uint32_t next_bits = ahead < word_end ? history.bitmap[ahead] : 0u;
+            const uint32_t rank0 = next_rank;
+            if (flags & 2u) next_rank = history.running[min(base + kWarps * 32u, word_end - 1u)];
+            const uint32_t mine = __popc(bits);
+            uint32_t incl = mine;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t up = __shfl_up_sync(kFullMask, incl, d);
+                if (lane >= (uint32_t)d) incl += up;
+            }
+            const uint32_t total = __shfl_sync(kFullMask, incl, 31);
+            uint32_t slot0 = 0;
+            if (lane == 0 && total != 0) slot0 = atomicAdd(&m.state.seen_count, total);
+            slot0 = __shfl_sync(kFullMask, slot0, 0);
+            for (uint32_t rest = bits, at = incl - mine; rest != 0; rest &= rest - 1)
+                queue[at++] = (uint16_t)(lane * 32u + (uint32_t)__ffs(rest) - 1u);
+            __syncwarp();
+            constexpr int kBatch = 8;  // columns per lane and trip, loaded before any is used
+            const uint32_t column0 = split_lo + base * 32u;
+            for (uint32_t i0 = lane; i0 < total; i0 += 32 * kBatch) {
+                uint32_t times[kBatch];
+                float raw[kBatch];
+#pragma unroll
+                for (int q = 0; q < kBatch; q++) {
+                    const uint32_t i = i0 + 32 * q;
+                    raw[q] = 0.0f;
+                    times[q] = 1;
+                    if (i < total) {
+                        raw[q] = Vector<T>::one(columns + column0 + queue[i]);
+                        if (flags & 2u) {
+                            const uint32_t at = min(rank0 + i, history.capacity - 1u);
+                            times[q] = history.wide ? static_cast<const uint32_t *>(history.dense)[at]
+                                                    : static_cast<const uint16_t *>(history.dense)[at];
+                        }
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < kBatch; q++) {
+                    const uint32_t i = i0 + 32 * q;
+                    if (i >= total) break;
+                    const float offset = flags & 2u ? penalty_offset(times[q], cfg.presence_penalty, cfg.frequency_penalty)
+                                                    : flat_offset;
+                    visit(column0 + queue[i], raw[q], penalise_with_offset(raw[q], offset, repetition), slot0 + i);
+                }
+            }
+            __syncwarp();
+            word = ahead;
+            bits = next_bits;
+        }
+    }
+}
+
+// After the raw logits have been counted: every seen column's raw value is taken back and its
+// penalised value counted instead, and kept with its column for the second pass.
+template <typename T, class P>
+__device__ __noinline__ Findings amend_seen(const NucleusParams &p, uint32_t row, const SamplerConfig cfg, uint32_t lo,
+                                            uint32_t n, float2 *seen, const Window window, const Team team) {
+    Counter<P> counter(window, team);
+    const SeenBits all_listed = {nullptr, 0, 1};
+    visit_seen<T>(p, row, cfg, lo, n, [&](uint32_t column, float raw, float penalised, uint32_t slot) {
+        if (fmaxf(raw, penalised) <= window.top && fminf(raw, penalised) >= window.bottom && raw == raw && penalised == penalised) {
+            counter.uncount(raw);
+            counter.count(penalised);
+        } else {
+            counter.take_back(raw);
+            counter.take(penalised, column, all_listed);
+        }
+        seen[slot] = make_float2(penalised, __uint_as_float(column));
+    });
+    return counter.found;
+}
+
+// The penalised row in scratch memory, for the long way.
+template <typename T>
+__device__ __noinline__ void write_scratch(const NucleusParams &p, uint32_t row, const SamplerConfig cfg, uint32_t lo,
+                                           uint32_t n, bool penalised, float *values) {
+    const T *columns = static_cast<const T *>(p.logits) + (size_t)row * p.row_stride;
+    for (uint32_t c = lo + threadIdx.x; c < lo + n; c += kNucleusThreads) values[c] = Vector<T>::one(columns + c);
+    __syncthreads();
+    if (penalised)
+        visit_seen<T>(p, row, cfg, lo, n, [&](uint32_t column, float, float value, uint32_t) { values[column] = value; });
+}
+
+// Sum over the warp of masses below 2^52.
+__device__ __forceinline__ unsigned long long warp_sum_mass(unsigned long long mass) {
+    const uint32_t low = __reduce_add_sync(kFullMask, (uint32_t)mass & 0x3ffffffu);
+    const uint32_t high = __reduce_add_sync(kFullMask, (uint32_t)(mass >> 26));
+    return ((unsigned long long)high << 26) + low;
+}
+
+// The factors of the moments in a bucket's masses, by kind of bucket.
+template <class P>
+struct MomentFactors {
+    double raw1, raw2, tempered1, tempered2;
+    __device__ __forceinline__ MomentFactors(const Window &window, uint32_t slot, double inv_t) {
+        float width;
+        window.middle_of(slot, width);
+        const double c = (double)width, ct = c * inv_t;
+        raw1 = c * (1.0 + c * c * 0.025) / (double)P::kFirstUnit;  // 0.15 / 6
+        tempered1 = ct * (1.0 + ct * ct * 0.025) / (double)P::kFirstUnit;
+        raw2 = 0.5 * c * c / (double)P::kSecondUnit;
+        tempered2 = 0.5 * ct * ct / (double)P::kSecondUnit;
+    }
+};
+__device__ __forceinline__ uint32_t kind_of_group(uint32_t group) {
+    return group < kFineSlots / 32 ? 0u : group < (kFineSlots + kMiddleSlots) / 32 ? 1u : 2u;
+}
+
+struct SlotMass {
+    unsigned long long raw, tempered;
+    uint32_t count;
+};
+// `raw_weight`, `tempered_weight`: the weights of the slot's middle, times 2^40.
+template <class P>
+__device__ __forceinline__ SlotMass slot_mass(uint32_t first, uint32_t second, const MomentFactors<P> &k,
+                                              double raw_weight, double tempered_weight) {
+    SlotMass s;
+    s.count = P::count(second);
+    const double n = (double)s.count, f = (double)P::sum_f(first, s.count), ff = (double)P::sum_ff(second);
+    // (an empty bucket: three zeros)
+    s.raw = __double2ull_rn(fma(k.raw2, ff, fma(k.raw1, f, n)) * raw_weight);
+    s.tempered = __double2ull_rn(fma(k.tempered2, ff, fma(k.tempered1, f, n)) * tempered_weight);
+    return s;
+}
+
+constexpr double kFixedOne = 1099511627776.0;  // 2^40
+
+// Masses and counts of this CTA's groups into m.raw, m.tempered, m.count (place 1 + group), and the
+// weights they are made with into m.edges, m.lanes; state.counted gets the sum of all counts.  All
+// threads call; ends synced.
+template <class P>
+__device__ __noinline__ void group_masses(const Window window, double best, double inv_t) {
+    ShortMemory &m = short_memory();
+    const uint32_t tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
+    constexpr uint32_t kWarps = kNucleusWarps;
+    static_assert(kNucleusThreads == 2 * kGroups && kGroups == 16 * kWarps, "an exponential per thread, 16 groups per warp");
+    static_assert(kFineSlots == 8 * 32 * kWarps && kMiddleSlots == 4 * 32 * kWarps, "four groups abreast are of one kind");
+    {
+        const uint32_t group = tid % kGroups, tempered = tid / kGroups;
+        const double x = window.middle(group * 32u) - best;
+        m.edges[tempered][group] = exp(tempered ? x * inv_t : x) * kFixedOne;
+        if (tid < 192u) {
+            const uint32_t kind = tid / 32u % 3u;
+            float width;
+            window.middle_of(kind == 0 ? 0u : kind == 1 ? kFineSlots : kFineSlots + kMiddleSlots, width);
+            const double away = -(double)lane * (double)width;
+            m.lanes[tid / 96u][kind][lane] = exp(tid < 96u ? away : away * inv_t);
+        }
+    }
+    __syncthreads();
+    uint32_t counted = 0;
+    // four groups abreast: their chains of conversions and reductions overlap
+#pragma unroll 1
+    for (uint32_t j = 0; j < 16; j += 4) {
+        const uint32_t group0 = j * kWarps + warp, kind = kind_of_group(group0);
+        uint32_t first[4], second[4], any = 0;
+#pragma unroll
+        for (uint32_t q = 0; q < 4; q++) {
+            const uint32_t at = swizzled((group0 + q * kWarps) * 32u + lane);
+            first[q] = m.first[at];
+            second[q] = m.second[at];
+            any |= second[q];
+        }
+        any = __any_sync(kFullMask, any != 0);
+        if (!any) {
+            if (lane < 4) {
+                const uint32_t place = 1 + group0 + lane * kWarps;
+                m.raw[place] = m.tempered[place] = 0;
+                m.count[place] = 0;
+            }
+            continue;
+        }
+        const MomentFactors<P> k(window, group0 * 32u, inv_t);
+        const double raw_lane = m.lanes[0][kind][lane], tempered_lane = m.lanes[1][kind][lane];
+#pragma unroll
+        for (uint32_t q = 0; q < 4; q++) {
+            const uint32_t group = group0 + q * kWarps;
+            const SlotMass s = slot_mass<P>(first[q], second[q], k, m.edges[0][group] * raw_lane, m.edges[1][group] * tempered_lane);
+            const unsigned long long raw = warp_sum_mass(s.raw), tempered = warp_sum_mass(s.tempered);
+            const uint32_t count = __reduce_add_sync(kFullMask, s.count);
+            if (lane == 0) {
+                m.raw[1 + group] = raw;
+                m.tempered[1 + group] = tempered;
+                m.count[1 + group] = count;
+            }
+            counted += count;
+        }
+    }
+    if (lane == 0) atomicAdd(&m.state.counted, counted);
+    __syncthreads();
+}
+
+// Among the 32 slots of a group, summed over the team: the first at which the running raw (or
+// tempered) mass reaches `target` (strict: exceeds it); the last with members when none does.
+// One warp calls.
+template <class P>
+__device__ __noinline__ SlotHit find_slot(const Team team, const Window window, uint32_t group,
+                                          double inv_t, unsigned long long raw_before,
+                                          unsigned long long tempered_before, uint32_t count_before,
+                                          unsigned long long target, bool tempered, bool strict) {
+    ShortMemory &m = short_memory();
+    const uint32_t lane = lane_id();
+    const MomentFactors<P> k(window, group * 32u, inv_t);
+    const uint32_t kind = kind_of_group(group);
+    const double raw_weight = m.edges[0][group] * m.lanes[0][kind][lane];
+    const double tempered_weight = m.edges[1][group] * m.lanes[1][kind][lane];
+    const uint32_t at = swizzled(group * 32u + lane);
+    SlotMass mine;
+    mine.raw = mine.tempered = 0;
+    mine.count = 0;
+    uint32_t far_first[kMostTeam], far_second[kMostTeam];
+#pragma unroll
+    for (uint32_t r = 0; r < kMostTeam; r++) {
+        far_first[r] = r < team.size ? *team.at(&m.first[at], r) : 0u;
+        far_second[r] = r < team.size ? *team.at(&m.second[at], r) : 0u;
+    }
+#pragma unroll
+    for (uint32_t r = 0; r < kMostTeam; r++) {
+        if (r >= team.size) break;
+        const SlotMass s = slot_mass<P>(far_first[r], far_second[r], k, raw_weight, tempered_weight);
+        mine.raw += s.raw;
+        mine.tempered += s.tempered;
+        mine.count += s.count;
+    }
+    unsigned long long raw = mine.raw, other = mine.tempered;
+    uint32_t count = mine.count;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const unsigned long long up_raw = __shfl_up_sync(kFullMask, raw, d), up_other = __shfl_up_sync(kFullMask, other, d);
+        const uint32_t up_count = __shfl_up_sync(kFullMask, count, d);
+        if (lane >= (uint32_t)d) {
+            raw += up_raw;
+            other += up_other;
+            count += up_count;
+        }
+    }
+    const unsigned long long here = tempered ? tempered_before + other : raw_before + raw;
+    const uint32_t reached = __ballot_sync(kFullMask, strict ? here > target : here >= target);
+    const uint32_t peopled = __ballot_sync(kFullMask, mine.count != 0);
+    const int lead = reached ? __ffs(reached) - 1 : (peopled ? 31 - __clz(peopled) : 0);
+    SlotHit hit;
+    hit.slot = group * 32u + (uint32_t)lead;
+    hit.count = __shfl_sync(kFullMask, mine.count, lead);
+    hit.count_before = count_before + __shfl_sync(kFullMask, count - mine.count, lead);
+    hit.raw_before = raw_before + __shfl_sync(kFullMask, raw - mine.raw, lead);
+    hit.tempered = __shfl_sync(kFullMask, mine.tempered, lead);
+    hit.tempered_before = tempered_before + __shfl_sync(kFullMask, other - mine.tempered, lead);
+    return hit;
+}
+
+// cumulative / sum >= top_p  <=>  cumulative >= top_p * sum
+__device__ __forceinline__ unsigned long long mass_target_of(double top_p, unsigned long long total) {
+    const unsigned long long t = (unsigned long long)ceil(top_p * (double)total);
+    return t > total ? total : t;
+}
+// the first element whose cumulative weight exceeds draw = u * sum
+__device__ __forceinline__ unsigned long long draw_target_of(double draw_at, unsigned long long total) {
+    return (unsigned long long)floor(draw_at * (double)total);
+}
+
+// The first CTA adds the team's masses up and finds the buckets the answer lies in.  All its
+// threads call; ends synced.
+template <class P>
+__device__ __noinline__ void make_plan(const Team team, const Window window, float best, double top_p, double inv_t,
+                                       double draw_at) {
+    ShortMemory &m = short_memory();
+    ShortShared &ss = m.state;
+    const NucleusShared &sh = m.scan;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const uint32_t over = min(ss.over_count, kOverCap);
+    bool crowded = false;
+    for (uint32_t r = 0; r < team.size; r++) crowded = crowded || team.at(&ss.share, r)->crowded != 0;
+    // place 0: the values above the window, each with its own weights
+    if (warp == kNucleusWarps - 1) {
+        unsigned long long raw = 0, tempered = 0;
+        for (uint32_t i = lane; i < over; i += 32) {
+            const double x = (double)m.over_value[i] - (double)best;
+            raw += exp_fixed(x, sh.table);
+            tempered += exp_fixed(x * inv_t, sh.table);
+        }
+        raw = warp_sum_mass(raw);
+        tempered = warp_sum_mass(tempered);
+        if (lane == 0) {
+            m.raw[0] = raw;
+            m.tempered[0] = tempered;
+            m.count[0] = over;
+        }
+    }
+    __syncthreads();
+    unsigned long long raw = 0, tempered = 0;
+    uint32_t count = 0;
+    if (tid < kPlaces) {
+        raw = m.raw[tid];
+        tempered = m.tempered[tid];
+        count = m.count[tid];
+        unsigned long long far_raw[kMostTeam], far_tempered[kMostTeam];  // (all on their way before one is used)
+        uint32_t far_count[kMostTeam];
+#pragma unroll
+        for (uint32_t r = 1; r < kMostTeam; r++) {
+            const bool there = tid > 0 && r < team.size;
+            far_raw[r] = there ? *team.at(&m.raw[tid], r) : 0ull;
+            far_tempered[r] = there ? *team.at(&m.tempered[tid], r) : 0ull;
+            far_count[r] = there ? *team.at(&m.count[tid], r) : 0u;
+        }
+#pragma unroll
+        for (uint32_t r = 1; r < kMostTeam; r++) {
+            raw += far_raw[r];
+            tempered += far_tempered[r];
+            count += far_count[r];
+        }
+    }
+    const unsigned long long own_raw = raw, own_tempered = tempered;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const unsigned long long up_raw = __shfl_up_sync(kFullMask, raw, d), up_tempered = __shfl_up_sync(kFullMask, tempered, d);
+        const uint32_t up_count = __shfl_up_sync(kFullMask, count, d);
+        if (lane >= (uint32_t)d) {
+            raw += up_raw;
+            tempered += up_tempered;
+            count += up_count;
+        }
+    }
+    if (lane == 31) {
+        ss.scan_raw[warp] = raw;
+        ss.scan_tempered[warp] = tempered;
+        ss.scan_count[warp] = count;
+    }
+    __syncthreads();
+    unsigned long long total_raw = 0;
+    constexpr uint32_t kScanWarps = (kPlaces + 31) / 32;
+#pragma unroll
+    for (uint32_t w = 0; w < kScanWarps; w++) {
+        const unsigned long long more = ss.scan_raw[w], more_tempered = ss.scan_tempered[w];
+        const uint32_t more_count = ss.scan_count[w];
+        total_raw += more;
+        raw += w < warp ? more : 0ull;
+        tempered += w < warp ? more_tempered : 0ull;
+        count += w < warp ? more_count : 0u;
+    }
+    const unsigned long long cut_target = mass_target_of(top_p, total_raw);
+    if (tid < kPlaces) {
+        m.raw[tid] = raw;
+        m.tempered[tid] = tempered;
+        m.count[tid] = count;
+        if (raw - own_raw < cut_target && raw >= cut_target) ss.cut_place = tid;  // exactly one thread when there is any mass
+    }
+    __syncthreads();
+    if (crowded || total_raw == 0) {
+        if (tid == 0) ss.plan.verdict = kLongWay;
+        __syncthreads();
+        return;
+    }
+    const uint32_t cut_place = ss.cut_place;
+    if (warp == 0) {
+        SlotHit cut;
+        cut.slot = 0;
+        cut.count = over;
+        cut.count_before = 0;
+        cut.raw_before = cut.tempered_before = 0;
+        cut.tempered = m.tempered[0];
+        if (cut_place != 0)
+            cut = find_slot<P>(team, window, cut_place - 1, inv_t, m.raw[cut_place - 1],
+                               m.tempered[cut_place - 1], m.count[cut_place - 1], cut_target, false, false);
+        if (lane == 0) {
+            ss.plan.cut = cut_place == 0 ? 0u : 1u + cut.slot;
+            ss.plan.cut_target = cut_target;
+            ss.plan.cut_before = cut.raw_before;
+            ss.plan.cut_tempered_before = cut.tempered_before;
+            ss.plan.cut_rank_before = cut.count_before;
+            ss.plan.cut_members = cut.count;
+            ss.plan.pick_before = cut.tempered;  // (handed on to the next step)
+            ss.pick_place[0] = ss.pick_place[1] = cut_place;
+        }
+    }
+    __syncthreads();
+    // The nucleus weighs at least what lies above the cut's bucket and at most that and the
+    // bucket: the draw lands between the two targets.
+    const unsigned long long least = ss.plan.cut_tempered_before, most = least + ss.plan.pick_before;
+    const unsigned long long target_first = draw_target_of(draw_at, least), target_last = draw_target_of(draw_at, most);
+    if (tid < kPlaces && tid < cut_place) {
+        const unsigned long long before = tempered - own_tempered;
+        if (before <= target_first && tempered > target_first) ss.pick_place[0] = tid;
+        if (before <= target_last && tempered > target_last) ss.pick_place[1] = tid;
+    }
+    __syncthreads();
+    __shared__ uint32_t ends[2], ends_count[2];
+    __shared__ unsigned long long ends_before;
+    if (warp < 2) {
+        const uint32_t place = ss.pick_place[warp];
+        const unsigned long long target = warp == 0 ? target_first : target_last;
+        uint32_t at = 0, edge = warp == 0 ? 0u : over;
+        unsigned long long before = 0;
+        if (place != 0) {
+            const SlotHit hit = find_slot<P>(team, window, place - 1, inv_t, m.raw[place - 1],
+                                             m.tempered[place - 1], m.count[place - 1], target, true, true);
+            at = 1u + hit.slot;
+            before = hit.tempered_before;
+            edge = warp == 0 ? hit.count_before : hit.count_before + hit.count;
+            if (at > ss.plan.cut) {  // (nothing below the cut takes part)
+                at = ss.plan.cut;
+                before = ss.plan.cut_tempered_before;
+                edge = warp == 0 ? ss.plan.cut_rank_before : ss.plan.cut_rank_before + ss.plan.cut_members;
+            }
+        }
+        if (lane == 0) {
+            ends[warp] = at;
+            ends_count[warp] = edge;
+            if (warp == 0) ends_before = before;
+        }
+    }
+    __syncthreads();
+    if (tid == 0) {
+        ss.plan.pick_first = ends[0];
+        ss.plan.pick_last = ends[1];
+        ss.plan.pick_before = ends_before;
+        ss.plan.pick_members = ends_count[1] - ends_count[0];
+        ss.plan.verdict = (ss.plan.cut != 0 && ss.plan.cut_members > kCutCap) || ss.plan.pick_members > kPickCap ? kLongWay : kDone;
+    }
+    __syncthreads();
+}
+
+// The second pass: the members of the plan's buckets onto the first CTA's two lists.
+struct Gatherer {
+    const Team team;
+    float cut_low, cut_high, pick_low, pick_high;  // whole buckets, both ends included
+
+    __device__ __forceinline__ Gatherer(const Team &team_, const Window &w) : team(team_) {
+        const Plan *plan = team.at(&short_memory().state.plan, 0);
+        cut_low = pick_low = __uint_as_float(0x7f800000u);  // nothing
+        cut_high = pick_high = __uint_as_float(0xff800000u);
+        if (plan->cut != 0) {
+            cut_low = w.lowest(plan->cut - 1);
+            cut_high = w.highest(plan->cut - 1);
+        }
+        if (plan->pick_last != 0) {
+            pick_low = w.lowest(plan->pick_last - 1);
+            pick_high = plan->pick_first != 0 ? w.highest(plan->pick_first - 1) : w.top;
+        }
+    }
+    __device__ __forceinline__ bool wanted(float v) const {
+        return (v >= cut_low && v <= cut_high) || (v >= pick_low && v <= pick_high);
+    }
+    // `skip`: columns that do not count
+    __device__ __forceinline__ void put(float v, uint32_t column, const SeenBits &skip) const {
+        if (skip.test(column)) return;
+        ShortMemory &m = short_memory();
+        if (v >= cut_low && v <= cut_high) {
+            const uint32_t slot = atomicAdd(team.at(&m.state.cut_count, 0), 1u);
+            if (slot < kCutCap) {
+                team.at(m.lists.cut_value, 0)[slot] = v;
+                team.at(m.lists.cut_id, 0)[slot] = column;
+            }
+        }
+        if (v >= pick_low && v <= pick_high) {
+            const uint32_t slot = atomicAdd(team.at(&m.state.pick_count, 0), 1u);
+            if (slot < kPickCap) {
+                team.at(m.lists.pick_value, 0)[slot] = v;
+                team.at(m.lists.pick_id, 0)[slot] = column;
+            }
+        }
+    }
+    template <int kPer>
+    __device__ __forceinline__ void take_vector(const float (&v)[kPer], uint32_t column, const SeenBits &skip) const {
+        uint32_t hits = 0;
+#pragma unroll
+        for (int j = 0; j < kPer; j++) hits |= wanted(v[j]) ? 1u << j : 0u;
+#pragma unroll 1
+        for (; hits != 0; hits &= hits - 1) {
+            const int j = __ffs(hits) - 1;
+            put(pick_element(v, j), column + j, skip);
+        }
+    }
+};
+
+// (`listed` seen columns with their penalised values; their raw logits do not count)
+template <typename T>
+__device__ __noinline__ void gather_members(const T *columns, uint32_t lo, uint32_t n, const Window window, const Team team,
+                                            const SeenBits bits, const float2 *seen, uint32_t listed) {
+    const Gatherer gather(team, window);
+    walk_logits<T>(
+        columns + lo, n, [&](const float (&v)[Vector<T>::kPer], uint32_t c) { gather.take_vector(v, lo + c, bits); },
+        [&](float v, uint32_t c) {
+            if (gather.wanted(v)) gather.put(v, lo + c, bits);
+        });
+    const SeenBits all_listed = {nullptr, 0, 1};
+    constexpr int kBatch = 4;
+    for (uint32_t i0 = threadIdx.x; i0 < listed; i0 += kBatch * kNucleusThreads) {
+        float2 pair[kBatch];
+#pragma unroll
+        for (int q = 0; q < kBatch; q++) {
+            const uint32_t i = i0 + q * kNucleusThreads;
+            pair[q] = i < listed ? seen[i] : make_float2(__uint_as_float(0x7fc00000u), 0.0f);
+        }
+#pragma unroll
+        for (int q = 0; q < kBatch; q++)
+            if (gather.wanted(pair[q].x)) gather.put(pair[q].x, __float_as_uint(pair[q].y), all_listed);
+    }
+}
+
+// The first CTA orders the gathered members and reports the row; leaves the verdict in the plan.
+// All its threads call; ends synced.
+__device__ __noinline__ void finish_short(float best, double inv_t, double draw_at, uint32_t row,
+                                          const SelectOutput &out) {
+    ShortMemory &m = short_memory();
+    ShortShared &ss = m.state;
+    NucleusShared &sh = m.scan;
+    const uint32_t tid = threadIdx.x;
+    const Plan plan = ss.plan;
+    const uint32_t over = min(ss.over_count, kOverCap);
+    // the ordering's work arrays lie where the buckets were
+    OrderWork work;
+    work.weight = reinterpret_cast<unsigned long long *>(m.first);
+    work.sorted_value = reinterpret_cast<float *>(work.weight + kOrderCap);
+    work.sorted_id = reinterpret_cast<uint32_t *>(work.sorted_value + kOrderCap);
+    static_assert(kOrderCap * 16 <= sizeof(m.first) + sizeof(m.second), "the ordering fits over the buckets");
+    work.value = plan.cut == 0 ? m.over_value : m.lists.cut_value;
+    work.id = plan.cut == 0 ? m.over_id : m.lists.cut_id;
+    Nucleus nucleus;
+    nucleus.everything = true;
+    nucleus.key = nucleus.id = 0;
+    unsigned long long tempered_inside = 0;
+    // (one copy of the ordering's code for both turns)
+    Position cut, pick;
+    cut.ok = pick.ok = false;
+    unsigned long long weight_sum = 0;
+    uint32_t members = plan.cut == 0 ? over : min(ss.cut_count, kCutCap);
+#pragma unroll 1
+    for (int turn = 0; turn < 2; turn++) {
+        const Position found = order_members(sh, work, members, turn == 0 ? 1.0 : inv_t, best, nucleus,
+                                             turn == 0 ? plan.cut_before : plan.pick_before,
+                                             turn == 0 ? plan.cut_rank_before : 0u,
+                                             turn == 0 ? plan.cut_target : draw_target_of(draw_at, weight_sum), turn != 0,
+                                             false, inv_t, turn == 0 ? &tempered_inside : nullptr);
+        if (turn != 0) {
+            pick = found;
+            break;
+        }
+        cut = found;
+        if (!cut.ok) break;
+        nucleus.everything = false;
+        nucleus.key = cut.key;
+        nucleus.id = cut.id;
+        weight_sum = plan.cut_tempered_before + tempered_inside;
+        members = min(ss.pick_count, kPickCap);
+        work.value = m.lists.pick_value;
+        work.id = m.lists.pick_id;
+        if (plan.pick_first == 0) {  // what lies above the window takes part
+            const uint32_t more = min(over, kPickCap - members);
+            for (uint32_t i = tid; i < more; i += kNucleusThreads) {
+                m.lists.pick_value[members + i] = m.over_value[i];
+                m.lists.pick_id[members + i] = m.over_id[i];
+            }
+            members += more;
         }
         __syncthreads();
+    }
+    const bool done = cut.ok && pick.ok && weight_sum != 0;
+    if (done && tid == 0) {
+        report_row(out, row, kOk, pick.id, pick.value);
+        if (out.dbg_count) out.dbg_count[row] = cut.rank;  // nucleus size; the list itself is not dumped
+    }
+    if (tid == 0) ss.plan.verdict = done ? kDone : kLongWay;
+    __syncthreads();
+}
+
+// One row's second half: masses, plan, gather, order.  All CTAs of the team call, with the
+// buckets filled; returns the verdict.
+template <typename T, class P>
+__device__ __forceinline__ uint32_t locate_and_pick(const NucleusParams &p, const Team &team, const Window &window,
+                                                    uint32_t row, uint32_t lo, uint32_t n, uint32_t counted,
+                                                    const SeenBits &bits, const float2 *seen, float best, double top_p,
+                                                    double inv_t, double draw_at) {
+    ShortShared &ss = short_memory().state;
+    group_masses<P>(window, (double)best, inv_t);
+    if (threadIdx.x == 0) ss.share.crowded = ss.counted != counted;
+    team.sync();
+    if (team.rank == 0) make_plan<P>(team, window, best, top_p, inv_t, draw_at);
+    team.sync();
+    if (team.at(&ss.plan, 0)->verdict == kDone) {
+        gather_members<T>(static_cast<const T *>(p.logits) + (size_t)row * p.row_stride, lo, n, window, team, bits, seen,
+                          ss.seen_count);
+        team.sync();
+        if (team.rank == 0) finish_short(best, inv_t, draw_at, row, p.out);
+        team.sync();
+    }
+    return team.at(&ss.plan, 0)->verdict;
+}
+
+// The largest of a few logits spread evenly over the row, NaN, infinities and seen columns left
+// out (so that the row's own maximum is no smaller): where the window goes.  All threads call.
+template <typename T>
+__device__ __forceinline__ float sample_row(const T *columns, uint32_t vocab, const SeenBits &seen) {
+    ShortShared &ss = short_memory().state;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    float best = __uint_as_float(0xff800000u);
+#pragma unroll
+    for (int j = 0; j < kSamples; j++) {
+        const uint32_t at = (uint32_t)(((uint64_t)(j * kNucleusThreads + tid) * vocab) / (kSamples * kNucleusThreads));
+        const float v = Vector<T>::one(columns + at);
+        if (!is_nonfinite(v) && !seen.test(at)) best = fmaxf(best, v);
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) best = fmaxf(best, __shfl_xor_sync(kFullMask, best, d));
+    if (lane == 0) ss.sample_max[warp] = best;
+    __syncthreads();
+    best = ss.sample_max[lane % kNucleusWarps];
+#pragma unroll
+    for (int d = kNucleusWarps / 2; d > 0; d >>= 1) best = fmaxf(best, __shfl_xor_sync(kFullMask, best, d));
+    return best;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kNucleusThreads, 2) nucleus_select_kernel(const __grid_constant__ NucleusParams p) {
+    constexpr bool kBf16 = sizeof(T) == 2;
+    ShortMemory &m = short_memory();
+    ShortShared &ss = m.state;
+    NucleusShared &sh = m.scan;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u;
+    Team team;
+    team.size = p.team;
+    team.rank = blockIdx.x % p.team;
+    const uint32_t teams = gridDim.x / p.team, team_index = blockIdx.x / p.team;
+    if (tid < 64) sh.table[tid] = exp2((double)tid / 64.0);
+    if (tid == 0) {
+        ss.over_count = ss.cut_count = ss.pick_count = 0;
+    }
+    float *values = p.scratch + (size_t)team_index * p.scratch_stride;
+    float2 *seen = p.seen + (size_t)blockIdx.x * p.seen_stride;
+    // the CTA's columns: ranges of a multiple of 64, so that every CTA's first column lies as
+    // the row's does to a 16-byte boundary
+    const uint32_t chunk = ((p.vocab + p.team - 1) / p.team + 63u) / 64u * 64u;
+    const uint32_t lo = min(p.vocab, team.rank * chunk);
+    const uint32_t n = min(chunk, p.vocab - lo);
+    team.sync();  // every CTA's lists are there before anybody adds to them
+
+    RowWalk walk(team_index);
+    uint32_t row;
+    while (walk.next(p, teams, row)) {
+        const SamplerConfig cfg = p.config_count > 1 ? p.configs[row] : p.config0;
+        const T *columns = static_cast<const T *>(p.logits) + (size_t)row * p.row_stride;
+        bool penalised = false;  // some column may be
+        uint32_t bad = 0;        // status a broken history earns the row
+        for (uint32_t split = 0; p.history_meta != nullptr && split < p.splits; split++) {
+            const uint2 meta = reinterpret_cast<const uint2 *>(p.history_meta)[(size_t)row * p.splits + split];
+            penalised = penalised || (meta.x & 1u);
+            if (meta.y) bad = meta.y;
+        }
+        if (bad) {  // src/output.c:610-612
+            if (tid == 0 && team.rank == 0) {
+                report_row(p.out, row, bad, kPaddingId, 0.0f);
+                if (p.out.dbg_count) p.out.dbg_count[row] = 0;
+            }
+            continue;
+        }
+        const double inv_t = 1.0 / (double)cfg.temperature, top_p = (double)cfg.top_p;
+        float u = p.uniforms[row];
+        if (is_nonfinite(u) || u < 0.0f) u = 0.0f;
+        if (u >= 1.0f) u = __uint_as_float(0x3f7fffffu);
+        const double draw_at = (double)u;
+
+        // (as many structures as splits in a row, one after the other)
+        const SeenBits bits = {penalised ? p.history_global + (size_t)row * p.splits * p.history_stride_words : nullptr,
+                               p.history_stride_words, p.split_len};
+        bool counting = cfg.temperature >= kShortColdest && cfg.temperature <= kShortHottest;
+        uint32_t finite = 1, verdict = kLongWay;
+        float reference = 0.0f;
+        if (counting) reference = sample_row(columns, p.vocab, bits);
+        if (is_nonfinite(reference)) reference = 0.0f;  // (nothing finite among the samples: any window will do)
+        for (uint32_t attempt = 0; counting; attempt++) {
+            const Window window(reference, cfg.temperature < kWideColdest ? 2.0f : 1.0f);
+            if (!window.usable) break;
+            uint4 *words = reinterpret_cast<uint4 *>(m.first);
+            for (uint32_t i = tid; i < 2 * kSlots / 4; i += kNucleusThreads) words[i] = make_uint4(0, 0, 0, 0);
+            if (tid == 0) {
+                ss.lost = ss.below = ss.above = 0;
+                ss.counted = ss.seen_count = 0;
+                ss.top_slot = kSlots;
+            }
+            __syncthreads();
+            // ---- first pass ----
+            Findings found = penalised ? count_logits<T, Packing<false>>(columns, lo, n, window, team, bits)
+                                       : count_logits<T, Packing<kBf16>>(columns, lo, n, window, team, bits);
+            if (penalised) {
+                __syncthreads();
+                const Findings more = amend_seen<T, Packing<false>>(p, row, cfg, lo, n, seen, window, team);
+                found.lost += more.lost;
+                found.below += more.below;
+                found.above += more.above;
+                __syncthreads();
+                // the raw maximum may have been a seen column's: the first bucket that holds anything
+                // now stands for it, and what lies above the window
+                uint32_t slot = tid;
+                while (slot < kSlots && m.second[swizzled(slot)] == 0) slot += kNucleusThreads;
+                slot = __reduce_min_sync(kFullMask, min(slot, kSlots));
+                if (lane == 0) atomicMin(&ss.top_slot, slot);
+                __syncthreads();
+                const float above = fmaxf(found.best > window.top ? found.best : -INFINITY, more.best > window.top ? more.best : -INFINITY);
+                const float within = ss.top_slot < kSlots ? window.highest(ss.top_slot) : -INFINITY;
+                if (fmaxf(above, within) > -INFINITY) found.best = fmaxf(above, within);
+            }
+            float my_best = found.best;
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) my_best = fmaxf(my_best, __shfl_xor_sync(kFullMask, my_best, d));
+            const int lost = __reduce_add_sync(kFullMask, found.lost);
+            const int below = __reduce_add_sync(kFullMask, found.below);
+            const int above = __reduce_add_sync(kFullMask, found.above);
+            if (lane == 0) {
+                ss.sample_max[tid >> 5] = my_best;
+                if (lost) atomicAdd(&ss.lost, lost);
+                if (below) atomicAdd(&ss.below, below);
+                if (above) atomicAdd(&ss.above, above);
+            }
+            __syncthreads();
+            if (tid < 32) {
+                my_best = ss.sample_max[lane % kNucleusWarps];
+#pragma unroll
+                for (int d = kNucleusWarps / 2; d > 0; d >>= 1) my_best = fmaxf(my_best, __shfl_xor_sync(kFullMask, my_best, d));
+                if (lane == 0) {
+                    ss.share.best = my_best;
+                    ss.share.finite = n - (uint32_t)ss.lost;
+                    ss.share.crowded = 0;
+                }
+            }
+            const uint32_t counted = n - (uint32_t)(ss.lost + ss.below + ss.above);
+            team.sync();
+            float best = -INFINITY;
+            finite = 0;
+            for (uint32_t r = 0; r < team.size; r++) {
+                const Share *share = team.at(&ss.share, r);
+                best = fmaxf(best, share->best);
+                finite += share->finite;
+            }
+            const uint32_t over = *team.at(&ss.over_count, 0);
+            if (finite == 0) break;
+            if (attempt == 0 && (over > kOverCap || best < reference)) {
+                // the sample said little: the window once more, from the true maximum
+                team.sync();
+                if (tid == 0) ss.over_count = 0;
+                reference = best;
+                team.sync();
+                continue;
+            }
+            if (over <= kOverCap)
+                verdict = penalised ? locate_and_pick<T, Packing<false>>(p, team, window, row, lo, n, counted, bits, seen,
+                                                                         best, top_p, inv_t, draw_at)
+                                    : locate_and_pick<T, Packing<kBf16>>(p, team, window, row, lo, n, counted, bits, seen,
+                                                                         best, top_p, inv_t, draw_at);
+            break;
+        }
+        if (finite == 0) {
+            // src/sampler.c:97 "sampler received no finite candidates"
+            if (tid == 0 && team.rank == 0) {
+                report_row(p.out, row, kErrFormat, kPaddingId, 0.0f);
+                if (p.out.dbg_count) p.out.dbg_count[row] = 0;
+            }
+        } else if (verdict == kLongWay) {
+            if (tid == 0) ss.seen_count = 0;
+            __syncthreads();
+            write_scratch<T>(p, row, cfg, lo, n, penalised, values);
+            team.sync();
+            if (team.rank == 0) {
+                if (tid == 0) {
+                    sh.mass = reinterpret_cast<unsigned long long *>(&m);
+                    sh.other_mass = sh.mass + kBuckets;
+                    sh.count = reinterpret_cast<uint32_t *>(sh.other_mass + kBuckets);
+                }
+                __syncthreads();
+                sample_the_long_way(sh, *reinterpret_cast<NucleusList *>(sh.count + kBuckets), values, p.vocab, cfg, u, row,
+                                    p.out);
+            }
+        }
+        // the row's lists are empty again before any CTA adds to them
+        if (tid == 0) ss.over_count = ss.cut_count = ss.pick_count = 0;
+        team.sync();
     }
 }
 
@@ -992,14 +2224,46 @@ __global__ void __launch_bounds__(kNucleusThreads, 1) nucleus_select_kernel(cons
 using namespace fgk;
 
 
-static constexpr size_t kNucleusDynamic = kNucleusHistogramBytes + sizeof(NucleusList);
+static constexpr size_t kNucleusDynamic = sizeof(ShortMemory);
+static_assert(kNucleusHistogramBytes + sizeof(NucleusList) <= offsetof(ShortMemory, state), "the long way fits over the short way's memory");
+static_assert(sizeof(ShortMemory) + 64 <= 113 * 1024, "two CTAs to an SM");
 
-extern "C" int fgk_nucleus_prepare(void) {
-    cudaError_t e = cudaFuncSetAttribute(nucleus_select_kernel<float>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kNucleusDynamic);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(nucleus_select_kernel<uint16_t>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kNucleusDynamic);
+static const void *nucleus_kernel(uint32_t dtype) {
+    return dtype == 1u ? reinterpret_cast<const void *>(nucleus_select_kernel<uint16_t>)
+                       : reinterpret_cast<const void *>(nucleus_select_kernel<float>);
+}
+
+static cudaLaunchConfig_t nucleus_config(uint32_t ctas, uint32_t team, cudaLaunchAttribute *cluster, cudaStream_t stream) {
+    cluster->id = cudaLaunchAttributeClusterDimension;
+    cluster->val.clusterDim.x = team;
+    cluster->val.clusterDim.y = 1;
+    cluster->val.clusterDim.z = 1;
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(ctas);
+    config.blockDim = dim3(kNucleusThreads);
+    config.dynamicSmemBytes = kNucleusDynamic;
+    config.stream = stream;
+    config.attrs = cluster;
+    config.numAttrs = 1;
+    return config;
+}
+
+extern "C" int fgk_nucleus_prepare(uint32_t most_teams[FGK_NUCLEUS_TEAM_SIZES]) {
+    cudaError_t e = cudaSuccess;
+    for (uint32_t i = 0; i < FGK_NUCLEUS_TEAM_SIZES; i++) most_teams[i] = 0xffffffffu;
+    for (uint32_t dtype = 0; dtype < 2u && e == cudaSuccess; dtype++) {
+        e = cudaFuncSetAttribute(nucleus_kernel(dtype), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kNucleusDynamic);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(nucleus_kernel(dtype), cudaFuncAttributePreferredSharedMemoryCarveout,
+                                     (int)cudaSharedmemCarveoutMaxShared);
+        for (uint32_t i = 0; i < FGK_NUCLEUS_TEAM_SIZES && e == cudaSuccess; i++) {
+            cudaLaunchAttribute cluster;
+            const cudaLaunchConfig_t config = nucleus_config(1u << i, 1u << i, &cluster, nullptr);
+            int teams = 0;
+            e = cudaOccupancyMaxActiveClusters(&teams, nucleus_kernel(dtype), &config);
+            if (e == cudaSuccess && (uint32_t)teams < most_teams[i]) most_teams[i] = (uint32_t)teams;
+        }
+    }
     return (int)e;
 }
 
@@ -1022,8 +2286,11 @@ extern "C" int fgk_launch_nucleus_select(const fgk_nucleus_launch *l, void *stre
     p.config0.seed = l->config0.seed;
     p.config_count = l->config_count;
     p.uniforms = l->uniforms;
+    p.team = l->team;
     p.scratch = l->scratch;
     p.scratch_stride = l->scratch_stride;
+    p.seen = static_cast<float2 *>(l->seen);
+    p.seen_stride = l->seen_stride;
     p.history_global = l->history_global;
     p.history_stride_words = l->history_stride_words;
     p.history_meta = l->history_meta;
@@ -1041,10 +2308,9 @@ extern "C" int fgk_launch_nucleus_select(const fgk_nucleus_launch *l, void *stre
     p.out.dbg_scores = l->out.dbg_scores;
     p.out.dbg_raw = l->out.dbg_raw;
     p.out.dbg_tempered = l->out.dbg_tempered;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (l->dtype == 1u)
-        nucleus_select_kernel<uint16_t><<<l->ctas, kNucleusThreads, kNucleusDynamic, s>>>(p);
-    else
-        nucleus_select_kernel<float><<<l->ctas, kNucleusThreads, kNucleusDynamic, s>>>(p);
-    return (int)cudaGetLastError();
+    cudaLaunchAttribute cluster;
+    const cudaLaunchConfig_t config = nucleus_config(l->ctas, l->team, &cluster, static_cast<cudaStream_t>(stream));
+    void *arguments[] = {&p};
+    const cudaError_t e = cudaLaunchKernelExC(&config, nucleus_kernel(l->dtype), arguments);
+    return (int)(e != cudaSuccess ? e : cudaGetLastError());
 }

@@ -22,6 +22,7 @@
 namespace fgk {
 
 constexpr int kThreads = 256;
+constexpr int kHistoryThreads = 1024;  // of the history pass: long histories are a chain of load latencies
 constexpr int kElemsPerThread = 16;
 constexpr int kTile = kThreads * kElemsPerThread;  // 4096 logits per CTA iteration
 constexpr int kCandCap = 1024;
@@ -69,7 +70,7 @@ struct StreamParams {
 struct StreamShared {
     CandidateBuffer<kCandCap> cand;
     FinishBuffer fin;
-    uint32_t scan[kThreads / 32];
+    uint32_t scan[kHistoryThreads / 32];
     uint32_t distinct;
     uint32_t bad_history;
     unsigned long long wild_key;  // greedy rows: min over NaN/Inf of (id << 32 | value bits)
@@ -299,6 +300,7 @@ constexpr uint32_t kWithCounts = 2u;   // ... and a frequency penalty, so counts
 // frequency * count + presence it will be charged (src/output.c:601-617 keeps a
 // vocabulary-wide count table per session instead).  Kept out of line so its
 // registers do not weigh on the streaming loop.
+template <int kCount>
 __device__ __noinline__ uint32_t build_history(const StreamParams &p, StreamShared &sh,
                                                uint32_t *dyn_smem, uint32_t row, uint32_t lo,
                                                uint32_t n, const SamplerConfig cfg) {
@@ -323,21 +325,22 @@ __device__ __noinline__ uint32_t build_history(const StreamParams &p, StreamShar
     const bool with_counts = seen_any && cfg.frequency_penalty != 0.0f && p.count_capacity != 0;
     if (!seen_any) return 0;
 
-    for (uint32_t w = tid; w < words; w += kThreads) bitmap[w] = 0;
+    for (uint32_t w = tid; w < words; w += kCount) bitmap[w] = 0;
     __syncthreads();
     const uint32_t first_global = p.vocab_offset + lo;
-    // four tokens per thread and trip, loaded before any is used: the loop is a chain of
+    // several tokens per thread and trip, loaded before any is used: the loop is a chain of
     // global-load latencies otherwise
-    for (uint32_t base = 0; base < history_len; base += 4 * kThreads) {
-        uint32_t token[4];
+    constexpr int kTrip = kCount == kHistoryThreads ? 8 : 4;
+    for (uint32_t base = 0; base < history_len; base += kTrip * kCount) {
+        uint32_t token[kTrip];
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const uint32_t i = base + q * kThreads + tid;
+        for (int q = 0; q < kTrip; q++) {
+            const uint32_t i = base + q * kCount + tid;
             token[q] = i < history_len ? history[i] : 0u;
         }
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            if (base + q * kThreads + tid >= history_len) continue;
+        for (int q = 0; q < kTrip; q++) {
+            if (base + q * kCount + tid >= history_len) continue;
             if (token[q] >= p.vocab_total) sh.bad_history = kErrFormat;
             const uint32_t local = token[q] - first_global;  // wraps for ids below the split
             if (local < n) {
@@ -350,7 +353,7 @@ __device__ __noinline__ uint32_t build_history(const StreamParams &p, StreamShar
     if (!with_counts) return kSeenAny;
 
     // exclusive running popcount per word: each thread owns a contiguous run of words
-    const uint32_t per = (words + kThreads - 1) / kThreads;
+    const uint32_t per = (words + kCount - 1) / kCount;
     const uint32_t w0 = min(tid * per, words), w1 = min(w0 + per, words);
     uint32_t mine = 0;
     for (uint32_t w = w0; w < w1; w++) mine += __popc(bitmap[w]);
@@ -364,7 +367,7 @@ __device__ __noinline__ uint32_t build_history(const StreamParams &p, StreamShar
     __syncthreads();
     uint32_t before = incl - mine;
     for (uint32_t q = 0; q < warp; q++) before += sh.scan[q];
-    if (tid == kThreads - 1) sh.distinct = before + mine;
+    if (tid == kCount - 1) sh.distinct = before + mine;
     for (uint32_t w = w0; w < w1; w++) {
         running[w] = (uint16_t)before;  // the host keeps count_capacity below 65,536
         before += __popc(bitmap[w]);
@@ -374,19 +377,19 @@ __device__ __noinline__ uint32_t build_history(const StreamParams &p, StreamShar
     const uint32_t distinct = min(sh.distinct, p.count_capacity);
     uint32_t *dense_words = static_cast<uint32_t *>(view.dense);
     const uint32_t dense_word_count = view.wide ? distinct : (distinct + 1) / 2;
-    for (uint32_t i = tid; i < dense_word_count; i += kThreads) dense_words[i] = 0;
+    for (uint32_t i = tid; i < dense_word_count; i += kCount) dense_words[i] = 0;
     __syncthreads();
-    for (uint32_t base = 0; base < history_len; base += 4 * kThreads) {
-        uint32_t token[4];
+    for (uint32_t base = 0; base < history_len; base += kTrip * kCount) {
+        uint32_t token[kTrip];
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const uint32_t i = base + q * kThreads + tid;
+        for (int q = 0; q < kTrip; q++) {
+            const uint32_t i = base + q * kCount + tid;
             token[q] = i < history_len ? history[i] : 0u;
         }
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
+        for (int q = 0; q < kTrip; q++) {
             const uint32_t local = token[q] - first_global;
-            if (base + q * kThreads + tid < history_len && local < n) {
+            if (base + q * kCount + tid < history_len && local < n) {
                 const uint32_t at = view.slot(local >> 5, bitmap[local >> 5], local & 31u);
                 // 16-bit counts share a word: add into the right half (a half cannot carry,
                 // a history that could overflow it uses 32-bit counts)
@@ -875,7 +878,7 @@ stream_select_kernel(const __grid_constant__ StreamParams p) {
     __syncthreads();
 
     // ---- 1. history slice -> bitmap / running popcount / offsets ----
-    state.flags = build_history(p, sh, dyn_smem, row, lo, state.n, cfg);
+    state.flags = build_history<kThreads>(p, sh, dyn_smem, row, lo, state.n, cfg);
 
     // ---- 2. stream the columns ----
     // Tiles 1 .. full-1 of a 16-byte aligned row take the fast loop below: 128-bit
@@ -925,7 +928,7 @@ struct alignas(8) HistoryMeta {
 
 // build_history in shared memory, then the structure is copied verbatim to the unit's
 // slot in global memory.
-__global__ void __launch_bounds__(kThreads) history_build_kernel(const __grid_constant__ StreamParams p) {
+__global__ void __launch_bounds__(kHistoryThreads) history_build_kernel(const __grid_constant__ StreamParams p) {
     extern __shared__ __align__(16) uint32_t dyn_smem[];
     __shared__ StreamShared sh;
     const uint32_t tid = threadIdx.x;
@@ -938,13 +941,13 @@ __global__ void __launch_bounds__(kThreads) history_build_kernel(const __grid_co
         sh.distinct = 0;
     }
     __syncthreads();
-    const uint32_t flags = build_history(p, sh, dyn_smem, row, lo, n, cfg);
+    const uint32_t flags = build_history<kHistoryThreads>(p, sh, dyn_smem, row, lo, n, cfg);
     __syncthreads();
     const size_t unit = (size_t)row * p.splits + split;
     if (flags) {
         uint32_t *out = p.history_global + unit * p.history_stride_words;
         const uint32_t words = (uint32_t)p.history_stride_words;
-        for (uint32_t i = tid; i < words; i += kThreads) out[i] = dyn_smem[i];
+        for (uint32_t i = tid; i < words; i += kHistoryThreads) out[i] = dyn_smem[i];
     }
     if (tid == 0) {
         HistoryMeta meta;
@@ -1200,7 +1203,7 @@ extern "C" int fgk_launch_stream_select(const fgk_stream_launch *l, void *stream
 extern "C" int fgk_launch_history_build(const fgk_stream_launch *l, void *stream) {
     const StreamParams p = to_stream_params(l);
     const size_t dynamic = fgk_stream_dynamic_smem(l->bitmap_words, l->count_capacity, l->dense_wide);
-    history_build_kernel<<<dim3(l->splits, l->rows), kThreads, dynamic, static_cast<cudaStream_t>(stream)>>>(p);
+    history_build_kernel<<<dim3(l->splits, l->rows), kHistoryThreads, dynamic, static_cast<cudaStream_t>(stream)>>>(p);
     return (int)cudaGetLastError();
 }
 

@@ -96,7 +96,7 @@ fg_status fg_cuda_context_create(int device, fg_cuda_context **out, fg_error *er
     if (!e) e = fgk_stream_create(&c->own_stream);
     if (!e) e = fgk_stream_prepare();
     if (!e) e = fgk_persistent_prepare();
-    if (!e) e = fgk_nucleus_prepare();
+    if (!e) e = fgk_nucleus_prepare(c->nucleus_teams);
     if (!e) e = fgk_malloc((void **)&c->first_error, 256u);
     if (e) {
         fg_status status = fg_cuda_fail(err, e, "opening the CUDA context");
@@ -555,7 +555,8 @@ static bool plan_stream(const fg_cuda_context *c, uint32_t rows, uint32_t vocab,
 }
 
 typedef struct batch_traits {
-    bool penalties, counts, sampled, nucleus, topk_rows;
+    bool penalties, counts, sampled, topk_rows;
+    uint32_t nucleus; /* rows without a top-k cut */
     bool raising; /* some row's penalties can raise a logit (or its repetition factor is extreme) */
 } batch_traits;
 
@@ -587,13 +588,14 @@ static fg_status check_batch(const fg_cuda_context *c, const fg_cuda_sample_args
         if (cfg->frequency_penalty != 0.0f) traits->counts = true;
         if (cfg->temperature != 0.0f) {
             traits->sampled = true;
-            if (cfg->top_k == 0u) traits->nucleus = true;
+            if (cfg->top_k == 0u) traits->nucleus++;
             else traits->topk_rows = true;
         } else {
             traits->topk_rows = true;
         }
     }
     if (shard) traits->topk_rows = true;
+    if (traits->nucleus && a->config_count == 1u) traits->nucleus = a->rows;
     if (traits->sampled && !shard && !a->uniforms) {
         fg_error_set(err, FG_ERR_ARGUMENT, "sampled rows need one uniform draw each");
         return FG_ERR_ARGUMENT;
@@ -796,8 +798,35 @@ static fg_status run_stream(fg_cuda_context *c, const fg_cuda_sample_args *a,
     return e ? fg_cuda_fail(err, e, "streaming select kernel") : FG_OK;
 }
 
+/* How many CTAs share a row without a top-k cut.  A row costs its CTAs a fixed time (barriers,
+ * prefix sums, ordering the candidates: about that of 160,000 columns) and a time that shrinks
+ * with the columns each has, but doubles once SMs hold two CTAs; the teams that fit the GPU work in
+ * rounds.  Measured on B200, vocabulary 151,936, fp32, teams of 1 / 2 / 4 / 8: one row - / 52 / 43 / 40 us,
+ * 32 rows - / 58 / 48 / 55, 64 rows - / 60 / 65 / 104, 148 rows 80 / 84 / 158 / -, 512 rows
+ * 238 / 277 / 435 / -. */
+static uint32_t plan_teams(const fg_cuda_context *c, uint32_t rows, uint32_t vocab, uint32_t *teams) {
+    uint32_t best = 1u;
+    double best_cost = 0.0;
+    *teams = rows < c->sm_count ? rows : c->sm_count;
+    if (rows == 0u) rows = 1u;
+    for (uint32_t i = 0; i < FGK_NUCLEUS_TEAM_SIZES; i++) {
+        const uint32_t most = c->nucleus_teams[i];
+        if (most == 0u) continue;
+        const double rounds = (double)((rows + most - 1u) / most);
+        const uint32_t abreast = rows < most ? rows : most;
+        const double share = (double)vocab / (double)(1u << i) * ((abreast << i) > c->sm_count ? 2.0 : 1.0);
+        const double cost = rounds * (160000.0 + share);
+        if (best_cost == 0.0 || cost < best_cost) {
+            best_cost = cost;
+            best = 1u << i;
+            *teams = abreast;
+        }
+    }
+    return best;
+}
+
 /* Rows without a top-k cut: history pass (when there are penalties), then the
- * persistent nucleus kernel, one scratch row per CTA. */
+ * persistent nucleus kernel, one scratch row per team of CTAs. */
 static fg_status run_nucleus(fg_cuda_context *c, const fg_cuda_sample_args *a,
                              const batch_traits *traits, fg_error *err) {
     fg_cuda_context planner = *c;
@@ -807,9 +836,10 @@ static fg_status run_nucleus(fg_cuda_context *c, const fg_cuda_sample_args *a,
         fg_error_set(err, FG_ERR_LIMIT, "history structure does not fit shared memory");
         return FG_ERR_LIMIT;
     }
-    const uint32_t ctas = a->rows < c->sm_count ? a->rows : c->sm_count;
+    uint32_t teams = 0u;
+    const uint32_t team = plan_teams(c, traits->nucleus, a->vocab, &teams);
     const size_t stride = (size_t)fg_align_up_u64(a->vocab, 64u);
-    fg_status status = fg_cuda_reserve(&c->nucleus, &c->nucleus_bytes, (size_t)ctas * stride * 4u, false, c, err);
+    fg_status status = fg_cuda_reserve(&c->nucleus, &c->nucleus_bytes, (size_t)teams * stride * 4u, false, c, err);
     const void *configs_device = NULL;
     if (status == FG_OK) status = upload_configs(c, a, &configs_device, err);
     if (status != FG_OK) return status;
@@ -828,19 +858,28 @@ static fg_status run_nucleus(fg_cuda_context *c, const fg_cuda_sample_args *a,
     n.uniforms = a->uniforms;
     n.scratch = c->nucleus;
     n.scratch_stride = stride;
-    n.ctas = ctas;
+    n.ctas = teams * team;
+    n.team = team;
     n.splits = plan.splits;
     n.split_len = plan.split_len;
     n.bitmap_words = plan.bitmap_words;
     n.count_capacity = plan.count_capacity;
     n.dense_wide = plan.dense_wide;
     fill_output(&n.out, c, a);
-    c->last_scratch_bytes = (size_t)ctas * stride * 4u;
+    c->last_scratch_bytes = (size_t)teams * stride * 4u;
     if (traits->penalties) {
         const size_t stride_words = plan.dynamic_smem / 4u;
         const size_t meta_at = (size_t)fg_align_up_u64(slots * stride_words * 4u, 256u);
-        status = fg_cuda_reserve(&c->history, &c->history_bytes, meta_at + slots * 8u, false, c, err);
+        /* behind the structures: every CTA's list of seen columns, as many as it has columns or
+         * the row has tokens */
+        const uint64_t columns = fg_align_up_u64((a->vocab + team - 1u) / team, 64u);
+        const uint64_t seen_stride = columns < a->history_max ? columns : a->history_max;
+        const size_t seen_at = (size_t)fg_align_up_u64(meta_at + slots * 8u, 256u);
+        const size_t history_bytes = seen_at + (size_t)seen_stride * 8u * teams * team;
+        status = fg_cuda_reserve(&c->history, &c->history_bytes, history_bytes, false, c, err);
         if (status != FG_OK) return status;
+        n.seen = (unsigned char *)c->history + seen_at;
+        n.seen_stride = seen_stride;
         fgk_stream_launch h;
         memset(&h, 0, sizeof(h));
         h.rows = a->rows;
@@ -866,7 +905,7 @@ static fg_status run_nucleus(fg_cuda_context *c, const fg_cuda_sample_args *a,
         n.history_global = c->history;
         n.history_stride_words = stride_words;
         n.history_meta = h.history_meta;
-        c->last_scratch_bytes += meta_at + slots * 8u;
+        c->last_scratch_bytes += history_bytes;
     }
     const int e = fgk_launch_nucleus_select(&n, c->stream);
     c->launches++;

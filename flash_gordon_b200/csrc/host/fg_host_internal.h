@@ -36,8 +36,9 @@ struct fg_cuda_context {
     size_t tickets_bytes;
     void *history;          /* ring path: history structures, one per (row, split) */
     size_t history_bytes;
-    void *nucleus;          /* one fp32 scratch row per persistent CTA of the nucleus kernel */
+    void *nucleus;          /* one fp32 scratch row per team of CTAs of the nucleus kernel */
     size_t nucleus_bytes;
+    uint32_t nucleus_teams[FGK_NUCLEUS_TEAM_SIZES]; /* how many teams of 1, 2, 4, 8 CTAs run at a time */
     void *configs;          /* per-row configs when they differ */
     size_t configs_bytes;
     uint64_t *first_error;  /* one device word */
