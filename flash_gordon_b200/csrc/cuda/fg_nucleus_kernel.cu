@@ -967,7 +967,7 @@ __device__ __noinline__ void sample_the_long_way(NucleusShared &sh, NucleusList 
 // latencies of 20 us, so two CTAs share an SM, one streaming while the other scans and sorts; for
 // few rows a row is spread over several CTAs instead.  A CTA per row and SM that added two fp64 weights
 // per logit to five shared-memory sums took, per call: 512 rows of 151,936 fp32 logits, histories
-// of 32,768 tokens 772 us (now 546), without history 600 (238); 32 rows bf16 410-560 (63).
+// of 32,768 tokens 772 us (now 546), without history 538 (238); 32 rows bf16 410-560 (63).
 // With histories the largest part is the seen columns' gather (amend_seen).
 //
 // A value's place: buckets 1/1024 wide over the top four units of the row's window, 1/256 wide over

@@ -219,25 +219,52 @@ topk_reduce_kernel(float *out_scores, uint32_t *out_ids, const float *scores, co
 // fp64 sum.  A NaN or +Inf logit makes the token's probabilities meaningless: the ids come
 // back as 0xffffffff and the weights as 0 (shaders/fg_router_top10.glsl:38-51), and the call
 // reports it.  One warp per token.
+//
+// Up to 32 * kPer experts the logits stay in registers, read once.  A round of the selection is
+// two warp-wide reductions: the largest 32-bit value key, then the smallest id that has it; only the lane
+// that gave its best away looks through its registers again.  The k weights are computed side
+// by side afterwards.  kPer == 0 takes any number of experts, reading the row again each round.
+// (What a token costs is mostly latency: a warp has about 25 instructions per logit, 16 of them
+// the fp64 exponential.)
+template <int kPer>
 __global__ void __launch_bounds__(128)
 router_topk_kernel(uint32_t *out_ids, float *out_weights, const float *logits, uint32_t tokens,
                    uint32_t experts, uint32_t k, uint32_t *bad) {
+    constexpr int kHeld = kPer ? kPer : 1;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t token = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (token >= tokens) return;
     const float *row = logits + (size_t)token * experts;
-    float top = __uint_as_float(0xff800000u);
+    const float lowest = __uint_as_float(0xff800000u);
+    float held[kHeld];  // expert j * 32 + lane
+    float top = lowest;
     bool broken = false;
-    for (uint32_t i = lane; i < experts; i += 32) {
-        const float v = row[i];
-        broken = broken || v != v || v == __uint_as_float(0x7f800000u);
-        top = fmaxf(top, v);
+    if (kPer) {
+#pragma unroll
+        for (int j = 0; j < kHeld; j++) held[j] = j * 32u + lane < experts ? __ldg(row + j * 32u + lane) : lowest;
+#pragma unroll
+        for (int j = 0; j < kHeld; j++) {
+            broken = broken || held[j] != held[j] || held[j] == __uint_as_float(0x7f800000u);
+            top = fmaxf(top, held[j]);
+        }
+    } else {
+        for (uint32_t i = lane; i < experts; i += 32) {
+            const float v = row[i];
+            broken = broken || v != v || v == __uint_as_float(0x7f800000u);
+            top = fmaxf(top, v);
+        }
     }
     broken = __any_sync(kFullMask, broken);
 #pragma unroll
     for (int d = 16; d >= 1; d >>= 1) top = fmaxf(top, __shfl_xor_sync(kFullMask, top, d));
     double total = 0.0;
-    for (uint32_t i = lane; i < experts; i += 32) total += exp((double)row[i] - (double)top);
+    if (kPer) {
+#pragma unroll
+        for (int j = 0; j < kHeld; j++)
+            if (j * 32u + lane < experts) total += exp((double)held[j] - (double)top);
+    } else {
+        for (uint32_t i = lane; i < experts; i += 32) total += exp((double)row[i] - (double)top);
+    }
 #pragma unroll
     for (int d = 16; d >= 1; d >>= 1) total += __shfl_xor_sync(kFullMask, total, d);
     if (broken || !(total > 0.0)) {
@@ -248,31 +275,56 @@ router_topk_kernel(uint32_t *out_ids, float *out_weights, const float *logits, u
         if (lane == 0) atomicMin(bad, token);
         return;
     }
-    // k rounds of "the best that is not taken yet"; a lane remembers what it gave away
-    uint64_t floor_key = ~0ull;  // keys at or above this have been taken
-    double picked_sum = 0.0;
-    float my_weight = 0.0f;
+    // k rounds of "the best that is not taken yet"; lane i remembers the i-th (k <= 32)
     uint32_t my_id = kPaddingId;
-    for (uint32_t slot = 0; slot < k; slot++) {
-        uint64_t best = 0;
-        for (uint32_t i = lane; i < experts; i += 32) {
-            const uint64_t candidate = ((uint64_t)float_key(row[i]) << 32) | (uint64_t)(~i);
-            if (candidate < floor_key && candidate > best) best = candidate;
-        }
+    if (kPer) {
+        // the lane's best: the largest key, of equal ones the smallest id (0: none left)
+        uint32_t taken = 0;  // bit j: held[j] has been given away
+        uint32_t best = 0, where = 0;
+        auto look = [&]() {
+            best = 0;
+            where = 0;
 #pragma unroll
-        for (int d = 16; d >= 1; d >>= 1) {
-            const uint64_t other = __shfl_xor_sync(kFullMask, best, d);
-            best = other > best ? other : best;
+            for (int j = 0; j < kHeld; j++) {
+                const uint32_t key = j * 32u + lane < experts && !((taken >> j) & 1u) ? float_key(held[j]) : 0u;
+                if (key > best) {
+                    best = key;
+                    where = (uint32_t)j;
+                }
+            }
+        };
+        look();
+        for (uint32_t slot = 0; slot < k; slot++) {
+            const uint32_t key = __reduce_max_sync(kFullMask, best);
+            const uint32_t id = __reduce_min_sync(kFullMask, best == key ? where * 32u + lane : kPaddingId);
+            if (lane == slot) my_id = id;
+            if (lane == (id & 31u)) {
+                taken |= 1u << (id >> 5);
+                look();
+            }
+            __syncwarp();
         }
-        floor_key = best;
-        const uint32_t id = ~(uint32_t)best;
-        const float weight = (float)(exp((double)row[id] - (double)top) / total);
-        picked_sum += (double)weight;
-        if (lane == slot % 32u) {  // (k <= 32: one slot per lane)
-            my_id = id;
-            my_weight = weight;
+    } else {
+        uint64_t floor_key = ~0ull;  // keys at or above this have been taken
+        for (uint32_t slot = 0; slot < k; slot++) {
+            uint64_t best = 0;
+            for (uint32_t i = lane; i < experts; i += 32) {
+                const uint64_t candidate = ((uint64_t)float_key(row[i]) << 32) | (uint64_t)(~i);
+                if (candidate < floor_key && candidate > best) best = candidate;
+            }
+#pragma unroll
+            for (int d = 16; d >= 1; d >>= 1) {
+                const uint64_t other = __shfl_xor_sync(kFullMask, best, d);
+                best = other > best ? other : best;
+            }
+            floor_key = best;
+            if (lane == slot) my_id = ~(uint32_t)best;
         }
     }
+    float my_weight = 0.0f;
+    if (lane < k) my_weight = (float)(exp((double)row[my_id] - (double)top) / total);
+    double picked_sum = 0.0;
+    for (uint32_t slot = 0; slot < k; slot++) picked_sum += (double)__shfl_sync(kFullMask, my_weight, (int)slot);
     if (lane < k) {
         out_ids[(size_t)token * k + lane] = my_id;
         out_weights[(size_t)token * k + lane] = (float)((double)my_weight / picked_sum);
@@ -395,7 +447,16 @@ extern "C" int fgk_launch_topk_reduce(float *out_scores, uint32_t *out_ids, cons
 extern "C" int fgk_launch_router_topk(uint32_t *out_ids, float *out_weights, const float *logits,
                                       uint32_t tokens, uint32_t experts, uint32_t k, uint32_t *bad,
                                       void *stream) {
-    router_topk_kernel<<<(tokens + 3) / 4, 128, 0, static_cast<cudaStream_t>(stream)>>>(
-        out_ids, out_weights, logits, tokens, experts, k, bad);
+    const cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const uint32_t blocks = (tokens + 3) / 4;
+    // registers for the next multiple of 128 experts; beyond 512 the row is read again each round
+    if (experts <= 128u)
+        router_topk_kernel<4><<<blocks, 128, 0, s>>>(out_ids, out_weights, logits, tokens, experts, k, bad);
+    else if (experts <= 256u)
+        router_topk_kernel<8><<<blocks, 128, 0, s>>>(out_ids, out_weights, logits, tokens, experts, k, bad);
+    else if (experts <= 512u)
+        router_topk_kernel<16><<<blocks, 128, 0, s>>>(out_ids, out_weights, logits, tokens, experts, k, bad);
+    else
+        router_topk_kernel<0><<<blocks, 128, 0, s>>>(out_ids, out_weights, logits, tokens, experts, k, bad);
     return (int)cudaGetLastError();
 }
