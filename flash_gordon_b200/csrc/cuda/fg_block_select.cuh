@@ -190,7 +190,9 @@ struct SelectOutput {
     uint32_t *tokens;
     float *token_logits;
     uint32_t *row_status;
-    unsigned long long *first_error;
+    unsigned long long *first_error;  // [0]: min over failing rows of (row << 8 | status), [1]: 1 when a wait ran out
+    unsigned long long *next_error;   // the next call's two words, set to "none" here (may be null)
+    uint32_t *noted;                  // host word: some row failed (may be null)
     uint32_t *dbg_count;
     uint32_t *dbg_ids;
     float *dbg_scores;
@@ -198,13 +200,28 @@ struct SelectOutput {
     double *dbg_tempered;
 };
 
+// A row failed: the smallest one's number and status stay in the device's words, and the host,
+// which looks at them only then, is told.
+__device__ __forceinline__ void note_error(const SelectOutput &out, uint32_t row, uint32_t status) {
+    atomicMin(out.first_error, ((unsigned long long)row << 8) | (unsigned long long)status);
+    if (out.noted != nullptr) *reinterpret_cast<volatile uint32_t *>(out.noted) = 1u;
+}
+
+// Calls use two pairs of error words in turn: the first block of every kernel clears the pair that
+// the call after this one will use (its last user has finished: calls are ordered by their stream).
+__device__ __forceinline__ void clear_next_error(const SelectOutput &out) {
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && out.next_error != nullptr) {
+        out.next_error[0] = ~0ull;
+        out.next_error[1] = ~0ull;
+    }
+}
+
 __device__ __forceinline__ void report_row(const SelectOutput &out, uint32_t row, uint32_t status,
                                            uint32_t token, float logit) {
     out.tokens[row] = token;
     out.token_logits[row] = logit;
     out.row_status[row] = status;
-    if (status != kOk)
-        atomicMin(out.first_error, ((unsigned long long)row << 8) | (unsigned long long)status);
+    if (status != kOk) note_error(out, row, status);
 }
 
 // x[0] + x[1] + ... + x[n-1] added from the left, one rounding per addition, as the C loops

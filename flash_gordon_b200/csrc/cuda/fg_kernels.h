@@ -31,6 +31,8 @@ int fgk_malloc(void **pointer, size_t bytes);
 int fgk_free(void *pointer);
 int fgk_host_alloc(void **pointer, size_t bytes); /* pinned */
 int fgk_host_free(void *pointer);
+/* whether the stream is being captured into a graph */
+int fgk_stream_capturing(void *stream, int *capturing);
 int fgk_memset_async(void *pointer, int value, size_t bytes, void *stream);
 int fgk_copy_to_device_async(void *device, const void *host, size_t bytes, void *stream);
 int fgk_copy_to_host_async(void *host, const void *device, size_t bytes, void *stream);
@@ -41,7 +43,9 @@ typedef struct fgk_select_output {
     uint32_t *tokens;
     float *token_logits;
     uint32_t *row_status;
-    uint64_t *first_error; /* device word: min over failing rows of (row << 8 | status) */
+    uint64_t *first_error; /* two device words: min over failing rows of (row << 8 | status), cause */
+    uint64_t *next_error;  /* two device words the kernel sets to all ones, or NULL */
+    uint32_t *noted;       /* pinned host word the kernel sets to 1 when a row fails, or NULL */
     uint32_t *dbg_count;
     uint32_t *dbg_ids;
     float *dbg_scores;
@@ -228,16 +232,19 @@ int fgk_launch_topk_select(float *out_scores, uint32_t *out_ids, const float *sc
 int fgk_launch_topk_reduce(float *out_scores, uint32_t *out_ids, const float *scores, const uint32_t *ids,
                            uint32_t count, uint32_t produced, void *stream);
 /* per token the k best of `experts` logits and their gate weights; *bad (device word, armed
- * with 0xffffffff) gets the lowest token whose logits hold a NaN or +Inf */
+ * with 0xffffffff) gets the lowest token whose logits hold a NaN or +Inf, and *noted (pinned host
+ * word) a 1 */
 int fgk_launch_router_topk(uint32_t *out_ids, float *out_weights, const float *logits, uint32_t tokens,
-                           uint32_t experts, uint32_t k, uint32_t *bad, void *stream);
+                           uint32_t experts, uint32_t k, uint32_t *bad, uint32_t *noted, void *stream);
 /* The executor's tables after a step: for every row that ended FG_OK and whose penalties are
  * active, the sampled token's count goes up by one (saturating) and its seen-bit is set in
- * the row's session (src/output.c:619-628, 742, 752).  `active` holds one byte per row. */
+ * the row's session (src/output.c:619-628, 742, 752).  `active` holds one byte per row.  Tokens
+ * and statuses also go to `host_tokens` and `host_status` (pinned host memory) unless NULL. */
 int fgk_launch_session_increment(uint32_t *slot_counts, uint32_t *slot_bitmaps, uint32_t vocab,
                                  uint32_t slot_bitmap_words, const uint32_t *row_slots,
                                  const uint32_t *tokens, const uint32_t *row_status,
-                                 const unsigned char *active, uint32_t rows, void *stream);
+                                 const unsigned char *active, uint32_t rows, uint32_t *host_tokens,
+                                 uint32_t *host_status, void *stream);
 /* one session's bitmap rebuilt from its count table */
 int fgk_launch_session_bitmap(uint32_t *bitmap, const uint32_t *counts, uint32_t vocab,
                               uint32_t bitmap_words, void *stream);

@@ -2064,6 +2064,7 @@ __global__ void __launch_bounds__(kNucleusThreads, 2) nucleus_select_kernel(cons
     team.size = p.team;
     team.rank = blockIdx.x % p.team;
     const uint32_t teams = gridDim.x / p.team, team_index = blockIdx.x / p.team;
+    clear_next_error(p.out);
     if (tid < 64) sh.table[tid] = exp2((double)tid / 64.0);
     if (tid == 0) {
         ss.over_count = ss.cut_count = ss.pick_count = 0;
@@ -2303,6 +2304,8 @@ extern "C" int fgk_launch_nucleus_select(const fgk_nucleus_launch *l, void *stre
     p.out.token_logits = l->out.token_logits;
     p.out.row_status = l->out.row_status;
     p.out.first_error = reinterpret_cast<unsigned long long *>(l->out.first_error);
+    p.out.next_error = reinterpret_cast<unsigned long long *>(l->out.next_error);
+    p.out.noted = l->out.noted;
     p.out.dbg_count = l->out.dbg_count;
     p.out.dbg_ids = l->out.dbg_ids;
     p.out.dbg_scores = l->out.dbg_scores;

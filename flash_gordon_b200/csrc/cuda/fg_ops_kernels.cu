@@ -229,7 +229,7 @@ topk_reduce_kernel(float *out_scores, uint32_t *out_ids, const float *scores, co
 template <int kPer>
 __global__ void __launch_bounds__(128)
 router_topk_kernel(uint32_t *out_ids, float *out_weights, const float *logits, uint32_t tokens,
-                   uint32_t experts, uint32_t k, uint32_t *bad) {
+                   uint32_t experts, uint32_t k, uint32_t *bad, uint32_t *noted) {
     constexpr int kHeld = kPer ? kPer : 1;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t token = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -272,7 +272,10 @@ router_topk_kernel(uint32_t *out_ids, float *out_weights, const float *logits, u
             out_ids[(size_t)token * k + slot] = kPaddingId;
             out_weights[(size_t)token * k + slot] = 0.0f;
         }
-        if (lane == 0) atomicMin(bad, token);
+        if (lane == 0) {
+            atomicMin(bad, token);
+            *reinterpret_cast<volatile uint32_t *>(noted) = 1u;
+        }
         return;
     }
     // k rounds of "the best that is not taken yet"; lane i remembers the i-th (k <= 32)
@@ -337,11 +340,16 @@ router_topk_kernel(uint32_t *out_ids, float *out_weights, const float *logits, u
 __global__ void __launch_bounds__(kOpThreads)
 session_increment_kernel(uint32_t *slot_counts, uint32_t *slot_bitmaps, uint32_t vocab,
                          uint32_t slot_bitmap_words, const uint32_t *row_slots, const uint32_t *tokens,
-                         const uint32_t *row_status, const unsigned char *active, uint32_t rows) {
+                         const uint32_t *row_status, const unsigned char *active, uint32_t rows,
+                         uint32_t *host_tokens, uint32_t *host_status) {
     const uint32_t row = blockIdx.x * blockDim.x + threadIdx.x;
-    if (row >= rows || !active[row] || row_status[row] != 0u) return;
-    const uint32_t token = tokens[row];
-    if (token >= vocab) return;
+    if (row >= rows) return;
+    const uint32_t token = tokens[row], status = row_status[row];
+    if (host_tokens != nullptr) {  // (pinned host memory: the step needs no copies back)
+        host_tokens[row] = token;
+        host_status[row] = status;
+    }
+    if (!active[row] || status != 0u || token >= vocab) return;
     uint32_t *counts = slot_counts + (size_t)row_slots[row] * vocab;
     uint32_t seen = counts[token];
     while (seen != 0xffffffffu) {  // two rows of a batch may share a session
@@ -420,12 +428,13 @@ extern "C" int fgk_launch_history_add(uint32_t *counts, uint32_t vocab, const ui
 extern "C" int fgk_launch_session_increment(uint32_t *slot_counts, uint32_t *slot_bitmaps, uint32_t vocab,
                                             uint32_t slot_bitmap_words, const uint32_t *row_slots,
                                             const uint32_t *tokens, const uint32_t *row_status,
-                                            const unsigned char *active, uint32_t rows, void *stream) {
+                                            const unsigned char *active, uint32_t rows, uint32_t *host_tokens,
+                                            uint32_t *host_status, void *stream) {
     if (rows == 0) return 0;
     session_increment_kernel<<<(rows + kOpThreads - 1) / kOpThreads, kOpThreads, 0,
                                static_cast<cudaStream_t>(stream)>>>(slot_counts, slot_bitmaps, vocab,
                                                                     slot_bitmap_words, row_slots, tokens,
-                                                                    row_status, active, rows);
+                                                                    row_status, active, rows, host_tokens, host_status);
     return (int)cudaGetLastError();
 }
 
@@ -446,17 +455,17 @@ extern "C" int fgk_launch_topk_reduce(float *out_scores, uint32_t *out_ids, cons
 
 extern "C" int fgk_launch_router_topk(uint32_t *out_ids, float *out_weights, const float *logits,
                                       uint32_t tokens, uint32_t experts, uint32_t k, uint32_t *bad,
-                                      void *stream) {
+                                      uint32_t *noted, void *stream) {
     const cudaStream_t s = static_cast<cudaStream_t>(stream);
     const uint32_t blocks = (tokens + 3) / 4;
     // registers for the next multiple of 128 experts; beyond 512 the row is read again each round
     if (experts <= 128u)
-        router_topk_kernel<4><<<blocks, 128, 0, s>>>(out_ids, out_weights, logits, tokens, experts, k, bad);
+        router_topk_kernel<4><<<blocks, 128, 0, s>>>(out_ids, out_weights, logits, tokens, experts, k, bad, noted);
     else if (experts <= 256u)
-        router_topk_kernel<8><<<blocks, 128, 0, s>>>(out_ids, out_weights, logits, tokens, experts, k, bad);
+        router_topk_kernel<8><<<blocks, 128, 0, s>>>(out_ids, out_weights, logits, tokens, experts, k, bad, noted);
     else if (experts <= 512u)
-        router_topk_kernel<16><<<blocks, 128, 0, s>>>(out_ids, out_weights, logits, tokens, experts, k, bad);
+        router_topk_kernel<16><<<blocks, 128, 0, s>>>(out_ids, out_weights, logits, tokens, experts, k, bad, noted);
     else
-        router_topk_kernel<0><<<blocks, 128, 0, s>>>(out_ids, out_weights, logits, tokens, experts, k, bad);
+        router_topk_kernel<0><<<blocks, 128, 0, s>>>(out_ids, out_weights, logits, tokens, experts, k, bad, noted);
     return (int)cudaGetLastError();
 }

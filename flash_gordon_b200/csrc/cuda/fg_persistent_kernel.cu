@@ -1238,7 +1238,7 @@ __device__ __noinline__ void close_unit(Shared &sh, uint32_t closer, Lists &L, c
         }
         if (lane == 0) {
             p.out.row_status[row] = bad_history;
-            if (bad_history) atomicMin(p.out.first_error, ((unsigned long long)row << 8) | bad_history);
+            if (bad_history) note_error(p.out, row, bad_history);
         }
         return;
     }
@@ -1351,6 +1351,7 @@ __global__ void __launch_bounds__(kBlock, 1) persistent_select_kernel(const __gr
     const uint32_t tiles = (p.vocab + kTileLogits - 1) / kTileLogits;
     const uint32_t polls = p.wait_polls ? p.wait_polls : kDefaultPolls;
     const uint32_t buffers = p.bitmap_buffers;
+    clear_next_error(p.out);
 
     if (tid == 0) {
         for (int w = 0; w < kWarps; w++)
@@ -1579,6 +1580,8 @@ static persist::Params to_persist_params(const fgk_stream_launch *l) {
     p.out.token_logits = l->out.token_logits;
     p.out.row_status = l->out.row_status;
     p.out.first_error = reinterpret_cast<unsigned long long *>(l->out.first_error);
+    p.out.next_error = reinterpret_cast<unsigned long long *>(l->out.next_error);
+    p.out.noted = l->out.noted;
     p.out.dbg_count = l->out.dbg_count;
     p.out.dbg_ids = l->out.dbg_ids;
     p.out.dbg_scores = l->out.dbg_scores;

@@ -28,6 +28,13 @@ extern "C" int fgk_stream_synchronize(void *stream) {
     return (int)cudaStreamSynchronize(static_cast<cudaStream_t>(stream));
 }
 
+extern "C" int fgk_stream_capturing(void *stream, int *capturing) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    const cudaError_t e = cudaStreamIsCapturing(static_cast<cudaStream_t>(stream), &status);
+    *capturing = status != cudaStreamCaptureStatusNone;
+    return (int)e;
+}
+
 extern "C" int fgk_malloc(void **pointer, size_t bytes) { return (int)cudaMalloc(pointer, bytes); }
 
 extern "C" int fgk_free(void *pointer) { return (int)cudaFree(pointer); }

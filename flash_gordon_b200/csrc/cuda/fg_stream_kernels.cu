@@ -659,8 +659,7 @@ __device__ __noinline__ void finish_split(const StreamParams &p, StreamShared &s
         }
         if (tid == 0) {
             p.out.row_status[row] = bad_history;
-            if (bad_history)
-                atomicMin(p.out.first_error, ((unsigned long long)row << 8) | bad_history);
+            if (bad_history) note_error(p.out, row, bad_history);
         }
         return;
     }
@@ -845,6 +844,7 @@ stream_select_kernel(const __grid_constant__ StreamParams p) {
 
     const uint32_t tid = threadIdx.x;
     const uint32_t split = blockIdx.x, row = blockIdx.y;
+    clear_next_error(p.out);
     const SamplerConfig cfg = p.config_count > 1 ? p.configs[row] : p.config0;
     const bool shard_mode = p.shard_k != 0;
     // (a shard of a greedy row keeps k_shard candidates like any other, and on top of them
@@ -984,6 +984,7 @@ struct MergeParams {
 __global__ void __launch_bounds__(kThreads) merge_select_kernel(const MergeParams p) {
     __shared__ StreamShared sh;
     const uint32_t tid = threadIdx.x, row = blockIdx.x;
+    clear_next_error(p.out);
     const SamplerConfig cfg = p.config_count > 1 ? p.configs[row] : p.config0;
     const bool greedy = cfg.temperature == 0.0f;
     const uint32_t k = greedy ? 1u : cfg.top_k;
@@ -1096,6 +1097,8 @@ static SelectOutput make_output(const fgk_select_output *o) {
     out.token_logits = o->token_logits;
     out.row_status = o->row_status;
     out.first_error = reinterpret_cast<unsigned long long *>(o->first_error);
+    out.next_error = reinterpret_cast<unsigned long long *>(o->next_error);
+    out.noted = o->noted;
     out.dbg_count = o->dbg_count;
     out.dbg_ids = o->dbg_ids;
     out.dbg_scores = o->dbg_scores;

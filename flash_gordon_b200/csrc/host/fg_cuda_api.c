@@ -97,12 +97,18 @@ fg_status fg_cuda_context_create(int device, fg_cuda_context **out, fg_error *er
     if (!e) e = fgk_stream_prepare();
     if (!e) e = fgk_persistent_prepare();
     if (!e) e = fgk_nucleus_prepare(c->nucleus_teams);
-    if (!e) e = fgk_malloc((void **)&c->first_error, 256u);
+    if (!e) e = fgk_malloc((void **)&c->errors, 256u);
+    if (!e) e = fgk_memset_async(c->errors, 0xff, 256u, c->own_stream);
+    if (!e) e = fgk_stream_synchronize(c->own_stream);
+    if (!e) e = fgk_host_alloc((void **)&c->noted, 64u);
     if (e) {
         fg_status status = fg_cuda_fail(err, e, "opening the CUDA context");
         fg_cuda_context_destroy(c);
         return status;
     }
+    c->noted[0] = c->noted[1] = 0u;
+    c->first_error = c->errors;
+    c->next_clean = true;
     c->stream = c->own_stream;
     c->sm_count = (uint32_t)sms;
     *out = c;
@@ -118,7 +124,8 @@ void fg_cuda_context_destroy(fg_cuda_context *c) {
         if (c->configs) fgk_free(c->configs);
         if (c->history) fgk_free(c->history);
         if (c->nucleus) fgk_free(c->nucleus);
-        if (c->first_error) fgk_free(c->first_error);
+        if (c->errors) fgk_free(c->errors);
+        if (c->noted) fgk_host_free((void *)c->noted);
         if (c->staging) fgk_free(c->staging);
         if (c->pinned) fgk_host_free(c->pinned);
         if (c->own_stream) fgk_stream_destroy(c->own_stream);
@@ -438,14 +445,18 @@ fg_status fg_cuda_router_topk(fg_cuda_context *c, fg_cuda_tensor *selected, fg_c
     }
     fg_status status = fg_cuda_enter(c, err);
     if (status != FG_OK) return status;
-    uint32_t *bad = (uint32_t *)c->first_error + 8; /* a word of the context's 256-byte block */
-    int e = fgk_memset_async(bad, 0xff, 4u, c->stream);
-    if (!e) e = fgk_launch_router_topk((uint32_t *)selected->base, (float *)gates->base,
-                                       (const float *)logits->base, tokens, experts, k, bad, c->stream);
+    uint32_t *bad = (uint32_t *)(c->errors + FG_ERROR_ROUTER); /* "none" between calls */
+    int e = fgk_launch_router_topk((uint32_t *)selected->base, (float *)gates->base, (const float *)logits->base,
+                                   tokens, experts, k, bad, (uint32_t *)&c->noted[1], c->stream);
     c->launches++;
-    uint32_t first_bad = UINT32_MAX;
-    if (!e) e = fgk_copy_to_host_async(&first_bad, bad, 4u, c->stream);
     if (!e) e = fgk_stream_synchronize(c->stream);
+    uint32_t first_bad = UINT32_MAX;
+    if (!e && c->noted[1] != 0u) { /* the word is fetched, and armed again, only then */
+        c->noted[1] = 0u;
+        e = fgk_copy_to_host_async(&first_bad, bad, 4u, c->stream);
+        if (!e) e = fgk_memset_async(bad, 0xff, 4u, c->stream);
+        if (!e) e = fgk_stream_synchronize(c->stream);
+    }
     if (e) return fg_cuda_fail(err, e, "router kernel");
     if (first_bad != UINT32_MAX) {  /* src/q38_math.c:61 */
         fg_error_set(err, FG_ERR_FORMAT, "router probabilities are not finite (token %u)", first_bad);
@@ -612,6 +623,8 @@ static void fill_output(fgk_select_output *out, const fg_cuda_context *c,
     out->token_logits = a->token_logits;
     out->row_status = a->row_status;
     out->first_error = c->first_error;
+    out->next_error = c->next_error;
+    out->noted = (uint32_t *)c->noted;
     if (a->debug) {
         out->dbg_count = a->debug->candidate_count;
         out->dbg_ids = a->debug->candidate_ids;
@@ -639,9 +652,12 @@ static fg_status upload_configs(fg_cuda_context *c, const fg_cuda_sample_args *a
  * after it says why a row ended with FG_ERR_LIMIT when it was not the history's length. */
 static fg_status collect_status(fg_cuda_context *c, fg_error *err) {
     uint64_t words[2] = {UINT64_MAX, UINT64_MAX};
-    int e = fgk_copy_to_host_async(words, c->first_error, 16u, c->stream);
+    int e = fgk_stream_synchronize(c->stream);
+    if (!e && c->noted[0] == 0u) return FG_OK; /* no row of any call since the last look */
+    if (!e) e = fgk_copy_to_host_async(words, c->first_error, 16u, c->stream);
     if (!e) e = fgk_stream_synchronize(c->stream);
     if (e) return fg_cuda_fail(err, e, "sampling kernels");
+    c->noted[0] = 0u;
     if (words[0] == UINT64_MAX) return FG_OK;
     const fg_status status = (fg_status)(words[0] & 0xffu);
     const uint64_t row = words[0] >> 8;
@@ -653,6 +669,33 @@ static fg_status collect_status(fg_cuda_context *c, fg_error *err) {
     else if (status == FG_ERR_ARGUMENT) why = "a penalty that can raise a logit reached the kernel for lowering penalties";
     fg_error_set(err, status, "row %llu: %s", (unsigned long long)row, why);
     return status;
+}
+
+/* Picks the call's pair of error words.  As a rule the previous call's kernel has cleared it; a
+ * memset does it when that call failed before its launch.  A captured call has a pair of its own and clears
+ * it in the graph, since it may be replayed any number of times between other calls. */
+static fg_status arm_first_error(fg_cuda_context *c, fg_error *err) {
+    int capturing = 0, e = fgk_stream_capturing(c->stream, &capturing);
+    if (!e && capturing) {
+        c->first_error = c->errors + FG_ERROR_CAPTURED;
+        c->next_error = NULL;
+        e = fgk_memset_async(c->first_error, 0xff, 16u, c->stream);
+    } else if (!e) {
+        uint64_t *pair = c->errors + FG_ERROR_PAIRS + (c->error_turn ? 0u : 2u);
+        if (!c->next_clean) e = fgk_memset_async(pair, 0xff, 16u, c->stream);
+        c->error_turn = !c->error_turn;
+        c->first_error = pair;
+        c->next_error = c->errors + FG_ERROR_PAIRS + (c->error_turn ? 0u : 2u);
+        c->next_clean = false;
+    }
+    return e ? fg_cuda_fail(err, e, "arming the error word") : FG_OK;
+}
+
+/* A sampling kernel has been launched: it clears the next call's words. */
+static int launched(fg_cuda_context *c, int e) {
+    c->launches++;
+    if (!e && c->next_error) c->next_clean = true;
+    return e;
 }
 
 static fg_status run_stream(fg_cuda_context *c, const fg_cuda_sample_args *a,
@@ -780,8 +823,7 @@ static fg_status run_stream(fg_cuda_context *c, const fg_cuda_sample_args *a,
         l.withhold_issue = c->ring_withhold_issue;
         c->last_scratch_bytes = part_slots * (64u * 8u + 16u) + (size_t)a->rows * 4u +
                                 (a->config_count > 1u ? (size_t)a->rows * sizeof(fg_sampler_config) : 0u);
-        const int e = fgk_launch_persistent_select(&l, ctas, c->stream);
-        c->launches++;
+        const int e = launched(c, fgk_launch_persistent_select(&l, ctas, c->stream));
         return e ? fg_cuda_fail(err, e, "persistent ring kernel") : FG_OK;
     }
     /* the streaming kernel's hand-off between the splits of a row, reserved only when it runs */
@@ -793,8 +835,7 @@ static fg_status run_stream(fg_cuda_context *c, const fg_cuda_sample_args *a,
         l.part_ids = (uint32_t *)(base + slots * 64u * 4u);
         l.part_meta = base + slots * 64u * 8u;
     }
-    const int e = fgk_launch_stream_select(&l, c->stream);
-    c->launches++;
+    const int e = launched(c, fgk_launch_stream_select(&l, c->stream));
     return e ? fg_cuda_fail(err, e, "streaming select kernel") : FG_OK;
 }
 
@@ -907,14 +948,8 @@ static fg_status run_nucleus(fg_cuda_context *c, const fg_cuda_sample_args *a,
         n.history_meta = h.history_meta;
         c->last_scratch_bytes += history_bytes;
     }
-    const int e = fgk_launch_nucleus_select(&n, c->stream);
-    c->launches++;
+    const int e = launched(c, fgk_launch_nucleus_select(&n, c->stream));
     return e ? fg_cuda_fail(err, e, "nucleus kernel") : FG_OK;
-}
-
-static fg_status arm_first_error(fg_cuda_context *c, fg_error *err) {
-    const int e = fgk_memset_async(c->first_error, 0xff, 16u, c->stream); /* the error word and its cause */
-    return e ? fg_cuda_fail(err, e, "arming the error word") : FG_OK;
 }
 
 fg_status fg_cuda_sample_batch(fg_cuda_context *c, const fg_cuda_sample_args *a, fg_error *err) {
@@ -1023,8 +1058,7 @@ fg_status fg_cuda_merge_select_layout(fg_cuda_context *c, const fg_cuda_sample_a
     l.config_count = a->config_count;
     l.uniforms = a->uniforms;
     fill_output(&l.out, c, a);
-    const int e = fgk_launch_merge_select(&l, c->stream);
-    c->launches++;
+    const int e = launched(c, fgk_launch_merge_select(&l, c->stream));
     return e ? fg_cuda_fail(err, e, "merge kernel") : FG_OK;
 }
 

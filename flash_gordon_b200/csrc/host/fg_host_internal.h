@@ -41,13 +41,24 @@ struct fg_cuda_context {
     uint32_t nucleus_teams[FGK_NUCLEUS_TEAM_SIZES]; /* how many teams of 1, 2, 4, 8 CTAs run at a time */
     void *configs;          /* per-row configs when they differ */
     size_t configs_bytes;
-    uint64_t *first_error;  /* one device word */
+    /* The sampling calls' error words.  `errors` is a device block of 256 bytes: three pairs of 64-bit
+     * words (calls use the first two in turn, captured calls the third), the router's 32-bit word
+     * and a pair nobody reads.  `first_error` is the pair of the call under way, `next_error` the one its kernels
+     * clear for the next call (NULL while capturing); `next_clean` says that a kernel that
+     * does so has been launched.  `noted` are pinned host words the kernels set when
+     * something failed: [0] sampling, [1] router. */
+    uint64_t *errors, *first_error, *next_error;
+    bool next_clean, error_turn;
+    volatile uint32_t *noted;
     void *staging;          /* host-entry inputs and outputs */
     size_t staging_bytes;
     void *pinned;           /* pinned host bounce buffer */
     size_t pinned_bytes;
     uint64_t last_scratch_bytes;
 };
+
+/* parts of the context's error block, in 64-bit words */
+enum { FG_ERROR_PAIRS = 0, FG_ERROR_CAPTURED = 8, FG_ERROR_ROUTER = 16, FG_ERROR_UNREAD = 24 };
 
 struct fg_cuda_tensor {
     fg_cuda_context *context;

@@ -192,8 +192,8 @@ fg_status fg_cuda_output_sample_sessions(fg_cuda_output_executor *x, const fg_cu
         host_sessions[r] = slots[r];
         host_active[r] = fg_sampler_penalties_active(&args->configs[args->config_count == 1u ? 0u : r]) ? 1u : 0u;
     }
-    int e = fgk_copy_to_device_async(device_sessions, host_sessions, (size_t)rows * 4u, c->stream);
-    if (!e) e = fgk_copy_to_device_async(device_active, host_active, rows, c->stream);
+    /* (the activity bytes follow the session indices on both sides) */
+    int e = fgk_copy_to_device_async(device_sessions, host_sessions, (size_t)rows * 5u, c->stream);
     if (e) return fg_cuda_fail(err, e, "staging the session indices");
 
     fg_cuda_sample_args call = *args;
@@ -243,17 +243,16 @@ fg_status fg_cuda_output_sample_sessions(fg_cuda_output_executor *x, const fg_cu
         *err = quiet;
     }
     if (status != FG_OK) return status;
+    /* tokens and statuses back, for the host's copy of the histories: the increment kernel
+     * stores them into the pinned staging (without an active row nobody asks for them) */
+    uint32_t *host_tokens = x->host_rows + 2u * rows, *host_status = x->host_rows + 3u * rows;
     if (any_active) {
         e = fgk_launch_session_increment(x->counts, x->bitmaps, x->vocab, x->bitmap_words, device_sessions,
-                                         args->tokens, args->row_status, device_active, rows, c->stream);
+                                         args->tokens, args->row_status, device_active, rows, host_tokens,
+                                         host_status, c->stream);
         c->launches++;
         if (e) return fg_cuda_fail(err, e, "session increment kernel");
     }
-    /* tokens and statuses back, for the host's copy of the histories */
-    uint32_t *host_tokens = x->host_rows + 2u * rows, *host_status = x->host_rows + 3u * rows;
-    e = fgk_copy_to_host_async(host_tokens, args->tokens, (size_t)rows * 4u, c->stream);
-    if (!e) e = fgk_copy_to_host_async(host_status, args->row_status, (size_t)rows * 4u, c->stream);
-    if (e) return fg_cuda_fail(err, e, "reading the step's tokens");
     status = fg_cuda_collect(c, err); /* waits for the stream */
     for (uint32_t r = 0; r < rows; r++) {
         if (!host_active[r] || host_status[r] != (uint32_t)FG_OK) continue;
@@ -282,7 +281,7 @@ fg_status fg_cuda_output_history_increment(fg_cuda_output_executor *x, uint32_t 
     uint32_t *device = x->device_rows;
     int e = fgk_copy_to_device_async(device, host, 16u, c->stream);
     if (!e) e = fgk_launch_session_increment(x->counts, x->bitmaps, x->vocab, x->bitmap_words, device, device + 2,
-                                             device + 3, (const unsigned char *)(device + 1), 1u, c->stream);
+                                             device + 3, (const unsigned char *)(device + 1), 1u, NULL, NULL, c->stream);
     c->launches++;
     if (!e) e = fgk_stream_synchronize(c->stream);
     if (e) return fg_cuda_fail(err, e, "session increment kernel");

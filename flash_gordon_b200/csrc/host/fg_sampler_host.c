@@ -158,38 +158,32 @@ fg_status fg_sampler_select(const fg_sampler_config *config, const float *scores
     fg_cuda_default_lock();
     fg_cuda_context *ctx = NULL;
     fg_status status = fg_cuda_default_context(&ctx, err);
-    /* device staging: scores[64] ids[64] uniform token logit status first_error */
+    /* pinned host memory, which the kernel reads and writes in place: no copies for half a KB.
+     * scores[64] ids[64] uniform token logit status */
     enum { SCORES = 0, IDS = 256, UNIFORM = 512, TOKEN = 528, LOGIT = 532, STATUS = 536, TOTAL = 544 };
-    if (status == FG_OK) status = fg_cuda_reserve(&ctx->staging, &ctx->staging_bytes, TOTAL, false, ctx, err);
     if (status == FG_OK) status = fg_cuda_reserve_pinned(ctx, TOTAL, err);
     if (status == FG_OK) {
-        unsigned char *pinned = ctx->pinned, *device = ctx->staging;
+        unsigned char *pinned = ctx->pinned;
         memcpy(pinned + SCORES, scores, (size_t)count * 4u);
         memcpy(pinned + IDS, ids, (size_t)count * 4u);
         memcpy(pinned + UNIFORM, &uniform, 4u);
-        const uint64_t none = UINT64_MAX;
         fgk_merge_launch launch;
         memset(&launch, 0, sizeof(launch));
-        launch.scores = (const float *)(device + SCORES);
-        launch.ids = (const uint32_t *)(device + IDS);
+        launch.scores = (const float *)(pinned + SCORES);
+        launch.ids = (const uint32_t *)(pinned + IDS);
         launch.rows = 1u;
         launch.shards = 1u;
         launch.k_shard = count;
         launch.check_spans = 0u;
         launch.config0 = *config;
         launch.config_count = 1u;
-        launch.uniforms = (const float *)(device + UNIFORM);
-        launch.out.tokens = (uint32_t *)(device + TOKEN);
-        launch.out.token_logits = (float *)(device + LOGIT);
-        launch.out.row_status = (uint32_t *)(device + STATUS);
-        launch.out.first_error = ctx->first_error;
-        int e = fgk_copy_to_device_async(device, pinned, UNIFORM + 4u, ctx->stream);
-        if (!e) e = fgk_copy_to_device_async(ctx->first_error, &none, 8u, ctx->stream);
-        if (!e) {
-            e = fgk_launch_merge_select(&launch, ctx->stream);
-            ctx->launches++;
-        }
-        if (!e) e = fgk_copy_to_host_async(pinned + TOKEN, device + TOKEN, 12u, ctx->stream);
+        launch.uniforms = (const float *)(pinned + UNIFORM);
+        launch.out.tokens = (uint32_t *)(pinned + TOKEN);
+        launch.out.token_logits = (float *)(pinned + LOGIT);
+        launch.out.row_status = (uint32_t *)(pinned + STATUS);
+        launch.out.first_error = ctx->errors + FG_ERROR_UNREAD; /* the row's status says it all */
+        int e = fgk_launch_merge_select(&launch, ctx->stream);
+        ctx->launches++;
         if (!e) e = fgk_stream_synchronize(ctx->stream);
         if (e) {
             status = fg_cuda_fail(err, e, "select kernel");
