@@ -234,6 +234,12 @@ __device__ __forceinline__ bool penalties_active(const SamplerConfig &c) {
            c.repetition_penalty != 1.0f;
 }
 
+// Penalties that can raise a logit (or push one to infinity); the others are monotone and lower it.
+__device__ __forceinline__ bool can_raise(const SamplerConfig &c) {
+    return penalties_active(c) && !(c.presence_penalty >= 0.0f && c.frequency_penalty >= 0.0f &&
+                                    c.repetition_penalty >= 1.0f && c.repetition_penalty <= 0x1p40f);
+}
+
 // Picture of the part of a row's history that falls into one column range, in shared
 // or global memory:
 //   bitmap   bit c set = column c occurs in the history            u32[bitmap_words]

@@ -77,6 +77,9 @@ typedef struct fgk_stream_launch {
     uint64_t row_stride;
     uint32_t vocab_offset, vocab_total;
     uint32_t splits, split_len;
+    uint32_t only_raising; /* streaming kernel: take only rows whose penalties can raise a logit */
+    uint32_t general;      /* ring kernel: rows need not begin or end on 16-byte boundaries, and ... */
+    uint32_t skip_raising; /* ... those rows may be left out */
     const uint32_t *history_tokens;
     const uint64_t *history_offsets;
     uint32_t history_max;

@@ -37,9 +37,17 @@
 // vocabulary-wide table per session): the entry keeps its raw logit, is ordered by the
 // charge for count = 1 -- an upper bound of its value -- and its occurrences are counted
 // in the token list only if that upper bound reaches the bound the row ends with.
-// Everything else (penalties that can raise a logit, rows that are not 16-byte aligned,
-// column splits) stays with stream_select_kernel.
+// Rows whose penalties can raise a logit, and column splits, stay with stream_select_kernel.
+//
+// The kernel has a second form (kGeneral) for batches with rows that do not begin or end on a
+// 16-byte boundary, or some of whose rows stay with the other kernel: tiles are counted from the
+// boundary before the row, the copy engine fetches the whole 16-byte granules inside the row, and
+// the warp that gets the first or the last tile writes the partial granule into its stage with
+// plain loads, -inf where the row is not.  (Such rows went element by element through the streaming
+// kernel before.  64 rows of 100,277 bf16 logits, histories of 512: 69 us there, 25 here; 512
+// rows 241 and 62; one row 42 and 25.)
 #include <cstring>
+#include <type_traits>
 
 #include "fg_block_select.cuh"
 #include "fg_kernels.h"
@@ -140,6 +148,7 @@ struct Params {
     const uint32_t *slot_bitmaps;   // [slots][slot_bitmap_words], a whole number of uint4 each
     const uint32_t *row_slots;      // [rows]
     uint32_t slot_bitmap_words;
+    uint32_t skip_raising;          // rows whose penalties can raise a logit are another kernel's
     uint32_t wait_polls;            // polls before a wait gives up
     uint32_t withhold_cta, withhold_issue;  // test seam: that CTA's warp 0 never asks for that tile
     SelectOutput out;
@@ -674,10 +683,18 @@ __device__ __noinline__ void raise_bound(Lists &L, const Tally tally, uint32_t k
 // one candidate) or is counted in the tally.  A list that is full is cut to its k best, which
 // lifts the bound too, and the lanes go on where they stopped.  All lanes call; returns the bound
 // the warp knows afterwards.
-template <typename T, bool kGreedy>
+// `columns` tells positions of a ragged row's tile that are not the row's.
+struct AnyColumn {  // rows that fill their vectors
+    __device__ __forceinline__ bool holds(uint32_t) const { return true; }
+};
+struct ColumnsBelow {
+    uint32_t count;
+    __device__ __forceinline__ bool holds(uint32_t column) const { return column < count; }
+};
+template <typename T, bool kGreedy, class Columns>
 __device__ __noinline__ uint64_t collect(Lists &L, const Row r, const uint32_t *bitmap, const unsigned char *tile,
                                          uint32_t column0, uint32_t valid_vectors, uint32_t w, uint32_t hot,
-                                         uint64_t bound, const Tally tally) {
+                                         uint64_t bound, const Tally tally, const Columns columns) {
     using V = Lanes<T>;
     constexpr int kPer = V::kPer;
     const uint32_t lane = lane_id();
@@ -705,6 +722,10 @@ __device__ __noinline__ uint64_t collect(Lists &L, const Row r, const uint32_t *
             const uint32_t position = ((e / kPer) * 32 + lane) * kPer + (e % kPer);
             const float x = tile_element<T>(tile, position);
             const uint32_t column = column0 + position;
+            if (!columns.holds(column)) {  // before the row's first logit or after its last
+                take &= take - 1;
+                continue;
+            }
             const uint32_t id = r.id_base + column;
             const bool wild = kGreedy && (__float_as_uint(x) & 0x7fffffffu) >= kHugeBits;
             const bool seen = r.seen_any && ((bitmap[column >> 5] >> (column & 31u)) & 1u);
@@ -789,58 +810,110 @@ __device__ __forceinline__ Row make_row(const Params &p, const SamplerConfig &cf
     return r;
 }
 
-// Does this kernel sample the row, or is it left to the kernel without a top-k cut?
-__device__ __forceinline__ bool row_is_ours(const SamplerConfig &cfg, bool shard_mode) {
-    return shard_mode || cfg.temperature == 0.0f || cfg.top_k != 0;
+// Does this kernel sample the row, or is it left to one of the others?
+template <bool kGeneral>
+__device__ __forceinline__ bool row_is_ours(const Params &p, const SamplerConfig &cfg, bool shard_mode) {
+    return (shard_mode || cfg.temperature == 0.0f || cfg.top_k != 0) &&
+           !(kGeneral && p.skip_raising && can_raise(cfg));
 }
 
 __device__ __forceinline__ SamplerConfig row_config(const Params &p, uint32_t row) {
     return p.config_count > 1 ? p.configs[row] : p.config0;
 }
 
+// How a row lies to the 16-byte boundaries its tiles are counted from.
+template <typename T, bool kGeneral>
+struct Lie {
+    const unsigned char *base;  // the boundary at or before the row's first logit
+    uint32_t off;               // logits between the two
+    uint32_t granule_end;       // whole granules end here (those of the row begin at 1 if off != 0)
+    uint32_t vectors;           // granules that hold some logit of the row end here
+    __device__ __forceinline__ Lie(const Params &p, uint32_t row) {
+        base = static_cast<const unsigned char *>(p.logits) + (size_t)row * p.row_stride * sizeof(T);
+        off = kGeneral ? (uint32_t)(reinterpret_cast<uintptr_t>(base) & 15u) / (uint32_t)sizeof(T) : 0u;
+        base -= off * sizeof(T);
+        granule_end = (off + p.vocab) / (uint32_t)Lanes<T>::kPer;
+        vectors = (off + p.vocab + (uint32_t)Lanes<T>::kPer - 1u) / (uint32_t)Lanes<T>::kPer;
+    }
+    // vectors of tile t that hold some logit of the row
+    __device__ __forceinline__ uint32_t valid(uint32_t t) const {
+        const uint32_t whole = tile_bytes<T>() / 16u;
+        return t * whole >= vectors ? 0u : min(whole, vectors - t * whole);
+    }
+    // The row's partial granules in tile t, written into the stage: -inf where the row is not.
+    __device__ __forceinline__ void patch(const Params &p, unsigned char *stage, uint32_t t) const {
+        if (!kGeneral) return;
+        const uint32_t whole = tile_bytes<T>() / 16u, lane = lane_id();
+        const bool head = off != 0 && t == 0, tail = vectors != granule_end && granule_end / whole == t;
+        if (!head && !tail) return;
+        constexpr uint32_t kPer = (uint32_t)Lanes<T>::kPer;
+        const uint32_t granule = head && lane < kPer ? 0u : granule_end;
+        if (lane < kPer ? head : (tail && lane < 2u * kPer)) {
+            const uint32_t at = granule * kPer + lane % kPer;  // counted from `base`
+            T value = sizeof(T) == 2 ? (T)0xff80u : (T)__uint_as_float(0xff800000u);
+            if (at >= off && at - off < p.vocab) value = __ldg(reinterpret_cast<const T *>(base) + at);
+            reinterpret_cast<T *>(stage)[at - t * whole * kPer] = value;
+        }
+        // (the copy engine writes here again later)
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+    }
+};
+
 // Walks the tiles one consumer warp asks the copy engine for -- every kWarps-th tile of
 // each of the CTA's units, unit after unit -- kStages ahead of the tile the warp looks at.
 struct Feeder {
     UnitWalk walk;
     Unit u;
-    const unsigned char *row;  // first byte of the unit's row
+    const unsigned char *row;  // where the unit's row is counted from
+    uint32_t granule_begin, granule_end;  // ragged rows: the whole granules of the row
     uint32_t t;
     uint32_t issued;
     bool live;
     __device__ __forceinline__ Feeder(const Params &p, uint32_t row_tiles) : walk(p, row_tiles), issued(0) {}
-    template <typename T>
+    template <typename T, bool kGeneral>
     __device__ __forceinline__ bool seek(const Params &p, uint32_t w, bool shard_mode) {
         while (walk.next(u)) {
-            if (!row_is_ours(row_config(p, u.row), shard_mode)) continue;
+            if (!row_is_ours<kGeneral>(p, row_config(p, u.row), shard_mode)) continue;
             t = u.first + w;
-            row = static_cast<const unsigned char *>(p.logits) + (size_t)u.row * p.row_stride * sizeof(T);
+            const Lie<T, kGeneral> lie(p, u.row);
+            row = lie.base;
+            granule_begin = lie.off != 0 ? 1u : 0u;
+            granule_end = lie.granule_end;
             if (t < u.end) return true;
         }
         return false;
     }
     // asks for the warp's next tile into `stage`; all lanes call, lane 0 talks to the engine
-    template <typename T>
+    template <typename T, bool kGeneral>
     __device__ __forceinline__ void issue(const Params &p, unsigned char *stage, uint64_t *full,
                                           uint32_t row_bytes, uint32_t w, bool shard_mode, uint64_t policy) {
         if (!live) return;
         if (lane_id() == 0) {
-            const uint32_t bytes = min(tile_bytes<T>(), row_bytes - t * tile_bytes<T>());
             const bool withheld = w == 0 && blockIdx.x == p.withhold_cta && issued == p.withhold_issue;
-            if (!withheld) {
+            if (kGeneral && !withheld) {
+                const uint32_t whole = tile_bytes<T>() / 16u;
+                const uint32_t from = max(t * whole, granule_begin), to = min((t + 1u) * whole, granule_end);
+                const uint32_t bytes = to > from ? (to - from) * 16u : 0u;  // (0: the tile's barrier completes at once)
+                mbarrier_expect(full, bytes);
+                if (bytes != 0)
+                    bulk_copy_to_shared_hinted(stage + (from - t * whole) * 16u, row + (size_t)from * 16u, bytes, full, policy);
+            } else if (!withheld) {
+                const uint32_t bytes = min(tile_bytes<T>(), row_bytes - t * tile_bytes<T>());
                 mbarrier_expect(full, bytes);
                 bulk_copy_to_shared_hinted(stage, row + (size_t)t * tile_bytes<T>(), bytes, full, policy);
             }
         }
         issued++;
         t += kWarps;
-        if (t >= u.end) live = seek<T>(p, w, shard_mode);
+        if (t >= u.end) live = seek<T, kGeneral>(p, w, shard_mode);
     }
 };
 
 // One consumer warp's share of one unit: its tiles against the bound, candidates onto its
 // list.  Per tile and lane: the 128-bit vectors of the tile, a maximum of each against the
 // bound's score.  Returns the number of tiles it has looked at.
-template <typename T, bool kGreedy>
+template <typename T, bool kGreedy, bool kGeneral>
 __device__ __forceinline__ uint32_t consume_unit(const Params &p, Shared &sh, Lists &L, const Row r, const Unit u,
                                               const uint32_t *bitmap, unsigned char *stages, Feeder &feeder,
                                               uint32_t consumed, uint32_t w, uint32_t tiles, uint32_t row_bytes,
@@ -853,6 +926,9 @@ __device__ __forceinline__ uint32_t consume_unit(const Params &p, Shared &sh, Li
     const uint32_t whole = tile_bytes<T>() / 16u;
     const uint32_t last_vectors = (row_bytes - (tiles - 1) * tile_bytes<T>()) / 16u;
     const uint32_t participants = min((uint32_t)kWarps, u.end - u.first);
+    const Lie<T, kGeneral> lie(p, u.row);
+    std::conditional_t<kGeneral, ColumnsBelow, AnyColumn> columns;
+    if constexpr (kGeneral) columns.count = p.vocab;
     uint64_t bound = 0;
     Tally tally;
     tally.base = 0;
@@ -863,8 +939,9 @@ __device__ __forceinline__ uint32_t consume_unit(const Params &p, Shared &sh, Li
         const uint32_t stage = consumed % kStages;
         tile_wait(sh, &sh.full[w][stage], (consumed / kStages) & 1u, polls);
         const unsigned char *tile = stages + (size_t)stage * kStageBytes;
-        const uint32_t valid_vectors = t + 1 == tiles ? last_vectors : whole;
-        const uint32_t column0 = t * kTileLogits;
+        if (kGeneral) lie.patch(p, stages + (size_t)stage * kStageBytes, t);
+        const uint32_t valid_vectors = kGeneral ? lie.valid(t) : (t + 1 == tiles ? last_vectors : whole);
+        const uint32_t column0 = t * kTileLogits - lie.off;  // (below 0 before a ragged row's first logit)
         if (done == 0) {
             const FirstBound first =
                 first_bound<T>(sh, L, r, bitmap, tile, column0, valid_vectors, participants, polls);
@@ -898,7 +975,7 @@ __device__ __forceinline__ uint32_t consume_unit(const Params &p, Shared &sh, Li
                 if ((uint32_t)(v8 * 32) + lane >= valid_vectors) hot &= ~(1u << v8);
         }
         if (__any_sync(kFullMask, hot != 0))
-            bound = collect<T, kGreedy>(L, r, bitmap, tile, column0, valid_vectors, w, hot, bound, tally);
+            bound = collect<T, kGreedy>(L, r, bitmap, tile, column0, valid_vectors, w, hot, bound, tally, columns);
         // The bound tightens as the row is read: the warps take turns, one after every round of
         // tiles, to see what the tally of all the warps' exact entries allows.  Nobody waits.
         if (r.k > 1u && done == turn) {
@@ -908,8 +985,8 @@ __device__ __forceinline__ uint32_t consume_unit(const Params &p, Shared &sh, Li
         done++;
         __syncwarp();
         consumed++;
-        feeder.template issue<T>(p, stages + (size_t)stage * kStageBytes, &sh.full[w][stage], row_bytes, w,
-                                 shard_mode, policy);
+        feeder.template issue<T, kGeneral>(p, stages + (size_t)stage * kStageBytes, &sh.full[w][stage], row_bytes, w,
+                                          shard_mode, policy);
     }
     return consumed;
 }
@@ -1336,7 +1413,7 @@ struct EverybodyMeets {
     }
 };
 
-template <typename T>
+template <typename T, bool kGeneral>
 __global__ void __launch_bounds__(kBlock, 1) persistent_select_kernel(const __grid_constant__ Params p) {
     extern __shared__ __align__(128) unsigned char dynamic[];
     __shared__ Shared sh;
@@ -1348,7 +1425,8 @@ __global__ void __launch_bounds__(kBlock, 1) persistent_select_kernel(const __gr
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const bool shard_mode = p.shard_k != 0;
     const uint32_t row_bytes = p.vocab * (uint32_t)sizeof(T);
-    const uint32_t tiles = (p.vocab + kTileLogits - 1) / kTileLogits;
+    // (a ragged row may reach one granule further; a tile without a logit of the row is empty)
+    const uint32_t tiles = (p.vocab + (kGeneral ? Lanes<T>::kPer - 1 : 0) + kTileLogits - 1) / kTileLogits;
     const uint32_t polls = p.wait_polls ? p.wait_polls : kDefaultPolls;
     const uint32_t buffers = p.bitmap_buffers;
     clear_next_error(p.out);
@@ -1385,7 +1463,7 @@ __global__ void __launch_bounds__(kBlock, 1) persistent_select_kernel(const __gr
         Unit u;
         while (walk.next(u)) {
             const SamplerConfig cfg = row_config(p, u.row);
-            if (!row_is_ours(cfg, shard_mode)) continue;
+            if (!row_is_ours<kGeneral>(p, cfg, shard_mode)) continue;
             if ((served & 1u) != closer) {
                 served++;
                 continue;
@@ -1428,7 +1506,7 @@ __global__ void __launch_bounds__(kBlock, 1) persistent_select_kernel(const __gr
         Unit u;
         while (walk.next(u)) {
             const SamplerConfig cfg = row_config(p, u.row);
-            if (!row_is_ours(cfg, shard_mode)) continue;
+            if (!row_is_ours<kGeneral>(p, cfg, shard_mode)) continue;
             uint32_t row_status;
             const Row r = make_row(p, cfg, u.row, shard_mode, &row_status);
             const uint32_t slot = served % buffers;
@@ -1460,17 +1538,18 @@ __global__ void __launch_bounds__(kBlock, 1) persistent_select_kernel(const __gr
     const uint64_t policy = l2_policy_evict_first();
     unsigned char *stages = ring + (size_t)w * kStages * kStageBytes;
     Feeder feeder(p, tiles);
-    feeder.live = feeder.template seek<T>(p, w, shard_mode);
+    feeder.live = feeder.template seek<T, kGeneral>(p, w, shard_mode);
 #pragma unroll
     for (int s = 0; s < kStages; s++)
-        feeder.template issue<T>(p, stages + (size_t)s * kStageBytes, &sh.full[w][s], row_bytes, w, shard_mode, policy);
+        feeder.template issue<T, kGeneral>(p, stages + (size_t)s * kStageBytes, &sh.full[w][s], row_bytes, w, shard_mode,
+                                          policy);
     {
         // The CTA's first unit: nothing has landed yet, so the consumer warps help the history
         // warps with its bitmap (every warp comes to the same decision from the same inputs).
         UnitWalk ahead(p, tiles);
         Unit u0;
         bool found = false;
-        while (!found && ahead.next(u0)) found = row_is_ours(row_config(p, u0.row), shard_mode);
+        while (!found && ahead.next(u0)) found = row_is_ours<kGeneral>(p, row_config(p, u0.row), shard_mode);
         if (found) {
             uint32_t ignored;
             const Row r0 = make_row(p, row_config(p, u0.row), u0.row, shard_mode, &ignored);
@@ -1486,7 +1565,7 @@ __global__ void __launch_bounds__(kBlock, 1) persistent_select_kernel(const __gr
     Unit u;
     while (walk.next(u)) {
         const SamplerConfig cfg = row_config(p, u.row);
-        if (!row_is_ours(cfg, shard_mode)) continue;
+        if (!row_is_ours<kGeneral>(p, cfg, shard_mode)) continue;
         uint32_t row_status;
         const Row r = make_row(p, cfg, u.row, shard_mode, &row_status);
         const uint32_t b = served % kListSets;
@@ -1503,9 +1582,9 @@ __global__ void __launch_bounds__(kBlock, 1) persistent_select_kernel(const __gr
         bounded_wait(sh, &sh.bitmap_ready[slot], (served / buffers) & 1u, polls);
         if (w == 0 && lane == 0) L.bad_history = sh.history_bad[slot];
         __syncwarp();
-        consumed = r.greedy ? consume_unit<T, true>(p, sh, L, r, u, bitmap, stages, feeder, consumed, w, tiles,
+        consumed = r.greedy ? consume_unit<T, true, kGeneral>(p, sh, L, r, u, bitmap, stages, feeder, consumed, w, tiles,
                                                     row_bytes, shard_mode, policy, polls)
-                            : consume_unit<T, false>(p, sh, L, r, u, bitmap, stages, feeder, consumed, w, tiles,
+                            : consume_unit<T, false, kGeneral>(p, sh, L, r, u, bitmap, stages, feeder, consumed, w, tiles,
                                                      row_bytes, shard_mode, policy, polls);
         __threadfence_block();
         __syncwarp();
@@ -1573,6 +1652,7 @@ static persist::Params to_persist_params(const fgk_stream_launch *l) {
     p.slot_bitmaps = l->slot_bitmaps;
     p.row_slots = l->row_slots;
     p.slot_bitmap_words = l->slot_bitmap_words;
+    p.skip_raising = l->skip_raising;
     p.wait_polls = l->wait_polls;
     p.withhold_cta = l->withhold_armed ? l->withhold_cta : 0xffffffffu;
     p.withhold_issue = l->withhold_issue;
@@ -1619,15 +1699,20 @@ extern "C" uint32_t fgk_persistent_max_parts(uint32_t k) {
     return (uint32_t)(persist::kWarps * persist::kListCap) / k;
 }
 
+using PersistentKernel = void (*)(const persist::Params);
+static PersistentKernel persistent_kernel(uint32_t dtype, bool general) {
+    if (dtype == 0) return general ? persist::persistent_select_kernel<float, true> : persist::persistent_select_kernel<float, false>;
+    return general ? persist::persistent_select_kernel<uint16_t, true> : persist::persistent_select_kernel<uint16_t, false>;
+}
+
 extern "C" int fgk_persistent_prepare(void) {
-    cudaError_t e = cudaFuncSetAttribute(persist::persistent_select_kernel<float>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(persist::kSharedLimit - sizeof(persist::Shared) - 256u));
-    if (e != cudaSuccess) return (int)e;
-    e = cudaFuncSetAttribute(persist::persistent_select_kernel<uint16_t>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(persist::kSharedLimit - sizeof(persist::Shared) - 256u));
-    return (int)e;
+    for (uint32_t i = 0; i < 4u; i++) {
+        const cudaError_t e = cudaFuncSetAttribute(persistent_kernel(i & 1u, i >= 2u),
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)(persist::kSharedLimit - sizeof(persist::Shared) - 256u));
+        if (e != cudaSuccess) return (int)e;
+    }
+    return (int)cudaSuccess;
 }
 
 extern "C" int fgk_launch_persistent_select(const fgk_stream_launch *l, uint32_t ctas, void *stream) {
@@ -1637,9 +1722,6 @@ extern "C" int fgk_launch_persistent_select(const fgk_stream_launch *l, uint32_t
     if (dynamic == 0) return (int)cudaErrorInvalidValue;
     p.bitmap_buffers = buffers;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (l->dtype == 0)
-        persist::persistent_select_kernel<float><<<ctas, persist::kBlock, dynamic, s>>>(p);
-    else
-        persist::persistent_select_kernel<uint16_t><<<ctas, persist::kBlock, dynamic, s>>>(p);
+    persistent_kernel(l->dtype, l->general != 0)<<<ctas, persist::kBlock, dynamic, s>>>(p);
     return (int)cudaGetLastError();
 }

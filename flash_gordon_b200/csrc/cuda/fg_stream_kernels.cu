@@ -56,6 +56,7 @@ struct StreamParams {
     uint32_t *part_ids;
     PartMeta *part_meta;            // [rows][splits]
     uint32_t *tickets;              // [rows], zero between launches
+    uint32_t only_raising;          // rows whose penalties cannot raise a logit are another kernel's
     uint32_t history_max;           // caller's bound on any row's history length
     uint32_t bitmap_words;          // shared-memory layout (0: no history structure)
     uint32_t count_capacity;        // entries of the dense count array (0: counts unused)
@@ -851,6 +852,7 @@ stream_select_kernel(const __grid_constant__ StreamParams p) {
     // notes the NaN/Inf the argmax order would put first: the merge must see it)
     const bool greedy = cfg.temperature == 0.0f;
     if (!shard_mode && !greedy && cfg.top_k == 0) return;  // rows without a top-k cut use the nucleus kernel
+    if (p.only_raising && !can_raise(cfg)) return;
 
     const uint32_t lo = split * p.split_len;
     const T *columns = static_cast<const T *>(p.logits) + (size_t)row * p.row_stride + lo;
@@ -1180,6 +1182,7 @@ static StreamParams to_stream_params(const fgk_stream_launch *l) {
     p.part_ids = l->part_ids;
     p.part_meta = reinterpret_cast<PartMeta *>(l->part_meta);
     p.tickets = l->tickets;
+    p.only_raising = l->only_raising;
     p.history_max = l->history_max;
     p.bitmap_words = l->bitmap_words;
     p.count_capacity = l->count_capacity;

@@ -568,7 +568,7 @@ static bool plan_stream(const fg_cuda_context *c, uint32_t rows, uint32_t vocab,
 typedef struct batch_traits {
     bool penalties, counts, sampled, topk_rows;
     uint32_t nucleus; /* rows without a top-k cut */
-    bool raising; /* some row's penalties can raise a logit (or its repetition factor is extreme) */
+    uint32_t raising; /* rows with a top-k cut whose penalties can raise a logit (or with an extreme repetition factor) */
 } batch_traits;
 
 static fg_status check_batch(const fg_cuda_context *c, const fg_cuda_sample_args *a, bool shard,
@@ -593,8 +593,9 @@ static fg_status check_batch(const fg_cuda_context *c, const fg_cuda_sample_args
         if (fg_sampler_penalties_active(cfg)) {
             traits->penalties = true;
             if (!(cfg->presence_penalty >= 0.0f && cfg->frequency_penalty >= 0.0f &&
-                  cfg->repetition_penalty >= 1.0f && cfg->repetition_penalty <= 0x1p40f))
-                traits->raising = true;
+                  cfg->repetition_penalty >= 1.0f && cfg->repetition_penalty <= 0x1p40f) &&
+                (shard || cfg->temperature == 0.0f || cfg->top_k != 0u))
+                traits->raising++;
         }
         if (cfg->frequency_penalty != 0.0f) traits->counts = true;
         if (cfg->temperature != 0.0f) {
@@ -702,8 +703,27 @@ static fg_status run_stream(fg_cuda_context *c, const fg_cuda_sample_args *a,
                             const batch_traits *traits, uint32_t vocab_offset,
                             uint32_t vocab_total, uint32_t shard_k, float *shard_scores,
                             uint32_t *shard_ids, uint32_t shard_stride, fg_error *err) {
+    /* Rows the copy engine can fetch whose penalties cannot raise a logit may go through the
+     * persistent ring kernel; rows whose penalties can, and anything the caller pinned to it, through the
+     * register-prefetch kernel.  A large batch with both kinds of rows goes through both, one after
+     * the other; a small one is faster through the second alone (measured with one row in eight
+     * raising, bf16, both against one kernel: 100,277 logits 148 rows 88 / 85 us, 200 rows 96 / 115, 400
+     * rows 129 / 227; 39,552 logits 300 rows 85 / 76, 400 rows 92 / 105). */
+    const size_t element = a->dtype == FG_CUDA_BF16 ? 2u : 4u;
+    const uint32_t whole_bitmap = traits->penalties ? (a->vocab + 31u) / 32u : 0u;
+    const uint32_t raising = !traits->penalties ? 0u : a->config_count == 1u && traits->raising ? a->rows : traits->raising;
+    const bool aligned = ((uintptr_t)a->logits % 16u) == 0u && (a->row_stride * element) % 16u == 0u &&
+                         ((size_t)a->vocab * element) % 16u == 0u;
+    const bool few_long_rows = a->rows * 4u < c->sm_count && fgk_persistent_row_tiles(a->dtype, a->vocab) > 512u;
+    const bool ring_ok = ((uintptr_t)a->logits % element) == 0u && c->forced_splits <= 1u &&
+                         (aligned || !few_long_rows) && /* (rows are cut at 16-byte boundaries) */
+                         fgk_persistent_dynamic_smem(whole_bitmap, NULL) != 0u;
+    const bool all_ring = ring_ok && raising == 0u;
+    const bool both = ring_ok && raising != 0u && raising < a->rows && a->config_count > 1u &&
+                      (uint64_t)(a->rows - traits->nucleus) * a->vocab >= 15000000u &&
+                      c->path == FG_CUDA_PATH_AUTO && !c->session_counts;
     stream_plan plan;
-    if (!plan_stream(c, a->rows, a->vocab, a->history_max, traits->penalties, traits->counts, &plan)) {
+    if (!plan_stream(c, both ? raising : a->rows, a->vocab, a->history_max, traits->penalties, traits->counts, &plan)) {
         fg_error_set(err, FG_ERR_LIMIT, "history structure does not fit shared memory");
         return FG_ERR_LIMIT;
     }
@@ -746,21 +766,12 @@ static fg_status run_stream(fg_cuda_context *c, const fg_cuda_sample_args *a,
     l.count_capacity = plan.count_capacity;
     l.dense_wide = plan.dense_wide;
     fill_output(&l.out, c, a);
-    /* Whole rows the copy engine can fetch (16-byte aligned starts and lengths) whose
-     * penalties cannot raise a logit may go through the persistent ring kernel; the
-     * rest, and anything the caller pinned to it, through the register-prefetch kernel. */
-    const size_t element = a->dtype == FG_CUDA_BF16 ? 2u : 4u;
-    const uint32_t whole_bitmap = traits->penalties ? (a->vocab + 31u) / 32u : 0u;
-    const bool ring_ok = ((uintptr_t)a->logits % 16u) == 0u && (a->row_stride * element) % 16u == 0u &&
-                         ((size_t)a->vocab * element) % 16u == 0u && c->forced_splits <= 1u &&
-                         !(traits->penalties && traits->raising) &&
-                         fgk_persistent_dynamic_smem(whole_bitmap, NULL) != 0u;
-    if (c->session_counts && !(ring_ok && c->path != FG_CUDA_PATH_REGISTERS && vocab_offset == 0u)) {
+    if (c->session_counts && !(all_ring && c->path != FG_CUDA_PATH_REGISTERS && vocab_offset == 0u)) {
         /* (the executor then falls back to token lists) */
         fg_error_set(err, FG_ERR_UNAVAILABLE, "session tables are read by the ring kernel only");
         return FG_ERR_UNAVAILABLE;
     }
-    if (c->path == FG_CUDA_PATH_RING && !ring_ok) {
+    if (c->path == FG_CUDA_PATH_RING && !(all_ring && aligned)) {
         fg_error_set(err, FG_ERR_ARGUMENT,
                      "the ring path needs whole 16-byte aligned rows and penalties that only lower logits");
         return FG_ERR_ARGUMENT;
@@ -768,7 +779,7 @@ static fg_status run_stream(fg_cuda_context *c, const fg_cuda_sample_args *a,
     /* AUTO: the persistent kernel whenever it can take the batch. */
     const uint32_t most = c->sm_count; /* one CTA per SM */
     const bool take_ring = c->path != FG_CUDA_PATH_REGISTERS;
-    if (ring_ok && take_ring) {
+    if (both || (all_ring && take_ring)) {
         /* When work goes out in tiles, every CTA gets the same number, so a row may be shared
          * by several CTAs.  A share is at least as long as the CTA's warps look at side by
          * side, and so long that no row has more parts than the merge takes. */
@@ -791,8 +802,7 @@ static fg_status run_stream(fg_cuda_context *c, const fg_cuda_sample_args *a,
          * its fixed work once per part and a merge through global memory, which only pays when a
          * single CTA would be alone with a row of a million logits.  (Measured on B200, vocabulary
          * 151,936: one row 39 against 69 us, 128 rows 51 against 67 us, 256 rows 47 against 63 us.) */
-        const bool few_long_rows = a->rows * 4u < most && row_tiles > 512u;
-        const bool whole_rows = c->ring_deal == 1u || (c->ring_deal == 0u && !few_long_rows);
+        const bool whole_rows = !aligned || both || c->ring_deal == 1u || (c->ring_deal == 0u && !few_long_rows);
         if (whole_rows) {
             per_cta = 0u;
             ctas = a->rows < most ? a->rows : most;
@@ -810,9 +820,12 @@ static fg_status run_stream(fg_cuda_context *c, const fg_cuda_sample_args *a,
             l.part_ids = (uint32_t *)(base + part_slots * 64u * 4u);
             l.part_meta = base + part_slots * 64u * 8u;
         }
+        fgk_stream_launch rest = l; /* for the rows the other kernel takes */
         l.splits = max_parts;
         l.split_len = (uint32_t)per_cta;
         l.bitmap_words = whole_bitmap;
+        l.general = !aligned || both;
+        l.skip_raising = both;
         l.slot_counts = c->session_counts;
         l.slot_bitmaps = c->session_bitmaps;
         l.row_slots = c->session_rows;
@@ -824,7 +837,10 @@ static fg_status run_stream(fg_cuda_context *c, const fg_cuda_sample_args *a,
         c->last_scratch_bytes = part_slots * (64u * 8u + 16u) + (size_t)a->rows * 4u +
                                 (a->config_count > 1u ? (size_t)a->rows * sizeof(fg_sampler_config) : 0u);
         const int e = launched(c, fgk_launch_persistent_select(&l, ctas, c->stream));
-        return e ? fg_cuda_fail(err, e, "persistent ring kernel") : FG_OK;
+        if (e) return fg_cuda_fail(err, e, "persistent ring kernel");
+        if (!both) return FG_OK;
+        l = rest;
+        l.only_raising = 1u;
     }
     /* the streaming kernel's hand-off between the splits of a row, reserved only when it runs */
     if (part_bytes) {

@@ -1,0 +1,80 @@
+"""Rows that do not begin or end on a 16-byte boundary in the ring kernel, and batches whose rows
+go through different kernels because some rows' penalties can raise a logit."""
+import numpy as np
+import pytest
+import torch
+
+from flash_gordon_b200 import FG_OK, SamplerConfig, synth
+from helpers import as_u32, assert_rows_equal, random_workload, run_gpu, run_oracle
+
+pytestmark = pytest.mark.gpu
+
+CONFIGS = {
+    "top_k": SamplerConfig.make(temperature=0.8, top_p=0.95, top_k=20),
+    "penalised": SamplerConfig.make(temperature=0.8, top_p=0.9, top_k=64, presence=0.4, frequency=0.3, repetition=1.1),
+    "greedy": SamplerConfig.make(temperature=0.0, top_p=1.0, top_k=1, repetition=1.2),
+}
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("kind", CONFIGS)
+@pytest.mark.parametrize("vocab,stride,start", [
+    (1, 3, 1), (5, 9, 3), (7, 8, 1), (9, 11, 2), (2041, 2049, 0), (2047, 2047, 5), (2048, 2055, 7), (2049, 2050, 1),
+    (16383, 16391, 3), (16385, 16385, 0), (100_277, 100_277, 0), (100_280, 100_283, 6),
+])
+def test_every_offset(context, dtype, kind, vocab, stride, start):
+    """`start` elements before the first row, `stride` between rows: nine rows meet every offset
+    of a row's first logit from a boundary.  What lies between the rows would win if it were
+    looked at; the rows' own ends hold large values, NaN and infinities."""
+    rows = 9
+    w = random_workload(rows, vocab, 40 if kind != "top_k" else 0, [CONFIGS[kind]], 31 * vocab + start,
+                        specials=2 if vocab > 16 else 0, dtype=dtype)
+    w.logits[1::3, 0] = 30.0
+    w.logits[2::3, -1] = 31.0
+    w.logits[0, -1] = float("nan")
+    if vocab > 1:
+        w.logits[3, 0] = float("inf")
+    expected = run_oracle(w)
+    block = torch.full((start + rows * stride + 16,), 99.0, dtype=dtype, device="cuda")
+    placed = torch.as_strided(block, (rows, vocab), (stride, 1), start)
+    placed.copy_(w.logits)
+    d = w.to("cuda")
+    result = context.sample_batch(placed, d.configs, d.uniforms, d.history_tokens, d.history_offsets, d.history_max)
+    torch.cuda.synchronize()
+    assert_rows_equal(result, expected, f"{kind} V={vocab}")
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("vocab", [12_346, 12_352])
+@pytest.mark.parametrize("raising", [1, 7, 30])
+def test_rows_of_one_batch_in_two_kernels(context, dtype, vocab, raising):
+    """`raising` of 30 rows have penalties that can raise a logit."""
+    rows = 30
+    configs = []
+    for r in range(rows):
+        lift = (r * 7) % rows < raising
+        configs.append(SamplerConfig.make(temperature=0.0 if r % 5 == 0 else 0.9, top_p=0.9, top_k=1 if r % 5 == 0 else 30,
+                                          presence=-0.7 if lift else 0.5, frequency=0.2 * (r % 2),
+                                          repetition=1.0 + 0.1 * (r % 3)))
+    w = random_workload(rows, vocab, 400, configs, 5 + raising, dtype=dtype)
+    assert_rows_equal(run_gpu(context, w), run_oracle(w), f"{raising} raising rows")
+
+
+def test_unaligned_shards(context):
+    """Two column ranges of unaligned rows, then the merge, against the whole rows."""
+    rows, vocab, k = 11, 9_001, 24
+    cfg = SamplerConfig.make(temperature=0.9, top_p=0.9, top_k=k, presence=0.3)
+    w = random_workload(rows, vocab, 200, [cfg], 77)
+    expected = run_oracle(w)
+    d = w.to("cuda")
+    scores = torch.empty(2, rows, k, device="cuda")
+    ids = torch.empty(2, rows, k, dtype=torch.int32, device="cuda")
+    first = [0, 4_503]
+    width = [4_503, vocab - 4_503]
+    for s in range(2):
+        part = d.logits[:, first[s]:first[s] + width[s]]
+        _, _, _, status = context.shard_topk(part, d.configs, first[s], vocab, k, d.history_tokens, d.history_offsets,
+                                             d.history_max, out=(scores[s], ids[s]))
+        assert status == FG_OK
+    result = context.merge_select(scores, ids, rows, 2, k, first, width, d.configs, d.uniforms)
+    assert np.array_equal(as_u32(result.tokens), expected[1])
