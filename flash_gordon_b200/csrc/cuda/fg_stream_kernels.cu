@@ -79,6 +79,7 @@ struct StreamShared {
     uint32_t wild_bits;
     uint32_t is_last;
     uint32_t overflow;            // a value found no slot in the candidate list
+    uint32_t part_count[kMaxSplits], part_before[kMaxSplits];  // the merge of a row's splits
 };
 
 template <typename T>
@@ -600,32 +601,57 @@ __device__ __noinline__ void finish_split(const StreamParams &p, StreamShared &s
         __syncthreads();
         if (!sh.is_last) return;
         __threadfence();
-        if (tid == 0) {
-            p.tickets[row] = 0;  // ready for the next launch
-            sh.cand.count = 0;
+        if (tid == 0) p.tickets[row] = 0;  // ready for the next launch
+        // Every split's survivors into the candidate buffer.  The splits' records and entries are
+        // asked for together: one trip to L2, not two per split.
+        const size_t first_slot = (size_t)row * p.splits;
+        uint4 meta = make_uint4(0, kPaddingId, 0, 0);
+        if (tid < p.splits) meta = __ldcg(reinterpret_cast<const uint4 *>(&p.part_meta[first_slot + tid]));
+        constexpr int kOwned = (int)(kMaxSplits * kMaxK) / kThreads;
+        float score[kOwned];
+        uint32_t id[kOwned];
+#pragma unroll
+        for (int q = 0; q < kOwned; q++) {
+            const uint32_t e = q * kThreads + tid;
+            const bool there = e < p.splits * (uint32_t)kMaxK;
+            score[q] = there ? __ldcg(&p.part_scores[first_slot * kMaxK + e]) : 0.0f;
+            id[q] = there ? __ldcg(&p.part_ids[first_slot * kMaxK + e]) : kPaddingId;
         }
-        // gather every split's survivors into the candidate buffer
-        uint32_t total = 0;
-        bad_history = 0;
-        wild_id = kPaddingId;
-        wild_bits = 0;
-        for (uint32_t s = 0; s < p.splits; s++) {
-            const size_t from = (size_t)row * p.splits + s;
-            const uint4 packed = __ldcg(reinterpret_cast<const uint4 *>(&p.part_meta[from]));
-            const uint32_t count = packed.x;
-            if (tid < count) {
-                sh.cand.score[total + tid] = __ldcg(&p.part_scores[from * kMaxK + tid]);
-                sh.cand.id[total + tid] = __ldcg(&p.part_ids[from * kMaxK + tid]);
+        if (tid < 32) {  // (at most 16 splits)
+            uint32_t before = meta.x;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t up = __shfl_up_sync(kFullMask, before, d);
+                if (tid >= (uint32_t)d) before += up;
             }
-            total += count;
-            if (packed.w) bad_history = packed.w;
-            if (packed.y < wild_id) {
-                wild_id = packed.y;
-                wild_bits = packed.z;
+            const uint32_t bad = __reduce_max_sync(kFullMask, meta.w);
+            const uint32_t wild = __reduce_min_sync(kFullMask, meta.y);
+            if (tid < p.splits) {
+                sh.part_count[tid] = meta.x;
+                sh.part_before[tid] = before - meta.x;
             }
+            if (tid == 31) sh.cand.count = before;
+            if (tid == 0) {
+                sh.bad_history = bad;
+                sh.wild_id = wild;
+                sh.wild_bits = 0;
+            }
+            __syncwarp();
+            if (wild != kPaddingId && meta.y == wild) sh.wild_bits = meta.z;
         }
         __syncthreads();
-        if (tid == 0) sh.cand.count = total;
+        const uint32_t total = sh.cand.count;
+        bad_history = sh.bad_history;
+        wild_id = sh.wild_id;
+        wild_bits = sh.wild_bits;
+#pragma unroll
+        for (int q = 0; q < kOwned; q++) {
+            const uint32_t e = q * kThreads + tid, s = e / kMaxK, i = e % kMaxK;
+            if (s < p.splits && i < sh.part_count[s]) {
+                sh.cand.score[sh.part_before[s] + i] = score[q];
+                sh.cand.id[sh.part_before[s] + i] = id[q];
+            }
+        }
         __syncthreads();
         held = compact_topk<kThreads, kCandCap>(sh.cand, total, k);
     }
