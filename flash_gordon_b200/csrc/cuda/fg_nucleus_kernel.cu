@@ -19,9 +19,9 @@
 // histogram pass, down to an MSB-first radix descent over the 32-bit monotone value key and,
 // among equal values, over the id.
 //
-// Masses are exp(s - max) as 2^-40 fixed point in 64-bit integers: integer addition is
-// associative, so the result does not depend on the order threads arrive in, and the 1e-12
-// grid is far below one element's weight.  The reference adds doubles left to right; the two
+// Masses are exp(s - max) as 2^-44 (the long way: 2^-40) fixed point in 64-bit integers: integer
+// addition is associative, so the result does not depend on the order threads arrive in, and
+// the grid is far below one element's weight.  The reference adds doubles left to right; the two
 // agree unless the top-p bound or the draw falls within ~1e-11 (relative) of an edge of the
 // CDF.
 #include <cooperative_groups.h>
@@ -79,10 +79,10 @@ struct NucleusShared {
     uint32_t hit_found;
 };
 
-// exp(x) * 2^40 for x <= 0 as a 64-bit integer (round to nearest): argument reduction
+// exp(x) * 2^bits for x <= 0 as a 64-bit integer (round to nearest): argument reduction
 // to n/64 * ln2 + r, |r| <= ln2/128, a 64-entry table of 2^(j/64) and a degree-5
 // polynomial (truncation 4e-17).  Below e^-70 the weight is under the fixed-point grid.
-__device__ __forceinline__ unsigned long long exp_fixed(double x, const double *table) {
+__device__ __forceinline__ unsigned long long exp_fixed(double x, const double *table, int bits = 40) {
     if (!(x > -70.0)) return 0ull;
     const double scaled = x * 92.33248261689366;                  // 64 / ln 2
     const double shifted = scaled + 6755399441055744.0;           // 1.5 * 2^52: rounds to nearest
@@ -96,7 +96,7 @@ __device__ __forceinline__ unsigned long long exp_fixed(double x, const double *
     p = fma(p, r, 1.0);
     p = fma(p, r, 1.0);                                           // 1 + r + r^2/2 + ... + r^5/120
     const int j = n & 63, k = n >> 6;                             // floor division for negative n
-    const double scale = __longlong_as_double((long long)(k + 40 + 1023) << 52);
+    const double scale = __longlong_as_double((long long)(k + bits + 1023) << 52);
     return __double2ull_rn(table[j] * p * scale);
 }
 
@@ -466,7 +466,7 @@ struct Position {
 __device__ __forceinline__ Position order_members(NucleusShared &sh, const OrderWork &list, uint32_t members, double inv_t, float top,
                                   const Nucleus inside, unsigned long long before, uint32_t rank_before,
                                   unsigned long long target, bool strict, bool clipped, double also_inv_t,
-                                  unsigned long long *also_sum) {
+                                  unsigned long long *also_sum, int bits) {
     const uint32_t tid = threadIdx.x;
     Position found;
     found.ok = false;
@@ -528,7 +528,7 @@ __device__ __forceinline__ Position order_members(NucleusShared &sh, const Order
         const float value = key_to_float((uint32_t)(mine >> 32));  // (-0.0 comes back as +0.0: see below)
         list.sorted_value[a] = value;
         list.sorted_id[a] = ~(uint32_t)mine;
-        list.weight[a] = exp_fixed(((double)value - (double)top) * inv_t, sh.table);
+        list.weight[a] = exp_fixed(((double)value - (double)top) * inv_t, sh.table, bits);
     }
     __syncthreads();
     // (what is not inside the nucleus comes last in the order)
@@ -601,7 +601,7 @@ __device__ __forceinline__ Position order_members(NucleusShared &sh, const Order
         // the other weight of the members up to the one found (order does not matter: integers)
         unsigned long long part = 0;
         for (uint32_t a = tid; a <= at; a += kNucleusThreads)
-            part += exp_fixed(((double)list.sorted_value[a] - (double)top) * also_inv_t, sh.table);
+            part += exp_fixed(((double)list.sorted_value[a] - (double)top) * also_inv_t, sh.table, bits);
         const uint32_t lane = tid & 31u, warp = tid >> 5;
 #pragma unroll
         for (int d = 16; d > 0; d >>= 1) part += __shfl_xor_sync(kFullMask, part, d);
@@ -644,7 +644,7 @@ __device__ Position resolve_bucket(NucleusShared &sh, NucleusList &list, const f
     members = min(list.count, kListCap);  // (inside may hold fewer of the bucket than the histogram counted)
     if (members == 0) return found;
     return order_members(sh, list.work(), members, inv_t, top, inside, before, rank_before, target, strict, clipped,
-                         also_inv_t, also_sum);
+                         also_inv_t, also_sum, 40);
 }
 
 // After a crossing search: the bucket it stopped in, or -- when the total never reaches the
@@ -967,21 +967,24 @@ __device__ __noinline__ void sample_the_long_way(NucleusShared &sh, NucleusList 
 // latencies of 20 us, so two CTAs share an SM, one streaming while the other scans and sorts; for
 // few rows a row is spread over several CTAs instead.  A CTA per row and SM that added two fp64 weights
 // per logit to five shared-memory sums took, per call: 512 rows of 151,936 fp32 logits, histories
-// of 32,768 tokens 772 us (now 546), without history 538 (238); 32 rows bf16 410-560 (63).
+// of 32,768 tokens 772 us (now 561), without history 538 (245); 32 rows bf16 410-560 (60).
 // With histories the largest part is the seen columns' gather (amend_seen).
 //
 // A value's place: buckets 1/1024 wide over the top four units of the row's window, 1/256 wide over
-// the next eight, 1/32 over the next 64 (all half as wide for temperatures below 0.36), with
-// their middles on the grid of multiples of the width, so that neither the bucket nor the
-// distance f from its middle depends on a subtraction that rounds: n = rint(v * 1024) by adding
-// and subtracting 1.5 * 2^23, f = v * 1024 - n in [-1/2, 1/2], both exact in fp32.  With
-// w = width * f the members' weights relative to the middle's add up to
+// the next eight, 1/64 over the next 32 (1/32 over 64 for temperatures above 1.42; all half as
+// wide for temperatures below 0.36), with their middles on the grid of multiples of the
+// width, so that neither the bucket nor the distance f from its middle depends on a
+// subtraction that rounds: n = rint(v * 1024) by adding and subtracting 1.5 * 2^23,
+// f = v * 1024 - n in [-1/2, 1/2], both exact in fp32.  With w = width * f the members' weights
+// relative to the middle's add up to
 //     sum exp(w) = N + c M1 + c^2/2 M2 + c^3/6 M3 + ...,   c = width (times 1/T: tempered)
 // M3 is not kept: f^3 is replaced by the nearest multiple of f (0.15 f over a bucket), which
 // leaves 0.019 c^3/6 (root mean square) of a member's weight: 3e-12 raw and 2.4e-11 at T = 0.5 in
-// the narrow buckets, at most 6e-12 of the largest weight in the wider ones (they begin 3.5
-// units below the sampled maximum, where a weight is e^-3.5 of it at most, e^-7 at T = 0.5),
-// against 6.7e-11 for weights rounded to 2^-32 of themselves.
+// the narrow buckets, less in the wider ones relative to the largest weight, against 6.7e-11
+// for weights rounded to 2^-32 of themselves, as they were before.  Largest error of the cumulative masses
+// over their total, rows of 151,936 logits of spread 0.5 to 4 (with and without Gumbel noise), fp32
+// and bf16, against extended precision: T = 0.5 7.5e-11 before, 1.4e-12 now; T = 1 5.8e-11 and
+// 2.0e-12; T = 1.4 3.5e-11 and 2.8e-12.
 //
 // A bucket is two 32-bit words that are added to, once each, per member:
 //     first    sum of f in units of 2^-22 (the bits of f * 2^22 + 1.5 * 2^23: the constant's
@@ -1001,8 +1004,7 @@ constexpr uint32_t kFineSlots = 4096, kMiddleSlots = 2048, kCoarseSlots = 2048;
 constexpr uint32_t kSlots = kFineSlots + kMiddleSlots + kCoarseSlots;
 constexpr uint32_t kGroups = kSlots / 32;      // the slots a warp looks at side by side
 constexpr uint32_t kPlaces = kGroups + 1;      // place 0: the values above the window
-constexpr float kFineScale = 1024.0f, kMiddleScale = 256.0f, kCoarseScale = 32.0f;
-constexpr int kFineSpan = 12301;               // from 32 times the topmost coarse middle to the topmost fine one
+constexpr float kFineScale = 1024.0f, kMiddleScale = 256.0f;
 constexpr float kMagic = 12582912.0f;          // 1.5 * 2^23: adding it rounds to a whole number
 constexpr uint32_t kMagicBits = 0x4b400000u;
 constexpr uint32_t kMostTeam = 8;              // CTAs that may share a row
@@ -1015,6 +1017,7 @@ constexpr int kSamples = 4;                    // logits a thread looks at to pl
 // it replaces (buckets half as wide take it down to half of the first); above, values under the window would
 // still weigh something.
 constexpr float kWideColdest = 0.36f, kShortColdest = 0.18f, kShortHottest = 2.6f;
+constexpr float kFarColdest = 1.42f;           // up to here 43 units under the maximum weigh less than the grid
 
 constexpr uint32_t inverse_mod(uint32_t a, uint32_t modulus) {  // a odd, modulus a power of two
     uint32_t x = 1;
@@ -1044,31 +1047,37 @@ struct Packing {
 // The window of a row: which values have a bucket, and which.
 struct Window {
     float sharp;                          // 1, or 2 for buckets half as wide
+    float coarse;                         // wide buckets in a unit (times sharp): 64, or 32 to reach further down
     float top, first_edge, second_edge;   // narrow buckets: [first_edge, top], middle: [second_edge, first_edge),
     float bottom;                         // wide: [bottom, second_edge)
-    int coarse_top;                       // the middle of the topmost wide bucket, in widths
+    int fine_top, middle_top, coarse_top; // the middle of the topmost bucket of each kind, in widths
     bool usable;
 
-    __device__ __forceinline__ explicit Window(float reference, float sharp_) : sharp(sharp_) {
+    __device__ __forceinline__ Window(float reference, float sharp_, float coarse_) : sharp(sharp_), coarse(coarse_) {
         usable = fabsf(reference) * sharp < kWindowLimit;
         const float at = usable ? reference * sharp : 0.0f, unit = 1.0f / sharp;  // (sharp: a power of two)
-        coarse_top = __float2int_rn(((at + kWindowMargin) * kFineScale - (float)kFineSpan) * 0.03125f);
-        top = (float)(32 * coarse_top + kFineSpan) * (1.0f / kFineScale) * unit;
-        first_edge = ((float)(8 * coarse_top + 2051) + 0.5f) * (1.0f / kMiddleScale) * unit;
-        second_edge = ((float)coarse_top + 0.5f) * (1.0f / kCoarseScale) * unit;
-        bottom = (float)(coarse_top - (int)(kCoarseSlots - 1)) * (1.0f / kCoarseScale) * unit;
+        const int ratio = (int)(kMiddleScale / coarse);                           // 4 or 8
+        // a kind's lowest bucket begins where the next kind's highest ends
+        const int span = 2 * ratio + 12285;                                       // 4 * (ratio / 2 + 2047.5) + 4095
+        coarse_top = __float2int_rn(((at + kWindowMargin) * kFineScale - (float)span) / (float)(4 * ratio));
+        middle_top = ratio * coarse_top + ratio / 2 + (int)(kMiddleSlots - 1);
+        fine_top = 4 * ratio * coarse_top + span;
+        top = (float)fine_top * (1.0f / kFineScale) * unit;
+        first_edge = ((float)middle_top + 0.5f) * (1.0f / kMiddleScale) * unit;
+        second_edge = ((float)coarse_top + 0.5f) / coarse * unit;
+        bottom = (float)(coarse_top - (int)(kCoarseSlots - 1)) / coarse * unit;
     }
     // the bucket of a value in [bottom, top], and its distance from the middle in widths
     __device__ __forceinline__ uint32_t slot(float v, float &f) const {
-        float scale = kCoarseScale * sharp;
+        float scale = coarse * sharp;
         uint32_t base = kMagicBits + kFineSlots + kMiddleSlots + (uint32_t)coarse_top;
         if (v >= second_edge) {
             scale = kMiddleScale * sharp;
-            base = kMagicBits + kFineSlots + (uint32_t)(8 * coarse_top + 2051);
+            base = kMagicBits + kFineSlots + (uint32_t)middle_top;
         }
         if (v >= first_edge) {
             scale = kFineScale * sharp;
-            base = kMagicBits + (uint32_t)(32 * coarse_top + kFineSpan);
+            base = kMagicBits + (uint32_t)fine_top;
         }
         const float shifted = __fmaf_rn(v, scale, kMagic);
         f = __fmaf_rn(v, scale, -__fsub_rn(shifted, kMagic));
@@ -1078,13 +1087,13 @@ struct Window {
     __device__ __forceinline__ int middle_of(uint32_t slot, float &width) const {
         if (slot < kFineSlots) {
             width = 1.0f / (kFineScale * sharp);
-            return 32 * coarse_top + kFineSpan - (int)slot;
+            return fine_top - (int)slot;
         }
         if (slot < kFineSlots + kMiddleSlots) {
             width = 1.0f / (kMiddleScale * sharp);
-            return 8 * coarse_top + 2051 - (int)(slot - kFineSlots);
+            return middle_top - (int)(slot - kFineSlots);
         }
-        width = 1.0f / (kCoarseScale * sharp);
+        width = 1.0f / (coarse * sharp);
         return coarse_top - (int)(slot - kFineSlots - kMiddleSlots);
     }
     __device__ __forceinline__ double middle(uint32_t slot) const {
@@ -1162,7 +1171,7 @@ struct ShortMemory {
     } lists;                                             // the first CTA's
     unsigned long long raw[kPlaces], tempered[kPlaces];  // masses per place, then their running sums
     uint32_t count[kPlaces];
-    double edges[2][kGroups];         // raw, tempered: the weight of a group's first middle, times 2^40
+    double edges[2][kGroups];         // raw, tempered: the weight of a group's first middle, times 2^bits
     double lanes[2][3][32];           // the weights of the 32 slots relative to it, by kind of bucket
     float over_value[kOverCap];
     uint32_t over_id[kOverCap];
@@ -1525,11 +1534,12 @@ __device__ __noinline__ void write_scratch(const NucleusParams &p, uint32_t row,
         visit_seen<T>(p, row, cfg, lo, n, [&](uint32_t column, float, float value, uint32_t) { values[column] = value; });
 }
 
-// Sum over the warp of masses below 2^52.
+// Sum over the warp of masses below 2^60 (4,095 members of 2^44 weigh less than 2^57).
 __device__ __forceinline__ unsigned long long warp_sum_mass(unsigned long long mass) {
-    const uint32_t low = __reduce_add_sync(kFullMask, (uint32_t)mass & 0x3ffffffu);
-    const uint32_t high = __reduce_add_sync(kFullMask, (uint32_t)(mass >> 26));
-    return ((unsigned long long)high << 26) + low;
+    const uint32_t low = __reduce_add_sync(kFullMask, (uint32_t)mass & 0xfffffu);
+    const uint32_t middle = __reduce_add_sync(kFullMask, (uint32_t)(mass >> 20) & 0xfffffu);
+    const uint32_t high = __reduce_add_sync(kFullMask, (uint32_t)(mass >> 40));
+    return ((unsigned long long)high << 40) + ((unsigned long long)middle << 20) + low;
 }
 
 // The factors of the moments in a bucket's masses, by kind of bucket.
@@ -1554,7 +1564,7 @@ struct SlotMass {
     unsigned long long raw, tempered;
     uint32_t count;
 };
-// `raw_weight`, `tempered_weight`: the weights of the slot's middle, times 2^40.
+// `raw_weight`, `tempered_weight`: the weights of the slot's middle, times 2^bits.
 template <class P>
 __device__ __forceinline__ SlotMass slot_mass(uint32_t first, uint32_t second, const MomentFactors<P> &k,
                                               double raw_weight, double tempered_weight) {
@@ -1567,13 +1577,16 @@ __device__ __forceinline__ SlotMass slot_mass(uint32_t first, uint32_t second, c
     return s;
 }
 
-constexpr double kFixedOne = 1099511627776.0;  // 2^40
+// Masses of the short way are 2^-44 fixed point (every one of 8,192 buckets is rounded to it, which
+// at 2^-40 was the largest error for peaked rows), unless a row has so many columns that their sum
+// might not fit: then 2^-40.
+constexpr uint32_t kFinestVocab = 1u << 18;
 
 // Masses and counts of this CTA's groups into m.raw, m.tempered, m.count (place 1 + group), and the
 // weights they are made with into m.edges, m.lanes; state.counted gets the sum of all counts.  All
 // threads call; ends synced.
 template <class P>
-__device__ __noinline__ void group_masses(const Window window, double best, double inv_t) {
+__device__ __noinline__ void group_masses(const Window window, double best, double inv_t, int bits) {
     ShortMemory &m = short_memory();
     const uint32_t tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
     constexpr uint32_t kWarps = kNucleusWarps;
@@ -1582,7 +1595,7 @@ __device__ __noinline__ void group_masses(const Window window, double best, doub
     {
         const uint32_t group = tid % kGroups, tempered = tid / kGroups;
         const double x = window.middle(group * 32u) - best;
-        m.edges[tempered][group] = exp(tempered ? x * inv_t : x) * kFixedOne;
+        m.edges[tempered][group] = exp(tempered ? x * inv_t : x) * (double)(1ull << bits);
         if (tid < 192u) {
             const uint32_t kind = tid / 32u % 3u;
             float width;
@@ -1706,7 +1719,7 @@ __device__ __forceinline__ unsigned long long draw_target_of(double draw_at, uns
 // threads call; ends synced.
 template <class P>
 __device__ __noinline__ void make_plan(const Team team, const Window window, float best, double top_p, double inv_t,
-                                       double draw_at) {
+                                       double draw_at, int bits) {
     ShortMemory &m = short_memory();
     ShortShared &ss = m.state;
     const NucleusShared &sh = m.scan;
@@ -1719,8 +1732,8 @@ __device__ __noinline__ void make_plan(const Team team, const Window window, flo
         unsigned long long raw = 0, tempered = 0;
         for (uint32_t i = lane; i < over; i += 32) {
             const double x = (double)m.over_value[i] - (double)best;
-            raw += exp_fixed(x, sh.table);
-            tempered += exp_fixed(x * inv_t, sh.table);
+            raw += exp_fixed(x, sh.table, bits);
+            tempered += exp_fixed(x * inv_t, sh.table, bits);
         }
         raw = warp_sum_mass(raw);
         tempered = warp_sum_mass(tempered);
@@ -1943,7 +1956,7 @@ __device__ __noinline__ void gather_members(const T *columns, uint32_t lo, uint3
 
 // The first CTA orders the gathered members and reports the row; leaves the verdict in the plan.
 // All its threads call; ends synced.
-__device__ __noinline__ void finish_short(float best, double inv_t, double draw_at, uint32_t row,
+__device__ __noinline__ void finish_short(float best, double inv_t, double draw_at, int bits, uint32_t row,
                                           const SelectOutput &out) {
     ShortMemory &m = short_memory();
     ShortShared &ss = m.state;
@@ -1974,7 +1987,7 @@ __device__ __noinline__ void finish_short(float best, double inv_t, double draw_
                                              turn == 0 ? plan.cut_before : plan.pick_before,
                                              turn == 0 ? plan.cut_rank_before : 0u,
                                              turn == 0 ? plan.cut_target : draw_target_of(draw_at, weight_sum), turn != 0,
-                                             false, inv_t, turn == 0 ? &tempered_inside : nullptr);
+                                             false, inv_t, turn == 0 ? &tempered_inside : nullptr, bits);
         if (turn != 0) {
             pick = found;
             break;
@@ -2015,16 +2028,17 @@ __device__ __forceinline__ uint32_t locate_and_pick(const NucleusParams &p, cons
                                                     const SeenBits &bits, const float2 *seen, float best, double top_p,
                                                     double inv_t, double draw_at) {
     ShortShared &ss = short_memory().state;
-    group_masses<P>(window, (double)best, inv_t);
+    const int grid = p.vocab <= kFinestVocab ? 44 : 40;
+    group_masses<P>(window, (double)best, inv_t, grid);
     if (threadIdx.x == 0) ss.share.crowded = ss.counted != counted;
     team.sync();
-    if (team.rank == 0) make_plan<P>(team, window, best, top_p, inv_t, draw_at);
+    if (team.rank == 0) make_plan<P>(team, window, best, top_p, inv_t, draw_at, grid);
     team.sync();
     if (team.at(&ss.plan, 0)->verdict == kDone) {
         gather_members<T>(static_cast<const T *>(p.logits) + (size_t)row * p.row_stride, lo, n, window, team, bits, seen,
                           ss.seen_count);
         team.sync();
-        if (team.rank == 0) finish_short(best, inv_t, draw_at, row, p.out);
+        if (team.rank == 0) finish_short(best, inv_t, draw_at, grid, row, p.out);
         team.sync();
     }
     return team.at(&ss.plan, 0)->verdict;
@@ -2112,7 +2126,8 @@ __global__ void __launch_bounds__(kNucleusThreads, 2) nucleus_select_kernel(cons
         if (counting) reference = sample_row(columns, p.vocab, bits);
         if (is_nonfinite(reference)) reference = 0.0f;  // (nothing finite among the samples: any window will do)
         for (uint32_t attempt = 0; counting; attempt++) {
-            const Window window(reference, cfg.temperature < kWideColdest ? 2.0f : 1.0f);
+            const Window window(reference, cfg.temperature < kWideColdest ? 2.0f : 1.0f,
+                                cfg.temperature <= kFarColdest ? 64.0f : 32.0f);
             if (!window.usable) break;
             uint4 *words = reinterpret_cast<uint4 *>(m.first);
             for (uint32_t i = tid; i < 2 * kSlots / 4; i += kNucleusThreads) words[i] = make_uint4(0, 0, 0, 0);
