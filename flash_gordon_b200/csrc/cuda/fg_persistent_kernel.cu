@@ -1447,11 +1447,12 @@ __global__ void __launch_bounds__(kBlock, 1) persistent_select_kernel(const __gr
             lists[b].first_count = 0;
             lists[b].first_top = 0;
             lists[b].bad_history = 0;
-            for (int i = 0; i < kTallyBins; i++) lists[b].tally[i] = 0;
         }
         mbarrier_fence_init();
         sh.ring_error = 0;
     }
+    for (uint32_t i = tid; i < (uint32_t)(kListSets * kTallyBins); i += kBlock)
+        lists[i / kTallyBins].tally[i % kTallyBins] = 0;
     __syncthreads();
 
     if (warp >= (uint32_t)(kWarps + kHistoryWarps)) {
