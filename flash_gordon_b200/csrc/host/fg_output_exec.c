@@ -13,7 +13,7 @@
  *
  * The token lists themselves are kept on the host as well: they are what
  * fg_output_history_reset is given, and what the register-prefetch kernel needs for the
- * batches the ring kernel does not take (penalties that can raise a logit, unaligned rows).
+ * batches the ring kernel does not take (penalties that can raise a logit).
  */
 #include "fg_host_internal.h"
 

@@ -68,7 +68,8 @@ fg_status fg_cuda_context_set_splits(fg_cuda_context *context, uint32_t splits, 
  * shared-memory ring fed by bulk copies (rows whose start, stride and length are
  * multiples of 16 bytes, penalties that cannot raise a logit), or the
  * register-prefetch kernel (anything).  AUTO is the library's choice: the ring
- * kernel whenever it can take the batch.  RING fails with FG_ERR_ARGUMENT on a
+ * kernel whenever it can take the batch, unaligned rows included, and for the
+ * rows it can take of a large batch with some raising penalties.  RING fails with FG_ERR_ARGUMENT on a
  * batch it cannot take, RING_IF_POSSIBLE falls back instead (as AUTO does).
  * Results never depend on it. */
 #define FG_CUDA_PATH_AUTO             0u

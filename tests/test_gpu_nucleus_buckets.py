@@ -66,6 +66,7 @@ PLAIN = (0.0, 0.0, 1.0)
     ("plain", 150, 9_000, 0.8, 1.0, 3000, (0.0, -0.2, 0.8)),
     ("plain", 2, 20_000, 1.0, 0.9, 70_000, (0.2, 0.1, 1.0)),    # 32-bit counts
     ("plain", 2, 70, 1.0, 0.7, 10, (0.2, 0.1, 1.0)),            # CTAs without a column
+    ("plain", 2, 300_001, 1.0, 0.95, 800, (0.2, 0.1, 1.0)),     # the coarser grid of masses
     ("plain", 2, 50_000, 0.36, 0.9, 0, PLAIN), ("plain", 2, 50_000, 0.35, 0.9, 0, PLAIN),
     ("plain", 2, 50_000, 0.18, 0.99, 90, (0.5, 0.1, 1.0)), ("plain", 2, 50_000, 0.17, 0.9, 0, PLAIN),
     ("plain", 2, 50_000, 2.6, 0.9, 0, PLAIN), ("plain", 2, 50_000, 2.7, 0.9, 40, (0.5, 0.1, 1.0)),
