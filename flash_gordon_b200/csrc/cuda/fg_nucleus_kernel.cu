@@ -1307,7 +1307,8 @@ __device__ __forceinline__ float pick_element(const float (&v)[kPer], int j) {
 
 // What a pass over one CTA's columns finds out beside the buckets.
 struct Findings {
-    float best;                     // largest finite value
+    float best;                     // largest value inside the window
+    float outside;                  // largest finite one outside (a seen id's raw logit is none)
     int lost, below, above;         // not finite, under the window, over it
 };
 
@@ -1332,7 +1333,7 @@ struct Counter {
     Findings found;
 
     __device__ __forceinline__ Counter(const Window &w, const Team &team_) : window(w), team(team_) {
-        found.best = -INFINITY;
+        found.best = found.outside = -INFINITY;
         found.lost = found.below = found.above = 0;
     }
     // a value inside the window
@@ -1362,7 +1363,7 @@ struct Counter {
             for (int j = 0; j < kPer; j++) take(pick_element(v, j), column + j, skip);
         }
     }
-    // `skip`: values above the window that are not listed (a seen id's raw logit)
+    // `skip`: columns whose value outside the window is not the row's (a seen id's raw logit)
     __device__ __forceinline__ void take(float v, uint32_t column, const SeenBits &skip) {
         if (v >= window.bottom && v <= window.top) {
             found.best = fmaxf(found.best, v);
@@ -1374,15 +1375,15 @@ struct Counter {
                 ShortMemory &m = short_memory();
                 found.above++;
                 if (skip.test(column)) return;
-                found.best = fmaxf(found.best, v);
+                found.outside = fmaxf(found.outside, v);
                 const uint32_t slot = atomicAdd(team.at(&m.state.over_count, 0), 1u);
                 if (slot < kOverCap) {
                     team.at(m.over_value, 0)[slot] = v;
                     team.at(m.over_id, 0)[slot] = column;
                 }
             } else {
-                found.best = fmaxf(found.best, v);
                 found.below++;
+                if (v > found.outside && !skip.test(column)) found.outside = v;
             }
         }
     }
@@ -2148,17 +2149,16 @@ __global__ void __launch_bounds__(kNucleusThreads, 2) nucleus_select_kernel(cons
                 found.above += more.above;
                 __syncthreads();
                 // the raw maximum may have been a seen column's: the first bucket that holds anything
-                // now stands for it, and what lies above the window
+                // now stands for it
                 uint32_t slot = tid;
                 while (slot < kSlots && m.second[swizzled(slot)] == 0) slot += kNucleusThreads;
                 slot = __reduce_min_sync(kFullMask, min(slot, kSlots));
                 if (lane == 0) atomicMin(&ss.top_slot, slot);
                 __syncthreads();
-                const float above = fmaxf(found.best > window.top ? found.best : -INFINITY, more.best > window.top ? more.best : -INFINITY);
-                const float within = ss.top_slot < kSlots ? window.highest(ss.top_slot) : -INFINITY;
-                if (fmaxf(above, within) > -INFINITY) found.best = fmaxf(above, within);
+                found.best = ss.top_slot < kSlots ? window.highest(ss.top_slot) : -INFINITY;
+                found.outside = fmaxf(found.outside, more.outside);
             }
-            float my_best = found.best;
+            float my_best = fmaxf(found.best, found.outside);
 #pragma unroll
             for (int d = 16; d > 0; d >>= 1) my_best = fmaxf(my_best, __shfl_xor_sync(kFullMask, my_best, d));
             const int lost = __reduce_add_sync(kFullMask, found.lost);
