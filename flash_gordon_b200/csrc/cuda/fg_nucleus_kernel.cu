@@ -30,6 +30,7 @@
 
 #include "fg_block_select.cuh"
 #include "fg_kernels.h"
+#include "fg_nucleus_window.cuh"
 
 namespace fgk {
 
@@ -1000,18 +1001,9 @@ __device__ __noinline__ void sample_the_long_way(NucleusShared &sh, NucleusList 
 // Slots are xor-swizzled inside their group of 32: bf16 values lie a power of two apart and
 // would meet in a few banks otherwise.
 
-constexpr uint32_t kFineSlots = 4096, kMiddleSlots = 2048, kCoarseSlots = 2048;
-constexpr uint32_t kSlots = kFineSlots + kMiddleSlots + kCoarseSlots;
-constexpr uint32_t kGroups = kSlots / 32;      // the slots a warp looks at side by side
-constexpr uint32_t kPlaces = kGroups + 1;      // place 0: the values above the window
-constexpr float kFineScale = 1024.0f, kMiddleScale = 256.0f;
-constexpr float kMagic = 12582912.0f;          // 1.5 * 2^23: adding it rounds to a whole number
-constexpr uint32_t kMagicBits = 0x4b400000u;
 constexpr uint32_t kMostTeam = 8;              // CTAs that may share a row
 constexpr uint32_t kOverCap = 768;             // values above the window that are kept one by one
 constexpr uint32_t kCutCap = 1024, kPickCap = kOrderCap;  // members of the cut's bucket and the draw's
-constexpr float kWindowMargin = 0.5f;          // how far the window reaches above the sample's maximum
-constexpr float kWindowLimit = 3900.0f;        // |v| * 1024 must stay below 2^22
 constexpr int kSamples = 4;                    // logits a thread looks at to place the window
 // Temperatures the short way takes: below, c^3 / T^3 would cost more precision than the rounding
 // it replaces (buckets half as wide take it down to half of the first); above, values under the window would
@@ -1042,78 +1034,6 @@ struct Packing {
     }
     static __device__ __forceinline__ int sum_f(uint32_t first, uint32_t n) { return (int)(first - n * kMagicBits); }
     static __device__ __forceinline__ uint32_t sum_ff(uint32_t second) { return second & ((1u << kCountShift) - 1u); }
-};
-
-// The window of a row: which values have a bucket, and which.
-struct Window {
-    float sharp;                          // 1, or 2 for buckets half as wide
-    float coarse;                         // wide buckets in a unit (times sharp): 64, or 32 to reach further down
-    float top, first_edge, second_edge;   // narrow buckets: [first_edge, top], middle: [second_edge, first_edge),
-    float bottom;                         // wide: [bottom, second_edge)
-    int fine_top, middle_top, coarse_top; // the middle of the topmost bucket of each kind, in widths
-    bool usable;
-
-    __device__ __forceinline__ Window(float reference, float sharp_, float coarse_) : sharp(sharp_), coarse(coarse_) {
-        usable = fabsf(reference) * sharp < kWindowLimit;
-        const float at = usable ? reference * sharp : 0.0f, unit = 1.0f / sharp;  // (sharp: a power of two)
-        const int ratio = (int)(kMiddleScale / coarse);                           // 4 or 8
-        // a kind's lowest bucket begins where the next kind's highest ends
-        const int span = 2 * ratio + 12285;                                       // 4 * (ratio / 2 + 2047.5) + 4095
-        coarse_top = __float2int_rn(((at + kWindowMargin) * kFineScale - (float)span) / (float)(4 * ratio));
-        middle_top = ratio * coarse_top + ratio / 2 + (int)(kMiddleSlots - 1);
-        fine_top = 4 * ratio * coarse_top + span;
-        top = (float)fine_top * (1.0f / kFineScale) * unit;
-        first_edge = ((float)middle_top + 0.5f) * (1.0f / kMiddleScale) * unit;
-        second_edge = ((float)coarse_top + 0.5f) / coarse * unit;
-        bottom = (float)(coarse_top - (int)(kCoarseSlots - 1)) / coarse * unit;
-    }
-    // the bucket of a value in [bottom, top], and its distance from the middle in widths
-    __device__ __forceinline__ uint32_t slot(float v, float &f) const {
-        float scale = coarse * sharp;
-        uint32_t base = kMagicBits + kFineSlots + kMiddleSlots + (uint32_t)coarse_top;
-        if (v >= second_edge) {
-            scale = kMiddleScale * sharp;
-            base = kMagicBits + kFineSlots + (uint32_t)middle_top;
-        }
-        if (v >= first_edge) {
-            scale = kFineScale * sharp;
-            base = kMagicBits + (uint32_t)fine_top;
-        }
-        const float shifted = __fmaf_rn(v, scale, kMagic);
-        f = __fmaf_rn(v, scale, -__fsub_rn(shifted, kMagic));
-        return base - __float_as_uint(shifted);
-    }
-    // a slot's middle in widths, and the width
-    __device__ __forceinline__ int middle_of(uint32_t slot, float &width) const {
-        if (slot < kFineSlots) {
-            width = 1.0f / (kFineScale * sharp);
-            return fine_top - (int)slot;
-        }
-        if (slot < kFineSlots + kMiddleSlots) {
-            width = 1.0f / (kMiddleScale * sharp);
-            return middle_top - (int)(slot - kFineSlots);
-        }
-        width = 1.0f / (coarse * sharp);
-        return coarse_top - (int)(slot - kFineSlots - kMiddleSlots);
-    }
-    __device__ __forceinline__ double middle(uint32_t slot) const {
-        float width;
-        const int n = middle_of(slot, width);
-        return (double)n * (double)width;
-    }
-    // the largest and the smallest value in the slot (half-way between two middles the even one takes it)
-    __device__ __forceinline__ float highest(uint32_t at) const {
-        float width, f;
-        const int n = middle_of(at, width);
-        const float edge = fminf(((float)n + 0.5f) * width, top);
-        return slot(edge, f) == at ? edge : key_to_float(float_key(edge) - 1u);
-    }
-    __device__ __forceinline__ float lowest(uint32_t at) const {
-        float width, f;
-        const int n = middle_of(at, width);
-        const float edge = fmaxf(((float)n - 0.5f) * width, bottom);
-        return slot(edge, f) == at ? edge : key_to_float(float_key(edge) + 1u);
-    }
 };
 
 __device__ __forceinline__ uint32_t swizzled(uint32_t slot) { return slot ^ ((slot >> 5) & 31u); }
@@ -1965,6 +1885,15 @@ __device__ __noinline__ void finish_short(float best, double inv_t, double draw_
     const uint32_t tid = threadIdx.x;
     const Plan plan = ss.plan;
     const uint32_t over = min(ss.over_count, kOverCap);
+    // (the lists hold what the plan has counted, or the row is not this way's to answer)
+    const uint32_t cut_listed = plan.cut == 0 ? over : ss.cut_count;
+    const uint32_t pick_listed = ss.pick_count + (plan.pick_first == 0 ? over : 0u);
+    if (cut_listed != plan.cut_members || pick_listed != plan.pick_members) {
+        __syncthreads();
+        if (tid == 0) ss.plan.verdict = kLongWay;
+        __syncthreads();
+        return;
+    }
     // the ordering's work arrays lie where the buckets were
     OrderWork work;
     work.weight = reinterpret_cast<unsigned long long *>(m.first);

@@ -48,3 +48,19 @@ def test_a_seen_raw_maximum_among_columns_without_another_value(context, rows):
     cfg = SamplerConfig.make(temperature=1.0, top_p=0.999, top_k=0, frequency=1.9)
     w = with_history(logits, cfg, {5: 32}, torch.rand(rows, generator=g).tolist())
     assert_rows_equal(run_gpu(context, w), run_oracle(w), f"{rows} rows")
+
+
+def test_three_ties_around_a_change_of_width(context):
+    """1000 logits each of 5943/1024, 5942/1024 and 5941.75/1024, interleaved, under one of 9.3 that
+    places the window so that the narrow buckets end at 5942/1024, in the middle of the last one."""
+    vocab = 3_001
+    logits = torch.empty(4, vocab)
+    logits[:, 0] = 9.3
+    for i, v in enumerate((5943.0, 5942.0, 5941.75)):
+        logits[:, 1 + i::3] = v / 1024.0
+    cfg = SamplerConfig.make(temperature=1.0, top_p=0.5, top_k=0)
+    w = synth.Workload("ties", logits, [cfg], torch.tensor([0.9, 0.95, 0.97, 0.999]), None, None, 0, allow_no_topk=True)
+    expected = run_oracle(w, want_candidates=True)
+    assert min(c.edge_margin for c in expected[4]) > 1e-9
+    for _ in range(5):
+        assert_rows_equal(run_gpu(context, w), expected, "ties")
