@@ -6,24 +6,24 @@
 // The vocabulary is never sorted.  A row belongs to a team of one, two, four or eight CTAs (a
 // thread-block cluster), each of which takes a range of its columns.
 //
-// The short way.  One pass over the logits counts the values into 16,384 narrow buckets in
-// shared memory.  A bucket holds the number of its members and the first two moments of
+// The short way.  One pass over the logits counts the values into 8,192 buckets of three
+// widths in shared memory.  A bucket holds the number of its members and the first two moments of
 // their distances from its middle, which give its raw and its tempered softmax mass alike
 // (a short series); prefix sums over the buckets' masses tell in which bucket the
 // cumulative mass reaches top_p and, to within a bucket or two, where the draw lands.  A
 // second pass (from L2) gathers the members of those buckets, a few hundred, which are
 // ordered exactly: the element at which top_p is reached, then the element drawn.
 //
-// The long way, for rows the short one cannot take (heavy ties, extreme temperatures): the
-// team's first CTA works on the penalised row in its scratch memory, histogram pass by
-// histogram pass, down to an MSB-first radix descent over the 32-bit monotone value key and,
-// among equal values, over the id.
+// The long way, for rows the short one cannot take (heavy ties, very low temperatures, masses that
+// would not be good enough): the team's first CTA works on the penalised row in scratch memory, histogram
+// pass by histogram pass, down to an MSB-first radix descent over the 32-bit monotone value key
+// and, among equal values, over the id.
 //
 // Masses are exp(s - max) as 2^-44 (the long way: 2^-40) fixed point in 64-bit integers: integer
 // addition is associative, so the result does not depend on the order threads arrive in, and
 // the grid is far below one element's weight.  The reference adds doubles left to right; the two
-// agree unless the top-p bound or the draw falls within ~1e-11 (relative) of an edge of the
-// CDF.
+// agree unless the top-p bound or the draw falls within 1e-10 (relative; as a rule 1e-12) of an edge
+// of the CDF: see the errors measured below.
 #include <cooperative_groups.h>
 
 #include <cstddef>
@@ -972,20 +972,27 @@ __device__ __noinline__ void sample_the_long_way(NucleusShared &sh, NucleusList 
 // With histories the largest part is the seen columns' gather (amend_seen).
 //
 // A value's place: buckets 1/1024 wide over the top four units of the row's window, 1/256 wide over
-// the next eight, 1/64 over the next 32 (1/32 over 64 for temperatures above 1.42; all half as
-// wide for temperatures below 0.36), with their middles on the grid of multiples of the
-// width, so that neither the bucket nor the distance f from its middle depends on a
-// subtraction that rounds: n = rint(v * 1024) by adding and subtracting 1.5 * 2^23,
-// f = v * 1024 - n in [-1/2, 1/2], both exact in fp32.  With w = width * f the members' weights
-// relative to the middle's add up to
+// the next eight, 1/64 over the next 32 (all half as wide for temperatures below 0.36, a quarter as
+// wide below 0.18, and so on), with their middles on the grid of multiples of the width, so that
+// neither the bucket nor the distance f from its middle depends on a subtraction that rounds:
+// n = rint(v * 1024) by adding and subtracting 1.5 * 2^23, f = v * 1024 - n in [-1/2, 1/2], both exact
+// in fp32.  With w = width * f the members' weights relative to the middle's add up to
 //     sum exp(w) = N + c M1 + c^2/2 M2 + c^3/6 M3 + ...,   c = width (times 1/T: tempered)
 // M3 is not kept: f^3 is replaced by the nearest multiple of f (0.15 f over a bucket), which
 // leaves 0.019 c^3/6 (root mean square) of a member's weight: 3e-12 raw and 2.4e-11 at T = 0.5 in
-// the narrow buckets, less in the wider ones relative to the largest weight, against 6.7e-11
-// for weights rounded to 2^-32 of themselves, as they were before.  Largest error of the cumulative masses
-// over their total, rows of 151,936 logits of spread 0.5 to 4 (with and without Gumbel noise), fp32
-// and bf16, against extended precision: T = 0.5 7.5e-11 before, 1.4e-12 now; T = 1 5.8e-11 and
-// 2.0e-12; T = 1.4 3.5e-11 and 2.8e-12.
+// the narrow buckets, against 6.7e-11 for weights rounded to 2^-32 of themselves, but 2e-10 and 1.2e-8 raw in
+// the wider ones.  So make_plan estimates how far off the masses are (place_error), and a row whose bulk
+// lies in wide buckets -- a peak above it placed the window -- is counted again with a window that has
+// its top at the 512th value, those above it being kept one by one.  What lies under a window (a cold
+// row's reaches only 44 units, halved as often as its buckets) counts as an error too.
+//
+// Largest error of the cumulative masses over their total against extended precision, this and weights
+// rounded to 2^-32 (the long way's): rows of 151,936 logits, spread 0.5 to 4 with and without Gumbel
+// noise, one token 6 to 20 above a body, 300 or 2,000 tokens 12 above it, bodies at -4 and -10, each
+// as fp32, bf16 and bf16 widened to fp32:
+//     T      0.2     0.5     1       1.4     2.5
+//     here   2e-11   1e-11   5e-12   2e-11   4e-11
+//     2^-32  7e-11   7e-11   7e-11   7e-11   7e-11
 //
 // A bucket is two 32-bit words that are added to, once each, per member:
 //     first    sum of f in units of 2^-22 (the bits of f * 2^22 + 1.5 * 2^23: the constant's
@@ -993,10 +1000,11 @@ __device__ __noinline__ void sample_the_long_way(NucleusShared &sh, NucleusList 
 //     second   low 22 bits: sum of f^2 in units of 2^-14; high 10 bits: N times an odd number
 //              (what the bits of the constant leave there), so N modulo 1024
 // Neither can overflow up to 1023 members.  A row whose counts do not add up to the number of
-// values counted had a bucket with more (a wrap loses 1024 and nothing can make up for it): it
-// goes the long way.  Rows of raw bf16 logits have at most eight significant bits, f is 0 above
-// 1/8, and many members share a value: they trade precision they have no use for against twelve
-// bits of count.
+// values counted had a bucket with more (a wrap loses 1024 and nothing can make up for it): its
+// window is placed anew or it goes the long way.  Rows of raw bf16 logits have at most eight significant
+// bits, so f is 0 beyond 128 widths from 0, and many members share a value: they trade precision for
+// twelve bits of count.  From 2,049 members at f = +-1/2 on, the sum of f^2 can run into the count there; the
+// total of the counts tells that as well (one carry changes a count by the inverse of the odd number).
 //
 // Slots are xor-swizzled inside their group of 32: bf16 values lie a power of two apart and
 // would meet in a few banks otherwise.
@@ -1005,11 +1013,15 @@ constexpr uint32_t kMostTeam = 8;              // CTAs that may share a row
 constexpr uint32_t kOverCap = 768;             // values above the window that are kept one by one
 constexpr uint32_t kCutCap = 1024, kPickCap = kOrderCap;  // members of the cut's bucket and the draw's
 constexpr int kSamples = 4;                    // logits a thread looks at to place the window
-// Temperatures the short way takes: below, c^3 / T^3 would cost more precision than the rounding
-// it replaces (buckets half as wide take it down to half of the first); above, values under the window would
-// still weigh something.
-constexpr float kWideColdest = 0.36f, kShortColdest = 0.18f, kShortHottest = 2.6f;
-constexpr float kFarColdest = 1.42f;           // up to here 43 units under the maximum weigh less than the grid
+constexpr uint32_t kBodyRank = 512;            // a window that is placed anew leaves that many values above it
+// Buckets are made narrower, halves at a time, until a narrow one is at most 1/369 of the temperature;
+// colder rows than the last go the long way (their window would reach less than 5.5 units down).
+constexpr float kWideColdest = 0.36f, kMostSharp = 8.0f;
+// How far off the cumulative masses may be beyond what weights rounded to 2^-32 of themselves would
+// be, by the estimate of make_plan and as a share of their total: a window that promises more is placed
+// anew, and a row that even then promises more than the second goes the long way.  (Of 2,560 rows of
+// spread 1 to 4 at T = 0.5 to 1.4 two in a thousand are counted again.)
+constexpr double kMassError = 8e-12, kMostMassError = 5e-11;
 
 constexpr uint32_t inverse_mod(uint32_t a, uint32_t modulus) {  // a odd, modulus a power of two
     uint32_t x = 1;
@@ -1020,6 +1032,7 @@ constexpr uint32_t inverse_mod(uint32_t a, uint32_t modulus) {  // a odd, modulu
 // How a bucket's words are packed: rows of raw bf16 logits, all others.
 template <bool kRawBf16>
 struct Packing {
+    static constexpr bool kCoarser = kRawBf16;
     static constexpr int kCountShift = kRawBf16 ? 20 : 22;
     static constexpr uint32_t kCountMask = (1u << (32 - kCountShift)) - 1u;
     static constexpr float kFirstUnit = kRawBf16 ? 1048576.0f : 4194304.0f;  // 2^20, 2^22
@@ -1027,6 +1040,8 @@ struct Packing {
     static constexpr float kSecondMagic = kRawBf16 ? 13631488.0f : kMagic;   // bits 0x4b500000: an odd count field
     static constexpr uint32_t kField = (kRawBf16 ? 0x4b500000u : kMagicBits) >> kCountShift;
     static_assert(kField & 1u, "the count can be read back");
+    // root mean square of f^3 less 0.15 f
+    static constexpr float kThirdError = kRawBf16 ? 0.03f : 0.019f;
     static constexpr uint32_t kInverse = inverse_mod(kField, kCountMask + 1u);
 
     static __device__ __forceinline__ uint32_t count(uint32_t second) {
@@ -1042,10 +1057,11 @@ __device__ __forceinline__ uint32_t swizzled(uint32_t slot) { return slot ^ ((sl
 struct Share {
     float best;          // largest finite value
     uint32_t finite;     // how many are finite
-    uint32_t crowded;    // a bucket had more members than its words take
+    double unseen;       // upper bound of what the values under the window weigh (a share of the largest
+                         // value's weight); infinite: a bucket had more members than its words take
 };
 
-enum Verdict : uint32_t { kDone, kLongWay };
+enum Verdict : uint32_t { kDone, kLongWay, kElsewhere };  // (kElsewhere: with the window placed anew)
 
 // What the team's first CTA has found out: in which buckets the answer lies.
 struct Plan {
@@ -1056,6 +1072,7 @@ struct Plan {
     uint32_t cut_rank_before, cut_members;
     unsigned long long pick_before;
     uint32_t pick_members;
+    float reference;              // where the window goes next, if the verdict is kElsewhere
 };
 
 // Result of looking for a crossing among the 32 slots of a group.
@@ -1073,9 +1090,11 @@ struct ShortShared {
     uint32_t seen_count;                          // seen columns of this CTA
     uint32_t top_slot;                            // the first bucket that holds anything
     uint32_t cut_place, pick_place[2];
-    float sample_max[kNucleusWarps];
+    float sample_max[kNucleusWarps], sample_next[kNucleusWarps];
     unsigned long long scan_raw[kNucleusWarps], scan_tempered[kNucleusWarps];
     uint32_t scan_count[kNucleusWarps];
+    float raw_error[kNucleusWarps], tempered_error[kNucleusWarps];
+    uint32_t poor;                                // the masses are not good enough
 };
 
 // Dynamic shared memory of the kernel: two CTAs' worth fit an SM.  The long way's memory lies over
@@ -1227,8 +1246,7 @@ __device__ __forceinline__ float pick_element(const float (&v)[kPer], int j) {
 
 // What a pass over one CTA's columns finds out beside the buckets.
 struct Findings {
-    float best;                     // largest value inside the window
-    float outside;                  // largest finite one outside (a seen id's raw logit is none)
+    float best;                     // largest finite value; with penalties, of those outside the window
     int lost, below, above;         // not finite, under the window, over it
 };
 
@@ -1246,14 +1264,14 @@ struct SeenBits {
 
 // The first pass over one CTA's columns: counts into the buckets, values above the window onto
 // the first CTA's list.
-template <class P>
+template <class P, bool kPenalised>
 struct Counter {
     const Window window;
     const Team team;
     Findings found;
 
     __device__ __forceinline__ Counter(const Window &w, const Team &team_) : window(w), team(team_) {
-        found.best = found.outside = -INFINITY;
+        found.best = -INFINITY;
         found.lost = found.below = found.above = 0;
     }
     // a value inside the window
@@ -1275,7 +1293,7 @@ struct Counter {
             low = fminf(low, v[j]);
         }
         if (high <= window.top && low >= window.bottom) {
-            found.best = fmaxf(found.best, high);
+            if (!kPenalised) found.best = fmaxf(found.best, high);
 #pragma unroll
             for (int j = 0; j < kPer; j++) count(v[j]);
         } else {
@@ -1286,7 +1304,7 @@ struct Counter {
     // `skip`: columns whose value outside the window is not the row's (a seen id's raw logit)
     __device__ __forceinline__ void take(float v, uint32_t column, const SeenBits &skip) {
         if (v >= window.bottom && v <= window.top) {
-            found.best = fmaxf(found.best, v);
+            if (!kPenalised) found.best = fmaxf(found.best, v);
             count(v);
         } else if (is_nonfinite(v)) {
             found.lost++;
@@ -1295,7 +1313,7 @@ struct Counter {
                 ShortMemory &m = short_memory();
                 found.above++;
                 if (skip.test(column)) return;
-                found.outside = fmaxf(found.outside, v);
+                found.best = fmaxf(found.best, v);
                 const uint32_t slot = atomicAdd(team.at(&m.state.over_count, 0), 1u);
                 if (slot < kOverCap) {
                     team.at(m.over_value, 0)[slot] = v;
@@ -1303,7 +1321,7 @@ struct Counter {
                 }
             } else {
                 found.below++;
-                if (v > found.outside && !skip.test(column)) found.outside = v;
+                if (v > found.best && !skip.test(column)) found.best = v;
             }
         }
     }
@@ -1328,10 +1346,10 @@ struct Counter {
     }
 };
 
-template <typename T, class P>
+template <typename T, class P, bool kPenalised>
 __device__ __noinline__ Findings count_logits(const T *columns, uint32_t lo, uint32_t n, const Window window,
                                               const Team team, const SeenBits seen) {
-    Counter<P> counter(window, team);
+    Counter<P, kPenalised> counter(window, team);
     walk_logits<T>(
         columns + lo, n,
         [&](const float (&v)[Vector<T>::kPer], uint32_t c) { counter.take_vector(v, lo + c, seen); },
@@ -1424,12 +1442,37 @@ __device__ __forceinline__ void visit_seen(const NucleusParams &p, uint32_t row,
     }
 }
 
+// Largest value under `bottom` among the CTA's columns, raw or (the `listed` seen ones) penalised:
+// a seen column's raw logit may be the one.  All threads call.
+template <typename T>
+__device__ __noinline__ float largest_under(const T *columns, uint32_t lo, uint32_t n, float bottom, const float2 *seen,
+                                            uint32_t listed) {
+    ShortShared &ss = short_memory().state;
+    float best = __uint_as_float(0xff800000u);
+    auto look = [&](float v) { best = v < bottom ? fmaxf(best, v) : best; };
+    walk_logits<T>(
+        columns + lo, n,
+        [&](const float (&v)[Vector<T>::kPer], uint32_t) {
+#pragma unroll
+            for (int j = 0; j < Vector<T>::kPer; j++) look(v[j]);
+        },
+        [&](float v, uint32_t) { look(v); });
+    for (uint32_t i = threadIdx.x; i < listed; i += kNucleusThreads) look(seen[i].x);
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) best = fmaxf(best, __shfl_xor_sync(kFullMask, best, d));
+    __syncthreads();
+    if (lane_id() == 0) ss.sample_max[threadIdx.x >> 5] = best;
+    __syncthreads();
+    for (uint32_t w = 0; w < (uint32_t)kNucleusWarps; w++) best = fmaxf(best, ss.sample_max[w]);
+    return best;
+}
+
 // After the raw logits have been counted: every seen column's raw value is taken back and its
 // penalised value counted instead, and kept with its column for the second pass.
 template <typename T, class P>
 __device__ __noinline__ Findings amend_seen(const NucleusParams &p, uint32_t row, const SamplerConfig cfg, uint32_t lo,
                                             uint32_t n, float2 *seen, const Window window, const Team team) {
-    Counter<P> counter(window, team);
+    Counter<P, true> counter(window, team);
     const SeenBits all_listed = {nullptr, 0, 1};
     visit_seen<T>(p, row, cfg, lo, n, [&](uint32_t column, float raw, float penalised, uint32_t slot) {
         if (fmaxf(raw, penalised) <= window.top && fminf(raw, penalised) >= window.bottom && raw == raw && penalised == penalised) {
@@ -1636,18 +1679,58 @@ __device__ __forceinline__ unsigned long long draw_target_of(double draw_at, uns
     return (unsigned long long)floor(draw_at * (double)total);
 }
 
-// The first CTA adds the team's masses up and finds the buckets the answer lies in.  All its
-// threads call; ends synced.
+// The window goes where all but a few hundred values lie under its top, those above it being kept
+// one by one.  First CTA, with the running sums of the counts; all its threads call.
+__device__ __noinline__ void place_anew(const Window window, bool sensible) {
+    Plan &plan = short_memory().state.plan;
+    const uint32_t tid = threadIdx.x;
+    const uint32_t places = __syncthreads_count(tid < kPlaces && short_memory().count[tid] <= kBodyRank);  // (the first ones)
+    if (tid == 0) {
+        float top = window.top;
+        if (places > 0 && places < kPlaces) top = window.highest((places - 1) * 32u);
+        plan.reference = top - kWindowMargin / window.sharp;
+        plan.verdict = sensible ? kElsewhere : kLongWay;
+    }
+    __syncthreads();
+}
+
+// What a place (not the first) adds to the square of the masses' error, less what weights rounded to
+// 2^-32 of themselves would: its members are off independently of one another, each by its weight
+// times the error of a bucket that is c wide.  `mass`: its running sums over the places.  `middle`:
+// that of the place's first bucket, in widths -- raw bf16 values have at most eight significant bits
+// and lie on their bucket's middle unless they are within 128 widths of 0.  (A row's largest weight
+// is no rounded one, and is left out.)
+template <class P>
+__device__ __forceinline__ float place_error(uint32_t place, float c, int middle, const unsigned long long *mass, float largest) {
+    constexpr float kSecond = 0.5f * 0x1p-14f * 0.28867513f, kThird = P::kThirdError / 6.0f, kWeight = 0x1p-32f * 0.28867513f;
+    const uint32_t *counts = short_memory().count;
+    const uint32_t before = place ? counts[place - 1] : 0u, count = counts[place] - before;
+    const float weight = __ull2float_rn(mass[place] - (place ? mass[place - 1] : 0ull));
+    const float second = c * c * kSecond, third = c * c * c * kThird;
+    const bool exact = P::kCoarser && (middle < -128 || middle > 128 + 31);
+    const float off = count && !exact ? (second * second + third * third) * weight * weight / (float)count : 0.0f;
+    const float others = before ? weight : weight - largest, rest = (float)(before ? count : count - 1u);
+    return off - (others > 0.0f && rest > 0.0f ? kWeight * kWeight * others * others / rest : 0.0f);
+}
+__device__ __forceinline__ float warp_sum(float v) {
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(kFullMask, v, d);
+    return v;
+}
+
+// The first CTA adds the team's masses up and finds the buckets the answer lies in.  `error`: how
+// far off the masses may be.  All its threads call; ends synced.
 template <class P>
 __device__ __noinline__ void make_plan(const Team team, const Window window, float best, double top_p, double inv_t,
-                                       double draw_at, int bits) {
+                                       double draw_at, int bits, double error) {
     ShortMemory &m = short_memory();
     ShortShared &ss = m.state;
     const NucleusShared &sh = m.scan;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t over = min(ss.over_count, kOverCap);
-    bool crowded = false;
-    for (uint32_t r = 0; r < team.size; r++) crowded = crowded || team.at(&ss.share, r)->crowded != 0;
+    double unseen = 0.0;
+    for (uint32_t r = 0; r < team.size; r++) unseen += team.at(&ss.share, r)->unseen;
+    const bool crowded = !(unseen < INFINITY);
     // place 0: the values above the window, each with its own weights
     if (warp == kNucleusWarps - 1) {
         unsigned long long raw = 0, tempered = 0;
@@ -1724,11 +1807,27 @@ __device__ __noinline__ void make_plan(const Team team, const Window window, flo
     }
     __syncthreads();
     if (crowded || total_raw == 0) {
-        if (tid == 0) ss.plan.verdict = kLongWay;
-        __syncthreads();
+        place_anew(window, crowded && !P::kCoarser);  // (the other packing takes fewer members)
         return;
     }
     const uint32_t cut_place = ss.cut_place;
+    constexpr uint32_t kErrorWarp = 2, kErrorWarps = kScanWarps;
+    static_assert(kErrorWarp + kErrorWarps <= (uint32_t)kNucleusWarps, "a thread per place beside the warps that look for slots");
+    if (warp >= kErrorWarp && warp < kErrorWarp + kErrorWarps) {
+        // meanwhile: how far off are the masses?
+        const uint32_t place = (warp - kErrorWarp) * 32 + lane;
+        const float largest = (float)(1ull << bits);
+        float width = 0.0f, raw_error = 0.0f, tempered_error = 0.0f;
+        const int middle = place != 0 ? window.middle_of((place - 1) * 32u, width) : 0;
+        if (place < kPlaces) raw_error = place_error<P>(place, width, middle, m.raw, largest);
+        if (place <= cut_place) tempered_error = place_error<P>(place, width * (float)inv_t, middle, m.tempered, largest);
+        raw_error = warp_sum(raw_error);
+        tempered_error = warp_sum(tempered_error);
+        if (lane == 0) {
+            ss.raw_error[warp - kErrorWarp] = raw_error;
+            ss.tempered_error[warp - kErrorWarp] = tempered_error;
+        }
+    }
     if (warp == 0) {
         SlotHit cut;
         cut.slot = 0;
@@ -1763,6 +1862,22 @@ __device__ __noinline__ void make_plan(const Team team, const Window window, flo
     __syncthreads();
     __shared__ uint32_t ends[2], ends_count[2];
     __shared__ unsigned long long ends_before;
+    if (warp == 2) {
+        // Are the masses good enough?  (Squares are compared; the nucleus weighs `most`, tempered.
+        // Values of raw bf16 rows tie, and ties are off by the same.)
+        float raw_off = 0.0f, tempered_off = 0.0f;
+#pragma unroll
+        for (uint32_t w = 0; w < kErrorWarps; w++) {
+            raw_off += ss.raw_error[w];
+            tempered_off += ss.tempered_error[w];
+        }
+        if (P::kCoarser) error *= 0.25;
+        const double raw_allowed = error * (double)total_raw, tempered_allowed = error * (double)most;
+        if (lane == 0)
+            ss.poor = (double)raw_off > raw_allowed * raw_allowed ||
+                      (double)tempered_off > tempered_allowed * tempered_allowed ||
+                      unseen * (double)(1ull << bits) > raw_allowed;
+    }
     if (warp < 2) {
         const uint32_t place = ss.pick_place[warp];
         const unsigned long long target = warp == 0 ? target_first : target_last;
@@ -1787,6 +1902,10 @@ __device__ __noinline__ void make_plan(const Team team, const Window window, flo
         }
     }
     __syncthreads();
+    if (ss.poor) {
+        place_anew(window, true);
+        return;
+    }
     if (tid == 0) {
         ss.plan.pick_first = ends[0];
         ss.plan.pick_last = ends[1];
@@ -1956,13 +2075,13 @@ template <typename T, class P>
 __device__ __forceinline__ uint32_t locate_and_pick(const NucleusParams &p, const Team &team, const Window &window,
                                                     uint32_t row, uint32_t lo, uint32_t n, uint32_t counted,
                                                     const SeenBits &bits, const float2 *seen, float best, double top_p,
-                                                    double inv_t, double draw_at) {
+                                                    double inv_t, double draw_at, double error) {
     ShortShared &ss = short_memory().state;
     const int grid = p.vocab <= kFinestVocab ? 44 : 40;
     group_masses<P>(window, (double)best, inv_t, grid);
-    if (threadIdx.x == 0) ss.share.crowded = ss.counted != counted;
+    if (threadIdx.x == 0 && ss.counted != counted) ss.share.unseen = INFINITY;
     team.sync();
-    if (team.rank == 0) make_plan<P>(team, window, best, top_p, inv_t, draw_at, grid);
+    if (team.rank == 0) make_plan<P>(team, window, best, top_p, inv_t, draw_at, grid, error);
     team.sync();
     if (team.at(&ss.plan, 0)->verdict == kDone) {
         gather_members<T>(static_cast<const T *>(p.logits) + (size_t)row * p.row_stride, lo, n, window, team, bits, seen,
@@ -1975,26 +2094,42 @@ __device__ __forceinline__ uint32_t locate_and_pick(const NucleusParams &p, cons
 }
 
 // The largest of a few logits spread evenly over the row, NaN, infinities and seen columns left
-// out (so that the row's own maximum is no smaller): where the window goes.  All threads call.
+// out (so that the row's own maximum is no smaller): where the window goes.  The second largest if
+// the largest is a peak as far above it as the narrow buckets reach: the bulk of the row would be left to
+// wide ones.  All threads call.
+struct TopTwo {
+    float first, second;
+    __device__ __forceinline__ void join(float a, float b) {  // (a >= b)
+        second = fmaxf(fminf(first, a), fmaxf(second, b));
+        first = fmaxf(first, a);
+    }
+};
 template <typename T>
-__device__ __forceinline__ float sample_row(const T *columns, uint32_t vocab, const SeenBits &seen) {
+__device__ __forceinline__ float sample_row(const T *columns, uint32_t vocab, const SeenBits &seen, float sharp) {
     ShortShared &ss = short_memory().state;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    float best = __uint_as_float(0xff800000u);
+    const float none = __uint_as_float(0xff800000u);
+    TopTwo best = {none, none};
 #pragma unroll
     for (int j = 0; j < kSamples; j++) {
         const uint32_t at = (uint32_t)(((uint64_t)(j * kNucleusThreads + tid) * vocab) / (kSamples * kNucleusThreads));
         const float v = Vector<T>::one(columns + at);
-        if (!is_nonfinite(v) && !seen.test(at)) best = fmaxf(best, v);
+        if (!is_nonfinite(v) && !seen.test(at)) best.join(v, none);
     }
 #pragma unroll
-    for (int d = 16; d > 0; d >>= 1) best = fmaxf(best, __shfl_xor_sync(kFullMask, best, d));
-    if (lane == 0) ss.sample_max[warp] = best;
+    for (int d = 16; d > 0; d >>= 1)
+        best.join(__shfl_xor_sync(kFullMask, best.first, d), __shfl_xor_sync(kFullMask, best.second, d));
+    if (lane == 0) {
+        ss.sample_max[warp] = best.first;
+        ss.sample_next[warp] = best.second;
+    }
     __syncthreads();
-    best = ss.sample_max[lane % kNucleusWarps];
+    best = {ss.sample_max[lane % kNucleusWarps], ss.sample_next[lane % kNucleusWarps]};
 #pragma unroll
-    for (int d = kNucleusWarps / 2; d > 0; d >>= 1) best = fmaxf(best, __shfl_xor_sync(kFullMask, best, d));
-    return best;
+    for (int d = kNucleusWarps / 2; d > 0; d >>= 1)
+        best.join(__shfl_xor_sync(kFullMask, best.first, d), __shfl_xor_sync(kFullMask, best.second, d));
+    const float reach = (float)kFineSlots / (kFineScale * sharp);
+    return best.second > none && best.first - best.second > reach ? best.second : best.first;
 }
 
 template <typename T>
@@ -2050,14 +2185,18 @@ __global__ void __launch_bounds__(kNucleusThreads, 2) nucleus_select_kernel(cons
         // (as many structures as splits in a row, one after the other)
         const SeenBits bits = {penalised ? p.history_global + (size_t)row * p.splits * p.history_stride_words : nullptr,
                                p.history_stride_words, p.split_len};
-        bool counting = cfg.temperature >= kShortColdest && cfg.temperature <= kShortHottest;
+        float sharp = 1.0f;
+        while (cfg.temperature * sharp < kWideColdest && sharp <= kMostSharp) sharp *= 2.0f;
+        const bool counting = sharp <= kMostSharp;
         uint32_t finite = 1, verdict = kLongWay;
         float reference = 0.0f;
-        if (counting) reference = sample_row(columns, p.vocab, bits);
+        if (counting) reference = sample_row(columns, p.vocab, bits, sharp);
         if (is_nonfinite(reference)) reference = 0.0f;  // (nothing finite among the samples: any window will do)
-        for (uint32_t attempt = 0; counting; attempt++) {
-            const Window window(reference, cfg.temperature < kWideColdest ? 2.0f : 1.0f,
-                                cfg.temperature <= kFarColdest ? 64.0f : 32.0f);
+        // The window is placed by the sample; if that said little, by the true maximum; if the masses
+        // it gives are not good enough, by the bulk of the values.
+        bool by_sample = true, by_bulk = false;
+        while (counting) {
+            const Window window(reference, sharp);
             if (!window.usable) break;
             uint4 *words = reinterpret_cast<uint4 *>(m.first);
             for (uint32_t i = tid; i < 2 * kSlots / 4; i += kNucleusThreads) words[i] = make_uint4(0, 0, 0, 0);
@@ -2068,8 +2207,10 @@ __global__ void __launch_bounds__(kNucleusThreads, 2) nucleus_select_kernel(cons
             }
             __syncthreads();
             // ---- first pass ----
-            Findings found = penalised ? count_logits<T, Packing<false>>(columns, lo, n, window, team, bits)
-                                       : count_logits<T, Packing<kBf16>>(columns, lo, n, window, team, bits);
+            const bool raw_form = kBf16 && !penalised;
+            Findings found = penalised  ? count_logits<T, Packing<false>, true>(columns, lo, n, window, team, bits)
+                             : raw_form ? count_logits<T, Packing<kBf16>, false>(columns, lo, n, window, team, bits)
+                                        : count_logits<T, Packing<false>, false>(columns, lo, n, window, team, bits);
             if (penalised) {
                 __syncthreads();
                 const Findings more = amend_seen<T, Packing<false>>(p, row, cfg, lo, n, seen, window, team);
@@ -2084,10 +2225,10 @@ __global__ void __launch_bounds__(kNucleusThreads, 2) nucleus_select_kernel(cons
                 slot = __reduce_min_sync(kFullMask, min(slot, kSlots));
                 if (lane == 0) atomicMin(&ss.top_slot, slot);
                 __syncthreads();
-                found.best = ss.top_slot < kSlots ? window.highest(ss.top_slot) : -INFINITY;
-                found.outside = fmaxf(found.outside, more.outside);
+                found.best = fmaxf(found.best, more.best);
+                if (ss.top_slot < kSlots) found.best = fmaxf(found.best, window.highest(ss.top_slot));
             }
-            float my_best = fmaxf(found.best, found.outside);
+            float my_best = found.best;
 #pragma unroll
             for (int d = 16; d > 0; d >>= 1) my_best = fmaxf(my_best, __shfl_xor_sync(kFullMask, my_best, d));
             const int lost = __reduce_add_sync(kFullMask, found.lost);
@@ -2106,8 +2247,8 @@ __global__ void __launch_bounds__(kNucleusThreads, 2) nucleus_select_kernel(cons
                 for (int d = kNucleusWarps / 2; d > 0; d >>= 1) my_best = fmaxf(my_best, __shfl_xor_sync(kFullMask, my_best, d));
                 if (lane == 0) {
                     ss.share.best = my_best;
+                    ss.share.unseen = 0.0;
                     ss.share.finite = n - (uint32_t)ss.lost;
-                    ss.share.crowded = 0;
                 }
             }
             const uint32_t counted = n - (uint32_t)(ss.lost + ss.below + ss.above);
@@ -2121,20 +2262,34 @@ __global__ void __launch_bounds__(kNucleusThreads, 2) nucleus_select_kernel(cons
             }
             const uint32_t over = *team.at(&ss.over_count, 0);
             if (finite == 0) break;
-            if (attempt == 0 && (over > kOverCap || best < reference)) {
+            if (by_sample && !by_bulk && (over > kOverCap || best < reference)) {
                 // the sample said little: the window once more, from the true maximum
                 team.sync();
                 if (tid == 0) ss.over_count = 0;
                 reference = best;
+                by_sample = false;
                 team.sync();
                 continue;
             }
-            if (over <= kOverCap)
-                verdict = penalised ? locate_and_pick<T, Packing<false>>(p, team, window, row, lo, n, counted, bits, seen,
-                                                                         best, top_p, inv_t, draw_at)
-                                    : locate_and_pick<T, Packing<kBf16>>(p, team, window, row, lo, n, counted, bits, seen,
-                                                                         best, top_p, inv_t, draw_at);
-            break;
+            if (over > kOverCap) break;
+            if (sharp > 1.0f && ss.below > 0) {
+                // (a window of more than 40 units needs no look at what lies under it)
+                const float under = largest_under<T>(columns, lo, n, window.bottom, seen, ss.seen_count);
+                if (tid == 0) ss.share.unseen = (double)ss.below * exp((double)under - (double)best);
+            }
+            const double error = by_bulk ? kMostMassError : kMassError;
+            verdict = raw_form ? locate_and_pick<T, Packing<kBf16>>(p, team, window, row, lo, n, counted, bits, seen, best,
+                                                                    top_p, inv_t, draw_at, error)
+                               : locate_and_pick<T, Packing<false>>(p, team, window, row, lo, n, counted, bits, seen, best,
+                                                                    top_p, inv_t, draw_at, error);
+            if (verdict != kElsewhere || by_bulk) break;
+            const float elsewhere = team.at(&ss.plan, 0)->reference;
+            if (elsewhere >= reference) break;
+            reference = elsewhere;
+            by_bulk = true;
+            team.sync();
+            if (tid == 0) ss.over_count = ss.cut_count = ss.pick_count = 0;
+            team.sync();
         }
         if (finite == 0) {
             // src/sampler.c:97 "sampler received no finite candidates"
@@ -2142,7 +2297,7 @@ __global__ void __launch_bounds__(kNucleusThreads, 2) nucleus_select_kernel(cons
                 report_row(p.out, row, kErrFormat, kPaddingId, 0.0f);
                 if (p.out.dbg_count) p.out.dbg_count[row] = 0;
             }
-        } else if (verdict == kLongWay) {
+        } else if (verdict != kDone) {
             if (tid == 0) ss.seen_count = 0;
             __syncthreads();
             write_scratch<T>(p, row, cfg, lo, n, penalised, values);

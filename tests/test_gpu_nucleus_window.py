@@ -64,3 +64,63 @@ def test_three_ties_around_a_change_of_width(context):
     assert min(c.edge_margin for c in expected[4]) > 1e-9
     for _ in range(5):
         assert_rows_equal(run_gpu(context, w), expected, "ties")
+
+
+def rows_like(kind, rows, vocab, seed):
+    g = torch.Generator().manual_seed(seed)
+    x = torch.randn(rows, vocab, generator=g)
+    if kind == "peak":           # one token far above the body: a sample of the row finds it or not
+        x[0::2, 0] = 13.3
+        x[1::2, 5] = 13.3
+    elif kind == "two peaks":    # ... and its neighbour in the sample
+        x[:, 0] = 14.0
+        x[:, vocab // 2] = 13.0
+    elif kind == "far peak":
+        x[:, 0] = 20.5
+    elif kind == "hill":         # thousands of values above the body
+        x[:, 7:2_007] = 12.0 + x[:, 7:2_007]
+    elif kind == "offset":       # a head whose logits are not centred
+        x = x * 1.5 - 4.0
+        x[:, ::501] += 9.0
+    return x
+
+
+def sizes_and_tokens_agree(context, w, least_margin=1e-10):
+    """Tokens, and the sizes of the nuclei, of the rows whose top_p and draw lie `least_margin` off
+    every edge of the cumulative distribution."""
+    expected = run_oracle(w, want_candidates=True)
+    clear = np.array([c.edge_margin for c in expected[4]]) > least_margin
+    assert clear.mean() > 0.5
+    result = run_gpu(context, w, debug=True)
+    sizes = np.array([c.nucleus for c in expected[4]])
+    assert np.array_equal(as_u32(result.row_status), expected[3])
+    assert np.array_equal(as_u32(result.tokens)[clear], expected[1][clear])
+    assert np.array_equal(as_u32(result.debug["count"])[clear], sizes[clear])
+
+
+@pytest.mark.parametrize("form", ["f32", "widened", "bf16"])
+@pytest.mark.parametrize("kind", ["peak", "two peaks", "far peak", "hill", "offset"])
+@pytest.mark.parametrize("rows,vocab,temperature,top_p", [
+    (2, 151_936, 1.0, 0.9), (34, 100_277, 2.0, 0.9), (150, 20_001, 0.5, 0.8), (3, 151_936, 0.3, 0.999_9), (2, 60_000, 0.2, 0.99),
+    (2, 151_936, 0.1, 0.95), (2, 60_000, 0.05, 0.9), (2, 60_000, 0.04, 0.9), (3, 100_277, 5.0, 0.9),
+])
+def test_windows_that_are_placed_anew(context, kind, form, rows, vocab, temperature, top_p):
+    x = rows_like(kind, rows, vocab, rows + vocab)
+    x = x.bfloat16() if form == "bf16" else x.bfloat16().float() if form == "widened" else x
+    cfg = SamplerConfig.make(temperature=temperature, top_p=top_p, top_k=0)
+    uniforms = torch.rand(rows, generator=torch.Generator().manual_seed(1))
+    w = synth.Workload(kind, x, [cfg], uniforms, None, None, 0, allow_no_topk=True)
+    sizes_and_tokens_agree(context, w)
+
+
+@pytest.mark.parametrize("form", ["f32", "bf16"])
+def test_what_lies_under_a_cold_row_s_window_is_not_forgotten(context, form):
+    """The lower part of a body 20 below the top weighs 7e-6 of a row of 151,936, each of its values
+    about 1e-9: that decides how many values top_p takes in.  (Masses on a grid of 2^-44, 8,192 of
+    them: about 1.5e-12.)"""
+    vocab = 151_936
+    x = rows_like("far peak", 4, vocab, 3)
+    x = x.bfloat16() if form == "bf16" else x
+    configs = [SamplerConfig.make(temperature=0.2, top_p=1.0 - k * 2.0 ** -24, top_k=0) for k in (100, 1_000, 3_000, 5_000)]
+    w = synth.Workload("under", x, configs, torch.tensor([0.1, 0.5, 0.9, 0.3]), None, None, 0, allow_no_topk=True)
+    sizes_and_tokens_agree(context, w, 2e-11)
