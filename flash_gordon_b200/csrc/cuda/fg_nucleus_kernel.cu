@@ -991,8 +991,8 @@ __device__ __noinline__ void sample_the_long_way(NucleusShared &sh, NucleusList 
 // noise, one token 6 to 20 above a body, 300 or 2,000 tokens 12 above it, bodies at -4 and -10, each
 // as fp32, bf16 and bf16 widened to fp32:
 //     T      0.2     0.5     1       1.4     2.5
-//     here   2e-11   1e-11   5e-12   2e-11   4e-11
-//     2^-32  7e-11   7e-11   7e-11   7e-11   7e-11
+//     here   1e-11   2e-11   9e-12   3e-11   5e-11
+//     2^-32  7e-11   7e-11   7e-11   7e-11   6e-11
 //
 // A bucket is two 32-bit words that are added to, once each, per member:
 //     first    sum of f in units of 2^-22 (the bits of f * 2^22 + 1.5 * 2^23: the constant's
@@ -1013,15 +1013,19 @@ constexpr uint32_t kMostTeam = 8;              // CTAs that may share a row
 constexpr uint32_t kOverCap = 768;             // values above the window that are kept one by one
 constexpr uint32_t kCutCap = 1024, kPickCap = kOrderCap;  // members of the cut's bucket and the draw's
 constexpr int kSamples = 4;                    // logits a thread looks at to place the window
+constexpr float kPeak = 1.5f;                  // the largest of them is left out if it is that far above the next
 constexpr uint32_t kBodyRank = 512;            // a window that is placed anew leaves that many values above it
 // Buckets are made narrower, halves at a time, until a narrow one is at most 1/369 of the temperature;
 // colder rows than the last go the long way (their window would reach less than 5.5 units down).
 constexpr float kWideColdest = 0.36f, kMostSharp = 8.0f;
 // How far off the cumulative masses may be beyond what weights rounded to 2^-32 of themselves would
 // be, by the estimate of make_plan and as a share of their total: a window that promises more is placed
-// anew, and a row that even then promises more than the second goes the long way.  (Of 2,560 rows of
-// spread 1 to 4 at T = 0.5 to 1.4 two in a thousand are counted again.)
-constexpr double kMassError = 8e-12, kMostMassError = 5e-11;
+// anew, and a row that even then promises more than the second goes the long way.  (The estimate is
+// up to seven times what is found, where few members decide, and down to a twentieth of it for raw bf16
+// rows, whose values tie: they are held to a twentieth.  At 8e-12 two rows in a hundred of 38,016 logits
+// of spread 3.8 with Gumbel noise, T = 0.54, were counted twice, 75 us instead of 39, for errors of
+// 1e-11; at 4e-11 none, and the errors above are the same.)
+constexpr double kMassError = 4e-11, kMostMassError = 6e-11;
 
 constexpr uint32_t inverse_mod(uint32_t a, uint32_t modulus) {  // a odd, modulus a power of two
     uint32_t x = 1;
@@ -1871,7 +1875,7 @@ __device__ __noinline__ void make_plan(const Team team, const Window window, flo
             raw_off += ss.raw_error[w];
             tempered_off += ss.tempered_error[w];
         }
-        if (P::kCoarser) error *= 0.25;
+        if (P::kCoarser) error *= 0.05;
         const double raw_allowed = error * (double)total_raw, tempered_allowed = error * (double)most;
         if (lane == 0)
             ss.poor = (double)raw_off > raw_allowed * raw_allowed ||
@@ -2095,8 +2099,10 @@ __device__ __forceinline__ uint32_t locate_and_pick(const NucleusParams &p, cons
 
 // The largest of a few logits spread evenly over the row, NaN, infinities and seen columns left
 // out (so that the row's own maximum is no smaller): where the window goes.  The second largest if
-// the largest is a peak as far above it as the narrow buckets reach: the bulk of the row would be left to
-// wide ones.  All threads call.
+// the largest is a peak well above it, which would leave the bulk of the row to wide buckets.  (With the
+// largest, or peaks of 4 units as the limit, the masses of 1 to 3 % of the rows whose maximum is in the
+// sample are estimated to be off by more than 1e-11; with this of none of 1,440.)
+// All threads call.
 struct TopTwo {
     float first, second;
     __device__ __forceinline__ void join(float a, float b) {  // (a >= b)
@@ -2128,8 +2134,7 @@ __device__ __forceinline__ float sample_row(const T *columns, uint32_t vocab, co
 #pragma unroll
     for (int d = kNucleusWarps / 2; d > 0; d >>= 1)
         best.join(__shfl_xor_sync(kFullMask, best.first, d), __shfl_xor_sync(kFullMask, best.second, d));
-    const float reach = (float)kFineSlots / (kFineScale * sharp);
-    return best.second > none && best.first - best.second > reach ? best.second : best.first;
+    return best.second > none && (best.first - best.second) * sharp > kPeak ? best.second : best.first;
 }
 
 template <typename T>
