@@ -15,7 +15,7 @@
 // ordered exactly: the element at which top_p is reached, then the element drawn.
 //
 // The long way, for rows the short one cannot take (heavy ties, very low temperatures, masses that
-// would not be good enough): the team's first CTA works on the penalised row in scratch memory, histogram
+// would not be good enough): the CTAs of the team work on the penalised row in scratch memory, histogram
 // pass by histogram pass, down to an MSB-first radix descent over the 32-bit monotone value key
 // and, among equal values, over the id.
 //
@@ -37,9 +37,7 @@ namespace fgk {
 
 constexpr int kNucleusThreads = 512;  // two CTAs to an SM: one streams while the other scans and sorts
 constexpr int kNucleusWarps = kNucleusThreads / 32;
-constexpr int kBuckets = 4096;
-// per bucket: two masses (raw and tempered weights) and a count
-constexpr size_t kNucleusHistogramBytes = kBuckets * (2 * sizeof(unsigned long long) + sizeof(uint32_t));
+constexpr int kBuckets = 4096;  // of the long way
 
 struct NucleusParams {
     const void *logits;
@@ -64,9 +62,8 @@ struct NucleusParams {
 };
 
 struct NucleusShared {
-    unsigned long long *mass;         // kBuckets entries, dynamic shared memory: the masses a crossing search walks
-    unsigned long long *other_mass;   // kBuckets entries: the tempered masses while `mass` holds the raw ones
-    uint32_t *count;                  // kBuckets entries
+    unsigned long long *mass;         // the long way's kBuckets masses and counts
+    uint32_t *count;
     double table[64];                 // 2^(j/64)
     unsigned long long scan_mass[kNucleusWarps];
     uint32_t scan_count[kNucleusWarps];
@@ -171,37 +168,42 @@ __device__ __forceinline__ void clear_histogram(NucleusShared &sh, uint32_t buck
     __syncthreads();
 }
 
-// Walks the scratch row: visit(value, index) for every element.  Eight values per thread
-// are in flight (two 128-bit loads) before the first is used: with one scalar load per
-// trip a pass over the row was a chain of L2 latencies.  Rows start 16-byte aligned.
+// Walks a scratch row: visit(value, index) for every element.  The next two quads of a thread are on
+// their way while it looks at two: a pass over the row is a chain of L2 latencies otherwise.  Rows
+// start 16-byte aligned.
 template <class Visit>
 __device__ __forceinline__ void walk_row(const float *values, uint32_t vocab, Visit visit) {
-    const uint32_t tid = threadIdx.x;
     const float4 *wide = reinterpret_cast<const float4 *>(values);
-    const uint32_t quads = vocab / 4u;
+    const uint32_t tid = threadIdx.x, quads = vocab / 4u;
+    auto visit_quad = [&](const float4 &v, uint32_t i) {
+        visit(v.x, i);
+        visit(v.y, i + 1u);
+        visit(v.z, i + 2u);
+        visit(v.w, i + 3u);
+    };
+    float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), b = a;
     uint32_t q = tid;
-    for (; q + kNucleusThreads < quads; q += 2 * kNucleusThreads) {
-        const float4 a = wide[q], b = wide[q + kNucleusThreads];
-        const uint32_t ia = q * 4u, ib = (q + kNucleusThreads) * 4u;
-        visit(a.x, ia);
-        visit(a.y, ia + 1u);
-        visit(a.z, ia + 2u);
-        visit(a.w, ia + 3u);
-        visit(b.x, ib);
-        visit(b.y, ib + 1u);
-        visit(b.z, ib + 2u);
-        visit(b.w, ib + 3u);
-    }
-    if (q < quads) {
-        const float4 a = wide[q];
-        const uint32_t ia = q * 4u;
-        visit(a.x, ia);
-        visit(a.y, ia + 1u);
-        visit(a.z, ia + 2u);
-        visit(a.w, ia + 3u);
+    if (q < quads) a = wide[q];
+    if (q + kNucleusThreads < quads) b = wide[q + kNucleusThreads];
+    for (; q < quads; q += 2 * kNucleusThreads) {
+        const float4 now_a = a, now_b = b;
+        const uint32_t next = q + 2 * kNucleusThreads;
+        if (next < quads) a = wide[next];
+        if (next + kNucleusThreads < quads) b = wide[next + kNucleusThreads];
+        visit_quad(now_a, q * 4u);
+        if (q + kNucleusThreads < quads) visit_quad(now_b, (q + kNucleusThreads) * 4u);
     }
     const uint32_t rest = quads * 4u + tid;
     if (rest < vocab) visit(values[rest], rest);
+}
+
+// *mass += w in shared memory by two 32-bit adds, the carry between them (a 64-bit one is a loop of
+// compare-and-swaps, which many values of one bucket make each other repeat).
+__device__ __forceinline__ void add_mass(unsigned long long *mass, unsigned long long w) {
+    uint32_t *half = reinterpret_cast<uint32_t *>(mass);
+    const uint32_t low = (uint32_t)w, before = atomicAdd(half, low);
+    const uint32_t high = (uint32_t)(w >> 32) + (before + low < low ? 1u : 0u);
+    if (high != 0) atomicAdd(half + 1, high);
 }
 
 // Which elements of the scratch row take part in a descent.
@@ -214,143 +216,6 @@ struct Nucleus {
     }
 };
 
-// One radix descent over the scratch row.  Weights are exp(value * inv_t - top * inv_t);
-// finds the first element of the (key descending, id ascending) order, restricted to
-// `inside`, at which the cumulative weight reaches `target` (strict: exceeds it).
-// When even the total does not, the last element inside is returned.  Outputs the
-// element's key and id, the cumulative weight up to and including it and its rank.
-// All threads of the CTA call it.
-__device__ void descend(NucleusShared &sh, const float *values, uint32_t vocab, double inv_t,
-                        double top, const Nucleus inside, unsigned long long target, bool strict,
-                        uint32_t *out_key, uint32_t *out_id, unsigned long long *out_mass,
-                        uint32_t *out_rank) {
-    const uint32_t tid = threadIdx.x;
-    const double top_scaled = top * inv_t;
-    uint32_t prefix = 0;  // key bits fixed so far
-    unsigned long long before = 0;
-    uint32_t rank_before = 0;
-    unsigned long long weight_of_key = 0;
-    uint32_t same_key = 0;
-    bool clipped = false;  // target beyond the total: steer to the last element inside
-    const int shifts[3] = {20, 8, 0};
-    const uint32_t widths[3] = {4096, 4096, 256};
-    for (int level = 0; level < 3; level++) {
-        const int shift = shifts[level];
-        const uint32_t buckets = widths[level];
-        clear_histogram(sh, buckets);
-        for (uint32_t i = tid; i < vocab; i += kNucleusThreads) {
-            const float v = values[i];
-            if (is_nonfinite(v)) continue;
-            const uint32_t key = float_key(v);
-            if (level > 0 && (key >> (shift + (level == 1 ? 12 : 8))) != prefix) continue;
-            if (!inside.holds(key, i)) continue;
-            const unsigned long long w = exp_fixed((double)v * inv_t - top_scaled, sh.table);
-            const uint32_t b = (key >> shift) & (buckets - 1);
-            atomicAdd(&sh.mass[b], w);
-            atomicAdd(&sh.count[b], 1u);
-        }
-        __syncthreads();
-        if (!clipped) {
-            find_crossing(sh, buckets, before, target, strict);
-            // the total stays below the target (rounding of the draw, or top_p = 1): the
-            // answer is the last element inside, i.e. the lowest non-empty bucket from here on
-            if (!sh.hit_found) clipped = true;
-            __syncthreads();
-        }
-        if (clipped) {
-            // lowest non-empty bucket: scan by thread 0 (rare path)
-            if (tid == 0) {
-                unsigned long long m = before;
-                uint32_t c = 0, last = 0;
-                bool any = false;
-                for (uint32_t at = 0; at < buckets; at++) {
-                    const uint32_t b = buckets - 1 - at;
-                    if (sh.count[b]) {
-                        if (any) {
-                            m += sh.mass[last];
-                            c += sh.count[last];
-                        }
-                        last = b;
-                        any = true;
-                    }
-                }
-                sh.hit_bucket = last;
-                sh.hit_mass_before = m;
-                sh.hit_count_before = c;
-                sh.hit_found = any ? 1u : 0u;
-            }
-            __syncthreads();
-        }
-        const uint32_t b = sh.hit_bucket;
-        before = sh.hit_mass_before;
-        rank_before += sh.hit_count_before;
-        weight_of_key = sh.mass[b];
-        same_key = sh.count[b];
-        prefix = (prefix << (level == 2 ? 8 : 12)) | b;
-        __syncthreads();
-    }
-    // `prefix` is now a full key; same_key elements share it, each weighing the same
-    const uint32_t key = prefix;
-    const unsigned long long each = same_key ? weight_of_key / same_key : 0;
-    uint32_t need = same_key;  // how many of the equal-valued elements it takes, 1-based
-    if (!clipped && each > 0) {
-        // smallest j with before + j*each reaching the target
-        const unsigned long long gap = target > before ? target - before : 0;
-        unsigned long long j = strict ? gap / each + 1 : (gap + each - 1) / each;
-        if (j < 1) j = 1;
-        if (j < need) need = (uint32_t)j;
-    }
-    // the need-th smallest id among the elements with this key that are inside
-    uint32_t id_prefix = 0, id_rank = need;
-    if (same_key > 1) {
-        for (int level = 0; level < 3; level++) {
-            const int shift = shifts[level];
-            const uint32_t buckets = widths[level];
-            clear_histogram(sh, buckets);
-            for (uint32_t i = tid; i < vocab; i += kNucleusThreads) {
-                const float v = values[i];
-                if (is_nonfinite(v) || float_key(v) != key || !inside.holds(key, i)) continue;
-                if (level > 0 && (i >> (shift + (level == 1 ? 12 : 8))) != id_prefix) continue;
-                // ascending ids: store reversed so the top-down walk visits small ids first
-                atomicAdd(&sh.count[buckets - 1 - ((i >> shift) & (buckets - 1))], 1u);
-                atomicAdd(&sh.mass[buckets - 1 - ((i >> shift) & (buckets - 1))], 1ull);
-            }
-            __syncthreads();
-            find_crossing(sh, buckets, 0, id_rank, false);
-            const uint32_t b = sh.hit_bucket;
-            id_rank -= (uint32_t)sh.hit_mass_before;
-            id_prefix = (id_prefix << (level == 2 ? 8 : 12)) | (buckets - 1 - b);
-            __syncthreads();
-        }
-    } else {
-        // the single element with this key: find its id
-        if (tid == 0) sh.hit_bucket = kPaddingId;
-        __syncthreads();
-        for (uint32_t i = tid; i < vocab; i += kNucleusThreads) {
-            const float v = values[i];
-            if (!is_nonfinite(v) && float_key(v) == key && inside.holds(key, i)) sh.hit_bucket = i;
-        }
-        __syncthreads();
-        id_prefix = sh.hit_bucket;
-        __syncthreads();
-    }
-    *out_key = key;
-    *out_id = id_prefix;
-    *out_mass = before + (unsigned long long)need * each;
-    *out_rank = rank_before + need;
-}
-
-// ---- the usual case: value buckets, then an exact look inside one bucket ----
-//
-// Buckets of equal width in the value itself, 1/256 wide and counted down from the
-// row's maximum (bucket 0 holds the largest values; everything 16 below the maximum,
-// where weights are below 2^-23, shares the last bucket).  Unlike the top bits of the
-// float key this spreads real logit rows over hundreds of buckets, which keeps the
-// shared-memory atomics apart.  One pass fills the histogram (this is where exp() is
-// paid), a prefix sum finds the bucket in which the target is reached, a second pass
-// gathers that bucket's members — a few hundred — and they are ordered exactly.
-
-constexpr uint32_t kListCap = 1024;    // members of a bucket the long way takes
 constexpr uint32_t kOrderCap = 2048;   // entries order_members takes
 
 // Entries to be ordered and the memory that takes.
@@ -361,24 +226,6 @@ struct OrderWork {
     uint32_t *sorted_id;
     unsigned long long *weight;  // of the sorted entries, then their running sum
 };
-
-struct NucleusList {
-    float value[kListCap];
-    uint32_t id[kListCap];
-    float sorted_value[kListCap];
-    uint32_t sorted_id[kListCap];
-    unsigned long long weight[kListCap];
-    uint32_t count;
-    __device__ __forceinline__ OrderWork work() { return {value, id, sorted_value, sorted_id, weight}; }
-};
-
-// (fp32 arithmetic: the bucket edges need not be exact, only the same in every pass and
-// monotone in v, which one rounded subtraction and an exact scaling are; the fp64 pipe is
-// what the histogram passes are short of)
-__device__ __forceinline__ uint32_t value_bucket(float v, float top) {
-    const float below = __fmul_rn(__fsub_rn(top, v), 256.0f);  // >= 0
-    return below >= (float)(kBuckets - 1) ? (uint32_t)(kBuckets - 1) : (uint32_t)below;
-}
 
 // Like find_crossing but walking the buckets upwards from 0; also leaves the sum of
 // all masses in sh.total_mass.  target_of(total) is evaluated once the total is known.
@@ -454,10 +301,6 @@ struct Position {
     bool ok;                     // false: fall back to the generic descent
 };
 
-// One phase: among the elements `inside`, weights exp((v - top) * inv_t), find the
-// first element of the (value descending, id ascending) order at which the running
-// weight reaches target_of(total) (strict: exceeds it); if it never does, the last
-// element inside.  All threads call.
 // The first `members` entries of the list, those of them that lie `inside`, ordered exactly, and
 // among them the first at which the running weight -- `before` plus the weights
 // exp((v - top) * inv_t) of the members so far -- reaches `target` (strict: exceeds it); the last
@@ -616,38 +459,6 @@ __device__ __forceinline__ Position order_members(NucleusShared &sh, const Order
     return found;
 }
 
-// The members of one value bucket (restricted to `inside`) gathered from the scratch row, then
-// order_members.  ok = false: the bucket is empty or holds more than the list takes.
-__device__ Position resolve_bucket(NucleusShared &sh, NucleusList &list, const float *values, uint32_t vocab,
-                                   double inv_t, float top, const Nucleus inside, uint32_t bucket,
-                                   uint32_t members, unsigned long long before, uint32_t rank_before,
-                                   unsigned long long target, bool strict, bool clipped, double also_inv_t,
-                                   unsigned long long *also_sum) {
-    const uint32_t tid = threadIdx.x;
-    Position found;
-    found.ok = false;
-    found.total = 0;
-    if (members == 0 || members > kListCap) return found;  // crowded bucket (heavy ties): generic path
-    if (tid == 0) list.count = 0;
-    __syncthreads();
-    walk_row(values, vocab, [&](float v, uint32_t i) {
-        // (a NaN or an infinity has no bucket: the conversion below sends them to the last one or
-        // to bucket 0, so they are looked at, and dropped, only there)
-        if (value_bucket(v, top) != bucket) return;
-        if (is_nonfinite(v) || !inside.holds(float_key(v), i)) return;
-        const uint32_t slot = atomicAdd(&list.count, 1u);
-        if (slot < kListCap) {
-            list.value[slot] = v;
-            list.id[slot] = i;
-        }
-    });
-    __syncthreads();
-    members = min(list.count, kListCap);  // (inside may hold fewer of the bucket than the histogram counted)
-    if (members == 0) return found;
-    return order_members(sh, list.work(), members, inv_t, top, inside, before, rank_before, target, strict, clipped,
-                         also_inv_t, also_sum, 40);
-}
-
 // After a crossing search: the bucket it stopped in, or -- when the total never reaches the
 // target (top_p = 1, a draw rounded up to the total) -- the last non-empty bucket.  Returns
 // whether it was clipped; all threads call.
@@ -674,290 +485,6 @@ __device__ bool settle_crossing(NucleusShared &sh) {
     }
     __syncthreads();
     return true;
-}
-
-// One phase: among the elements `inside`, weights exp((v - top) * inv_t), find the
-// first element of the (value descending, id ascending) order at which the running
-// weight reaches target_of(total) (strict: exceeds it); if it never does, the last
-// element inside.  All threads call.
-template <typename TargetOf>
-__device__ Position locate(NucleusShared &sh, NucleusList &list, const float *values, uint32_t vocab,
-                           double inv_t, float top, const Nucleus inside, TargetOf target_of,
-                           bool strict) {
-    clear_histogram(sh, kBuckets);
-    walk_row(values, vocab, [&](float v, uint32_t i) {
-        if (is_nonfinite(v) || !inside.holds(float_key(v), i)) return;
-        const unsigned long long w = exp_fixed(((double)v - (double)top) * inv_t, sh.table);
-        const uint32_t b = value_bucket(v, top);
-        atomicAdd(&sh.mass[b], w);
-        atomicAdd(&sh.count[b], 1u);
-    });
-    __syncthreads();
-    const unsigned long long target = find_crossing_up(sh, target_of, strict);
-    const unsigned long long total = sh.total_mass;
-    const bool clipped = settle_crossing(sh);
-    const uint32_t bucket = sh.hit_bucket;
-    const unsigned long long before = sh.hit_mass_before;
-    const uint32_t rank_before = sh.hit_count_before;
-    const uint32_t members = sh.count[bucket];
-    __syncthreads();
-    Position found = resolve_bucket(sh, list, values, vocab, inv_t, top, inside, bucket, members, before,
-                                    rank_before, target, strict, clipped, 0.0, nullptr);
-    found.total = total;
-    return found;
-}
-
-// exp(x) for |x| <= 1/64 by its series to the sixth power (the next term is below 1e-16).
-__device__ __forceinline__ double exp_small(double x) {
-    double p = fma(x, 1.0 / 720.0, 1.0 / 120.0);
-    p = fma(p, x, 1.0 / 24.0);
-    p = fma(p, x, 1.0 / 6.0);
-    p = fma(p, x, 0.5);
-    p = fma(p, x, 1.0);
-    return fma(p, x, 1.0);
-}
-
-// One pass over the row for both phases: per value bucket the count, the raw weights
-// exp(v - top) and the tempered weights exp((v - top) * inv_t) of its members.  A member's
-// weight is taken relative to the bucket's upper edge -- an argument of at most 1/256 (times
-// inv_t), a short series instead of a full exp() -- as 2^-32 fixed point, and summed in two
-// 16-bit halves with 32-bit shared-memory adds (a bucket of up to 65,535 members cannot
-// overflow them; integer sums do not depend on the order of arrival).  The rounding of one
-// member is 2^-33 of a member's weight; a whole row's worth stays below 1e-4 of one member's
-// weight, three orders of magnitude under the smallest distance to an edge of the cumulative
-// distribution that decides a row.  Afterwards every bucket's sums are scaled by the weight of
-// its edge, exp(-b/256) (and its power inv_t), into the row's 2^-40 fixed point.  The last
-// bucket (everything 16 below the maximum) and rows with inv_t > 4 take the full exp().
-// Returns false when a bucket holds too many members for its sums (heavy ties).
-__device__ bool fill_both(NucleusShared &sh, const float *values, uint32_t vocab, double inv_t, float top) {
-    const uint32_t tid = threadIdx.x;
-    // the two mass arrays, seen as four arrays of 32-bit sums
-    uint32_t *raw_low = reinterpret_cast<uint32_t *>(sh.mass), *raw_high = raw_low + kBuckets;
-    uint32_t *tempered_low = reinterpret_cast<uint32_t *>(sh.other_mass), *tempered_high = tempered_low + kBuckets;
-    for (uint32_t b = tid; b < kBuckets; b += kNucleusThreads) {
-        sh.mass[b] = 0;
-        sh.other_mass[b] = 0;
-        sh.count[b] = 0;
-    }
-    if (tid == 0) sh.hit_found = 0;
-    __syncthreads();
-    const bool series = inv_t <= 4.0;  // (1/256) * inv_t <= 1/64
-    const double top_d = (double)top;
-    constexpr double kOne = 4294967296.0;  // 2^32
-    walk_row(values, vocab, [&](float v, uint32_t i) {
-        if (is_nonfinite(v)) return;
-        const uint32_t b = value_bucket(v, top);
-        // v - (top - b/256): at most a bucket's width (and a rounding of the bucket's number) from 0
-        const double x = ((double)v - top_d) + (double)b * (1.0 / 256.0);
-        // (a weight of 1 and a rounding above it saturate at 2^32 - 1: half a unit, like any rounding)
-        uint32_t r, t;
-        if (series && b != (uint32_t)(kBuckets - 1)) {
-            r = (uint32_t)min(__double2ull_rn(exp_small(x) * kOne), 0xffffffffull);
-            t = (uint32_t)min(__double2ull_rn(exp_small(x * inv_t) * kOne), 0xffffffffull);
-        } else {
-            r = (uint32_t)min((exp_fixed(x, sh.table) + 128ull) >> 8, 0xffffffffull);
-            t = (uint32_t)min((exp_fixed(x * inv_t, sh.table) + 128ull) >> 8, 0xffffffffull);
-        }
-        atomicAdd(&raw_low[b], r & 0xffffu);
-        atomicAdd(&raw_high[b], r >> 16);
-        atomicAdd(&tempered_low[b], t & 0xffffu);
-        atomicAdd(&tempered_high[b], t >> 16);
-        atomicAdd(&sh.count[b], 1u);
-    });
-    __syncthreads();
-    // the halves back together (every thread reads the sums of its buckets before any of them is
-    // overwritten: the 64-bit masses take the place of the 32-bit sums), scaled by the edge's
-    // weight into the row's fixed point: 2^-32 -> 2^-40 is a factor 256
-    constexpr int kOwn = kBuckets / kNucleusThreads;
-    unsigned long long raw[kOwn], tempered[kOwn];
-#pragma unroll
-    for (int j = 0; j < kOwn; j++) {
-        const uint32_t b = j * kNucleusThreads + tid;
-        raw[j] = ((unsigned long long)raw_high[b] << 16) + raw_low[b];
-        tempered[j] = ((unsigned long long)tempered_high[b] << 16) + tempered_low[b];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < kOwn; j++) {
-        const uint32_t b = j * kNucleusThreads + tid;
-        const uint32_t members = sh.count[b];
-        if (members > 65535u) sh.hit_found = 1;  // (reused as "a bucket overflowed")
-        const double edge = -(double)b * (1.0 / 256.0);
-        sh.mass[b] = members ? __double2ull_rn((double)raw[j] * 256.0 * exp(edge)) : 0ull;
-        sh.other_mass[b] = members ? __double2ull_rn((double)tempered[j] * 256.0 * exp(edge * inv_t)) : 0ull;
-    }
-    __syncthreads();
-    const bool fits = sh.hit_found == 0;
-    __syncthreads();
-    return fits;
-}
-
-// The long way, by one CTA over the whole penalised row in scratch memory (see the top of the
-// file).  All threads call.
-__device__ __noinline__ void sample_the_long_way(NucleusShared &sh, NucleusList &list, const float *values,
-                                                 uint32_t vocab, const SamplerConfig cfg, float uniform,
-                                                 uint32_t row, const SelectOutput &out) {
-    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    float best = -INFINITY;
-    walk_row(values, vocab, [&](float v, uint32_t) {
-        if (!is_nonfinite(v)) best = fmaxf(best, v);
-    });
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) best = fmaxf(best, __shfl_xor_sync(kFullMask, best, d));
-    if (lane == 0) sh.reduce_max[warp] = best;
-    __syncthreads();
-    for (int w = 0; w < kNucleusThreads / 32; w++) best = fmaxf(best, sh.reduce_max[w]);
-    if (best == -INFINITY) {  // src/sampler.c:97 "sampler received no finite candidates"
-        if (tid == 0) {
-            report_row(out, row, kErrFormat, kPaddingId, 0.0f);
-            if (out.dbg_count) out.dbg_count[row] = 0;
-        }
-        __syncthreads();
-        return;
-    }
-    // ---- top-p on the un-tempered softmax: where does the mass reach top_p? ----
-    Nucleus all;
-    all.everything = true;
-    all.key = 0;
-    all.id = 0;
-    const double top_p = (double)cfg.top_p;
-    // cumulative / sum >= top_p  <=>  cumulative >= top_p * sum
-    auto mass_target = [top_p](unsigned long long total) {
-        const unsigned long long t = (unsigned long long)ceil(top_p * (double)total);
-        return t > total ? total : t;
-    };
-    Nucleus nucleus;
-    nucleus.everything = false;
-    unsigned long long raw_sum, mass_at_cut;
-    uint32_t size;
-    const double inv_t = 1.0 / (double)cfg.temperature;
-    float u = uniform;
-    if (is_nonfinite(u) || u < 0.0f) u = 0.0f;
-    if (u >= 1.0f) u = __uint_as_float(0x3f7fffffu);
-    const double draw_at = (double)u;
-    // first element whose cumulative weight exceeds draw = u * sum
-    auto draw_target = [draw_at](unsigned long long total) {
-        return (unsigned long long)floor(draw_at * (double)total);
-    };
-    uint32_t picked_id = kPaddingId;
-    unsigned long long weight_sum = 0;
-
-    // ---- the usual way: one pass fills both histograms, each phase then looks into one bucket ----
-    bool done = false;
-    {
-        const bool filled = fill_both(sh, values, vocab, inv_t, best);
-        const unsigned long long cut_target = find_crossing_up(sh, mass_target, false);
-        raw_sum = sh.total_mass;
-        const bool cut_clipped = settle_crossing(sh);
-        const uint32_t cut_bucket = sh.hit_bucket;
-        const unsigned long long cut_before = sh.hit_mass_before;
-        const uint32_t cut_rank_before = sh.hit_count_before;
-        const uint32_t cut_members = sh.count[cut_bucket];
-        __syncthreads();
-        unsigned long long tempered_inside = 0;  // tempered weight of the bucket's members inside the nucleus
-        const Position cut = resolve_bucket(sh, list, values, vocab, 1.0, best, all, cut_bucket, cut_members,
-                                            cut_before, cut_rank_before, cut_target, false, cut_clipped, inv_t,
-                                            &tempered_inside);
-        if (filled && cut.ok) {
-            nucleus.key = cut.key;
-            nucleus.id = cut.id;
-            mass_at_cut = cut.mass;
-            size = cut.rank;
-            // the tempered masses of the nucleus: whole buckets above the cut's, that bucket as
-            // far as the nucleus reaches into it, nothing below
-            if (tid == 0) {
-                unsigned long long *raw = sh.mass;
-                sh.mass = sh.other_mass;
-                sh.other_mass = raw;
-            }
-            __syncthreads();
-            for (uint32_t b = tid; b < kBuckets; b += kNucleusThreads) {
-                if (b > cut_bucket) {
-                    sh.mass[b] = 0;
-                    sh.count[b] = 0;
-                } else if (b == cut_bucket) {
-                    sh.mass[b] = tempered_inside;
-                }
-            }
-            __syncthreads();
-            const unsigned long long pick_target = find_crossing_up(sh, draw_target, true);
-            weight_sum = sh.total_mass;
-            const bool pick_clipped = settle_crossing(sh);
-            const uint32_t pick_bucket = sh.hit_bucket;
-            const unsigned long long pick_before = sh.hit_mass_before;
-            const uint32_t pick_members = sh.count[pick_bucket];
-            __syncthreads();
-            const Position pick = resolve_bucket(sh, list, values, vocab, inv_t, best, nucleus, pick_bucket,
-                                                 pick_members, pick_before, 0u, pick_target, true, pick_clipped,
-                                                 0.0, nullptr);
-            if (pick.ok) {
-                picked_id = pick.id;
-                done = true;
-            }
-        }
-    }
-    if (!done) {
-        // ---- a bucket too crowded to order in shared memory: phase by phase, with the exact descent ----
-        const Position cut = locate(sh, list, values, vocab, 1.0, best, all, mass_target, false);
-        if (cut.ok) {
-            nucleus.key = cut.key;
-            nucleus.id = cut.id;
-            raw_sum = cut.total;
-            mass_at_cut = cut.mass;
-            size = cut.rank;
-        } else {
-            // a bucket too crowded to order in shared memory: the generic radix descent
-            unsigned long long partial = 0;
-            for (uint32_t i = tid; i < vocab; i += kNucleusThreads) {
-                const float v = values[i];
-                if (!is_nonfinite(v)) partial += exp_fixed((double)v - (double)best, sh.table);
-            }
-#pragma unroll
-            for (int d = 16; d > 0; d >>= 1) partial += __shfl_xor_sync(kFullMask, partial, d);
-            if (lane == 0) sh.scan_mass[warp] = partial;
-            __syncthreads();
-            raw_sum = 0;
-            for (int w = 0; w < kNucleusThreads / 32; w++) raw_sum += sh.scan_mass[w];
-            __syncthreads();
-            descend(sh, values, vocab, 1.0, (double)best, all, mass_target(raw_sum), false, &nucleus.key,
-                    &nucleus.id, &mass_at_cut, &size);
-        }
-
-        // ---- temperature weights of the nucleus, then the draw ----
-        const Position pick = locate(sh, list, values, vocab, inv_t, best, nucleus, draw_target, true);
-        if (pick.ok) {
-            picked_id = pick.id;
-            weight_sum = pick.total;
-        } else {
-            unsigned long long partial = 0;
-            for (uint32_t i = tid; i < vocab; i += kNucleusThreads) {
-                const float v = values[i];
-                if (is_nonfinite(v)) continue;
-                if (nucleus.holds(float_key(v), i))
-                    partial += exp_fixed(((double)v - (double)best) * inv_t, sh.table);
-            }
-#pragma unroll
-            for (int d = 16; d > 0; d >>= 1) partial += __shfl_xor_sync(kFullMask, partial, d);
-            if (lane == 0) sh.scan_mass[warp] = partial;
-            __syncthreads();
-            weight_sum = 0;
-            for (int w = 0; w < kNucleusThreads / 32; w++) weight_sum += sh.scan_mass[w];
-            __syncthreads();
-            uint32_t picked_key, picked_rank;
-            unsigned long long picked_mass;
-            descend(sh, values, vocab, inv_t, (double)best, nucleus, draw_target(weight_sum), true,
-                    &picked_key, &picked_id, &picked_mass, &picked_rank);
-        }
-    }
-    if (tid == 0) {
-        if (weight_sum == 0 || raw_sum == 0 || picked_id >= vocab) {
-            report_row(out, row, kErrFormat, kPaddingId, 0.0f);
-        } else {
-            report_row(out, row, kOk, picked_id, values[picked_id]);
-        }
-        if (out.dbg_count) out.dbg_count[row] = size;  // nucleus size; the list itself is not dumped
-    }
-    __syncthreads();
 }
 
 // ================================================================== the short way
@@ -1085,6 +612,19 @@ struct SlotHit {
     unsigned long long raw_before, tempered_before, tempered;
 };
 
+// What the first CTA of a team asks of all of them on the long way, and what they need for it.
+struct LongStep {
+    enum What : uint32_t { kStop, kLargest, kWeighBoth, kWeigh, kWeighAll, kWeighKeys, kCountIds, kListMembers, kFindOnly };
+    uint32_t what, bucket, level, prefix, key;
+    float top;
+    double inv_t;
+    Nucleus inside;
+};
+// the levels of a descent over 32 bits: 12, 12 and 8
+__device__ __forceinline__ int descent_bits(uint32_t level) { return level < 2u ? 12 : 8; }
+__device__ __forceinline__ int descent_shift(uint32_t level) { return level == 0u ? 20 : level == 1u ? 8 : 0; }
+__device__ __forceinline__ uint32_t descent_buckets(uint32_t level) { return 1u << descent_bits(level); }
+
 struct ShortShared {
     Share share;
     Plan plan;
@@ -1099,6 +639,8 @@ struct ShortShared {
     uint32_t scan_count[kNucleusWarps];
     float raw_error[kNucleusWarps], tempered_error[kNucleusWarps];
     uint32_t poor;                                // the masses are not good enough
+    LongStep step;                                // the first CTA's
+    uint32_t only_id;
 };
 
 // Dynamic shared memory of the kernel: two CTAs' worth fit an SM.  The long way's memory lies over
@@ -1491,15 +1033,35 @@ __device__ __noinline__ Findings amend_seen(const NucleusParams &p, uint32_t row
     return counter.found;
 }
 
-// The penalised row in scratch memory, for the long way.
+// The penalised row in scratch memory, for the long way.  Returns the thread's largest finite raw logit.
 template <typename T>
-__device__ __noinline__ void write_scratch(const NucleusParams &p, uint32_t row, const SamplerConfig cfg, uint32_t lo,
+__device__ __noinline__ float write_scratch(const NucleusParams &p, uint32_t row, const SamplerConfig cfg, uint32_t lo,
                                            uint32_t n, bool penalised, float *values) {
     const T *columns = static_cast<const T *>(p.logits) + (size_t)row * p.row_stride;
-    for (uint32_t c = lo + threadIdx.x; c < lo + n; c += kNucleusThreads) values[c] = Vector<T>::one(columns + c);
+    constexpr int kPer = Vector<T>::kPer;
+    float best = __uint_as_float(0xff800000u);
+    walk_logits<T>(
+        columns + lo, n,
+        [&](const float (&v)[kPer], uint32_t c) {
+            float *to = values + lo + c;
+#pragma unroll
+            for (int j = 0; j < kPer; j++) best = is_nonfinite(v[j]) ? best : fmaxf(best, v[j]);
+            if ((c & 3u) == 0) {  // (`lo` is a multiple of 64)
+#pragma unroll
+                for (int j = 0; j < kPer; j += 4) *reinterpret_cast<float4 *>(to + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < kPer; j++) to[j] = v[j];
+            }
+        },
+        [&](float v, uint32_t c) {
+            values[lo + c] = v;
+            best = is_nonfinite(v) ? best : fmaxf(best, v);
+        });
     __syncthreads();
     if (penalised)
         visit_seen<T>(p, row, cfg, lo, n, [&](uint32_t column, float, float value, uint32_t) { values[column] = value; });
+    return best;
 }
 
 // Sum over the warp of masses below 2^60 (4,095 members of 2^44 weigh less than 2^57).
@@ -2097,6 +1659,611 @@ __device__ __forceinline__ uint32_t locate_and_pick(const NucleusParams &p, cons
     return team.at(&ss.plan, 0)->verdict;
 }
 
+// ================================================================== the long way
+//
+// For rows the short way cannot take: the row with its penalties applied lies in the team's scratch
+// memory, and every CTA of the team goes over its own columns again and again, step by step as the
+// first CTA asks; what the steps leave (histograms, members of a bucket) the first CTA adds up.
+//
+// Buckets of equal width in the value itself, 1/256 wide and counted down from the row's maximum
+// (bucket 0 holds the largest values; everything 16 below the maximum, where weights are below
+// 2^-23, shares the last bucket).  Unlike the top bits of the float key this spreads real logit rows
+// over hundreds of buckets, which keeps the shared-memory atomics apart.  One pass fills the
+// histograms of both phases, a prefix sum finds the bucket in which the target is reached, a second
+// pass gathers that bucket's members, which are ordered exactly.  A bucket too crowded for that
+// is taken apart by its members' keys, and equal keys by their ids (descend).
+//
+// What bounds it: the passes' instruction issue, and latency where a row has one CTA.  Measured with 1 /
+// 32 / 148 / 512 rows of 151,936 bf16 logits N(-10, 1.5^2), whose ties fill buckets: 381 / 572 / 1278 /
+// 4181 us.  By the first CTA alone, one value in flight per thread in the descents and 64-bit adds in
+// shared memory: 1887 / 1974 / 2146 / 6413; by a CTA of 1,024 threads a row: 1032 / 1270 / 1342 / 4522.
+// Continuous rows of spread 0.03 315 / 366 / 828 / 2838 (1136 / 1150 / 1442 / 4492; 846 / 860 / 880 / 3423).
+
+// Which values share a bucket.  (fp32 arithmetic: the bucket edges need not be exact, only the same
+// in every pass and monotone in v, which one rounded subtraction and an exact scaling are.)
+__device__ __forceinline__ uint32_t value_bucket(float v, float top) {
+    const float below = __fmul_rn(__fsub_rn(top, v), 256.0f);  // >= 0
+    return below >= (float)(kBuckets - 1) ? (uint32_t)(kBuckets - 1) : (uint32_t)below;
+}
+
+constexpr uint32_t kListCap = kOrderCap;  // members of a bucket that are ordered in shared memory
+
+// Lies over the short way's memory; the ordering works where the masses were.
+struct LongMemory {
+    unsigned long long mass[kBuckets], other_mass[kBuckets];  // raw and tempered, or the one asked for
+    uint32_t count[kBuckets];
+    float value[kListCap];  // the first CTA's list
+    uint32_t id[kListCap];
+};
+static_assert(sizeof(LongMemory) <= offsetof(ShortMemory, state), "the long way fits over the short way's memory");
+static_assert(kOrderCap * 16 <= sizeof(LongMemory::mass), "the ordering fits over the masses");
+
+// exp(x) for |x| <= 1/64 by its series to the sixth power (the next term is below 1e-16).
+__device__ __forceinline__ double exp_small(double x) {
+    double p = fma(x, 1.0 / 720.0, 1.0 / 120.0);
+    p = fma(p, x, 1.0 / 24.0);
+    p = fma(p, x, 1.0 / 6.0);
+    p = fma(p, x, 0.5);
+    p = fma(p, x, 1.0);
+    return fma(p, x, 1.0);
+}
+
+// One CTA's part of a row in scratch memory.
+struct LongWay {
+    const Team team;
+    const float *const values;  // of its columns
+    const uint32_t lo, n;
+    __device__ __forceinline__ LongMemory &memory() const { return *reinterpret_cast<LongMemory *>(&short_memory()); }
+
+    template <class Visit>
+    __device__ __forceinline__ void walk(Visit visit) const {
+        const uint32_t first = lo;
+        walk_row(values, n, [&](float v, uint32_t i) { visit(v, first + i); });
+    }
+    // The largest of the threads' values, into the CTA's share.
+    __device__ __forceinline__ void share_largest(float best) const {
+        ShortShared &ss = short_memory().state;
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) best = fmaxf(best, __shfl_xor_sync(kFullMask, best, d));
+        if (lane_id() == 0) ss.sample_max[threadIdx.x >> 5] = best;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int w = 0; w < kNucleusWarps; w++) best = fmaxf(best, ss.sample_max[w]);
+            ss.share.best = best;
+        }
+    }
+    __device__ __noinline__ void largest() const {
+        float best = -INFINITY;
+        walk([&](float v, uint32_t) {
+            if (!is_nonfinite(v)) best = fmaxf(best, v);
+        });
+        share_largest(best);
+    }
+    // Per value bucket the count, the raw weights exp(v - top) and the tempered weights
+    // exp((v - top) * inv_t) of its members.  A member's weight is taken relative to the bucket's
+    // upper edge -- an argument of at most 1/256 (times inv_t), a short series instead of a full
+    // exp() -- as 2^-32 fixed point, and summed in two 16-bit halves with 32-bit shared-memory adds
+    // (a bucket of up to 65,535 members cannot overflow them; integer sums do not depend on the
+    // order of arrival).  The rounding of one member is 2^-33 of a member's weight.  The last bucket
+    // (everything 16 below the maximum) and the tempered weights for inv_t > 4 take the full exp().  A bucket with
+    // more members than the sums take (heavy ties) is noted in the CTA's share.
+    __device__ __noinline__ void weigh_both(const LongStep &step) const {
+        LongMemory &m = memory();
+        const NucleusShared &sh = short_memory().scan;
+        const uint32_t tid = threadIdx.x;
+        // the two mass arrays, seen as four arrays of 32-bit sums
+        uint32_t *raw_low = reinterpret_cast<uint32_t *>(m.mass), *raw_high = raw_low + kBuckets;
+        uint32_t *tempered_low = reinterpret_cast<uint32_t *>(m.other_mass), *tempered_high = tempered_low + kBuckets;
+        for (uint32_t b = tid; b < kBuckets; b += kNucleusThreads) {
+            m.mass[b] = 0;
+            m.other_mass[b] = 0;
+            m.count[b] = 0;
+        }
+        if (tid == 0) short_memory().state.share.unseen = 0.0;
+        __syncthreads();
+        const float top = step.top;
+        const double inv_t = step.inv_t, top_d = (double)top;
+        // (65,535 members 40 temperatures below the maximum weigh less than half a unit of the row's
+        // 2^-40 fixed point: what they weigh tempered need not be known)
+        const uint32_t weightless = (uint32_t)fmin(ceil(40.0 * 256.0 / inv_t), (double)kBuckets);
+        const bool series = inv_t <= 4.0;  // (1/256) * inv_t <= 1/64
+        constexpr double kOne = 4294967296.0;  // 2^32
+        walk([&](float v, uint32_t) {
+            if (is_nonfinite(v)) return;
+            const uint32_t b = value_bucket(v, top);
+            // v - (top - b/256): at most a bucket's width (and a rounding of the bucket's number) from 0
+            const double x = ((double)v - top_d) + (double)b * (1.0 / 256.0);
+            // (a weight of 1 and a rounding above it saturate at 2^32 - 1: half a unit, like any rounding)
+            const bool last = b == (uint32_t)(kBuckets - 1);
+            const uint32_t r = (uint32_t)min(last ? (exp_fixed(x, sh.table) + 128ull) >> 8
+                                                  : __double2ull_rn(exp_small(x) * kOne), 0xffffffffull);
+            atomicAdd(&raw_low[b], r & 0xffffu);
+            atomicAdd(&raw_high[b], r >> 16);
+            if (b < weightless) {
+                const uint32_t t = (uint32_t)min(last || !series ? (exp_fixed(x * inv_t, sh.table) + 128ull) >> 8
+                                                                 : __double2ull_rn(exp_small(x * inv_t) * kOne), 0xffffffffull);
+                atomicAdd(&tempered_low[b], t & 0xffffu);
+                atomicAdd(&tempered_high[b], t >> 16);
+            }
+            atomicAdd(&m.count[b], 1u);
+        });
+        __syncthreads();
+        // the halves back together (every thread reads the sums of its buckets before any of them is
+        // overwritten: the 64-bit masses take the place of the 32-bit sums)
+        constexpr int kOwn = kBuckets / kNucleusThreads;
+        unsigned long long raw[kOwn], tempered[kOwn];
+#pragma unroll
+        for (int j = 0; j < kOwn; j++) {
+            const uint32_t b = j * kNucleusThreads + tid;
+            raw[j] = ((unsigned long long)raw_high[b] << 16) + raw_low[b];
+            tempered[j] = ((unsigned long long)tempered_high[b] << 16) + tempered_low[b];
+            if (m.count[b] > 65535u) short_memory().state.share.unseen = INFINITY;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < kOwn; j++) {
+            const uint32_t b = j * kNucleusThreads + tid;
+            m.mass[b] = raw[j];
+            m.other_mass[b] = tempered[j];
+        }
+    }
+    // The weights exp((v - top) * inv_t) inside `step.inside`, per value bucket.
+    __device__ __noinline__ void weigh(const LongStep &asked) const {
+        const LongStep step = asked;
+        LongMemory &m = memory();
+        const NucleusShared &sh = short_memory().scan;
+        clear_histogram(short_memory().scan, kBuckets);
+        walk([&](float v, uint32_t i) {
+            if (is_nonfinite(v) || !step.inside.holds(float_key(v), i)) return;
+            const unsigned long long w = exp_fixed(((double)v - (double)step.top) * step.inv_t, sh.table);
+            const uint32_t b = value_bucket(v, step.top);
+            add_mass(&m.mass[b], w);
+            atomicAdd(&m.count[b], 1u);
+        });
+    }
+    // ... all of them together
+    __device__ __noinline__ void weigh_all(const LongStep &asked) const {
+        const LongStep step = asked;
+        NucleusShared &sh = short_memory().scan;
+        unsigned long long sum = 0;
+        walk([&](float v, uint32_t i) {
+            if (!is_nonfinite(v) && step.inside.holds(float_key(v), i))
+                sum += exp_fixed(((double)v - (double)step.top) * step.inv_t, sh.table);
+        });
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(kFullMask, sum, d);
+        if (lane_id() == 0) sh.scan_mass[threadIdx.x >> 5] = sum;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < kNucleusWarps; w++) sum += sh.scan_mass[w];
+            sh.total_mass = sum;
+        }
+    }
+    // One level of a descent over the keys: those that begin with `step.prefix`, by their next bits.
+    __device__ __noinline__ void weigh_keys(const LongStep &asked) const {
+        const LongStep step = asked;
+        LongMemory &m = memory();
+        const NucleusShared &sh = short_memory().scan;
+        const int shift = descent_shift(step.level);
+        const uint32_t buckets = descent_buckets(step.level);
+        clear_histogram(short_memory().scan, buckets);
+        walk([&](float v, uint32_t i) {
+            if (is_nonfinite(v)) return;
+            const uint32_t key = float_key(v);
+            if (step.level > 0 && (key >> (shift + descent_bits(step.level))) != step.prefix) return;
+            if (!step.inside.holds(key, i)) return;
+            const unsigned long long w = exp_fixed((double)v * step.inv_t - (double)step.top * step.inv_t, sh.table);
+            const uint32_t b = (key >> shift) & (buckets - 1);
+            add_mass(&m.mass[b], w);
+            atomicAdd(&m.count[b], 1u);
+        });
+    }
+    // One level of a descent over the ids of the values with key `step.key`, small ones first: the
+    // buckets are numbered backwards.
+    __device__ __noinline__ void count_ids(const LongStep &asked) const {
+        const LongStep step = asked;
+        LongMemory &m = memory();
+        const int shift = descent_shift(step.level);
+        const uint32_t buckets = descent_buckets(step.level);
+        clear_histogram(short_memory().scan, buckets);
+        walk([&](float v, uint32_t i) {
+            if (is_nonfinite(v) || float_key(v) != step.key || !step.inside.holds(step.key, i)) return;
+            if (step.level > 0 && (i >> (shift + descent_bits(step.level))) != step.prefix) return;
+            const uint32_t b = buckets - 1 - ((i >> shift) & (buckets - 1));
+            atomicAdd(&m.count[b], 1u);
+            add_mass(&m.mass[b], 1ull);
+        });
+    }
+    // The members of a value bucket inside `step.inside` onto the first CTA's list.
+    __device__ __noinline__ void list_members(const LongStep &asked) const {
+        const LongStep step = asked;
+        LongMemory &m = memory();
+        ShortShared &ss = short_memory().state;
+        walk([&](float v, uint32_t i) {
+            // (a NaN or an infinity has no bucket: the conversion sends them to the last one or to
+            // bucket 0, so they are looked at, and dropped, only there)
+            if (value_bucket(v, step.top) != step.bucket) return;
+            if (is_nonfinite(v) || !step.inside.holds(float_key(v), i)) return;
+            const uint32_t slot = atomicAdd(team.at(&ss.cut_count, 0), 1u);
+            if (slot < kListCap) {
+                team.at(m.value, 0)[slot] = v;
+                team.at(m.id, 0)[slot] = i;
+            }
+        });
+    }
+    // The id of the one value with key `step.key`.
+    __device__ __noinline__ void find_only(const LongStep &asked) const {
+        const LongStep step = asked;
+        ShortShared &ss = short_memory().state;
+        walk([&](float v, uint32_t i) {
+            if (!is_nonfinite(v) && float_key(v) == step.key && step.inside.holds(step.key, i)) *team.at(&ss.only_id, 0) = i;
+        });
+    }
+    __device__ __forceinline__ void take(const LongStep &step) const {
+        switch (step.what) {
+        case LongStep::kLargest: largest(); break;
+        case LongStep::kWeighBoth: weigh_both(step); break;
+        case LongStep::kWeigh: weigh(step); break;
+        case LongStep::kWeighAll: weigh_all(step); break;
+        case LongStep::kWeighKeys: weigh_keys(step); break;
+        case LongStep::kCountIds: count_ids(step); break;
+        case LongStep::kListMembers: list_members(step); break;
+        case LongStep::kFindOnly: find_only(step); break;
+        default: break;
+        }
+    }
+
+    // ---- the other CTAs of the team: whatever the first one asks for ----
+    __device__ __forceinline__ void follow() const {
+        for (;;) {
+            team.sync();
+            const LongStep step = *team.at(&short_memory().state.step, 0);
+            if (step.what == LongStep::kStop) return;
+            take(step);
+            team.sync();
+        }
+    }
+    // ---- the first CTA; all its threads call these ----
+    __device__ __forceinline__ void stop() const {
+        if (threadIdx.x == 0) short_memory().state.step.what = LongStep::kStop;
+        team.sync();
+    }
+    __device__ __noinline__ void all(const LongStep step) const {
+        __syncthreads();
+        if (threadIdx.x == 0) short_memory().state.step = step;
+        team.sync();
+        take(step);
+        team.sync();
+    }
+    // the team's histograms added up in the first CTA's
+    __device__ __noinline__ void add_up(uint32_t buckets, bool both) const {
+        LongMemory &m = memory();
+        for (uint32_t b = threadIdx.x; b < buckets; b += kNucleusThreads) {
+            unsigned long long mass = m.mass[b], other = both ? m.other_mass[b] : 0ull;
+            uint32_t count = m.count[b];
+#pragma unroll
+            for (uint32_t r = 1; r < kMostTeam; r++) {
+                if (r >= team.size) break;
+                mass += *team.at(&m.mass[b], r);
+                if (both) other += *team.at(&m.other_mass[b], r);
+                count += *team.at(&m.count[b], r);
+            }
+            m.mass[b] = mass;
+            if (both) m.other_mass[b] = other;
+            m.count[b] = count;
+        }
+        __syncthreads();
+    }
+    // Both phases' masses as 2^-40 fixed point, scaled by the weight of the bucket's edge,
+    // exp(-b/256) (and its power inv_t): 2^-32 -> 2^-40 is a factor 256.  false: a bucket holds
+    // too many members for its sums.
+    __device__ __noinline__ bool fill_both(double inv_t, float top) const {
+        LongMemory &m = memory();
+        LongStep step;
+        step.what = LongStep::kWeighBoth;
+        step.inv_t = inv_t;
+        step.top = top;
+        all(step);
+        add_up(kBuckets, true);
+        for (uint32_t b = threadIdx.x; b < kBuckets; b += kNucleusThreads) {
+            const uint32_t members = m.count[b];
+            const double edge = -(double)b * (1.0 / 256.0);
+            m.mass[b] = members ? __double2ull_rn((double)m.mass[b] * 256.0 * exp(edge)) : 0ull;
+            m.other_mass[b] = members ? __double2ull_rn((double)m.other_mass[b] * 256.0 * exp(edge * inv_t)) : 0ull;
+        }
+        double unseen = 0.0;
+        for (uint32_t r = 0; r < team.size; r++) unseen += team.at(&short_memory().state.share, r)->unseen;
+        __syncthreads();
+        return unseen == 0.0;
+    }
+    // The members of one value bucket (restricted to `inside`), then order_members.  ok = false: the
+    // bucket is empty or holds more than the list takes.
+    __device__ __noinline__ Position resolve_bucket(double inv_t, float top, const Nucleus inside, uint32_t bucket,
+                                                    uint32_t members, unsigned long long before, uint32_t rank_before,
+                                                    unsigned long long target, bool strict, bool clipped,
+                                                    double also_inv_t, unsigned long long *also_sum) const {
+        LongMemory &m = memory();
+        ShortShared &ss = short_memory().state;
+        Position found;
+        found.ok = false;
+        found.total = 0;
+        if (members == 0 || members > kListCap) return found;  // (heavy ties)
+        if (threadIdx.x == 0) ss.cut_count = 0;
+        LongStep step;
+        step.what = LongStep::kListMembers;
+        step.top = top;
+        step.inside = inside;
+        step.bucket = bucket;
+        all(step);
+        members = min(ss.cut_count, kListCap);  // (inside may hold fewer of the bucket than the histogram counted)
+        if (members == 0) return found;
+        OrderWork work;
+        work.weight = m.mass;
+        work.sorted_value = reinterpret_cast<float *>(work.weight + kOrderCap);
+        work.sorted_id = reinterpret_cast<uint32_t *>(work.sorted_value + kOrderCap);
+        work.value = m.value;
+        work.id = m.id;
+        return order_members(short_memory().scan, work, members, inv_t, top, inside, before, rank_before, target, strict,
+                             clipped, also_inv_t, also_sum, 40);
+    }
+    // One phase: among the elements `inside`, weights exp((v - top) * inv_t), find the first
+    // element of the (value descending, id ascending) order at which the running weight reaches
+    // target_of(total) (strict: exceeds it); if it never does, the last element inside.
+    template <typename TargetOf>
+    __device__ __forceinline__ Position locate(double inv_t, float top, const Nucleus inside, TargetOf target_of,
+                                               bool strict) const {
+        NucleusShared &sh = short_memory().scan;
+        LongStep step;
+        step.what = LongStep::kWeigh;
+        step.inv_t = inv_t;
+        step.top = top;
+        step.inside = inside;
+        all(step);
+        add_up(kBuckets, false);
+        const unsigned long long target = find_crossing_up(sh, target_of, strict);
+        const unsigned long long total = sh.total_mass;
+        const bool clipped = settle_crossing(sh);
+        const uint32_t bucket = sh.hit_bucket;
+        const unsigned long long before = sh.hit_mass_before;
+        const uint32_t rank_before = sh.hit_count_before;
+        const uint32_t members = sh.count[bucket];
+        __syncthreads();
+        Position found = resolve_bucket(inv_t, top, inside, bucket, members, before, rank_before, target, strict, clipped,
+                                        0.0, nullptr);
+        found.total = total;
+        return found;
+    }
+    __device__ __noinline__ unsigned long long total(double inv_t, float top, const Nucleus inside) const {
+        LongStep step;
+        step.what = LongStep::kWeighAll;
+        step.inv_t = inv_t;
+        step.top = top;
+        step.inside = inside;
+        all(step);
+        unsigned long long sum = 0;
+        for (uint32_t r = 0; r < team.size; r++) sum += *team.at(&short_memory().scan.total_mass, r);
+        __syncthreads();
+        return sum;
+    }
+    // One radix descent.  Weights are exp(value * inv_t - top * inv_t); finds the first element of
+    // the (key descending, id ascending) order, restricted to `inside`, at which the cumulative
+    // weight reaches `target` (strict: exceeds it).  When even the total does not, the last element
+    // inside is returned.  Outputs the element's key and id, the cumulative weight up to and
+    // including it and its rank.
+    __device__ __noinline__ void descend(double inv_t, float top, const Nucleus inside, unsigned long long target,
+                                         bool strict, uint32_t *out_key, uint32_t *out_id,
+                                         unsigned long long *out_mass, uint32_t *out_rank) const {
+        NucleusShared &sh = short_memory().scan;
+        ShortShared &ss = short_memory().state;
+        const uint32_t tid = threadIdx.x;
+        unsigned long long before = 0;
+        uint32_t rank_before = 0;
+        unsigned long long weight_of_key = 0;
+        uint32_t same_key = 0;
+        bool clipped = false;  // target beyond the total: steer to the last element inside
+        LongStep step;
+        step.what = LongStep::kWeighKeys;
+        step.inv_t = inv_t;
+        step.top = top;
+        step.inside = inside;
+        step.prefix = 0;  // key bits fixed so far
+        for (step.level = 0; step.level < 3; step.level++) {
+            const uint32_t buckets = descent_buckets(step.level);
+            all(step);
+            add_up(buckets, false);
+            if (!clipped) {
+                find_crossing(sh, buckets, before, target, strict);
+                // the total stays below the target (rounding of the draw, or top_p = 1): the
+                // answer is the last element inside, i.e. the lowest non-empty bucket from here on
+                if (!sh.hit_found) clipped = true;
+                __syncthreads();
+            }
+            if (clipped) {
+                // lowest non-empty bucket: scan by thread 0 (rare path)
+                if (tid == 0) {
+                    unsigned long long m = before;
+                    uint32_t c = 0, last = 0;
+                    bool any = false;
+                    for (uint32_t at = 0; at < buckets; at++) {
+                        const uint32_t b = buckets - 1 - at;
+                        if (sh.count[b]) {
+                            if (any) {
+                                m += sh.mass[last];
+                                c += sh.count[last];
+                            }
+                            last = b;
+                            any = true;
+                        }
+                    }
+                    sh.hit_bucket = last;
+                    sh.hit_mass_before = m;
+                    sh.hit_count_before = c;
+                    sh.hit_found = any ? 1u : 0u;
+                }
+                __syncthreads();
+            }
+            const uint32_t b = sh.hit_bucket;
+            before = sh.hit_mass_before;
+            rank_before += sh.hit_count_before;
+            weight_of_key = sh.mass[b];
+            same_key = sh.count[b];
+            step.prefix = (step.prefix << descent_bits(step.level)) | b;
+        }
+        // the prefix is now a full key; same_key elements share it, each weighing the same
+        step.key = step.prefix;
+        const unsigned long long each = same_key ? weight_of_key / same_key : 0;
+        uint32_t need = same_key;  // how many of the equal-valued elements it takes, 1-based
+        if (!clipped && each > 0) {
+            // smallest j with before + j*each reaching the target
+            const unsigned long long gap = target > before ? target - before : 0;
+            unsigned long long j = strict ? gap / each + 1 : (gap + each - 1) / each;
+            if (j < 1) j = 1;
+            if (j < need) need = (uint32_t)j;
+        }
+        // the need-th smallest id among the elements with this key that are inside
+        step.prefix = 0;
+        if (same_key > 1) {
+            uint32_t id_rank = need;
+            step.what = LongStep::kCountIds;
+            for (step.level = 0; step.level < 3; step.level++) {
+                const uint32_t buckets = descent_buckets(step.level);
+                all(step);
+                add_up(buckets, false);
+                find_crossing(sh, buckets, 0, id_rank, false);
+                id_rank -= (uint32_t)sh.hit_mass_before;
+                step.prefix = (step.prefix << descent_bits(step.level)) | (buckets - 1 - sh.hit_bucket);
+            }
+            *out_id = step.prefix;
+        } else {
+            step.what = LongStep::kFindOnly;
+            if (tid == 0) ss.only_id = kPaddingId;
+            all(step);
+            *out_id = ss.only_id;
+        }
+        *out_key = step.key;
+        *out_mass = before + (unsigned long long)need * each;
+        *out_rank = rank_before + need;
+        __syncthreads();
+    }
+
+    __device__ __noinline__ void sample(const SamplerConfig cfg, float u, const float *row_values, uint32_t vocab,
+                                        uint32_t row, bool penalised, const SelectOutput &out) const {
+        NucleusShared &sh = short_memory().scan;
+        LongMemory &m = memory();
+        const uint32_t tid = threadIdx.x;
+        if (penalised) {  // (otherwise the raw logits' maximum has been shared)
+            LongStep step;
+            step.what = LongStep::kLargest;
+            all(step);
+        }
+        float best = -INFINITY;
+        for (uint32_t r = 0; r < team.size; r++) best = fmaxf(best, team.at(&short_memory().state.share, r)->best);
+        if (best == -INFINITY) {  // src/sampler.c:97 "sampler received no finite candidates"
+            if (tid == 0) {
+                report_row(out, row, kErrFormat, kPaddingId, 0.0f);
+                if (out.dbg_count) out.dbg_count[row] = 0;
+            }
+            return;
+        }
+        // ---- top-p on the un-tempered softmax: where does the mass reach top_p? ----
+        Nucleus everything;
+        everything.everything = true;
+        everything.key = 0;
+        everything.id = 0;
+        const double top_p = (double)cfg.top_p, inv_t = 1.0 / (double)cfg.temperature, draw_at = (double)u;
+        auto mass_target = [top_p](unsigned long long total) { return mass_target_of(top_p, total); };
+        auto draw_target = [draw_at](unsigned long long total) { return draw_target_of(draw_at, total); };
+        Nucleus nucleus;
+        nucleus.everything = false;
+        unsigned long long raw_sum, mass_at_cut;
+        uint32_t size;
+        uint32_t picked_id = kPaddingId;
+        unsigned long long weight_sum = 0;
+
+        // ---- the usual way: one pass fills both histograms, each phase then looks into one bucket ----
+        bool done = false;
+        {
+            const bool filled = fill_both(inv_t, best);
+            const unsigned long long cut_target = find_crossing_up(sh, mass_target, false);
+            raw_sum = sh.total_mass;
+            const bool cut_clipped = settle_crossing(sh);
+            const uint32_t cut_bucket = sh.hit_bucket;
+            const unsigned long long cut_before = sh.hit_mass_before;
+            const uint32_t cut_rank_before = sh.hit_count_before;
+            const uint32_t cut_members = sh.count[cut_bucket];
+            __syncthreads();
+            unsigned long long tempered_inside = 0;  // tempered weight of the bucket's members inside the nucleus
+            Position cut;
+            cut.ok = false;
+            if (filled)
+                cut = resolve_bucket(1.0, best, everything, cut_bucket, cut_members, cut_before, cut_rank_before, cut_target,
+                                     false, cut_clipped, inv_t, &tempered_inside);
+            if (cut.ok) {
+                nucleus.key = cut.key;
+                nucleus.id = cut.id;
+                mass_at_cut = cut.mass;
+                size = cut.rank;
+                // the tempered masses of the nucleus: whole buckets above the cut's, that bucket as
+                // far as the nucleus reaches into it, nothing below
+                for (uint32_t b = tid; b < kBuckets; b += kNucleusThreads) {
+                    m.mass[b] = b < cut_bucket ? m.other_mass[b] : b == cut_bucket ? tempered_inside : 0ull;
+                    if (b > cut_bucket) m.count[b] = 0;
+                }
+                __syncthreads();
+                const unsigned long long pick_target = find_crossing_up(sh, draw_target, true);
+                weight_sum = sh.total_mass;
+                const bool pick_clipped = settle_crossing(sh);
+                const uint32_t pick_bucket = sh.hit_bucket;
+                const unsigned long long pick_before = sh.hit_mass_before;
+                const uint32_t pick_members = sh.count[pick_bucket];
+                __syncthreads();
+                const Position pick = resolve_bucket(inv_t, best, nucleus, pick_bucket, pick_members, pick_before, 0u,
+                                                     pick_target, true, pick_clipped, 0.0, nullptr);
+                if (pick.ok) {
+                    picked_id = pick.id;
+                    done = true;
+                }
+            }
+        }
+        if (!done) {
+            // ---- a bucket too crowded to order in shared memory: phase by phase, with the exact descent ----
+            const Position cut = locate(1.0, best, everything, mass_target, false);
+            if (cut.ok) {
+                nucleus.key = cut.key;
+                nucleus.id = cut.id;
+                raw_sum = cut.total;
+                mass_at_cut = cut.mass;
+                size = cut.rank;
+            } else {
+                raw_sum = total(1.0, best, everything);
+                descend(1.0, best, everything, mass_target(raw_sum), false, &nucleus.key, &nucleus.id, &mass_at_cut, &size);
+            }
+            // ---- temperature weights of the nucleus, then the draw ----
+            const Position pick = locate(inv_t, best, nucleus, draw_target, true);
+            if (pick.ok) {
+                picked_id = pick.id;
+                weight_sum = pick.total;
+            } else {
+                weight_sum = total(inv_t, best, nucleus);
+                uint32_t picked_key, picked_rank;
+                unsigned long long picked_mass;
+                descend(inv_t, best, nucleus, draw_target(weight_sum), true, &picked_key, &picked_id, &picked_mass,
+                        &picked_rank);
+            }
+        }
+        if (tid == 0) {
+            if (weight_sum == 0 || raw_sum == 0 || picked_id >= vocab) {
+                report_row(out, row, kErrFormat, kPaddingId, 0.0f);
+            } else {
+                // (from L2: another CTA may have written it)
+                report_row(out, row, kOk, picked_id, __ldcg(row_values + picked_id));
+            }
+            if (out.dbg_count) out.dbg_count[row] = size;  // nucleus size; the list itself is not dumped
+        }
+        __syncthreads();
+    }
+};
+
 // The largest of a few logits spread evenly over the row, NaN, infinities and seen columns left
 // out (so that the row's own maximum is no smaller): where the window goes.  The second largest if
 // the largest is a peak well above it, which would leave the bulk of the row to wide buckets.  (With the
@@ -2137,6 +2304,30 @@ __device__ __forceinline__ float sample_row(const T *columns, uint32_t vocab, co
     return best.second > none && (best.first - best.second) * sharp > kPeak ? best.second : best.first;
 }
 
+// One row the long way; all CTAs of its team call.
+template <typename T>
+__device__ __noinline__ void go_the_long_way(const NucleusParams &p, const Team team, uint32_t row, const SamplerConfig cfg,
+                                             uint32_t lo, uint32_t n, bool penalised, float u) {
+    ShortMemory &m = short_memory();
+    if (threadIdx.x == 0) {
+        m.state.seen_count = 0;
+        m.scan.mass = reinterpret_cast<LongMemory *>(&m)->mass;
+        m.scan.count = reinterpret_cast<LongMemory *>(&m)->count;
+    }
+    __syncthreads();
+    float *values = p.scratch + (size_t)(blockIdx.x / p.team) * p.scratch_stride;
+    const float largest = write_scratch<T>(p, row, cfg, lo, n, penalised, values);
+    const LongWay way = {team, values + lo, lo, n};
+    way.share_largest(largest);
+    team.sync();
+    if (team.rank == 0) {
+        way.sample(cfg, u, values, p.vocab, row, penalised, p.out);
+        way.stop();
+    } else {
+        way.follow();
+    }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kNucleusThreads, 2) nucleus_select_kernel(const __grid_constant__ NucleusParams p) {
     constexpr bool kBf16 = sizeof(T) == 2;
@@ -2153,7 +2344,6 @@ __global__ void __launch_bounds__(kNucleusThreads, 2) nucleus_select_kernel(cons
     if (tid == 0) {
         ss.over_count = ss.cut_count = ss.pick_count = 0;
     }
-    float *values = p.scratch + (size_t)team_index * p.scratch_stride;
     float2 *seen = p.seen + (size_t)blockIdx.x * p.seen_stride;
     // the CTA's columns: ranges of a multiple of 64, so that every CTA's first column lies as
     // the row's does to a 16-byte boundary
@@ -2303,20 +2493,7 @@ __global__ void __launch_bounds__(kNucleusThreads, 2) nucleus_select_kernel(cons
                 if (p.out.dbg_count) p.out.dbg_count[row] = 0;
             }
         } else if (verdict != kDone) {
-            if (tid == 0) ss.seen_count = 0;
-            __syncthreads();
-            write_scratch<T>(p, row, cfg, lo, n, penalised, values);
-            team.sync();
-            if (team.rank == 0) {
-                if (tid == 0) {
-                    sh.mass = reinterpret_cast<unsigned long long *>(&m);
-                    sh.other_mass = sh.mass + kBuckets;
-                    sh.count = reinterpret_cast<uint32_t *>(sh.other_mass + kBuckets);
-                }
-                __syncthreads();
-                sample_the_long_way(sh, *reinterpret_cast<NucleusList *>(sh.count + kBuckets), values, p.vocab, cfg, u, row,
-                                    p.out);
-            }
+            go_the_long_way<T>(p, team, row, cfg, lo, n, penalised, u);
         }
         // the row's lists are empty again before any CTA adds to them
         if (tid == 0) ss.over_count = ss.cut_count = ss.pick_count = 0;
@@ -2330,7 +2507,6 @@ using namespace fgk;
 
 
 static constexpr size_t kNucleusDynamic = sizeof(ShortMemory);
-static_assert(kNucleusHistogramBytes + sizeof(NucleusList) <= offsetof(ShortMemory, state), "the long way fits over the short way's memory");
 static_assert(sizeof(ShortMemory) + 64 <= 113 * 1024, "two CTAs to an SM");
 
 static const void *nucleus_kernel(uint32_t dtype) {

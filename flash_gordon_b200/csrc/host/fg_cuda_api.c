@@ -859,8 +859,10 @@ static fg_status run_stream(fg_cuda_context *c, const fg_cuda_sample_args *a,
  * prefix sums, ordering the candidates: about that of 160,000 columns) and a time that shrinks
  * with the columns each has, but doubles once SMs hold two CTAs; the teams that fit the GPU work in
  * rounds.  Measured on B200, vocabulary 151,936, fp32, teams of 1 / 2 / 4 / 8: one row - / 52 / 43 / 40 us,
- * 32 rows - / 58 / 48 / 55, 64 rows - / 60 / 65 / 104, 148 rows 80 / 84 / 158 / -, 512 rows
- * 238 / 277 / 435 / -. */
+ * 32 rows - / 58 / 48 / 55, 64 rows - / 60 / 65 / 104, 90 rows 89 / 88, 148 rows 94 / 99, 512 rows
+ * 238 / 277 / 435 / -.  A row that goes the long way, or whose window is placed anew, costs half as much
+ * with two CTAs (148 rows, bf16 ties 1500 / 1289 us, one such row among them 153 / 120; histories of 4,096
+ * tokens 171 / 146), so up to half the GPU's places no row has one alone. */
 static uint32_t plan_teams(const fg_cuda_context *c, uint32_t rows, uint32_t vocab, uint32_t *teams) {
     uint32_t best = 1u;
     double best_cost = 0.0;
@@ -872,6 +874,7 @@ static uint32_t plan_teams(const fg_cuda_context *c, uint32_t rows, uint32_t voc
         const double rounds = (double)((rows + most - 1u) / most);
         const uint32_t abreast = rows < most ? rows : most;
         const double share = (double)vocab / (double)(1u << i) * ((abreast << i) > c->sm_count ? 2.0 : 1.0);
+        if (i == 0u && c->nucleus_teams[1] != 0u && rows <= most / 2u) continue;
         const double cost = rounds * (160000.0 + share);
         if (best_cost == 0.0 || cost < best_cost) {
             best_cost = cost;

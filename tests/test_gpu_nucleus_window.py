@@ -124,3 +124,33 @@ def test_what_lies_under_a_cold_row_s_window_is_not_forgotten(context, form):
     configs = [SamplerConfig.make(temperature=0.2, top_p=1.0 - k * 2.0 ** -24, top_k=0) for k in (100, 1_000, 3_000, 5_000)]
     w = synth.Workload("under", x, configs, torch.tensor([0.1, 0.5, 0.9, 0.3]), None, None, 0, allow_no_topk=True)
     sizes_and_tokens_agree(context, w, 2e-11)
+
+
+@pytest.mark.parametrize("rows", [1, 20, 60, 150])
+@pytest.mark.parametrize("kind", ["narrow", "ties", "equal", "cold", "ties with history"])
+def test_rows_of_the_long_way_shared_by_teams(context, kind, rows):
+    """Buckets with more members than their words or the lists take, and temperatures below the range:
+    every CTA of a team does its part of every step."""
+    vocab = 140_001 if rows < 60 else 40_001
+    g = torch.Generator().manual_seed(rows)
+    x = torch.randn(rows, vocab, generator=g)
+    temperature, top_p = 0.9, 0.7501
+    if kind == "narrow":
+        x *= 0.002
+    elif kind == "equal":
+        x[:, :] = 0.5
+        x[:, ::3] = -0.25
+    elif kind == "cold":
+        temperature, top_p = 0.02, 0.9
+    else:
+        x = torch.round(x * 2.0) * 0.5 - 20.0
+    x[:, 3] = float("nan")
+    x[:, 77] = float("-inf")
+    cfg = SamplerConfig.make(temperature=temperature, top_p=top_p, top_k=0,
+                             presence=0.3 if "history" in kind else 0.0, frequency=0.1 if "history" in kind else 0.0)
+    uniforms = torch.rand(rows, generator=g).tolist()
+    if "history" in kind:
+        w = with_history(x, cfg, {int(i): 1 + int(i) % 3 for i in torch.randperm(vocab, generator=g)[:900]}, uniforms)
+    else:
+        w = synth.Workload(kind, x, [cfg], torch.tensor(uniforms), None, None, 0, allow_no_topk=True)
+    sizes_and_tokens_agree(context, w)
