@@ -2386,7 +2386,9 @@ __global__ void __launch_bounds__(kNucleusThreads, 2) nucleus_select_kernel(cons
         uint32_t finite = 1, verdict = kLongWay;
         float reference = 0.0f;
         if (counting) reference = sample_row(columns, p.vocab, bits, sharp);
-        if (is_nonfinite(reference)) reference = 0.0f;  // (nothing finite among the samples: any window will do)
+        // (nothing finite among the samples, or nothing but a mask's value: any window will do, and the
+        // pass finds the true maximum)
+        if (is_nonfinite(reference) || !Window(reference, sharp).usable) reference = 0.0f;
         // The window is placed by the sample; if that said little, by the true maximum; if the masses
         // it gives are not good enough, by the bulk of the values.
         bool by_sample = true, by_bulk = false;

@@ -154,3 +154,20 @@ def test_rows_of_the_long_way_shared_by_teams(context, kind, rows):
     else:
         w = synth.Workload(kind, x, [cfg], torch.tensor(uniforms), None, None, 0, allow_no_topk=True)
     sizes_and_tokens_agree(context, w)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("temperature", [1.0, 0.2])
+@pytest.mark.parametrize("offset", [0.0, -30.0])
+def test_a_mask_s_value_in_every_sample(context, dtype, temperature, offset):
+    """Sixty values left by a mask of the type's lowest value: the samples see nothing else."""
+    vocab = 151_936
+    g = torch.Generator().manual_seed(9)
+    x = torch.full((4, vocab), torch.finfo(dtype).min, dtype=dtype)
+    sampled = torch.arange(2_048) * vocab // 2_048
+    at = torch.randperm(vocab, generator=g)[:60]
+    at = at[~torch.isin(at, sampled)]
+    x[:, at] = (torch.randn(4, len(at), generator=g) * 3.0 + offset).to(dtype)
+    cfg = SamplerConfig.make(temperature=temperature, top_p=0.95, top_k=0)
+    w = synth.Workload("masked", x, [cfg], torch.rand(4, generator=g), None, None, 0, allow_no_topk=True)
+    sizes_and_tokens_agree(context, w)
