@@ -699,6 +699,28 @@ static int launched(fg_cuda_context *c, int e) {
     return e;
 }
 
+/* Whether counting tokens costs rows more in the ring kernel than its faster pass over the logits
+ * saves.  The ring kernel does not tabulate a history: its closing warp scans the token list for entries that may
+ * be among the k best, more of them the more of the vocabulary has been seen.  The streaming kernel counts
+ * in shared memory, and its time grows with the logits.  Fitted to 1,248 batches (B200, fp32, unaligned rows;
+ * vocabularies of 32,001 to 199,999, histories of 2,048 to 8,192 uniform or Zipf tokens, k 8 to 64, 1 to 700
+ * rows) such that none is more than 1.09 times slower than in the streaming kernel, which took all
+ * unaligned rows before; without the rule up to 3.1 times: 64 rows of 32,001 logits with 8,192 uniform tokens,
+ * k = 64, 168 us in the ring kernel and 53 (148 rows of 100,277 97 and 115, and left to it).  Zipf
+ * histories repeat few ids and would be up to 2.1 times faster in the ring kernel, 7 % on average,
+ * but whether ids repeat is not known here. */
+static bool scans_cost_more(const fg_cuda_sample_args *a) {
+    uint32_t k = 0u;
+    for (uint32_t i = 0; i < a->config_count; i++) {
+        const fg_sampler_config *cfg = &a->configs[i];
+        const uint32_t wanted = cfg->temperature == 0.0f ? 1u : cfg->top_k;
+        if (cfg->frequency_penalty != 0.0f && wanted > k) k = wanted;
+    }
+    const double kilotokens = (double)a->history_max / 1024.0;
+    const double scans = (double)k * kilotokens * kilotokens * sqrt(kilotokens) / ((double)a->vocab / 100000.0);
+    return scans > 2900.0 && (double)a->rows * (double)a->vocab < 19.0 * scans * sqrt(scans);
+}
+
 static fg_status run_stream(fg_cuda_context *c, const fg_cuda_sample_args *a,
                             const batch_traits *traits, uint32_t vocab_offset,
                             uint32_t vocab_total, uint32_t shard_k, float *shard_scores,
@@ -717,6 +739,8 @@ static fg_status run_stream(fg_cuda_context *c, const fg_cuda_sample_args *a,
     const bool few_long_rows = a->rows * 4u < c->sm_count && fgk_persistent_row_tiles(a->dtype, a->vocab) > 512u;
     const bool ring_ok = ((uintptr_t)a->logits % element) == 0u && c->forced_splits <= 1u &&
                          (aligned || !few_long_rows) && /* (rows are cut at 16-byte boundaries) */
+                         (aligned || c->path != FG_CUDA_PATH_AUTO || c->session_counts || !traits->counts ||
+                          !scans_cost_more(a)) &&
                          fgk_persistent_dynamic_smem(whole_bitmap, NULL) != 0u;
     const bool all_ring = ring_ok && raising == 0u;
     const bool both = ring_ok && raising != 0u && raising < a->rows && a->config_count > 1u &&

@@ -60,6 +60,25 @@ def test_rows_of_one_batch_in_two_kernels(context, dtype, vocab, raising):
     assert_rows_equal(run_gpu(context, w), run_oracle(w), f"{raising} raising rows")
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("vocab", [3_001, 3_008, 32_001])
+@pytest.mark.parametrize("history", [700, 8_192, 70_000])
+@pytest.mark.parametrize("k,top_p", [(20, 0.9), (64, 1.0)])
+def test_most_of_the_best_have_been_seen(context, dtype, vocab, history, k, top_p):
+    """Uniform histories, up to many times the vocabulary, with a frequency penalty: much to count, by
+    the kernel that is faster at it (the streaming kernel for unaligned rows and long histories)."""
+    configs = [SamplerConfig.make(temperature=0.0 if r == 2 else 0.8, top_p=top_p, top_k=1 if r == 2 else k, presence=0.1 * r,
+                                  frequency=0.02 + 0.1 * (r % 2), repetition=1.0 + 0.05 * (r % 3)) for r in range(5)]
+    w = random_workload(5, vocab, history, configs, vocab + history + k, dtype=dtype)
+    expected = run_oracle(w)
+    for path in (0, 3):  # (3: the ring kernel wherever it can)
+        context.set_path(path)
+        try:
+            assert_rows_equal(run_gpu(context, w), expected, f"V={vocab} H={history} path {path}")
+        finally:
+            context.set_path(0)
+
+
 def test_unaligned_shards(context):
     """Two column ranges of unaligned rows, then the merge, against the whole rows."""
     rows, vocab, k = 11, 9_001, 24
