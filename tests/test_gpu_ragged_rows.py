@@ -47,17 +47,66 @@ def test_every_offset(context, dtype, kind, vocab, stride, start):
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("vocab", [12_346, 12_352])
 @pytest.mark.parametrize("raising", [1, 7, 30])
-def test_rows_of_one_batch_in_two_kernels(context, dtype, vocab, raising):
-    """`raising` of 30 rows have penalties that can raise a logit."""
+def test_some_rows_of_a_small_batch_raise(context, dtype, vocab, raising):
+    """`raising` of 30 rows have penalties that can raise a logit (a batch so small goes through the
+    streaming kernel whole)."""
     rows = 30
+    w = random_workload(rows, vocab, 400, some_raising(rows, raising), 5 + raising, dtype=dtype)
+    assert_rows_equal(run_gpu(context, w), run_oracle(w), f"{raising} raising rows")
+
+
+def some_raising(rows, raising, nucleus_every=0):
     configs = []
     for r in range(rows):
         lift = (r * 7) % rows < raising
-        configs.append(SamplerConfig.make(temperature=0.0 if r % 5 == 0 else 0.9, top_p=0.9, top_k=1 if r % 5 == 0 else 30,
+        nucleus = nucleus_every and r % nucleus_every == 2
+        greedy = r % 5 == 0 and not nucleus
+        configs.append(SamplerConfig.make(temperature=0.0 if greedy else 0.9, top_p=0.9,
+                                          top_k=0 if nucleus else 1 if greedy else 30,
                                           presence=-0.7 if lift else 0.5, frequency=0.2 * (r % 2),
                                           repetition=1.0 + 0.1 * (r % 3)))
-    w = random_workload(rows, vocab, 400, configs, 5 + raising, dtype=dtype)
-    assert_rows_equal(run_gpu(context, w), run_oracle(w), f"{raising} raising rows")
+    return configs
+
+
+@pytest.mark.parametrize("rows,vocab,dtype,raising,nucleus_every", [
+    (160, 100_277, torch.bfloat16, 20, 0), (180, 100_277, torch.bfloat16, 1, 8), (128, 131_072, torch.float32, 127, 0),
+    (175, 98_049, torch.float32, 31, 11),
+])
+def test_rows_of_a_large_batch_in_two_kernels(context, rows, vocab, dtype, raising, nucleus_every):
+    """Above 15 million logits the raising rows go through the streaming kernel and the others through
+    the ring kernel: one launch more than with a single kernel."""
+    w = random_workload(rows, vocab, 300, some_raising(rows, raising, nucleus_every), raising, dtype=dtype, specials=1)
+    w.allow_no_topk = bool(nucleus_every)
+    expected = run_oracle(w)
+    before = context.launches
+    assert_rows_equal(run_gpu(context, w), expected, f"{raising} raising rows")
+    mixed = context.launches - before
+    context.set_path(1)
+    try:
+        before = context.launches
+        assert_rows_equal(run_gpu(context, w), expected, "streaming kernel")
+        assert mixed == context.launches - before + 1
+    finally:
+        context.set_path(0)
+
+
+def test_rows_of_a_large_shard_in_two_kernels(context):
+    """The same for the columns of a shard: the lists of both kernels' rows are the whole rows' parts."""
+    rows, vocab, width, k = 300, 104_000, 52_000, 24
+    configs = [SamplerConfig.make(temperature=0.9, top_p=0.9, top_k=k, presence=-0.6 if r % 9 == 4 else 0.4, frequency=0.1)
+               for r in range(rows)]
+    w = random_workload(rows, vocab, 200, configs, 78)
+    expected = run_oracle(w)
+    d = w.to("cuda")
+    scores = torch.empty(2, rows, k, device="cuda")
+    ids = torch.empty(2, rows, k, dtype=torch.int32, device="cuda")
+    for s in range(2):
+        before = context.launches
+        _, _, _, status = context.shard_topk(d.logits[:, s * width:(s + 1) * width], d.configs, s * width, vocab, k,
+                                             d.history_tokens, d.history_offsets, d.history_max, out=(scores[s], ids[s]))
+        assert status == FG_OK and context.launches - before == 2
+    result = context.merge_select(scores, ids, rows, 2, k, [0, width], [width, width], d.configs, d.uniforms)
+    assert np.array_equal(as_u32(result.tokens), expected[1])
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
