@@ -727,10 +727,12 @@ static fg_status run_stream(fg_cuda_context *c, const fg_cuda_sample_args *a,
                             uint32_t *shard_ids, uint32_t shard_stride, fg_error *err) {
     /* Rows the copy engine can fetch whose penalties cannot raise a logit may go through the
      * persistent ring kernel; rows whose penalties can, and anything the caller pinned to it, through the
-     * register-prefetch kernel.  A large batch with both kinds of rows goes through both, one after
-     * the other; a small one is faster through the second alone (measured with one row in eight
-     * raising, bf16, both against one kernel: 100,277 logits 148 rows 88 / 85 us, 200 rows 96 / 115, 400
-     * rows 129 / 227; 39,552 logits 300 rows 85 / 76, 400 rows 92 / 105). */
+     * register-prefetch kernel.  A large batch with few raising rows goes through both, one after
+     * the other; a small one, or one with more of them, is faster through the second alone.  Measured (both
+     * against one kernel, us): one row in eight raising, bf16, 100,277 logits 148 rows 88 / 85, 200 rows 87 / 130, 400
+     * rows 119 / 234; 39,552 logits 300 rows 85 / 76, 500 rows 94 / 116.  One in four, 152 rows of 100,277 91 / 112, 300
+     * of 151,936 137 / 147, 900 of 39,552 147 / 174; every other one 118 / 111, 161 / 151, 166 / 196;
+     * three in four 133 / 111, 179 / 144, 186 / 175. */
     const size_t element = a->dtype == FG_CUDA_BF16 ? 2u : 4u;
     const uint32_t whole_bitmap = traits->penalties ? (a->vocab + 31u) / 32u : 0u;
     const uint32_t raising = !traits->penalties ? 0u : a->config_count == 1u && traits->raising ? a->rows : traits->raising;
@@ -743,7 +745,7 @@ static fg_status run_stream(fg_cuda_context *c, const fg_cuda_sample_args *a,
                           !scans_cost_more(a)) &&
                          fgk_persistent_dynamic_smem(whole_bitmap, NULL) != 0u;
     const bool all_ring = ring_ok && raising == 0u;
-    const bool both = ring_ok && raising != 0u && raising < a->rows && a->config_count > 1u &&
+    const bool both = ring_ok && raising != 0u && raising <= (a->rows - traits->nucleus) / 4u && a->config_count > 1u &&
                       (uint64_t)(a->rows - traits->nucleus) * a->vocab >= 15000000u &&
                       c->path == FG_CUDA_PATH_AUTO && !c->session_counts;
     stream_plan plan;
