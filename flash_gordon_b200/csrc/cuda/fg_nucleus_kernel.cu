@@ -495,7 +495,7 @@ __device__ bool settle_crossing(NucleusShared &sh) {
 // latencies of 20 us, so two CTAs share an SM, one streaming while the other scans and sorts; for
 // few rows a row is spread over several CTAs instead.  A CTA per row and SM that added two fp64 weights
 // per logit to five shared-memory sums took, per call: 512 rows of 151,936 fp32 logits, histories
-// of 32,768 tokens 772 us (now 561), without history 538 (245); 32 rows bf16 410-560 (60).
+// of 32,768 tokens 772 us (now 571), without history 538 (250); 32 rows bf16 410-560 (64).
 // With histories the largest part is the seen columns' gather (amend_seen).
 //
 // A value's place: buckets 1/1024 wide over the top four units of the row's window, 1/256 wide over

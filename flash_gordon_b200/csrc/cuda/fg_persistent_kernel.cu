@@ -45,7 +45,8 @@
 // the warp that gets the first or the last tile writes the partial granule into its stage with
 // plain loads, -inf where the row is not.  (Such rows went element by element through the streaming
 // kernel before.  64 rows of 100,277 bf16 logits, histories of 512: 69 us there, 25 here; 512
-// rows 241 and 62; one row 42 and 25.)
+// rows 241 and 62; one row 42 and 25.  With long histories whose occurrences have to be counted that kernel
+// can be the faster one, and the host sends such batches there.)
 #include <cstring>
 #include <type_traits>
 

@@ -68,9 +68,11 @@ fg_status fg_cuda_context_set_splits(fg_cuda_context *context, uint32_t splits, 
  * shared-memory ring fed by bulk copies (rows whose start, stride and length are
  * multiples of 16 bytes, penalties that cannot raise a logit), or the
  * register-prefetch kernel (anything).  AUTO is the library's choice: the ring
- * kernel whenever it can take the batch, unaligned rows included, and for the
- * rows it can take of a large batch with some raising penalties.  RING fails with FG_ERR_ARGUMENT on a
- * batch it cannot take, RING_IF_POSSIBLE falls back instead (as AUTO does).
+ * kernel whenever it can take the batch, unaligned rows included (unless long
+ * histories with a frequency penalty make the other one faster for them), and for
+ * the rows it can take of a large batch with few raising penalties.  RING fails
+ * with FG_ERR_ARGUMENT on a batch it cannot take or whose rows are not aligned,
+ * RING_IF_POSSIBLE falls back instead (as AUTO does).
  * Results never depend on it. */
 #define FG_CUDA_PATH_AUTO             0u
 #define FG_CUDA_PATH_REGISTERS        1u

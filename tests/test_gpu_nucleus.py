@@ -1,9 +1,10 @@
 """Rows sampled without a top-k cut (top_k == 0 under FG_CUDA_SAMPLE_ALLOW_NO_TOPK):
 top-p over the whole vocabulary.  The reference's select stops at 64 candidates, so
 the oracle here is the repository's generalisation of it (fgo_select_general): same
-order, same fp64 formulas, any number of candidates.  The GPU accumulates masses as
-2^-40 fixed point instead of left-to-right doubles; ids agree unless top_p or the
-draw lies within ~1e-11 of an edge of the CDF, which these seeds do not hit."""
+order, same fp64 formulas, any number of candidates.  The GPU has masses per bucket of
+values, from moments (or weights rounded to 2^-32), as fixed point instead of left-to-right
+doubles; they are off by up to 6e-11 of their total, and ids agree unless top_p or the draw
+lies that close to an edge of the CDF, which these seeds do not hit."""
 import numpy as np
 import pytest
 import torch
@@ -25,12 +26,12 @@ def test_config5_reduced_rows(context):
 
 
 def test_config5_a_wave_of_rows_with_their_edge_margins(context, capsys):
-    """More rows than the GPU has SMs (the kernel is one CTA per SM), full vocabulary, the
+    """More rows than the GPU has SMs, full vocabulary, the
     benchmark's 32,768-token histories.  The oracle also reports, per row, how far top_p and
     the draw lie from the nearest edge of the cumulative distribution (in units of the total
-    mass): ids can only differ where that is within the rounding of a sum -- about 1e-12 for
-    the 2^-40 fixed point here, 1e-16 per term for the oracle's doubles -- so the smallest
-    margin of the run is printed and must be far above it."""
+    mass): ids can only differ where that is within the error of a sum -- 6e-11 at most here (flat
+    rows like these 1e-12), 1e-16 per term for the oracle's doubles -- so the smallest margin of
+    the run is printed and must be above it."""
     w = synth.config5(rows=160)
     expected = run_oracle(w, want_candidates=True)
     assert expected[0] == FG_OK
