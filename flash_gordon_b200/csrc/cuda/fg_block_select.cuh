@@ -37,9 +37,6 @@ struct FinishBuffer {
     uint32_t id[kMaxK];
     double raw[kMaxK];
     double tempered[kMaxK];
-    uint32_t cutoff;
-    uint32_t picked;
-    uint32_t status;
 };
 
 // How the threads that share a candidate list meet: the whole CTA by default; a
@@ -224,47 +221,39 @@ __device__ __forceinline__ void report_row(const SelectOutput &out, uint32_t row
     if (status != kOk) note_error(out, row, status);
 }
 
-// x[0] + x[1] + ... + x[n-1] added from the left, one rounding per addition, as the C loops
-// of src/sampler.c:99-111 do; the loads of four terms go ahead of their additions.
-__device__ __forceinline__ double ordered_sum(const double *x, uint32_t n) {
+// x[i] becomes x[0] + ... + x[i], added from the left with one rounding per addition, as the C
+// loops of src/sampler.c:99-111 do; the loads of four terms go ahead of their additions.  Returns
+// the sum of all n.
+__device__ __forceinline__ double running_sums(double *x, uint32_t n) {
     double sum = 0.0;
     uint32_t i = 0;
     for (; i + 4 <= n; i += 4) {
         const double a = x[i], b = x[i + 1], c = x[i + 2], d = x[i + 3];
-        sum += a;
-        sum += b;
-        sum += c;
-        sum += d;
-    }
-    for (; i < n; i++) sum += x[i];
-    return sum;
-}
-
-// The first i whose running sum x[0] + ... + x[i] (added from the left) satisfies
-// `sum >= limit` (kStrictlyAbove: `limit < sum`); n when none does.
-template <bool kStrictlyAbove>
-__device__ __forceinline__ uint32_t ordered_reach(const double *x, uint32_t n, double limit) {
-    double sum = 0.0;
-    uint32_t i = 0;
-    for (; i + 4 <= n; i += 4) {
-        const double a = x[i], b = x[i + 1], c = x[i + 2], d = x[i + 3];
-        const double s0 = sum + a, s1 = s0 + b, s2 = s1 + c, s3 = s2 + d;
-        if (kStrictlyAbove ? limit < s0 : s0 >= limit) return i;
-        if (kStrictlyAbove ? limit < s1 : s1 >= limit) return i + 1;
-        if (kStrictlyAbove ? limit < s2 : s2 >= limit) return i + 2;
-        if (kStrictlyAbove ? limit < s3 : s3 >= limit) return i + 3;
-        sum = s3;
+        const double s0 = sum + a, s1 = s0 + b, s2 = s1 + c;
+        sum = s2 + d;
+        x[i] = s0;
+        x[i + 1] = s1;
+        x[i + 2] = s2;
+        x[i + 3] = sum;
     }
     for (; i < n; i++) {
         sum += x[i];
-        if (kStrictlyAbove ? limit < sum : sum >= limit) return i;
+        x[i] = sum;
     }
-    return n;
+    return sum;
 }
 
-// Final step for one row; called by warp 0 of the CTA (all 32 lanes) with the
+// Final step for one row; called by one warp of the CTA (all 32 lanes) with the
 // candidates already in sampling order in fin.score/id[0..n), n = min(top_k,
 // #finite).  Greedy rows never come here.
+//
+// What bounds it: the additions, which have to be made one after the other in the reference's order.
+// There are two chains of n of them.  The raw weights' sum and the tempered weights' running sums are
+// made side by side by two lanes (how far the nucleus reaches is not known by then, but a running
+// sum is there for every length); the quotients' running sums follow.  Both edges -- where top_p is
+// reached, where the draw lands -- are then compares of all lanes.  (Four chains of one lane, two of
+// them with a compare and a branch per addition, took 1.5 us longer: 64 rows of 151,936 logits, k = 20, 26.1 us
+// a call then and 24.6 now; 1024 rows, k = 50, 143.7 and 140.5.)
 __device__ inline void finish_select(FinishBuffer &fin, uint32_t n, const SamplerConfig &cfg,
                               float uniform, uint32_t row, const SelectOutput &out) {
     const uint32_t lane = lane_id();
@@ -275,9 +264,8 @@ __device__ inline void finish_select(FinishBuffer &fin, uint32_t n, const Sample
         }
         return;
     }
-    // Every lane has at most two candidates (n <= 64).  Their four exponentials -- the raw
-    // and the tempered weight of each, the latter wanted only below the top-p cut, which is not
-    // known yet -- do not wait for one another, so they are all started here.
+    // Every lane has at most two candidates (n <= 64), whose exponentials -- the raw and the tempered
+    // weight of each -- do not wait for one another.
     static_assert(kMaxK <= 64, "two candidates per lane");
     const double top_raw = (double)fin.score[0];
     const double temperature = (double)cfg.temperature;
@@ -285,75 +273,71 @@ __device__ inline void finish_select(FinishBuffer &fin, uint32_t n, const Sample
     const uint32_t i0 = lane, i1 = lane + 32;
     const double s0 = i0 < n ? (double)fin.score[i0] : top_raw;
     const double s1 = i1 < n ? (double)fin.score[i1] : top_raw;
-    double raw0 = exp(s0 - top_raw), raw1 = exp(s1 - top_raw);
-    const double tempered0 = exp(s0 / temperature - top_tempered);
-    const double tempered1 = exp(s1 / temperature - top_tempered);
+    double raw0 = exp(s0 - top_raw), tempered0 = exp(s0 / temperature - top_tempered);
+    double raw1 = 1.0, tempered1 = 1.0;
+    if (n > 32) {
+        raw1 = exp(s1 - top_raw);
+        tempered1 = exp(s1 / temperature - top_tempered);
+    }
+    if (i0 < n) {
+        fin.raw[i0] = raw0;
+        fin.tempered[i0] = tempered0;
+    }
+    if (i1 < n) {
+        fin.raw[i1] = raw1;
+        fin.tempered[i1] = tempered1;
+    }
+    __syncwarp();
+    double raw_sum = 0.0;
+    if (lane < 2) raw_sum = running_sums(lane == 0 ? fin.raw : fin.tempered, n);
+    raw_sum = __shfl_sync(kFullMask, raw_sum, 0);
+    if (!(raw_sum > 0.0) || isinf(raw_sum) || isnan(raw_sum)) {  // "sampler raw softmax failed"
+        if (lane == 0) {
+            report_row(out, row, kErrFormat, kPaddingId, 0.0f);
+            if (out.dbg_count) out.dbg_count[row] = 0;
+        }
+        return;
+    }
+    raw0 = raw0 / raw_sum;
+    raw1 = raw1 / raw_sum;
     if (i0 < n) fin.raw[i0] = raw0;
     if (i1 < n) fin.raw[i1] = raw1;
     __syncwarp();
-    // the sums run left to right on one lane, as the C code's loops do; the divisions
-    // are independent of one another and spread over the warp
-    double raw_sum = 0.0;
-    if (lane == 0) raw_sum = ordered_sum(fin.raw, n);
-    raw_sum = __shfl_sync(kFullMask, raw_sum, 0);
-    const bool raw_ok = raw_sum > 0.0 && !isinf(raw_sum) && !isnan(raw_sum);
-    if (raw_ok) {
-        raw0 = raw0 / raw_sum;
-        raw1 = raw1 / raw_sum;
-        if (i0 < n) fin.raw[i0] = raw0;
-        if (i1 < n) fin.raw[i1] = raw1;
-    }
+    if (lane == 0) running_sums(fin.raw, n);
     __syncwarp();
-    if (lane == 0) {
-        uint32_t cutoff = n;
-        if (raw_ok) cutoff = min(n, ordered_reach<false>(fin.raw, n, (double)cfg.top_p) + 1u);
-        fin.cutoff = cutoff;
-        fin.status = raw_ok ? kOk : kErrFormat;  // "sampler raw softmax failed"
-    }
-    __syncwarp();
-    if (fin.status != kOk) {
+    // the first of the 64 places at which something holds; `otherwise` when at none
+    auto first_place = [](bool here0, bool here1, uint32_t otherwise) {
+        const uint32_t low = __ballot_sync(kFullMask, here0), high = __ballot_sync(kFullMask, here1);
+        return low ? (uint32_t)__ffs(low) - 1u : high ? (uint32_t)__ffs(high) + 31u : otherwise;
+    };
+    const double top_p = (double)cfg.top_p;
+    const uint32_t cutoff = first_place(i0 < n && fin.raw[i0] >= top_p, i1 < n && fin.raw[i1] >= top_p, n - 1u) + 1u;
+    const double weight_sum = fin.tempered[cutoff - 1u];
+    if (!(weight_sum > 0.0) || isinf(weight_sum) || isnan(weight_sum)) {  // "sampler temperature softmax failed"
         if (lane == 0) {
-            report_row(out, row, fin.status, kPaddingId, 0.0f);
+            report_row(out, row, kErrFormat, kPaddingId, 0.0f);
             if (out.dbg_count) out.dbg_count[row] = 0;
         }
         return;
     }
-    const uint32_t cutoff = fin.cutoff;
-    if (i0 < n) fin.tempered[i0] = i0 < cutoff ? tempered0 : 0.0;
-    if (i1 < n) fin.tempered[i1] = i1 < cutoff ? tempered1 : 0.0;
-    __syncwarp();
-    if (lane == 0) {
-        const double weight_sum = ordered_sum(fin.tempered, cutoff);
-        if (!(weight_sum > 0.0) || isinf(weight_sum) || isnan(weight_sum)) {
-            fin.status = kErrFormat;  // "sampler temperature softmax failed"
-        } else {
-            float u = uniform;
-            if (is_nonfinite(u) || u < 0.0f) u = 0.0f;
-            if (u >= 1.0f) u = __uint_as_float(0x3f7fffffu);  // nextafterf(1, 0)
-            const double draw = (double)u * weight_sum;
-            fin.picked = min(cutoff - 1u, ordered_reach<true>(fin.tempered, cutoff, draw));
-            if (out.dbg_tempered)
-                for (uint32_t i = 0; i < cutoff; i++) fin.tempered[i] = fin.tempered[i] / weight_sum;
-        }
-    }
-    __syncwarp();
-    if (fin.status != kOk) {
-        if (lane == 0) {
-            report_row(out, row, fin.status, kPaddingId, 0.0f);
-            if (out.dbg_count) out.dbg_count[row] = 0;
-        }
-        return;
-    }
-    if (lane == 0) report_row(out, row, kOk, fin.id[fin.picked], fin.score[fin.picked]);
+    float u = uniform;
+    if (is_nonfinite(u) || u < 0.0f) u = 0.0f;
+    if (u >= 1.0f) u = __uint_as_float(0x3f7fffffu);  // nextafterf(1, 0)
+    const double draw = (double)u * weight_sum;
+    const uint32_t picked = first_place(i0 < cutoff && draw < fin.tempered[i0], i1 < cutoff && draw < fin.tempered[i1],
+                                        cutoff - 1u);
+    if (lane == 0) report_row(out, row, kOk, fin.id[picked], fin.score[picked]);
     if (out.dbg_count) {
         if (lane == 0) out.dbg_count[row] = n;
-        for (uint32_t i = lane; i < kMaxK; i += 32) {
-            const size_t at = (size_t)row * kMaxK + i;
+        const size_t at = (size_t)row * kMaxK;
+#pragma unroll
+        for (uint32_t h = 0; h < 2; h++) {
+            const uint32_t i = lane + 32 * h;
             const bool live = i < n;
-            if (out.dbg_ids) out.dbg_ids[at] = live ? fin.id[i] : kPaddingId;
-            if (out.dbg_scores) out.dbg_scores[at] = live ? fin.score[i] : 0.0f;
-            if (out.dbg_raw) out.dbg_raw[at] = live ? fin.raw[i] : 0.0;
-            if (out.dbg_tempered) out.dbg_tempered[at] = live ? fin.tempered[i] : 0.0;
+            if (out.dbg_ids) out.dbg_ids[at + i] = live ? fin.id[i] : kPaddingId;
+            if (out.dbg_scores) out.dbg_scores[at + i] = live ? fin.score[i] : 0.0f;
+            if (out.dbg_raw) out.dbg_raw[at + i] = live ? (h ? raw1 : raw0) : 0.0;
+            if (out.dbg_tempered) out.dbg_tempered[at + i] = i < cutoff ? (h ? tempered1 : tempered0) / weight_sum : 0.0;
         }
     }
 }
