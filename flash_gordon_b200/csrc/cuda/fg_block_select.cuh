@@ -223,8 +223,9 @@ __device__ __forceinline__ void report_row(const SelectOutput &out, uint32_t row
 
 // x[i] becomes x[0] + ... + x[i], added from the left with one rounding per addition, as the C
 // loops of src/sampler.c:99-111 do; the loads of four terms go ahead of their additions.  Returns
-// the sum of all n.
-__device__ __forceinline__ double running_sums(double *x, uint32_t n) {
+// the sum of all n.  With `limit` it stops soon after a sum that has reached it: later places keep
+// their terms.
+__device__ __forceinline__ double running_sums(double *x, uint32_t n, const double *limit = nullptr) {
     double sum = 0.0;
     uint32_t i = 0;
     for (; i + 4 <= n; i += 4) {
@@ -235,6 +236,7 @@ __device__ __forceinline__ double running_sums(double *x, uint32_t n) {
         x[i + 1] = s1;
         x[i + 2] = s2;
         x[i + 3] = sum;
+        if (limit != nullptr && sum >= *limit) return sum;
     }
     for (; i < n; i++) {
         sum += x[i];
@@ -243,17 +245,33 @@ __device__ __forceinline__ double running_sums(double *x, uint32_t n) {
     return sum;
 }
 
+// Inclusive sums over the lanes' terms of up to 64 places (the second 32 only if `two`).
+__device__ __forceinline__ void scan_places(double &low, double &high, bool two) {
+    const uint32_t lane = lane_id();
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const double up = __shfl_up_sync(kFullMask, low, d);
+        low += lane >= (uint32_t)d ? up : 0.0;
+        if (two) {
+            const double up_high = __shfl_up_sync(kFullMask, high, d);
+            high += lane >= (uint32_t)d ? up_high : 0.0;
+        }
+    }
+    high += __shfl_sync(kFullMask, low, 31);
+}
+
 // Final step for one row; called by one warp of the CTA (all 32 lanes) with the
 // candidates already in sampling order in fin.score/id[0..n), n = min(top_k,
 // #finite).  Greedy rows never come here.
 //
-// What bounds it: the additions, which have to be made one after the other in the reference's order.
-// There are two chains of n of them.  The raw weights' sum and the tempered weights' running sums are
-// made side by side by two lanes (how far the nucleus reaches is not known by then, but a running
-// sum is there for every length); the quotients' running sums follow.  Both edges -- where top_p is
-// reached, where the draw lands -- are then compares of all lanes.  (Four chains of one lane, two of
-// them with a compare and a branch per addition, took 1.5 us longer: 64 rows of 151,936 logits, k = 20, 26.1 us
-// a call then and 24.6 now; 1024 rows, k = 50, 143.7 and 140.5.)
+// What bounds it: chains of fp64 operations, 30 cycles each; in the reference's order n additions for
+// the raw weights' sum and n more for the quotients' (the tempered weights' running sums are made
+// beside the first).  But those sums decide no more than where one of them passes top_p and where the
+// draw lands.  So they are first made by a scan over the lanes, and only if one of the two edges lies
+// within 1e-13 (of the total) of a sum -- the two ways of adding 64 positive terms differ by 2e-14 at
+// most, see below -- or if the quotients are asked for, the chains decide.  (2.2 thousand cycles for 20
+// candidates instead of 3.1, 2.9 instead of 4.6 for 50; 1024 rows 144.6 us a call before, 142.7 now, 256 rows of a
+// shard and their merge 37.4 and 35.5.)
 __device__ inline void finish_select(FinishBuffer &fin, uint32_t n, const SamplerConfig &cfg,
                               float uniform, uint32_t row, const SelectOutput &out) {
     const uint32_t lane = lane_id();
@@ -279,6 +297,37 @@ __device__ inline void finish_select(FinishBuffer &fin, uint32_t n, const Sample
         raw1 = exp(s1 - top_raw);
         tempered1 = exp(s1 / temperature - top_tempered);
     }
+    // the first of the 64 places at which something holds; `otherwise` when at none
+    auto first_place = [](bool here0, bool here1, uint32_t otherwise) {
+        const uint32_t low = __ballot_sync(kFullMask, here0), high = __ballot_sync(kFullMask, here1);
+        return low ? (uint32_t)__ffs(low) - 1u : high ? (uint32_t)__ffs(high) + 31u : otherwise;
+    };
+    float u = uniform;
+    if (is_nonfinite(u) || u < 0.0f) u = 0.0f;
+    if (u >= 1.0f) u = __uint_as_float(0x3f7fffffu);  // nextafterf(1, 0)
+    const double top_p = (double)cfg.top_p;
+    if (out.dbg_count == nullptr) {
+        // A sum of n <= 64 positive terms added from the left is off by at most n 2^-53 of itself, 7.1e-15,
+        // one added by the scan by 8 * 2^-53; the reference compares sums of quotients by such a sum with
+        // top_p (1.5e-14 together), and such a sum with a multiple of another (the same).
+        constexpr double kMargin = 1e-13;
+        double r0 = i0 < n ? raw0 : 0.0, r1 = i1 < n ? raw1 : 0.0;
+        double t0 = i0 < n ? tempered0 : 0.0, t1 = i1 < n ? tempered1 : 0.0;
+        scan_places(r0, r1, n > 32);
+        scan_places(t0, t1, n > 32);
+        const double sum = __shfl_sync(kFullMask, r1, 31), edge = top_p * sum, margin = kMargin * sum;
+        const uint32_t last = first_place(i0 < n && r0 >= edge, i1 < n && r1 >= edge, n - 1u);
+        bool near = fabs(r0 - edge) <= margin || fabs(r1 - edge) <= margin || !(sum > 0.0 && sum < 1e300);
+        const double low = __shfl_sync(kFullMask, t0, (int)(last & 31u)), high = __shfl_sync(kFullMask, t1, (int)(last & 31u));
+        const double weights = last < 32u ? low : high, draw = (double)u * weights, slack = kMargin * weights;
+        near = near || (i0 <= last && fabs(t0 - draw) <= slack) || (i1 <= last && fabs(t1 - draw) <= slack) ||
+               !(weights > 0.0 && weights < 1e300);
+        if (!__any_sync(kFullMask, near)) {
+            const uint32_t picked = first_place(i0 <= last && draw < t0, i1 <= last && draw < t1, last);
+            if (lane == 0) report_row(out, row, kOk, fin.id[picked], fin.score[picked]);
+            return;
+        }
+    }
     if (i0 < n) {
         fin.raw[i0] = raw0;
         fin.tempered[i0] = tempered0;
@@ -303,14 +352,8 @@ __device__ inline void finish_select(FinishBuffer &fin, uint32_t n, const Sample
     if (i0 < n) fin.raw[i0] = raw0;
     if (i1 < n) fin.raw[i1] = raw1;
     __syncwarp();
-    if (lane == 0) running_sums(fin.raw, n);
+    if (lane == 0) running_sums(fin.raw, n, &top_p);  // (the sums grow: the first that reaches it counts)
     __syncwarp();
-    // the first of the 64 places at which something holds; `otherwise` when at none
-    auto first_place = [](bool here0, bool here1, uint32_t otherwise) {
-        const uint32_t low = __ballot_sync(kFullMask, here0), high = __ballot_sync(kFullMask, here1);
-        return low ? (uint32_t)__ffs(low) - 1u : high ? (uint32_t)__ffs(high) + 31u : otherwise;
-    };
-    const double top_p = (double)cfg.top_p;
     const uint32_t cutoff = first_place(i0 < n && fin.raw[i0] >= top_p, i1 < n && fin.raw[i1] >= top_p, n - 1u) + 1u;
     const double weight_sum = fin.tempered[cutoff - 1u];
     if (!(weight_sum > 0.0) || isinf(weight_sum) || isnan(weight_sum)) {  // "sampler temperature softmax failed"
@@ -320,9 +363,6 @@ __device__ inline void finish_select(FinishBuffer &fin, uint32_t n, const Sample
         }
         return;
     }
-    float u = uniform;
-    if (is_nonfinite(u) || u < 0.0f) u = 0.0f;
-    if (u >= 1.0f) u = __uint_as_float(0x3f7fffffu);  // nextafterf(1, 0)
     const double draw = (double)u * weight_sum;
     const uint32_t picked = first_place(i0 < cutoff && draw < fin.tempered[i0], i1 < cutoff && draw < fin.tempered[i1],
                                         cutoff - 1u);
