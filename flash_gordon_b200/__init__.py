@@ -173,8 +173,9 @@ def load_library() -> ctypes.CDLL:
         "fg_cuda_output_greedy": (c_int, [P, P, POINTER(u32), POINTER(c_float), E]),
         "fg_cuda_output_sample": (c_int, [P, P, CFG, c_float, POINTER(u32), POINTER(c_float), E]),
         "fg_cuda_output_sample_sessions": (c_int, [P, POINTER(SampleArgs), P, E]),
-        # test seam of the ring kernel (csrc/host/fg_host_internal.h; not in the public headers)
+        # test seams of the ring and the team kernel (csrc/host/fg_host_internal.h; not in the public headers)
         "fg_cuda_internal_ring_controls": (c_int, [P, u32, u32, u32, u32, u32]),
+        "fg_cuda_internal_team_controls": (c_int, [P, u32, u32]),
     }
     for name, (restype, argtypes) in sig.items():
         fn = getattr(lib, name)

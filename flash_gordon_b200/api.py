@@ -130,6 +130,13 @@ class Context:
         if status != FG_OK:
             raise FgStatusError(status, "invalid ring controls")
 
+    def team_controls(self, team: int = 0, form: int = 0) -> None:
+        """Test seam of the team kernel: how many of its CTAs share a row (0 planner, 1, 2, 4, 8; 255: it is
+        not used) and its form (0 planner, 1 or 2)."""
+        status = self.lib.fg_cuda_internal_team_controls(self.handle, team, form)
+        if status != FG_OK:
+            raise FgStatusError(status, "invalid team controls")
+
     def set_path(self, path: int) -> None:
         """0 automatic, 1 register-prefetch kernel, 2 shared-memory ring kernel, 3 ring where rows allow."""
         err = FgError()

@@ -25,7 +25,8 @@ OBJ_DIR = PKG / "build"
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 CC = os.environ.get("CC", "gcc")
 
-CUDA_SOURCES = ["fg_stream_kernels.cu", "fg_persistent_kernel.cu", "fg_nucleus_kernel.cu", "fg_ops_kernels.cu",
+CUDA_SOURCES = ["fg_stream_kernels.cu", "fg_persistent_kernel.cu", "fg_team_kernel.cu", "fg_nucleus_kernel.cu",
+                "fg_ops_kernels.cu",
                 "fg_runtime.cu", "fg_nccl.cu"]
 HOST_SOURCES = ["fg_util.c", "fg_sampler_host.c", "fg_cuda_api.c", "fg_dist.c", "fg_output_wire.c",
                 "fg_request.c", "fg_output_exec.c"]

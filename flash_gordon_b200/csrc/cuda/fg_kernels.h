@@ -103,16 +103,16 @@ typedef struct fgk_stream_launch {
     uint32_t *history_global;
     uint64_t history_stride_words;
     void *history_meta; /* 8 bytes per (row, split); NULL when the batch has no history */
-    /* persistent kernel only: session tables in place of token lists (the stateful executor):
+    /* persistent and team kernel: session tables in place of token lists (the stateful executor):
      * counts [slots][vocab] and seen-bitmaps [slots][slot_bitmap_words], row r uses session
      * row_slots[r]; all three NULL otherwise */
     const uint32_t *slot_counts;
     const uint32_t *slot_bitmaps;
     const uint32_t *row_slots;
     uint32_t slot_bitmap_words;
-    /* persistent kernel only: polls before a device-side wait gives up (0 = the default, about
+    /* persistent and team kernel: polls before a device-side wait gives up (0 = the default, about
      * two seconds), and the test seam that makes one wait run out: warp 0 of CTA withhold_cta
-     * never asks the copy engine for its withhold_issue-th tile */
+     * never makes its withhold_issue-th request to the copy engine */
     uint32_t wait_polls;
     uint32_t withhold_armed, withhold_cta, withhold_issue;
     fgk_select_output out;
@@ -140,6 +140,23 @@ uint32_t fgk_persistent_tiles_abreast(void);
 uint32_t fgk_persistent_max_parts(uint32_t k);
 int fgk_persistent_prepare(void);
 int fgk_launch_persistent_select(const fgk_stream_launch *launch, uint32_t ctas, void *stream);
+
+/* ---- team kernel (fg_team_kernel.cu) ----
+ * Takes a fgk_stream_launch whose rows have a frequency penalty >= 0 and a repetition factor
+ * between 2^-40 and 2^40 (any alignment of the logits, any presence penalty); `team` CTAs (1, 2, 4 or
+ * 8) share a row, each with `chunk` columns (a multiple of 128), `bitmap_words` (a multiple of 32, 0 without
+ * a history) are those of a CTA's columns.  `which`: all rows, those whose penalties cannot raise a
+ * logit, or the others.  Needs no scratch. */
+enum { FGK_TEAM_ALL_ROWS = 0, FGK_TEAM_LOWERING_ROWS = 1, FGK_TEAM_RAISING_ROWS = 2 };
+#define FGK_TEAM_MOST 8u
+/* `form`: 0 as a rule, 1 holds more of a row at a time; whether a CTA's bitmap fits the form's shared memory,
+ * and the columns a CTA holds at a time */
+#define FGK_TEAM_FORMS 2u
+int fgk_team_fits(uint32_t form, uint32_t bitmap_words);
+uint32_t fgk_team_turn(uint32_t dtype, uint32_t form);
+int fgk_team_prepare(void);
+int fgk_launch_team_select(const fgk_stream_launch *launch, uint32_t team, uint32_t chunk, uint32_t form,
+                           uint32_t which, void *stream);
 
 typedef struct fgk_merge_launch {
     const float *scores;

@@ -52,6 +52,7 @@
 
 #include "fg_block_select.cuh"
 #include "fg_kernels.h"
+#include "fg_row_scan.cuh"
 
 namespace fgk {
 namespace persist {
@@ -69,35 +70,8 @@ constexpr int kTallyBins = 256;                 // bins of the per-unit score ta
 constexpr int kBlock = (kWarps + kHistoryWarps + kClosers) * 32;
 constexpr uint32_t kDefaultPolls = 1u << 21;    // polls before a wait gives up: a second or two
 constexpr uint32_t kNapNanoseconds = 400;       // sleep between two polls of a wait that may be long
-constexpr uint32_t kHugeBits = 0x6b000000u;     // |x| >= 2^87: a repetition factor <= 2^40 may reach inf
 constexpr uint32_t kSharedLimit = 227u * 1024u; // shared memory one CTA may ask for
 
-template <typename T>
-struct Lanes;
-template <>
-struct Lanes<float> {
-    static constexpr int kPer = 4;  // logits per 128-bit vector
-    static __device__ __forceinline__ void unpack(const uint4 &raw, float *v) {
-        v[0] = __uint_as_float(raw.x);
-        v[1] = __uint_as_float(raw.y);
-        v[2] = __uint_as_float(raw.z);
-        v[3] = __uint_as_float(raw.w);
-    }
-};
-template <>
-struct Lanes<uint16_t> {  // bf16 bit patterns
-    static constexpr int kPer = 8;
-    static __device__ __forceinline__ void unpack(const uint4 &raw, float *v) {
-        v[0] = __uint_as_float(raw.x << 16);
-        v[1] = __uint_as_float(raw.x & 0xffff0000u);
-        v[2] = __uint_as_float(raw.y << 16);
-        v[3] = __uint_as_float(raw.y & 0xffff0000u);
-        v[4] = __uint_as_float(raw.z << 16);
-        v[5] = __uint_as_float(raw.z & 0xffff0000u);
-        v[6] = __uint_as_float(raw.w << 16);
-        v[7] = __uint_as_float(raw.w & 0xffff0000u);
-    }
-};
 // A tile is kTileLogits logits whatever their type: 8 KB of fp32, 4 KB of bf16.
 template <typename T>
 __host__ __device__ constexpr uint32_t tile_bytes() { return kTileLogits * (uint32_t)sizeof(T); }
@@ -247,17 +221,6 @@ struct Row {
     bool greedy, seen_any, with_counts;
 };
 
-// Shared words that warps watch while others change them.
-__device__ __forceinline__ uint32_t peek(const uint32_t *word) {
-    return *reinterpret_cast<const volatile uint32_t *>(word);
-}
-__device__ __forceinline__ unsigned long long peek64(const unsigned long long *word) {
-    return *reinterpret_cast<const volatile unsigned long long *>(word);
-}
-__device__ __forceinline__ void poke(uint32_t *word, uint32_t value) {
-    *reinterpret_cast<volatile uint32_t *>(word) = value;
-}
-
 // Waits for a phase of an mbarrier, at most `polls` polls with a short sleep between them, and
 // not at all once another wait of the CTA has run out.  A wait that runs out raises
 // ring_error: the CTA's rows then end with FG_ERR_LIMIT and every later wait returns at
@@ -282,70 +245,6 @@ __device__ __forceinline__ bool tile_wait(Shared &sh, uint64_t *barrier, uint32_
     return false;
 }
 
-
-__device__ __forceinline__ uint64_t warp_max_u64(uint64_t v) {
-#pragma unroll
-    for (int d = 16; d >= 1; d >>= 1) {
-        const uint64_t other = __shfl_xor_sync(kFullMask, v, d);
-        v = other > v ? other : v;
-    }
-    return v;
-}
-__device__ __forceinline__ uint64_t warp_min_u64(uint64_t v) {
-#pragma unroll
-    for (int d = 16; d >= 1; d >>= 1) {
-        const uint64_t other = __shfl_xor_sync(kFullMask, v, d);
-        v = other < v ? other : v;
-    }
-    return v;
-}
-
-// Largest of three; a NaN loses against a number, as with fmaxf.
-__device__ __forceinline__ float fmax3(float a, float b, float c) {
-    float d;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-    return d;
-}
-
-// max(m, v...) that turns NaN as soon as one operand is NaN.
-template <int N>
-__device__ __forceinline__ float propagating_max(float m, const float (&v)[N]) {
-#pragma unroll
-    for (int i = 0; i < N; i++) asm("max.NaN.f32 %0, %0, %1;" : "+f"(m) : "f"(v[i]));
-    return m;
-}
-
-// Smallest of N values; a NaN loses against a number, as with fminf.
-template <int N>
-__device__ __forceinline__ float smallest(const float (&v)[N]) {
-    float m = v[0];
-#pragma unroll
-    for (int i = 1; i < N; i++) m = fminf(m, v[i]);
-    return m;
-}
-
-// Largest of N values, three at a time (a short tree instead of a chain of N - 1).
-template <int N>
-__device__ __forceinline__ float largest(const float (&v)[N]) {
-    float level[N];
-#pragma unroll
-    for (int i = 0; i < N; i++) level[i] = v[i];
-    int n = N;
-#pragma unroll
-    for (int round = 0; round < 6; round++) {
-        if (n <= 1) break;
-        int m = 0;
-#pragma unroll
-        for (int i = 0; i < N; i += 3) {
-            if (i >= n) break;
-            if (i + 2 < n) level[m++] = fmax3(level[i], level[i + 1], level[i + 2]);
-            else if (i + 1 < n) level[m++] = fmaxf(level[i], level[i + 1]);
-            else level[m++] = level[i];
-        }
-        n = m;
-    }
-    return level[0];
-}
 
 // One logit of a tile in shared memory, by its position in the tile.
 template <typename T>
@@ -1220,6 +1119,7 @@ __device__ __noinline__ void close_unit(Shared &sh, uint32_t closer, Lists &L, c
                                         const SamplerConfig cfg, bool shard_mode, uint32_t row_status) {
     const uint32_t lane = lane_id();
     const uint32_t row = u.row;
+    const float uniform = shard_mode || r.greedy ? 0.0f : __ldg(&p.uniforms[row]);  // (on its way meanwhile)
     FinishBuffer &fin = sh.fin[closer];
     uint32_t kept = settle_lists(fin, sh.hist[closer], &sh.gathered[closer], L, r);
     uint32_t bad_history = row_status ? row_status : L.bad_history;
@@ -1286,76 +1186,12 @@ __device__ __noinline__ void close_unit(Shared &sh, uint32_t closer, Lists &L, c
         __syncwarp();
         kept = settle_lists(fin, sh.hist[closer], &sh.gathered[closer], L, r);
     }
-    // ---- the row's result ----
-    if (shard_mode) {
-        // a greedy row's NaN/Inf with the smallest id goes first, as the slice's argmax
-        // cascade of src/output.c:320-344 would report it; the finite ones follow
-        const uint32_t lead = r.greedy && wild_id != kPaddingId ? 1u : 0u;
-        for (uint32_t i = lane; i < r.k; i += 32) {
-            const size_t at = ((size_t)row * r.k + i) * p.shard_stride;
-            const bool ok = i >= lead && i - lead < kept && !bad_history;
-            float score = ok ? fin.score[i - lead] : __uint_as_float(0xff800000u);
-            uint32_t id = ok ? fin.id[i - lead] : kPaddingId;
-            if (lead && i == 0 && !bad_history) {
-                score = __uint_as_float(wild_bits);
-                id = wild_id;
-            }
-            if (p.push.ranks != 0) {
-                // the fused exchange: the block lands in every rank's window, this one's too
-                for (uint32_t t = 0; t < p.push.ranks; t++)
-                    *p.push.pair(t, row, r.k, i) = make_uint2(__float_as_uint(score), id);
-            } else {
-                p.shard_scores[at] = score;
-                p.shard_ids[at] = id;
-            }
-        }
-        if (p.push.ranks != 0) {
-            __threadfence_system();  // the pairs are visible on the peers before the arrivals are
-            __syncwarp();
-            if (lane < p.push.ranks) atomicAdd_system(p.push.arrived(lane, row), 1u);
-        }
-        if (lane == 0) {
-            p.out.row_status[row] = bad_history;
-            if (bad_history) note_error(p.out, row, bad_history);
-        }
-        return;
-    }
-    if (bad_history) {  // "history token ... is outside vocabulary", src/output.c:610-612
-        if (lane == 0) {
-            report_row(p.out, row, bad_history, kPaddingId, 0.0f);
-            if (p.out.dbg_count) p.out.dbg_count[row] = 0;
-        }
-        return;
-    }
-    if (r.greedy) {
-        if (lane == 0) {
-            uint32_t status = kOk, token;
-            float logit;
-            if (wild_id != kPaddingId) {
-                // a NaN/Inf beats every finite logit in the argmax order and is then
-                // rejected: src/output.c:593 (no penalties) / 737-739 (penalised)
-                status = penalties_active(cfg) ? kErrFormat : kErrMismatch;
-                token = wild_id;
-                logit = __uint_as_float(wild_bits);
-            } else if (kept == 0) {
-                status = kErrMismatch;
-                token = kPaddingId;
-                logit = 0.0f;
-            } else {
-                token = fin.id[0];
-                logit = fin.score[0];
-            }
-            report_row(p.out, row, status, token, logit);
-            if (p.out.dbg_count) {
-                const bool ok = status == kOk;
-                p.out.dbg_count[row] = ok ? 1u : 0u;
-                if (p.out.dbg_ids) p.out.dbg_ids[(size_t)row * kMaxK] = ok ? token : kPaddingId;
-                if (p.out.dbg_scores) p.out.dbg_scores[(size_t)row * kMaxK] = ok ? logit : 0.0f;
-            }
-        }
-        return;
-    }
-    finish_select(fin, kept, cfg, p.uniforms[row], row, p.out);
+    RowResult result;
+    result.kept = kept;
+    result.wild_id = wild_id;
+    result.wild_bits = wild_bits;
+    result.bad_history = bad_history;
+    finish_row(p, fin, result, r.k, r.greedy, cfg, uniform, row);
 }
 
 // One warp's share (`part` of `parts`) of a unit's history bitmap.  First the words of the

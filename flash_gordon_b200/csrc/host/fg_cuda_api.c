@@ -96,6 +96,7 @@ fg_status fg_cuda_context_create(int device, fg_cuda_context **out, fg_error *er
     if (!e) e = fgk_stream_create(&c->own_stream);
     if (!e) e = fgk_stream_prepare();
     if (!e) e = fgk_persistent_prepare();
+    if (!e) e = fgk_team_prepare();
     if (!e) e = fgk_nucleus_prepare(c->nucleus_teams);
     if (!e) e = fgk_malloc((void **)&c->errors, 256u);
     if (!e) e = fgk_memset_async(c->errors, 0xff, 256u, c->own_stream);
@@ -186,6 +187,17 @@ fg_status fg_cuda_internal_ring_controls(fg_cuda_context *c, uint32_t deal, uint
     c->ring_withhold_armed = armed;
     c->ring_withhold_cta = cta;
     c->ring_withhold_issue = issue;
+    return FG_OK;
+}
+
+/* Test seam (declared in fg_host_internal.h only): how many CTAs of the team kernel share a row
+ * (0 as the planner likes, 1, 2, 4 or 8; 255: that kernel is not used) and which of its forms is
+ * taken where its shared memory suffices (0 as the planner likes, else one more than the form). */
+fg_status fg_cuda_internal_team_controls(fg_cuda_context *c, uint32_t team, uint32_t form) {
+    if (!c || (team != 255u && (team > FGK_TEAM_MOST || (team & (team - 1u)) != 0u)) || form > FGK_TEAM_FORMS)
+        return FG_ERR_ARGUMENT;
+    c->team_size = team;
+    c->team_form = form;
     return FG_OK;
 }
 
@@ -569,6 +581,7 @@ typedef struct batch_traits {
     bool penalties, counts, sampled, topk_rows;
     uint32_t nucleus; /* rows without a top-k cut */
     uint32_t raising; /* rows with a top-k cut whose penalties can raise a logit (or with an extreme repetition factor) */
+    uint32_t wild;    /* those of them whose charge does not grow with the count, or with an extreme factor */
 } batch_traits;
 
 static fg_status check_batch(const fg_cuda_context *c, const fg_cuda_sample_args *a, bool shard,
@@ -594,8 +607,12 @@ static fg_status check_batch(const fg_cuda_context *c, const fg_cuda_sample_args
             traits->penalties = true;
             if (!(cfg->presence_penalty >= 0.0f && cfg->frequency_penalty >= 0.0f &&
                   cfg->repetition_penalty >= 1.0f && cfg->repetition_penalty <= 0x1p40f) &&
-                (shard || cfg->temperature == 0.0f || cfg->top_k != 0u))
+                (shard || cfg->temperature == 0.0f || cfg->top_k != 0u)) {
                 traits->raising++;
+                if (!(cfg->frequency_penalty >= 0.0f && cfg->repetition_penalty >= 0x1p-40f &&
+                      cfg->repetition_penalty <= 0x1p40f))
+                    traits->wild++;
+            }
         }
         if (cfg->frequency_penalty != 0.0f) traits->counts = true;
         if (cfg->temperature != 0.0f) {
@@ -721,6 +738,37 @@ static bool scans_cost_more(const fg_cuda_sample_args *a) {
     return scans > 2900.0 && (double)a->rows * (double)a->vocab < 19.0 * scans * sqrt(scans);
 }
 
+/* How many CTAs of the team kernel share a row, each one's columns and the kernel's form; 0: the batch is not for
+ * that kernel.  It beats the ring kernel everywhere but in large fp32 batches, which are bound by HBM and
+ * take fewer steps there.  Measured (B200, us a call, rows of 151,936; ring kernel / teams of 1 / 2 / 4 / 8 CTAs):
+ * fp32, k = 20, 512 tokens: 1 row 23 / 25 / 17 / 14 / 12, 32 rows 25 / 30 / 18 / 15 / 15, 64 rows 25 / 30 / 19 / 18 / 27,
+ * 148 rows 28 / 33 / 26 / 40 / 49, 296 rows 43 / 45 / 46, 512 rows 71 / 73 / 78, 1024 rows 118 / 131; k = 50,
+ * 4,096 tokens to be counted: 1 row 29 / 33 / 25 / 21 / 19, 148 rows 44 / 40 / 38, 512 rows 92 / 86, 1024 rows
+ * 147 / 153; greedy: 1 row 16 / 17 / 12 / 10 / 8, 512 rows 58 / 53, 1024 rows 97 / 100; bf16, k = 20: 64 rows
+ * 26 / 21 / 16 / 18, 1024 rows 115 / 80. */
+static uint32_t plan_team(const fg_cuda_context *c, const fg_cuda_sample_args *a, const batch_traits *traits,
+                          bool ring, uint32_t *chunk, uint32_t *form, uint32_t *bitmap_words) {
+    const size_t element = a->dtype == FG_CUDA_BF16 ? 2u : 4u;
+    if (c->team_size == 255u || c->path != FG_CUDA_PATH_AUTO || c->forced_splits != 0u || c->ring_deal != 0u ||
+        (c->ring_withhold_armed && !c->team_size) || traits->wild != 0u || ((uintptr_t)a->logits % element) != 0u)
+        return 0u;
+    uint32_t team = c->team_size;
+    if (!team) {
+        if (a->vocab > (1u << 20)) return 0u;
+        if (ring && a->dtype == FG_CUDA_F32 && (uint64_t)a->rows * a->vocab > 100000000u) return 0u;
+        team = a->rows * 8u <= c->sm_count ? 8u : a->rows * 4u <= 2u * c->sm_count ? 4u : a->rows <= c->sm_count ? 2u : 1u;
+        while (team > 1u && a->vocab / team < 4096u) team /= 2u;
+    }
+    for (;; team *= 2u) {
+        *chunk = (uint32_t)fg_align_up_u64((a->vocab + team - 1u) / team, 128u);
+        *bitmap_words = traits->penalties ? (*chunk / 32u + 31u) / 32u * 32u : 0u;
+        *form = *chunk > fgk_team_turn(a->dtype, 0u) && fgk_team_fits(1u, *bitmap_words) ? 1u : 0u;
+        if (c->team_form && fgk_team_fits(c->team_form - 1u, *bitmap_words)) *form = c->team_form - 1u;
+        if (fgk_team_fits(*form, *bitmap_words)) return team;
+        if (team == FGK_TEAM_MOST) return 0u;
+    }
+}
+
 static fg_status run_stream(fg_cuda_context *c, const fg_cuda_sample_args *a,
                             const batch_traits *traits, uint32_t vocab_offset,
                             uint32_t vocab_total, uint32_t shard_k, float *shard_scores,
@@ -801,6 +849,22 @@ static fg_status run_stream(fg_cuda_context *c, const fg_cuda_sample_args *a,
         fg_error_set(err, FG_ERR_ARGUMENT,
                      "the ring path needs whole 16-byte aligned rows and penalties that only lower logits");
         return FG_ERR_ARGUMENT;
+    }
+    uint32_t chunk = 0u, form = 0u, team_words = 0u;
+    const uint32_t team = both ? 0u : plan_team(c, a, traits, all_ring && aligned, &chunk, &form, &team_words);
+    if (team != 0u) {
+        l.bitmap_words = team_words;
+        l.slot_counts = c->session_counts;
+        l.slot_bitmaps = c->session_bitmaps;
+        l.row_slots = c->session_rows;
+        l.slot_bitmap_words = c->session_bitmap_words;
+        l.wait_polls = c->ring_wait_polls;
+        l.withhold_armed = c->ring_withhold_armed;
+        l.withhold_cta = c->ring_withhold_cta;
+        l.withhold_issue = c->ring_withhold_issue;
+        c->last_scratch_bytes = a->config_count > 1u ? (size_t)a->rows * sizeof(fg_sampler_config) : 0u;
+        const int e = launched(c, fgk_launch_team_select(&l, team, chunk, form, FGK_TEAM_ALL_ROWS, c->stream));
+        return e ? fg_cuda_fail(err, e, "team kernel") : FG_OK;
     }
     /* AUTO: the persistent kernel whenever it can take the batch. */
     const uint32_t most = c->sm_count; /* one CTA per SM */

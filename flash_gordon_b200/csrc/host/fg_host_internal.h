@@ -16,6 +16,7 @@ struct fg_cuda_context {
     uint32_t path;          /* FG_CUDA_PATH_* */
     /* test seam of the ring kernel (fg_cuda_internal_ring_controls) */
     uint32_t ring_deal, ring_wait_polls, ring_withhold_armed, ring_withhold_cta, ring_withhold_issue;
+    uint32_t team_size, team_form; /* test seam of the team kernel (fg_cuda_internal_team_controls) */
 
     /* Set by the stateful executor around a call: the batch's penalties come from session
      * tables (counts [slots][vocab], seen-bitmaps [slots][words], one session index per row)
@@ -81,6 +82,7 @@ void fg_cuda_default_lock(void);
 void fg_cuda_default_unlock(void);
 fg_status fg_cuda_internal_ring_controls(fg_cuda_context *context, uint32_t deal, uint32_t wait_polls,
                                          uint32_t armed, uint32_t cta, uint32_t issue);
+fg_status fg_cuda_internal_team_controls(fg_cuda_context *context, uint32_t team, uint32_t form);
 /* The two steps of the vocabulary-sharded mode with an explicit candidate layout (stride 1:
  * separate score and id arrays; 2: interleaved (value, id) pairs); both only enqueue.  The
  * multi-GPU layer calls them with its exchange buffers. */

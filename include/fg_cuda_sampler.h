@@ -63,16 +63,16 @@ uint64_t fg_cuda_context_launches(const fg_cuda_context *context);
  * fused path (0 = chosen per call from rows, vocabulary and SM count; at most
  * 16).  Results never depend on it. */
 fg_status fg_cuda_context_set_splits(fg_cuda_context *context, uint32_t splits, fg_error *err);
-/* Tuning knob, no reference counterpart: which of the two fused kernels a batch
+/* Tuning knob, no reference counterpart: which of the fused kernels a batch
  * with a top-k cut takes — the persistent kernel that streams rows through a
  * shared-memory ring fed by bulk copies (rows whose start, stride and length are
  * multiples of 16 bytes, penalties that cannot raise a logit), or the
- * register-prefetch kernel (anything).  AUTO is the library's choice: the ring
- * kernel whenever it can take the batch, unaligned rows included (unless long
- * histories with a frequency penalty make the other one faster for them), and for
- * the rows it can take of a large batch with few raising penalties.  RING fails
+ * register-prefetch kernel (anything).  AUTO is the library's choice: as a rule a third kernel, in which
+ * up to eight CTAs share a row; for large fp32 batches the ring kernel, with the register-prefetch
+ * kernel for raising penalties, and that one alone for what neither of the others takes (negative
+ * frequency penalties, extreme repetition factors).  RING fails
  * with FG_ERR_ARGUMENT on a batch it cannot take or whose rows are not aligned,
- * RING_IF_POSSIBLE falls back instead (as AUTO does).
+ * RING_IF_POSSIBLE falls back to the register-prefetch kernel instead.
  * Results never depend on it. */
 #define FG_CUDA_PATH_AUTO             0u
 #define FG_CUDA_PATH_REGISTERS        1u
