@@ -963,8 +963,8 @@ __global__ void __launch_bounds__(kThreads, 2) team_select_kernel(const __grid_c
             }
         }
     }
-    const uint32_t share = 2u * vectors.span;  // a warp's vectors of the turn
-    const uint32_t warps = max(1u, min((uint32_t)kWarps, (vectors.count + share - 1u) / share));
+    // (a last warp with less than half a warp's vectors has too few keys to bound the others)
+    const uint32_t warps = max(1u, min((uint32_t)kWarps, (vectors.count + vectors.span) / (2u * vectors.span)));
     uint32_t top;
     uint32_t low = bound_of_lanes(key, k, warps, k > 1u && !one_turn, &top);
     if (k == 1u) low = top;

@@ -745,9 +745,14 @@ static bool scans_cost_more(const fg_cuda_sample_args *a) {
  * 148 rows 28 / 33 / 26 / 40 / 49, 296 rows 43 / 45 / 46, 512 rows 71 / 73 / 78, 1024 rows 118 / 131; k = 50,
  * 4,096 tokens to be counted: 1 row 29 / 33 / 25 / 21 / 19, 148 rows 44 / 40 / 38, 512 rows 92 / 86, 1024 rows
  * 147 / 153; greedy: 1 row 16 / 17 / 12 / 10 / 8, 512 rows 58 / 53, 1024 rows 97 / 100; bf16, k = 20: 64 rows
- * 26 / 21 / 16 / 18, 1024 rows 115 / 80. */
+ * 26 / 21 / 16 / 18, 1024 rows 115 / 80.
+ * What the ring kernel does not take was the streaming kernel's, which tabulates histories: that pays when they
+ * cover much of a vocabulary (48 batches of up to 60 M logits with a token for every column, us there / here: 0.3 to
+ * 2.2 times, 0.8 in the mean; with half as many 1.1, with a tenth 1.6, with fewer 2.4).  Greedy rows whose
+ * history covers an eighth of the vocabulary or more have few unseen logits at the top: the ring kernel's bound,
+ * which rises with every one it meets, is the better one (73 rows of 19,200 logits, 5,277 tokens 15 us there, 29 here). */
 static uint32_t plan_team(const fg_cuda_context *c, const fg_cuda_sample_args *a, const batch_traits *traits,
-                          bool ring, uint32_t *chunk, uint32_t *form, uint32_t *bitmap_words) {
+                          bool ring, uint32_t rows, uint32_t *chunk, uint32_t *form, uint32_t *bitmap_words) {
     const size_t element = a->dtype == FG_CUDA_BF16 ? 2u : 4u;
     if (c->team_size == 255u || c->path != FG_CUDA_PATH_AUTO || c->forced_splits != 0u || c->ring_deal != 0u ||
         (c->ring_withhold_armed && !c->team_size) || traits->wild != 0u || ((uintptr_t)a->logits % element) != 0u)
@@ -755,8 +760,10 @@ static uint32_t plan_team(const fg_cuda_context *c, const fg_cuda_sample_args *a
     uint32_t team = c->team_size;
     if (!team) {
         if (a->vocab > (1u << 20)) return 0u;
-        if (ring && a->dtype == FG_CUDA_F32 && (uint64_t)a->rows * a->vocab > 100000000u) return 0u;
-        team = a->rows * 8u <= c->sm_count ? 8u : a->rows * 4u <= 2u * c->sm_count ? 4u : a->rows <= c->sm_count ? 2u : 1u;
+        if (ring && a->dtype == FG_CUDA_F32 && (uint64_t)rows * a->vocab > 100000000u) return 0u;
+        if (!ring && traits->penalties && a->history_max > a->vocab / 2u) return 0u;
+        if (ring && !traits->sampled && traits->penalties && !c->session_counts && a->history_max > a->vocab / 8u) return 0u;
+        team = rows * 8u <= c->sm_count ? 8u : rows * 4u <= 2u * c->sm_count ? 4u : rows <= c->sm_count ? 2u : 1u;
         while (team > 1u && a->vocab / team < 4096u) team /= 2u;
     }
     for (;; team *= 2u) {
@@ -850,21 +857,29 @@ static fg_status run_stream(fg_cuda_context *c, const fg_cuda_sample_args *a,
                      "the ring path needs whole 16-byte aligned rows and penalties that only lower logits");
         return FG_ERR_ARGUMENT;
     }
-    uint32_t chunk = 0u, form = 0u, team_words = 0u;
-    const uint32_t team = both ? 0u : plan_team(c, a, traits, all_ring && aligned, &chunk, &form, &team_words);
-    if (team != 0u) {
-        l.bitmap_words = team_words;
-        l.slot_counts = c->session_counts;
-        l.slot_bitmaps = c->session_bitmaps;
-        l.row_slots = c->session_rows;
-        l.slot_bitmap_words = c->session_bitmap_words;
-        l.wait_polls = c->ring_wait_polls;
-        l.withhold_armed = c->ring_withhold_armed;
-        l.withhold_cta = c->ring_withhold_cta;
-        l.withhold_issue = c->ring_withhold_issue;
-        c->last_scratch_bytes = a->config_count > 1u ? (size_t)a->rows * sizeof(fg_sampler_config) : 0u;
-        const int e = launched(c, fgk_launch_team_select(&l, team, chunk, form, FGK_TEAM_ALL_ROWS, c->stream));
-        return e ? fg_cuda_fail(err, e, "team kernel") : FG_OK;
+    l.slot_counts = c->session_counts;
+    l.slot_bitmaps = c->session_bitmaps;
+    l.row_slots = c->session_rows;
+    l.slot_bitmap_words = c->session_bitmap_words;
+    l.wait_polls = c->ring_wait_polls;
+    l.withhold_armed = c->ring_withhold_armed;
+    l.withhold_cta = c->ring_withhold_cta;
+    l.withhold_issue = c->ring_withhold_issue;
+    {
+        fgk_stream_launch t = l;
+        uint32_t chunk = 0u, form = 0u;
+        const uint32_t others = both ? a->rows - traits->nucleus - raising : a->rows;
+        uint32_t team = plan_team(c, a, traits, all_ring && aligned, others, &chunk, &form, &t.bitmap_words);
+        if (team != 0u) {
+            c->last_scratch_bytes = a->config_count > 1u ? (size_t)a->rows * sizeof(fg_sampler_config) : 0u;
+            int e = launched(c, fgk_launch_team_select(&t, team, chunk, form, both ? FGK_TEAM_LOWERING_ROWS : FGK_TEAM_ALL_ROWS,
+                                                       c->stream));
+            if (!e && both) { /* (more CTAs for fewer rows: a raising row looks at more of its logits) */
+                team = plan_team(c, a, traits, false, raising * 2u, &chunk, &form, &t.bitmap_words);
+                e = launched(c, fgk_launch_team_select(&t, team, chunk, form, FGK_TEAM_RAISING_ROWS, c->stream));
+            }
+            return e ? fg_cuda_fail(err, e, "team kernel") : FG_OK;
+        }
     }
     /* AUTO: the persistent kernel whenever it can take the batch. */
     const uint32_t most = c->sm_count; /* one CTA per SM */
@@ -916,14 +931,6 @@ static fg_status run_stream(fg_cuda_context *c, const fg_cuda_sample_args *a,
         l.bitmap_words = whole_bitmap;
         l.general = !aligned || both;
         l.skip_raising = both;
-        l.slot_counts = c->session_counts;
-        l.slot_bitmaps = c->session_bitmaps;
-        l.row_slots = c->session_rows;
-        l.slot_bitmap_words = c->session_bitmap_words;
-        l.wait_polls = c->ring_wait_polls;
-        l.withhold_armed = c->ring_withhold_armed;
-        l.withhold_cta = c->ring_withhold_cta;
-        l.withhold_issue = c->ring_withhold_issue;
         c->last_scratch_bytes = part_slots * (64u * 8u + 16u) + (size_t)a->rows * 4u +
                                 (a->config_count > 1u ? (size_t)a->rows * sizeof(fg_sampler_config) : 0u);
         const int e = launched(c, fgk_launch_persistent_select(&l, ctas, c->stream));
