@@ -780,11 +780,13 @@ static fg_status run_stream(fg_cuda_context *c, const fg_cuda_sample_args *a,
                             const batch_traits *traits, uint32_t vocab_offset,
                             uint32_t vocab_total, uint32_t shard_k, float *shard_scores,
                             uint32_t *shard_ids, uint32_t shard_stride, fg_error *err) {
-    /* Rows the copy engine can fetch whose penalties cannot raise a logit may go through the
-     * persistent ring kernel; rows whose penalties can, and anything the caller pinned to it, through the
-     * register-prefetch kernel.  A large batch with few raising rows goes through both, one after
-     * the other; a small one, or one with more of them, is faster through the second alone.  Measured (both
-     * against one kernel, us): one row in eight raising, bf16, 100,277 logits 148 rows 88 / 85, 200 rows 87 / 130, 400
+    /* Most batches are taken by the team kernel (plan_team).  What it leaves goes on as follows.  Rows the
+     * copy engine can fetch whose penalties cannot raise a logit may go through the persistent ring kernel;
+     * rows whose penalties can, and anything the caller pinned to it, through the register-prefetch kernel.
+     * A large batch with few raising rows (`both`) is two launches, one per kind of row: of the team kernel
+     * where it takes the rows, else of the ring and the register-prefetch kernel.  A small batch, or one
+     * with more raising rows, is faster through one launch.  Measured with the latter two kernels (both
+     * against one, us): one row in eight raising, bf16, 100,277 logits 148 rows 88 / 85, 200 rows 87 / 130, 400
      * rows 119 / 234; 39,552 logits 300 rows 85 / 76, 500 rows 94 / 116.  One in four, 152 rows of 100,277 91 / 112, 300
      * of 151,936 137 / 147, 900 of 39,552 147 / 174; every other one 118 / 111, 161 / 151, 166 / 196;
      * three in four 133 / 111, 179 / 144, 186 / 175. */
