@@ -709,8 +709,8 @@ __device__ __forceinline__ void conclude(const Params &p, uint32_t row, uint32_t
     Shared &sh = shared();
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, team = p.team;
     const uint32_t k = sh.row.k, first_id = sh.row.id_base;
-    float uniform = 0.0f;  // (on its way meanwhile)
-    if (rank == 0 && warp == 0 && p.uniforms != nullptr) uniform = __ldg(&p.uniforms[row]);
+    float uniform = 0.0f;  // (on its way meanwhile; rows that draw nothing may not have one)
+    if (rank == 0 && warp == 0 && p.shard_k == 0 && !sh.row.greedy) uniform = __ldg(&p.uniforms[row]);
     const uint32_t total = min(sh.count, kListCap);
     if (sh.row.with_counts && sh.row.counts == nullptr) settle(true);
     const uint64_t mine = tid < total ? sh.key[tid] : 0ull;  // (a thread's own entry)

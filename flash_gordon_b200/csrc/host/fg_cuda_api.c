@@ -839,7 +839,7 @@ static fg_status run_stream(fg_cuda_context *c, const fg_cuda_sample_args *a,
     l.config0 = a->configs[0];
     l.config_count = a->config_count;
     l.shard_k = shard_k;
-    l.uniforms = a->uniforms;
+    l.uniforms = !shard_k && traits->sampled ? a->uniforms : NULL; /* (else whatever the caller left there) */
     l.shard_scores = shard_scores;
     l.shard_ids = shard_ids;
     l.shard_stride = shard_stride;
