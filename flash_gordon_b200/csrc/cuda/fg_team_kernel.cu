@@ -1062,7 +1062,9 @@ extern "C" int fgk_team_prepare(void) {
 
 extern "C" int fgk_launch_team_select(const fgk_stream_launch *l, uint32_t team_size, uint32_t chunk, uint32_t form,
                                       uint32_t which, void *stream) {
-    if (!fgk_team_fits(form, l->bitmap_words)) return (int)cudaErrorInvalidValue;
+    if (team_size == 0 || team_size > team::kMostTeam || (team_size & (team_size - 1u)) != 0 || chunk % 128u != 0 ||
+        (uint64_t)team_size * chunk < l->vocab || !fgk_team_fits(form, l->bitmap_words))
+        return (int)cudaErrorInvalidValue;
     team::Params p;
     memset(&p, 0, sizeof(p));
     p.logits = l->logits;

@@ -868,18 +868,20 @@ static fg_status run_stream(fg_cuda_context *c, const fg_cuda_sample_args *a,
     l.withhold_cta = c->ring_withhold_cta;
     l.withhold_issue = c->ring_withhold_issue;
     {
-        fgk_stream_launch t = l;
-        uint32_t chunk = 0u, form = 0u;
+        /* (both launches are planned before the first is made: the team kernel takes all of a batch or nothing) */
+        fgk_stream_launch t = l, second = l;
+        uint32_t chunk = 0u, form = 0u, second_chunk = 0u, second_form = 0u, second_team = 0u;
         const uint32_t others = both ? a->rows - traits->nucleus - raising : a->rows;
-        uint32_t team = plan_team(c, a, traits, all_ring && aligned, others, &chunk, &form, &t.bitmap_words);
-        if (team != 0u) {
+        const uint32_t team = plan_team(c, a, traits, all_ring && aligned, others, &chunk, &form, &t.bitmap_words);
+        if (both) /* (more CTAs for fewer rows: a raising row looks at more of its logits) */
+            second_team = plan_team(c, a, traits, false, raising * 2u, &second_chunk, &second_form, &second.bitmap_words);
+        if (team != 0u && (!both || second_team != 0u)) {
             c->last_scratch_bytes = a->config_count > 1u ? (size_t)a->rows * sizeof(fg_sampler_config) : 0u;
             int e = launched(c, fgk_launch_team_select(&t, team, chunk, form, both ? FGK_TEAM_LOWERING_ROWS : FGK_TEAM_ALL_ROWS,
                                                        c->stream));
-            if (!e && both) { /* (more CTAs for fewer rows: a raising row looks at more of its logits) */
-                team = plan_team(c, a, traits, false, raising * 2u, &chunk, &form, &t.bitmap_words);
-                e = launched(c, fgk_launch_team_select(&t, team, chunk, form, FGK_TEAM_RAISING_ROWS, c->stream));
-            }
+            if (!e && both)
+                e = launched(c, fgk_launch_team_select(&second, second_team, second_chunk, second_form, FGK_TEAM_RAISING_ROWS,
+                                                       c->stream));
             return e ? fg_cuda_fail(err, e, "team kernel") : FG_OK;
         }
     }

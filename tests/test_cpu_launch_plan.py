@@ -67,3 +67,12 @@ def test_draws_that_no_row_uses_are_not_read(plan):
                 assert status == FG_OK and launches and all(l.endswith("uniforms=0") for l in launches), launches
             status, launches = plan([TOP_K], rows, vocab, offset=offset)
             assert status == FG_OK and all(l.endswith("uniforms=1") for l in launches), launches
+
+
+@pytest.mark.parametrize("team,chunk,form", [(0, 1024, 0), (3, 1024, 0), (16, 1024, 0), (2, 384, 0), (4, 200, 0), (1, 1024, 2)])
+def test_plans_that_cannot_be_launched_are_refused(library, team, chunk, form):
+    """Before anything is enqueued: no CTAs, a number that is no cluster's, columns that do not cover the row."""
+    launch = (c_uint32 * 512)()  # (larger than fgk_stream_launch)
+    launch[3], launch[4] = 1, 1000  # rows, vocab
+    refused = library.fgk_launch_team_select(launch, c_uint32(team), c_uint32(chunk), c_uint32(form), c_uint32(0), None)
+    assert refused == 1  # cudaErrorInvalidValue
