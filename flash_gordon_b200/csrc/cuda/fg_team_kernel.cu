@@ -13,7 +13,13 @@
 //   4. what reaches the bound, penalised if the history has seen its id, goes on a list, one entry to a
 //      thread.  Columns that did not fit shared memory at once come after that, turn by turn: vectors that hold
 //      something at or above the bound go into a queue as they are, so that the scan does not wait for what it
-//      finds, and from there on the list; when that grows long it is cut to its k best, which lifts the bound;
+//      finds, and from there on the list; when that grows long it is cut to its k best, which lifts the bound.
+//      A bound that lets whole vectors through -- a mask leaves fewer than k of the CTA's logits, they are all the same, or
+//      each is larger than those before -- shows in that most lanes find something.  Such vectors are sifted first
+//      (`sift`, `crowded`): logits equal to the bound count up to its id, those under it if the history has
+//      seen them, infinities never.  (64 fp32 rows of 151,936, 40 ids allowed, k = 50, us a call without it / with it / ring
+//      kernel: mask of -inf 66 / 17 / 118, of the lowest value 150 / 35 / 148, with penalties that raise 182 / 52 / 103
+//      (streaming kernel); rows that rise 220 / 134 / 219; ordinary ones 18.7 with and without);
 //   5. occurrences, if they matter, are counted in one walk over the tokens, with the entries' ids in a
 //      hash table (an entry is on the list by the most it can be worth, which is the charge for one occurrence);
 //   6. every CTA ranks its entries by counting the larger ones and hands its k best, in order, to the
@@ -52,6 +58,8 @@ constexpr uint32_t kQueueLong = 128;            // it is worked off between two 
 constexpr uint32_t kMostTeam = 8;
 constexpr uint32_t kMostRounds = 11;            // keys a warp contributes to a tight bound
 constexpr uint32_t kHashBits = 9, kHashSlots = 1u << kHashBits;  // twice the list
+constexpr uint32_t kLooseMost = 32;             // candidates that a loose bound is for: with more the list runs over at times
+constexpr float kFarApart = 64.0f;              // a bound so far below the largest logit is a mask's, and made tight
 constexpr uint32_t kDefaultPolls = 1u << 21;    // polls before a wait gives up: a second or two
 
 // Which rows a launch takes.
@@ -97,6 +105,7 @@ struct Row {
     uint32_t k;
     float flat_offset;             // charge for count = 1 (the exact charge when frequency is +-0)
     float presence, frequency, repetition;
+    uint32_t odd;                  // bits of |x| from here on: greedy rows must see it
     bool greedy, seen_any, with_counts, raises;
 };
 
@@ -121,7 +130,7 @@ struct alignas(128) Shared {
         struct {
             uint32_t id[kHashSlots], count[kHashSlots];
         } hash;                             // for counting
-        uint64_t order[kMostTeam * kMaxK];  // for ranking
+        alignas(16) uint64_t order[kMostTeam * kMaxK];  // for ranking
         struct {
             uint4 vector[kQueueCap];
             uint32_t column[kQueueCap];
@@ -163,6 +172,18 @@ __device__ __forceinline__ bool seen_column(const Row &r, uint32_t column) {
     return (seen_bitmap()[column >> 5] >> (column & 31u)) & 1u;
 }
 
+// The larger of `best` and a vector's largest finite logit among those the history has not seen.
+template <int N>
+__device__ __forceinline__ float largest_unseen(const float (&v)[N], uint32_t column, float best) {
+    const float most = largest(v);
+    if (!(most > best)) return best;
+    if (!shared().row.seen_any && !is_nonfinite(most)) return most;
+#pragma unroll
+    for (int j = 0; j < N; j++)
+        if (v[j] > best && !is_nonfinite(v[j]) && !seen_column(shared().row, column + (uint32_t)j)) best = v[j];
+    return best;
+}
+
 // Raw logits under this cannot reach tau: unseen ones are their own value; of a seen one `most` is
 // the most it can be worth, and that grows with the logit.
 __device__ __noinline__ float raw_floor(float tau) {
@@ -179,17 +200,82 @@ __device__ __noinline__ float raw_floor(float tau) {
     }
     return __uint_as_float(0xff800000u);
 }
-__device__ __forceinline__ float floor_of(uint64_t bound) {
-    const float tau = key_to_float((uint32_t)(bound >> 32));
-    return shared().row.raises ? raw_floor(tau) : tau;
+
+// What a bound asks of a raw logit.  An unseen one must be larger than `tau`, or equal to it with an id up
+// to `last_id`; a seen one must reach `floor`, which is tau unless penalties may raise it.
+struct Gate {
+    uint64_t bound;
+    float tau, floor;
+    __device__ __forceinline__ uint32_t last_id() const { return ~(uint32_t)bound; }
+};
+__device__ __forceinline__ Gate gate_of(uint64_t bound) {
+    Gate g;
+    g.bound = bound;
+    g.tau = key_to_float((uint32_t)(bound >> 32));
+    g.floor = shared().row.raises ? raw_floor(g.tau) : g.tau;
+    return g;
+}
+// What the largest logit of a vector must be for a look at it, when no id in there is below `first_id`.  (An infinity is
+// no candidate: greedy rows find it otherwise.)
+__device__ __forceinline__ float gate_of_vectors(const Gate &g, uint32_t first_id) {
+    const bool ties_lose = !shared().row.raises && first_id > g.last_id();
+    const float at_least = ties_lose ? key_to_float((uint32_t)(g.bound >> 32) + 1u) : g.floor;
+    return fmaxf(at_least, -3.402823466e38f);
 }
 
 // NaN, infinities and magnitudes a repetition factor of 2^-40 to 2^40 could push there: greedy rows
-// must see them.
-__device__ __forceinline__ bool odd_value(float x) { return (__float_as_uint(x) & 0x7fffffffu) >= kHugeBits; }
+// must see them.  (The charge cannot: penalties are 2 at most, so it is less than the last place of such a
+// value, and whether the value becomes infinite does not depend on the count.)
+__device__ __forceinline__ bool odd_value(float x, uint32_t odd) { return (__float_as_uint(x) & 0x7fffffffu) >= odd; }
 template <int N>
-__device__ __forceinline__ bool odd_values(const float (&v)[N]) {
-    return !(propagating_max(v[0], v) < __uint_as_float(kHugeBits)) || smallest(v) <= -__uint_as_float(kHugeBits);
+__device__ __forceinline__ bool odd_values(const float (&v)[N], uint32_t odd) {
+    return !(propagating_max(v[0], v) < __uint_as_float(odd)) || smallest(v) <= -__uint_as_float(odd);
+}
+
+// A gate with what else decides over whole vectors, for where a mask, equal logits or a penalty that raises let many
+// through: few elements of theirs are left then.
+struct Sieve {
+    Gate gate;
+    uint32_t first_id, odd;
+    bool greedy, marked;  // marked: it makes a difference whether the history has seen a column
+};
+__device__ __forceinline__ Sieve sieve_of(const Gate &gate) {
+    const Row &r = shared().row;
+    return Sieve{gate, r.id_base, r.odd, r.greedy, r.seen_any && (r.greedy || r.raises)};
+}
+// Which of a vector's columns the history has seen, a bit each.
+template <int N>
+__device__ __forceinline__ uint32_t seen_columns(uint32_t column) {
+    const uint32_t word = column >> 5, shift = column & 31u;
+    const uint32_t *bitmap = seen_bitmap();
+    uint32_t seen = bitmap[word] >> shift;
+    if (shift + N > 32u) seen |= bitmap[word + 1u] << (32u - shift);  // (the vector ends in there)
+    return seen & ((1u << N) - 1u);
+}
+// Whether any element of a vector may be worth the bound.
+template <int N>
+__device__ __forceinline__ bool may_pass(const float (&v)[N], uint32_t column, const Sieve &s) {
+    const float most = largest(v);
+    return s.greedy || most > s.gate.tau || (most == s.gate.tau && s.first_id + column <= s.gate.last_id()) ||
+           (s.marked && seen_columns<N>(column) != 0);
+}
+// Which of them, a bit each.  Greedy rows also look at the first NaN or infinity (the smallest id counts) and at what
+// a penalty may turn into one.
+template <int N>
+__device__ __forceinline__ uint32_t passing(const float (&v)[N], uint32_t column, const Sieve &s) {
+    const uint32_t first = s.first_id + column, last = s.gate.last_id(), seen = s.marked ? seen_columns<N>(column) : 0u;
+    uint32_t pass = 0, wild = 0;
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+        const bool was_seen = (seen >> j) & 1u, finite = !is_nonfinite(v[j]);
+        const bool take = v[j] > s.gate.tau || (v[j] == s.gate.tau && first + (uint32_t)j <= last) ||
+                          (was_seen && (v[j] >= s.gate.floor || (s.greedy && odd_value(v[j], s.odd))));
+        pass |= (take && finite ? 1u : 0u) << j;
+        wild |= (finite ? 0u : 1u) << j;
+    }
+    if (s.greedy && wild != 0 && first + (uint32_t)__ffs(wild) - 1u < (uint32_t)(peek64(&shared().wild) >> 32))
+        pass |= wild & (0u - wild);
+    return pass;
 }
 
 // A bound for k lanes' keys: at least k of them are as large.  Loosely: every warp's j-th largest, j = ceil(k /
@@ -276,20 +362,16 @@ __device__ __forceinline__ Worth worth_of(float raw, uint32_t column, uint64_t b
     if (!is_nonfinite(w.value)) {
         w.key = select_key(w.value, id);
         if (w.key < bound) w.key = 0;
-    } else if (!w.waits && r.greedy) {
-        atomicMin(&sh.wild, ((unsigned long long)id << 32) | __float_as_uint(w.value));
+    } else if (r.greedy) {
+        atomicMin(&sh.wild, ((unsigned long long)id << 32) | __float_as_uint(w.value));  // (for any count: see odd_value)
     }
-    if (w.waits) {
-        if (r.greedy && w.key == 0 && (is_nonfinite(w.value) || odd_value(raw))) w.key = ~0ull;  // (to be looked at when it is counted)
-        w.value = raw;
-    }
+    if (w.waits) w.value = raw;
     return w;
 }
 __device__ __forceinline__ bool entry_waits(const Shared &sh, uint32_t i) { return (sh.waiting[i >> 5] >> (i & 31u)) & 1u; }
 
 // Counts the occurrences of the entries that wait for it, and gives them their exact value.  One that
-// the penalty turns into NaN/Inf (greedy rows note it) or that does not reach the bound is dead.  All
-// threads call; ends synced.  `last`: no id is looked up any more, and the
+// does not reach the bound is dead.  All threads call; ends synced.  `last`: no id is looked up any more, and the
 // bitmap of seen columns becomes one of those that are to be counted, which few tokens pass.
 __device__ __noinline__ void settle(bool last) {
     Shared &sh = shared();
@@ -356,9 +438,7 @@ __device__ __noinline__ void settle(bool last) {
             const uint32_t times = sh.hash.count[place];
             const float exact = times == 0 ? raw
                 : penalise_with_offset(raw, penalty_offset(times, r.presence, r.frequency), make_repetition(r.repetition));
-            uint64_t key = 0;
-            if (!is_nonfinite(exact)) key = select_key(exact, id);
-            else if (r.greedy) atomicMin(&sh.wild, ((unsigned long long)id << 32) | __float_as_uint(exact));
+            const uint64_t key = select_key(exact, id);  // (finite, as what it was listed by: see odd_value)
             sh.value[tid] = exact;
             sh.key[tid] = key >= peek64(&sh.bound) ? key : 0ull;
         }
@@ -372,13 +452,16 @@ __device__ __noinline__ void settle(bool last) {
 __device__ __forceinline__ void rank_entries(Shared &sh, uint32_t n) {
     const uint32_t tid = threadIdx.x;
     const uint32_t bits = n <= 32u ? 5u : n <= 64u ? 6u : n <= 128u ? 7u : 8u, parts = kThreads >> bits;
-    const uint32_t each = (n + parts - 1u) / parts;
+    const uint32_t each = ((n + parts - 1u) / parts + 1u) & ~1u;  // (two keys to a load)
     const uint32_t at = tid & ((1u << bits) - 1u), from = (tid >> bits) * each, to = min(n, from + each);
     if (at < n) {
         const uint64_t key = sh.order[at];
         uint32_t larger = 0;
-#pragma unroll 8
-        for (uint32_t j = from; j < to; j++) larger += sh.order[j] > key ? 1u : 0u;
+#pragma unroll 4
+        for (uint32_t j = from; j < to; j += 2) {  // (behind the last entry: zero)
+            const ulonglong2 two = *reinterpret_cast<const ulonglong2 *>(&sh.order[j]);
+            larger += (two.x > key ? 1u : 0u) + (two.y > key ? 1u : 0u);
+        }
         if (larger != 0) atomicAdd(&sh.rank[at], larger);
     }
     __syncthreads();
@@ -487,11 +570,12 @@ __device__ __forceinline__ uint32_t list_elements(const float (&v)[Lanes<T>::kPe
     constexpr int kPer = Lanes<T>::kPer;
     Shared &sh = shared();
     const uint32_t lane = lane_id();
+    const uint32_t odd = greedy ? sh.row.odd : 0u;
     uint32_t hits = 0, left = 0;
 #pragma unroll
     for (int j = 0; j < kPer; j++) {
         bool take = v[j] >= floor;
-        if (greedy) take = take || odd_value(v[j]);
+        if (greedy) take = take || odd_value(v[j], odd);
         hits |= (take ? 1u : 0u) << j;
     }
     hits &= mask;
@@ -546,9 +630,8 @@ __device__ __forceinline__ void list_all(const uint4 raw, uint32_t left, uint32_
     Lanes<T>::unpack(raw, v);
     bool hard = false;
     for (;;) {
-        const uint64_t bound = peek64(&sh.bound);
-        const float floor = floor_of(bound);
-        left = list_elements<T>(v, left, column, floor, bound, r.greedy);
+        const Gate gate = gate_of(peek64(&sh.bound));
+        left = list_elements<T>(v, left, column, gate.floor, gate.bound, r.greedy);
         if (!__syncthreads_or(left != 0)) break;
         tighten(hard);
         hard = true;  // (whatever the first cut has left: the next one makes room)
@@ -584,20 +667,95 @@ __device__ __noinline__ void work_off() {
     if (__syncthreads_or(sh.count > kListLong)) tighten(false);
 }
 
-// The queue is worked off, and what found it full (`pending`: vectors of the turn at `base`, a bit each)
-// put there after all.  All threads call; ends synced.
+// More than the queue holds is worth a look (`pending`: vectors of the turn at `base`, a bit each): the queue is worked
+// off, which lifts the bound, and filled with what still passes, until nothing is left.  After the first turn, whose
+// bound comes from all its lanes' largest logits, those of the pending vectors lift it before that.  All
+// threads call; ends synced.
 template <typename T, int kHalf>
 __device__ __noinline__ void crowded(const Vectors<T, kHalf> vectors, uint32_t base, uint32_t pending) {
+    constexpr int kPer = Lanes<T>::kPer;
+    constexpr int kBatch = 4;  // vectors on their way at a time
     Shared &sh = shared();
+    if (base != 0 && __syncthreads_or(pending != 0)) {
+        float best = __uint_as_float(0xff800000u);
+#pragma unroll 1
+        for (uint32_t rest = pending; rest != 0;) {
+            uint4 raw[kBatch];
+            uint32_t column[kBatch];
+#pragma unroll
+            for (int q = 0; q < kBatch; q++) {
+                const uint32_t number = vectors.number(base, (uint32_t)__ffs(rest != 0 ? rest : pending) - 1u);
+                raw[q] = vectors.fetch(number);
+                column[q] = vectors.column(number);
+                rest &= rest - 1u;
+            }
+#pragma unroll
+            for (int q = 0; q < kBatch; q++) {
+                float v[kPer];
+                Lanes<T>::unpack(raw[q], v);
+                best = largest_unseen(v, column[q], best);
+            }
+        }
+        uint32_t top;
+        const uint32_t key = bound_of_lanes(is_nonfinite(best) ? 0u : float_key(best), sh.row.k, kWarps, true, &top);
+        if (threadIdx.x == 0 && key != 0) atomicMax(&sh.bound, (unsigned long long)key << 32);
+    }
     do {
         work_off<T>();
+        const Sieve sieve = sieve_of(gate_of(peek64(&sh.bound)));
         uint32_t left = 0;
-        for (; pending != 0; pending &= pending - 1) {
-            const uint32_t u = (uint32_t)__ffs(pending) - 1u, number = vectors.number(base, u);
-            if (!enqueue(sh, vectors.fetch(number), vectors.column(number), (1u << Lanes<T>::kPer) - 1u)) left |= 1u << u;
+#pragma unroll 1
+        for (uint32_t rest = pending; rest != 0;) {
+            if (peek(&sh.queue_count) >= kQueueCap) {
+                left |= rest;
+                break;
+            }
+            uint4 raw[kBatch];
+            uint32_t bit[kBatch];
+#pragma unroll
+            for (int q = 0; q < kBatch; q++) {
+                bit[q] = rest & (0u - rest);
+                raw[q] = vectors.fetch(vectors.number(base, (uint32_t)__ffs(rest != 0 ? rest : pending) - 1u));
+                rest &= rest - 1u;
+            }
+#pragma unroll
+            for (int q = 0; q < kBatch; q++) {
+                if (bit[q] == 0) continue;
+                const uint32_t column = vectors.column(vectors.number(base, (uint32_t)__ffs(bit[q]) - 1u));
+                float v[kPer];
+                Lanes<T>::unpack(raw[q], v);
+                if (!may_pass(v, column, sieve)) continue;
+                const uint32_t mask = passing(v, column, sieve);
+                if (mask != 0 && !enqueue(sh, raw[q], column, mask)) left |= bit[q];
+            }
         }
         pending = left;
     } while (__syncthreads_or(pending != 0));
+}
+
+// A warp's half of a turn in which most lanes have found something: what passes goes into the queue.  Returns the
+// vectors that found it full, a bit each.  All lanes call.
+template <typename T, int kHalf>
+__device__ __noinline__ uint32_t sift(const uint4 *stage, uint32_t column, uint32_t hot, const Gate gate) {
+    constexpr int kPer = Lanes<T>::kPer;
+    const Sieve sieve = sieve_of(gate);
+    uint32_t full = 0, rest = 0;
+#pragma unroll
+    for (uint32_t u = 0; u < (uint32_t)kHalf; u++) {
+        float v[kPer];
+        Lanes<T>::unpack(stage[u * 32u], v);
+        if (((hot >> u) & 1u) && may_pass(v, column + u * 32u * kPer, sieve)) rest |= 1u << u;
+    }
+#pragma unroll 1
+    for (; rest != 0; rest &= rest - 1) {
+        const uint32_t u = (uint32_t)__ffs(rest) - 1u, at = column + u * 32u * kPer;
+        const uint4 raw = stage[u * 32u];
+        float v[kPer];
+        Lanes<T>::unpack(raw, v);
+        const uint32_t mask = passing(v, at, sieve);
+        if (mask != 0 && !enqueue(shared(), raw, at, mask)) full |= 1u << u;
+    }
+    return full;
 }
 
 // The turns of the scan after the first.  The warps run freely; when the queue has become long all stop
@@ -607,10 +765,11 @@ __device__ __forceinline__ void scan(const Params &p, Vectors<T, kHalf> &vectors
     constexpr int kPer = Lanes<T>::kPer;
     constexpr uint32_t kTurn = 2u * kHalf * kThreads;  // (more than one turn: whole ones)
     Shared &sh = shared();
+    const uint32_t odd = sh.row.odd;
     uint32_t base = kTurn, h = 0, parity = 1;
     for (;;) {
         uint32_t pending = 0;
-        const float floor = floor_of(peek64(&sh.bound));
+        const Gate gate = gate_of(peek64(&sh.bound));
         bool stopped = false;  // with a half looked at
         while (vectors.first_of(base, h) < vectors.count && !__any_sync(kFullMask, peek(&sh.queue_count) > kQueueLong)) {
             if (!vectors.wait(p, base, h, parity)) {
@@ -620,21 +779,27 @@ __device__ __forceinline__ void scan(const Params &p, Vectors<T, kHalf> &vectors
             const uint4 *stage = vectors.stage(p, h) + lane_id();
             const uint32_t first = vectors.number(base, h * kHalf);
             const int here = vectors.extent(base, h);
+            const float at_least = gate_of_vectors(gate, sh.row.id_base + vectors.column(vectors.first_of(base, h)));
             uint32_t hot = 0;
 #pragma unroll
             for (int u = 0; u < kHalf; u++) {
                 float v[kPer];
                 Lanes<T>::unpack(stage[u * 32], v);
-                bool look = largest(v) >= floor;
-                if (kGreedy) look = look || odd_values(v);
+                bool look = largest(v) >= at_least;
+                if (kGreedy) look = look || odd_values(v, odd);
                 hot |= (look && u * 32 < here ? 1u : 0u) << u;
             }
-            if (__any_sync(kFullMask, hot != 0)) {
+            const uint32_t finders = __ballot_sync(kFullMask, hot != 0);
+            if (finders != 0) {
+                if (__popc(finders) > 16) {  // (not what a row as such has to offer)
+                    pending |= sift<T, kHalf>(stage, vectors.column(first), hot, gate) << (h * kHalf);
+                } else {
 #pragma unroll 1
-                for (; hot != 0; hot &= hot - 1) {
-                    const uint32_t u = (uint32_t)__ffs(hot) - 1u;
-                    if (!enqueue(sh, stage[u * 32u], vectors.column(first + u * 32u), (1u << kPer) - 1u))
-                        pending |= 1u << (h * kHalf + u);
+                    for (; hot != 0; hot &= hot - 1) {
+                        const uint32_t u = (uint32_t)__ffs(hot) - 1u;
+                        if (!enqueue(sh, stage[u * 32u], vectors.column(first + u * 32u), (1u << kPer) - 1u))
+                            pending |= 1u << (h * kHalf + u);
+                    }
                 }
                 __syncwarp();
                 stopped = __any_sync(kFullMask, pending != 0);
@@ -866,6 +1031,7 @@ __global__ void __launch_bounds__(kThreads, 2) team_select_kernel(const __grid_c
         r.frequency = cfg.frequency_penalty;
         r.repetition = cfg.repetition_penalty;
         r.raises = raises;
+        r.odd = cfg.repetition_penalty != 1.0f && (length != 0 || tabled) ? kHugeBits : 0x7f800000u;
         r.tokens = tokens;
         r.counts = tabled ? p.slot_counts + (size_t)session * p.vocab_total + lo : nullptr;
         r.history_len = length;
@@ -910,6 +1076,7 @@ __global__ void __launch_bounds__(kThreads, 2) team_select_kernel(const __grid_c
     const float none = __uint_as_float(0xff800000u);
     float most[2 * kHalf];  // the thread's vectors' largest values
     uint32_t odd = 0;
+    const uint32_t odd_from = sh.row.odd;
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         const bool landed = vectors.wait(p, 0, h, 0);
@@ -921,7 +1088,7 @@ __global__ void __launch_bounds__(kThreads, 2) team_select_kernel(const __grid_c
             Lanes<T>::unpack(stage[u * 32], v);
             const bool there = u * 32 < here;
             most[h * kHalf + u] = there ? largest(v) : none;  // (a NaN never wins)
-            if (greedy && there && odd_values(v)) odd |= 1u << (h * kHalf + u);
+            if (greedy && there && odd_values(v, odd_from)) odd |= 1u << (h * kHalf + u);
         }
         __syncwarp();
         if (landed) vectors.ask(p, vectors.turn(), h);
@@ -947,30 +1114,35 @@ __global__ void __launch_bounds__(kThreads, 2) team_select_kernel(const __grid_c
             if (seen_column(sh.row, vectors.column(vectors.number(0, where)) + j)) key = 0;
         }
     }
-    // Where the history has seen most of the best, the lanes' largest unseen ones are looked for.  (Rows that
-    // it covers so densely are short.)
-    if (one_turn && __popc(__ballot_sync(kFullMask, key == 0 && best > none)) > 8) {
-        if (key == 0) {
+    // Where the history has seen so many of the best that the warp's j-th largest key (j = ceil(k / warps)) would lie
+    // low, the lanes' largest unseen ones are looked for.  (Rows that it covers so densely are short.)
+    if (one_turn && sh.row.seen_any && 2u * __popc(__ballot_sync(kFullMask, key != 0)) < 5u * ((k + kWarps - 1u) / kWarps)) {
+        if (key == 0 && best > none) {
+            float unseen = none;
 #pragma unroll 1
             for (uint32_t u = 0; u < 2u * kHalf; u++) {
                 if ((int)(u % kHalf * 32u) >= vectors.extent(0, u / kHalf)) continue;
                 float v[kPer];
                 Lanes<T>::unpack(vector_of(u), v);
-                const uint32_t column = vectors.column(vectors.number(0, u));
-#pragma unroll
-                for (int j = 0; j < kPer; j++)
-                    if (!is_nonfinite(v[j]) && !seen_column(sh.row, column + (uint32_t)j)) key = max(key, float_key(v[j]));
+                unseen = largest_unseen(v, vectors.column(vectors.number(0, u)), unseen);
             }
+            key = is_nonfinite(unseen) ? 0u : float_key(unseen);
         }
     }
     // (a last warp with less than half a warp's vectors has too few keys to bound the others)
     const uint32_t warps = max(1u, min((uint32_t)kWarps, (vectors.count + vectors.span) / (2u * vectors.span)));
     uint32_t top;
-    uint32_t low = bound_of_lanes(key, k, warps, k > 1u && !one_turn, &top);
-    if (k == 1u) low = top;
+    const bool tight = k > 1u && (!one_turn || (k > kLooseMost && warps == (uint32_t)kWarps));  // (fewer warps have too few keys)
+    uint32_t low = bound_of_lanes(key, k, warps, tight, &top);
+    if (k == 1u) {
+        low = top;
+    } else if (!tight && !(key_to_float(top) - key_to_float(low) < kFarApart)) {
+        __syncthreads();  // (everybody has read what the second bound is made over)
+        low = max(low, bound_of_lanes(key, k, warps, true, &top));
+    }
     const uint64_t bound = (uint64_t)low << 32;
     if (tid == 0) sh.bound = bound;
-    const float tau = key_to_float(low), floor = raises ? raw_floor(tau) : tau;
+    const Gate gate = gate_of(bound);
     // the columns before the first boundary and after the last: one for some threads of two warps
     const uint32_t tail = vectors.column(vectors.count);
     if (vectors.head != 0 || tail < n) {
@@ -979,7 +1151,7 @@ __global__ void __launch_bounds__(kThreads, 2) team_select_kernel(const __grid_c
         if (tid >= 32u && tail + (tid - 32u) < n) single = tail + (tid - 32u);
         if (single != kPaddingId) {
             const float x = sizeof(T) == 2 ? bf16_bits_to_float((uint32_t)__ldg(columns + single)) : (float)__ldg(columns + single);
-            if (x >= floor || (greedy && odd_value(x))) {
+            if (x >= gate.floor || (greedy && odd_value(x, sh.row.odd))) {
                 const Worth w = worth_of(x, single, bound);
                 if (w.key != 0) {
                     const uint32_t slot = atomicAdd(&sh.count, 1u);
@@ -997,12 +1169,14 @@ __global__ void __launch_bounds__(kThreads, 2) team_select_kernel(const __grid_c
         // vectors after it)
         uint32_t hot = odd, part = 0, part_of = 0;
 #pragma unroll
-        for (int u = 0; u < 2 * kHalf; u++) hot |= (most[u] >= floor && most[u] > none ? 1u : 0u) << u;
-        while (__any_sync(kFullMask, hot != 0) && !__any_sync(kFullMask, part != 0)) {
+        for (int u = 0; u < 2 * kHalf; u++) hot |= (most[u] >= gate.floor && most[u] > none ? 1u : 0u) << u;
+        // (a flood is not what a row as such has to offer: left to `crowded`, which sifts it)
+        const bool flood = __any_sync(kFullMask, odd != 0 || __popc(hot) > kHalf);
+        while (!flood && __any_sync(kFullMask, hot != 0) && !__any_sync(kFullMask, part != 0)) {
             part_of = hot != 0 ? (uint32_t)__ffs(hot) - 1u : 0u;
             float v[kPer] = {};
             if (hot != 0) Lanes<T>::unpack(vector_of(part_of), v);
-            part = list_elements<T>(v, hot != 0 ? (1u << kPer) - 1u : 0u, vectors.column(vectors.number(0, part_of)), floor, bound,
+            part = list_elements<T>(v, hot != 0 ? (1u << kPer) - 1u : 0u, vectors.column(vectors.number(0, part_of)), gate.floor, bound,
                                     greedy);
             hot &= hot - 1u;
         }

@@ -89,6 +89,26 @@ def test_most_of_the_vocabulary_has_been_seen(context, team, vocab, dtype):
         check(context, w, f"V={vocab} k={k} team={team}")
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("vocab", [4_099, 33_000, 151_936])
+@pytest.mark.parametrize("fill", ["-inf", "lowest", "one"])
+def test_most_of_a_row_is_one_value(context, team, vocab, dtype, fill):
+    """Rows under a mask, and rows of equal logits: next to nothing, fewer than k, or more than k logits stand out, and
+    with a mask of finite values or none the ties are won by the smallest ids."""
+    value = {"-inf": float("-inf"), "lowest": torch.finfo(dtype).min, "one": 1.0}[fill]
+    for i, penalties in enumerate((dict(temperature=0.9, top_p=0.9), CONFIGS["lowering"], CONFIGS["raising"],
+                                   dict(temperature=0.0, top_p=1.0, frequency=0.3, presence=-0.5),
+                                   dict(temperature=0.0, top_p=1.0, repetition=1.2))):
+        k = 1 if penalties["temperature"] == 0.0 else 50
+        w = random_workload(4, vocab, 200, [SamplerConfig.make(top_k=k, **penalties)], vocab + i, dtype=dtype)
+        allowed = torch.zeros(w.logits.shape, dtype=torch.bool)
+        for r, few in enumerate((1, 30, 2000, 300)):
+            where = torch.randint(0, vocab, (few,), generator=torch.Generator().manual_seed(r))
+            allowed[r, where if r < 3 else torch.arange(vocab // 3, vocab // 3 + few)] = True
+        w.logits = torch.where(allowed, w.logits, torch.full_like(w.logits, value))
+        check(context, w, f"{fill} V={vocab} team={team} {penalties}")
+
+
 def test_mixed_settings_in_one_batch(context, team):
     """Every row its own settings; rows without a top-k cut are left to their kernel."""
     rows, vocab = 40, 20_011
