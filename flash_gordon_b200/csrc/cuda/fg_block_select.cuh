@@ -317,7 +317,9 @@ __device__ inline void finish_select(FinishBuffer &fin, uint32_t n, const Sample
         scan_places(t0, t1, n > 32);
         const double sum = __shfl_sync(kFullMask, r1, 31), edge = top_p * sum, margin = kMargin * sum;
         const uint32_t last = first_place(i0 < n && r0 >= edge, i1 < n && r1 >= edge, n - 1u);
-        bool near = fabs(r0 - edge) <= margin || fabs(r1 - edge) <= margin || !(sum > 0.0 && sum < 1e300);
+        // (The last place is never in doubt: whether its sum reaches top_p or no sum does, all n are kept.)
+        bool near = (i0 + 1u < n && fabs(r0 - edge) <= margin) || (i1 + 1u < n && fabs(r1 - edge) <= margin) ||
+                    !(sum > 0.0 && sum < 1e300);
         const double low = __shfl_sync(kFullMask, t0, (int)(last & 31u)), high = __shfl_sync(kFullMask, t1, (int)(last & 31u));
         const double weights = last < 32u ? low : high, draw = (double)u * weights, slack = kMargin * weights;
         near = near || (i0 <= last && fabs(t0 - draw) <= slack) || (i1 <= last && fabs(t1 - draw) <= slack) ||
