@@ -739,20 +739,27 @@ static bool scans_cost_more(const fg_cuda_sample_args *a) {
 }
 
 /* How many CTAs of the team kernel share a row, each one's columns and the kernel's form; 0: the batch is not for
- * that kernel.  It beats the ring kernel everywhere but in large fp32 batches, which are bound by HBM and
- * take fewer steps there.  Measured (B200, us a call, rows of 151,936; ring kernel / teams of 1 / 2 / 4 / 8 CTAs):
+ * that kernel.  `lowering`: the launch's rows are such as the ring kernel takes, and that kernel's if this one
+ * refuses.  Measured (B200, us a call, rows of 151,936; ring kernel / teams of 1 / 2 / 4 / 8 CTAs):
  * fp32, k = 20, 512 tokens: 1 row 23 / 25 / 17 / 14 / 12, 32 rows 25 / 30 / 18 / 15 / 15, 64 rows 25 / 30 / 19 / 18 / 27,
- * 148 rows 28 / 33 / 26 / 40 / 49, 296 rows 43 / 45 / 46, 512 rows 71 / 73 / 78, 1024 rows 118 / 131; k = 50,
- * 4,096 tokens to be counted: 1 row 29 / 33 / 25 / 21 / 19, 148 rows 44 / 40 / 38, 512 rows 92 / 86, 1024 rows
- * 147 / 153; greedy: 1 row 16 / 17 / 12 / 10 / 8, 512 rows 58 / 53, 1024 rows 97 / 100; bf16, k = 20: 64 rows
- * 26 / 21 / 16 / 18, 1024 rows 115 / 80.
+ * 148 rows 28 / 33 / 26 / 40 / 49; k = 50, 4,096 tokens to be counted: 1 row 29 / 33 / 25 / 21 / 19, 148 rows
+ * 44 / 40 / 38; greedy: 1 row 16 / 17 / 12 / 10 / 8; bf16, k = 20: 64 rows 26 / 21 / 16 / 18, 1024 rows 115 / 80.
+ * Batches with more rows than CTAs run at a time (two to an SM) are taken in waves.  The ring kernel, whose CTAs take
+ * row after row, is faster at long fp32 rows when the last wave is not nearly full (ring / team: 400 rows of 151,936,
+ * 512 tokens 58 / 72, 640 rows 89 / 100, 320 rows of 128,256 0.89 of the team kernel's time, 444 rows of 202,048 0.82;
+ * 512 rows of 151,936 without penalties 69 / 67, 444 rows of 81,920 1.0, 350 of 65,536 1.15), unaligned rows alike; and at
+ * aligned fp32 batches of more than 100 M logits, which are bound by HBM (1024 rows 118 / 131, 500 of 202,048 the
+ * same).  Unaligned ones of that size are as fast in either (1024 rows of 151,937 0.95 to 1.0, of 100,277 1.05 to 1.09), bf16
+ * rows 1.04 to 1.5 times as fast here (greedy ones 0.89 to 1.07).  The lowering rows of a batch split in two stay here:
+ * 296 to 1024 rows, one in 4 to one in 256 raising, ring and streaming kernel 0.95 to 2.3 times the time of two
+ * launches of this kernel, 1.3 in the mean.
  * What the ring kernel does not take was the streaming kernel's, which tabulates histories: that pays when they
  * cover much of a vocabulary (48 batches of up to 60 M logits with a token for every column, us there / here: 0.3 to
  * 2.2 times, 0.8 in the mean; with half as many 1.1, with a tenth 1.6, with fewer 2.4).  Greedy rows whose
  * history covers an eighth of the vocabulary or more have few unseen logits at the top: the ring kernel's bound,
  * which rises with every one it meets, is the better one (73 rows of 19,200 logits, 5,277 tokens 15 us there, 29 here). */
 static uint32_t plan_team(const fg_cuda_context *c, const fg_cuda_sample_args *a, const batch_traits *traits,
-                          bool ring, uint32_t rows, uint32_t *chunk, uint32_t *form, uint32_t *bitmap_words) {
+                          bool lowering, bool aligned, uint32_t rows, uint32_t *chunk, uint32_t *form, uint32_t *bitmap_words) {
     const size_t element = a->dtype == FG_CUDA_BF16 ? 2u : 4u;
     if (c->team_size == 255u || c->path != FG_CUDA_PATH_AUTO || c->forced_splits != 0u || c->ring_deal != 0u ||
         (c->ring_withhold_armed && !c->team_size) || traits->wild != 0u || ((uintptr_t)a->logits % element) != 0u)
@@ -760,7 +767,12 @@ static uint32_t plan_team(const fg_cuda_context *c, const fg_cuda_sample_args *a
     uint32_t team = c->team_size;
     if (!team) {
         if (a->vocab > (1u << 20)) return 0u;
-        if (ring && a->dtype == FG_CUDA_F32 && (uint64_t)rows * a->vocab > 100000000u) return 0u;
+        const bool ring = lowering && aligned;
+        if (lowering && a->dtype == FG_CUDA_F32) {
+            const uint64_t abreast = 2u * c->sm_count, waves = (rows + abreast - 1u) / abreast;
+            if (aligned && (uint64_t)rows * a->vocab > 100000000u) return 0u;
+            if (a->vocab > 100000u && rows > abreast && rows * 20u < waves * abreast * 17u) return 0u;
+        }
         if (!ring && traits->penalties && a->history_max > a->vocab / 2u) return 0u;
         if (ring && !traits->sampled && traits->penalties && !c->session_counts && a->history_max > a->vocab / 8u) return 0u;
         team = rows * 8u <= c->sm_count ? 8u : rows * 4u <= 2u * c->sm_count ? 4u : rows <= c->sm_count ? 2u : 1u;
@@ -872,9 +884,9 @@ static fg_status run_stream(fg_cuda_context *c, const fg_cuda_sample_args *a,
         fgk_stream_launch t = l, second = l;
         uint32_t chunk = 0u, form = 0u, second_chunk = 0u, second_form = 0u, second_team = 0u;
         const uint32_t others = both ? a->rows - traits->nucleus - raising : a->rows;
-        const uint32_t team = plan_team(c, a, traits, all_ring && aligned, others, &chunk, &form, &t.bitmap_words);
+        const uint32_t team = plan_team(c, a, traits, all_ring, aligned, others, &chunk, &form, &t.bitmap_words);
         if (both) /* (more CTAs for fewer rows: a raising row looks at more of its logits) */
-            second_team = plan_team(c, a, traits, false, raising * 2u, &second_chunk, &second_form, &second.bitmap_words);
+            second_team = plan_team(c, a, traits, false, aligned, raising * 2u, &second_chunk, &second_form, &second.bitmap_words);
         if (team != 0u && (!both || second_team != 0u)) {
             c->last_scratch_bytes = a->config_count > 1u ? (size_t)a->rows * sizeof(fg_sampler_config) : 0u;
             int e = launched(c, fgk_launch_team_select(&t, team, chunk, form, both ? FGK_TEAM_LOWERING_ROWS : FGK_TEAM_ALL_ROWS,

@@ -69,6 +69,49 @@ def test_draws_that_no_row_uses_are_not_read(plan):
             assert status == FG_OK and all(l.endswith("uniforms=1") for l in launches), launches
 
 
+def kernels(launches):
+    return [line.split()[0] for line in launches]
+
+
+@pytest.mark.parametrize("rows,vocab,dtype,offset,kernel", [
+    (1, 151_936, "f32", 0, "team"), (296, 151_936, "f32", 0, "team"), (320, 151_936, "f32", 0, "ring"),
+    (444, 151_936, "f32", 1, "ring"), (512, 151_936, "f32", 0, "team"), (512, 151_936, "f32", 1, "team"),
+    (640, 128_256, "f32", 0, "ring"), (592, 128_256, "f32", 0, "team"), (400, 100_000, "f32", 0, "team"),
+    (400, 151_936, "bf16", 0, "team"), (1024, 151_936, "f32", 0, "ring"), (1024, 151_936, "f32", 1, "team"),
+    (1024, 151_936, "bf16", 0, "team"), (800, 100_352, "f32", 0, "team"), (2, 1_048_576, "f32", 0, "team"),
+])
+def test_kernel_of_a_lowering_batch(plan, rows, vocab, dtype, offset, kernel):
+    """Long fp32 rows whose last wave of teams would be half empty, and large aligned fp32 batches, are the ring kernel's."""
+    for configs, history in (([TOP_K], 0), ([LOWERING], 512)):
+        status, launches = plan(configs, rows, vocab, dtype, history, offset)
+        assert status == FG_OK and kernels(launches) == [kernel], launches
+
+
+def mixed(rows, every, odd=None):
+    """One row in `every` raises; `odd` overrides the last of those."""
+    configs = [SamplerConfig.make(temperature=0.8, top_p=0.9, top_k=20, presence=-0.4 if r % every == 0 else 0.4) for r in range(rows)]
+    if odd:
+        configs[(rows - 1) // every * every] = SamplerConfig.make(temperature=0.8, top_p=0.9, top_k=20, **odd)
+    return configs
+
+
+@pytest.mark.parametrize("offset", [0, 1])
+def test_kernels_of_a_batch_with_some_raising_rows(plan, offset):
+    rows, vocab = 400, 151_936
+    status, launches = plan(mixed(rows, 8), rows, vocab, history=512, offset=offset)
+    assert status == FG_OK and [line.split()[:2] for line in launches] == [["team", "which=1"], ["team", "which=2"]]
+    # a charge that does not grow with the count, an extreme factor, a history over half the vocabulary
+    for odd, history in ((dict(frequency=-0.5), 512), (dict(repetition=2.0 ** -41), 512), (dict(repetition=2.0 ** 41), 512),
+                         (None, vocab // 2 + 1)):
+        status, launches = plan(mixed(rows, 8, odd), rows, vocab, history=history, offset=offset)
+        assert status == FG_OK
+        assert [line.split()[:2] for line in launches] == [["ring", "skip_raising=1"], ["stream", "only_raising=1"]]
+    # many raising rows, and a small batch: one launch
+    assert kernels(plan(mixed(rows, 2), rows, vocab, history=512, offset=offset)[1]) == ["team"]
+    assert kernels(plan(mixed(30, 8), 30, vocab, history=512, offset=offset)[1]) == ["team"]
+    assert kernels(plan(mixed(30, 8, dict(frequency=-0.5)), 30, vocab, history=512, offset=offset)[1]) == ["stream"]
+
+
 @pytest.mark.parametrize("team,chunk,form", [(0, 1024, 0), (3, 1024, 0), (16, 1024, 0), (2, 384, 0), (4, 200, 0), (1, 1024, 2)])
 def test_plans_that_cannot_be_launched_are_refused(library, team, chunk, form):
     """Before anything is enqueued: no CTAs, a number that is no cluster's, columns that do not cover the row."""
