@@ -13,6 +13,14 @@ from helpers import as_u32, run_oracle
 pytestmark = pytest.mark.gpu
 
 
+@pytest.fixture(params=[0, 255], ids=["automatic choice", "without the team kernel"], autouse=True)
+def kernels(context, request):
+    """The tables are read by the team kernel, and by the ring kernel for what that one leaves to it."""
+    context.team_controls(request.param)
+    yield request.param
+    context.team_controls()
+
+
 def oracle_step(logits, configs, uniforms, histories):
     tokens = torch.tensor([t for h in histories for t in h], dtype=torch.int32)
     offsets = torch.tensor(np.cumsum([0] + [len(h) for h in histories]), dtype=torch.int64)
@@ -21,7 +29,7 @@ def oracle_step(logits, configs, uniforms, histories):
     return run_oracle(w)
 
 
-@pytest.mark.parametrize("vocab", [151_936, 9_001])  # (9,001 fp32 rows are not 16-byte aligned: the other kernel)
+@pytest.mark.parametrize("vocab", [151_936, 9_001])  # (9,001 fp32 logits: rows are not 16-byte aligned)
 def test_sixty_four_steps_of_eight_sessions(context, vocab):
     rows, steps, slots = 8, 64, 11
     g = torch.Generator().manual_seed(vocab)

@@ -215,10 +215,11 @@ def test_ring_refuses_what_it_cannot_take(context):
 
 
 def test_shapes_the_planner_treats_differently(context):
-    """Through the automatic choice: a few rows of more than a million logits (dealt out in tiles
-    and merged), the same with a history (its bitmap does not fit beside the ring: the other
-    kernel), long rows in a small batch, many one-tile rows, a ragged one-tile row."""
+    """Through the automatic choice, the team kernel left out: a few rows of more than a million logits
+    (dealt out in tiles and merged), the same with a history (its bitmap does not fit beside the ring: the
+    streaming kernel), long rows in a small batch, many one-tile rows, a ragged one-tile row."""
     context.set_path(PATH_AUTO)
+    context.team_controls(255)
     try:
         for rows, vocab, history, cfg in (
                 (3, 1_200_000, 0, SamplerConfig.make(0.9, 0.9, 50)),
@@ -231,4 +232,5 @@ def test_shapes_the_planner_treats_differently(context):
             assert_rows_equal(run_gpu(context, w), run_oracle(w), f"{rows} x {vocab}")
     finally:
         context.set_path(PATH_RING)
+        context.team_controls()
 

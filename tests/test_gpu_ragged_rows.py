@@ -1,5 +1,6 @@
-"""Rows that do not begin or end on a 16-byte boundary in the ring kernel, and batches whose rows
-go through different kernels because some rows' penalties can raise a logit."""
+"""Rows that do not begin or end on a 16-byte boundary, and batches whose rows go through different
+launches because some rows' penalties can raise a logit: by the automatic choice, which is mostly the team
+kernel, and by the ring and the streaming kernel, which take over where that one does not."""
 import numpy as np
 import pytest
 import torch
@@ -14,6 +15,13 @@ CONFIGS = {
     "penalised": SamplerConfig.make(temperature=0.8, top_p=0.9, top_k=64, presence=0.4, frequency=0.3, repetition=1.1),
     "greedy": SamplerConfig.make(temperature=0.0, top_p=1.0, top_k=1, repetition=1.2),
 }
+
+
+@pytest.fixture(params=[0, 255], ids=["automatic choice", "without the team kernel"], autouse=True)
+def kernels(context, request):
+    context.team_controls(request.param)
+    yield request.param
+    context.team_controls()
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
@@ -48,8 +56,7 @@ def test_every_offset(context, dtype, kind, vocab, stride, start):
 @pytest.mark.parametrize("vocab", [12_346, 12_352])
 @pytest.mark.parametrize("raising", [1, 7, 30])
 def test_some_rows_of_a_small_batch_raise(context, dtype, vocab, raising):
-    """`raising` of 30 rows have penalties that can raise a logit (a batch so small goes through the
-    streaming kernel whole)."""
+    """`raising` of 30 rows have penalties that can raise a logit (a batch so small is one launch)."""
     rows = 30
     w = random_workload(rows, vocab, 400, some_raising(rows, raising), 5 + raising, dtype=dtype)
     assert_rows_equal(run_gpu(context, w), run_oracle(w), f"{raising} raising rows")
@@ -73,8 +80,9 @@ def some_raising(rows, raising, nucleus_every=0):
     (175, 98_049, torch.float32, 31, 11), (128, 131_072, torch.float32, 70, 0),
 ])
 def test_rows_of_a_large_batch_in_two_kernels(context, rows, vocab, dtype, raising, nucleus_every):
-    """Above 15 million logits up to a quarter of the rows, the raising ones, go through the streaming
-    kernel and the others through the ring kernel: one launch more than with a single kernel."""
+    """Above 15 million logits up to a quarter of the rows, the raising ones, are a launch of their own: of the
+    team kernel like the others', or of the streaming kernel beside the ring kernel's.  One launch more
+    than with a single kernel."""
     w = random_workload(rows, vocab, 300, some_raising(rows, raising, nucleus_every), raising, dtype=dtype, specials=1)
     w.allow_no_topk = bool(nucleus_every)
     expected = run_oracle(w)
@@ -91,7 +99,7 @@ def test_rows_of_a_large_batch_in_two_kernels(context, rows, vocab, dtype, raisi
 
 
 def test_rows_of_a_large_shard_in_two_kernels(context):
-    """The same for the columns of a shard: the lists of both kernels' rows are the whole rows' parts."""
+    """The same for the columns of a shard: the lists of both launches' rows are the whole rows' parts."""
     rows, vocab, width, k = 300, 104_000, 52_000, 24
     configs = [SamplerConfig.make(temperature=0.9, top_p=0.9, top_k=k, presence=-0.6 if r % 9 == 4 else 0.4, frequency=0.1)
                for r in range(rows)]
@@ -109,13 +117,30 @@ def test_rows_of_a_large_shard_in_two_kernels(context):
     assert np.array_equal(as_u32(result.tokens), expected[1])
 
 
+@pytest.mark.parametrize("vocab,history,wild", [
+    (100_280, 300, dict(frequency=-0.5)), (100_277, 300, dict(frequency=-0.02, presence=0.4)),
+    (100_280, 300, dict(repetition=2.0 ** 50)), (100_280, 300, dict(repetition=2.0 ** -60)),
+    (30_000, 16_000, dict(presence=-0.5)), (30_001, 16_000, dict(presence=-0.5)),
+])
+def test_rows_that_only_the_streaming_kernel_takes(context, vocab, history, wild):
+    """A charge that shrinks with the count, an extreme repetition factor, a raising row with a history of half
+    the vocabulary: those rows go through the streaming kernel, the others of a large batch through the
+    ring kernel, a small batch whole."""
+    for rows in (12, 15_500_000 // vocab):
+        configs = some_raising(rows, rows // 9)
+        configs[rows // 2] = SamplerConfig.make(temperature=0.9, top_p=0.9, top_k=30, **wild)
+        configs[3] = SamplerConfig.make(0.0, 1.0, 1, **wild)
+        w = random_workload(rows, vocab, history, configs, vocab + rows, uniform_history=False)
+        assert_rows_equal(run_gpu(context, w), run_oracle(w), f"{rows} rows, {wild}")
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("vocab", [3_001, 3_008, 32_001])
 @pytest.mark.parametrize("history", [700, 8_192, 70_000])
 @pytest.mark.parametrize("k,top_p", [(20, 0.9), (64, 1.0)])
 def test_most_of_the_best_have_been_seen(context, dtype, vocab, history, k, top_p):
     """Uniform histories, up to many times the vocabulary, with a frequency penalty: much to count, by
-    the kernel that is faster at it (the streaming kernel for unaligned rows and long histories)."""
+    the kernel that is faster at it."""
     configs = [SamplerConfig.make(temperature=0.0 if r == 2 else 0.8, top_p=top_p, top_k=1 if r == 2 else k, presence=0.1 * r,
                                   frequency=0.02 + 0.1 * (r % 2), repetition=1.0 + 0.05 * (r % 3)) for r in range(5)]
     w = random_workload(5, vocab, history, configs, vocab + history + k, dtype=dtype)

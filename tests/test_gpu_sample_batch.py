@@ -17,11 +17,14 @@ pytestmark = pytest.mark.gpu
 PROBABILITY_RTOL = 1e-5
 
 
-@pytest.fixture(params=["ring_if_possible", "registers"], autouse=True)
+PATHS = {"automatic": 0, "ring_if_possible": 3, "registers": 1}
+
+
+@pytest.fixture(params=PATHS, autouse=True)
 def kernel_path(context, request):
-    """Every case runs twice: through the shared-memory ring kernel wherever rows are
-    16-byte aligned, and pinned to the register-prefetch kernel."""
-    context.set_path(3 if request.param == "ring_if_possible" else 1)
+    """Every case runs three times: by the automatic choice (the team kernel for most of them), through the
+    shared-memory ring kernel wherever it takes the rows, and pinned to the register-prefetch kernel."""
+    context.set_path(PATHS[request.param])
     yield request.param
     context.set_path(0)
 

@@ -15,9 +15,12 @@ from helpers import (as_u32, assert_candidates_close, assert_rows_equal, logits_
 pytestmark = pytest.mark.gpu
 
 
-@pytest.fixture(params=["ring_if_possible", "registers"], autouse=True)
+PATHS = {"automatic": 0, "ring_if_possible": 3, "registers": 1}
+
+
+@pytest.fixture(params=PATHS, autouse=True)
 def kernel_path(context, request):
-    context.set_path(3 if request.param == "ring_if_possible" else 1)
+    context.set_path(PATHS[request.param])
     yield request.param
     context.set_path(0)
 

@@ -195,3 +195,16 @@ def test_edges_that_are_met_exactly(context, team, count):
         cfg = SamplerConfig.make(0.5, top_p, count)
         w = synth.Workload("exact", logits, [cfg], torch.tensor(draws), None, None, 0)
         assert_rows_equal(run_gpu(context, w), run_oracle(w), f"{count} equal weights, top_p {top_p}")
+
+
+@pytest.mark.parametrize("gap", [20.0, 29.0, 29.93, 31.0, 36.0, 40.0, 800.0])
+def test_sums_that_stand_still(context, gap):
+    """All candidates are asked for, and the last ones weigh so little that the sum reaches top_p before them, or
+    not at all."""
+    vocab, draws = 3_000, [0.0, 0.3, 0.999999]
+    logits = torch.full((len(draws), vocab), -900.0)
+    logits[:, 5:10] = torch.tensor([0.0, -0.5, -gap, -gap - 0.25, -gap - 7.0])
+    for k in (3, 4, 5, 40):
+        for top_p in (1.0, float(np.nextafter(np.float32(1.0), np.float32(0.0)))):
+            w = synth.Workload("tails", logits, [SamplerConfig.make(1.0, top_p, k)], torch.tensor(draws), None, None, 0)
+            assert_rows_equal(run_gpu(context, w), run_oracle(w), f"gap {gap}, top_p {top_p}, k {k}")
