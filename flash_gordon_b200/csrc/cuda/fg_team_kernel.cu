@@ -215,12 +215,21 @@ __device__ __forceinline__ Gate gate_of(uint64_t bound) {
     g.floor = shared().row.raises ? raw_floor(g.tau) : g.tau;
     return g;
 }
-// What the largest logit of a vector must be for a look at it, when no id in there is below `first_id`.  (An infinity is
-// no candidate: greedy rows find it otherwise.)
-__device__ __forceinline__ float gate_of_vectors(const Gate &g, uint32_t first_id) {
-    const bool ties_lose = !shared().row.raises && first_id > g.last_id();
-    const float at_least = ties_lose ? key_to_float((uint32_t)(g.bound >> 32) + 1u) : g.floor;
-    return fmaxf(at_least, -3.402823466e38f);
+// What the largest logit of a vector must be for a look at it: `at_least`, or `above` if no id in there is below
+// `ties_lose`.  (An infinity is no candidate: greedy rows find it otherwise.)
+struct VectorGate {
+    float at_least, above;
+    uint32_t ties_lose;  // a column of the CTA's
+};
+__device__ __forceinline__ VectorGate gate_of_vectors(const Gate &g) {
+    const Row &r = shared().row;
+    constexpr float kLowest = -3.402823466e38f;
+    VectorGate v;
+    v.at_least = fmaxf(g.floor, kLowest);
+    v.above = fmaxf(key_to_float((uint32_t)(g.bound >> 32) + 1u), kLowest);
+    const uint32_t last = g.last_id();
+    v.ties_lose = r.raises || last >= r.id_base + r.columns ? 0xffffffffu : last < r.id_base ? 0u : last - r.id_base + 1u;
+    return v;
 }
 
 // NaN, infinities and magnitudes a repetition factor of 2^-40 to 2^40 could push there: greedy rows
@@ -278,46 +287,53 @@ __device__ __forceinline__ uint32_t passing(const float (&v)[N], uint32_t column
     return pass;
 }
 
-// A bound for k lanes' keys: at least k of them are as large.  Loosely: every warp's j-th largest, j = ceil(k /
-// warps), of the `warps` first warps; the smallest of them (twice k keys or so are as large).  With
-// `tight` every warp contributes three more, and of all those the k-th largest is taken (k and a few keys are as
-// large: worth a step more when much of the row is still to come).  `largest`: the largest of all lanes'
-// keys.  All threads call; syncs once, in the middle, or twice.
-__device__ __forceinline__ uint32_t bound_of_lanes(uint32_t key, uint32_t k, uint32_t warps, bool tight, uint32_t *largest) {
+// Bounds for k lanes' keys: at least k of them are as large.  `largest`: the largest of all lanes' keys.  All
+// threads call.
+//
+// Every warp contributes three more than k / warps, and of all those the k-th largest is taken (k and a few keys are as
+// large: worth a step more when much of the row is still to come).  Syncs twice.  One copy for all its users:
+// instructions that have not run before come from L2.
+__device__ __noinline__ uint2 tight_bound(uint32_t key, uint32_t k) {
     Shared &sh = shared();
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    const uint32_t each = (k + warps - 1u) / warps;
+    const uint32_t rounds = min((k + kWarps - 1u) / kWarps + 3u, kMostRounds), keys = rounds * kWarps;
+    uint32_t found = __reduce_max_sync(kFullMask, key);
+    for (uint32_t i = 0;; i++) {
+        if (lane == 0) sh.warp_key[i * kWarps + warp] = found;
+        if (i + 1u >= rounds) break;
+        const unsigned owners = __ballot_sync(kFullMask, key == found);
+        if ((int)lane == __ffs(owners) - 1) key = 0;
+        found = __reduce_max_sync(kFullMask, key);
+    }
+    if (tid == 0) sh.tight_key = 0;
+    __syncthreads();
+    if (tid < keys) {
+        // (equal keys are counted together, so that somebody finds the k-th)
+        const uint32_t mine = sh.warp_key[tid];
+        uint32_t larger = 0, equal = 0;
+        for (uint32_t i = 0; i < keys; i += 4) {
+            const uint4 four = *reinterpret_cast<const uint4 *>(&sh.warp_key[i]);
+            larger += (four.x > mine) + (four.y > mine) + (four.z > mine) + (four.w > mine);
+            equal += (four.x == mine) + (four.y == mine) + (four.z == mine) + (four.w == mine);
+        }
+        if (larger < k && larger + equal >= k) sh.tight_key = mine;
+        if (larger == 0) sh.warp_top[0] = mine;
+    }
+    __syncthreads();
+    return make_uint2(sh.tight_key, sh.warp_top[0]);
+}
+
+// Every warp's j-th largest, j = ceil(k / warps), of the `warps` first warps; the smallest of them (twice k keys or so
+// are as large).  Syncs once, in the middle.
+__device__ __forceinline__ uint2 loose_bound(uint32_t key, uint32_t k, uint32_t warps) {
+    Shared &sh = shared();
+    const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
     uint32_t found = __reduce_max_sync(kFullMask, key);
     const uint32_t top = found;
-    if (each > 1u || tight) {
-        const uint32_t rounds = tight ? min(each + 3u, kMostRounds) : each;
-        for (uint32_t i = 0;; i++) {
-            if (tight && lane == 0) sh.warp_key[i * kWarps + warp] = found;
-            if (i + 1u >= rounds) break;
-            const unsigned owners = __ballot_sync(kFullMask, key == found);
-            if ((int)lane == __ffs(owners) - 1) key = 0;
-            found = __reduce_max_sync(kFullMask, key);
-        }
-        if (tight) {
-            const uint32_t keys = rounds * kWarps;
-            if (tid == 0) sh.tight_key = 0;
-            __syncthreads();
-            if (tid < keys) {
-                // (equal keys are counted together, so that somebody finds the k-th)
-                const uint32_t mine = sh.warp_key[tid];
-                uint32_t larger = 0, equal = 0;
-                for (uint32_t i = 0; i < keys; i += 4) {
-                    const uint4 four = *reinterpret_cast<const uint4 *>(&sh.warp_key[i]);
-                    larger += (four.x > mine) + (four.y > mine) + (four.z > mine) + (four.w > mine);
-                    equal += (four.x == mine) + (four.y == mine) + (four.z == mine) + (four.w == mine);
-                }
-                if (larger < k && larger + equal >= k) sh.tight_key = mine;
-                if (larger == 0) sh.warp_top[0] = mine;
-            }
-            __syncthreads();
-            *largest = sh.warp_top[0];
-            return sh.tight_key;
-        }
+    for (uint32_t each = (k + warps - 1u) / warps; each > 1u; each--) {
+        const unsigned owners = __ballot_sync(kFullMask, key == found);
+        if ((int)lane == __ffs(owners) - 1) key = 0;
+        found = __reduce_max_sync(kFullMask, key);
     }
     if (lane == 0) {
         sh.warp_key[warp] = found;
@@ -333,8 +349,7 @@ __device__ __forceinline__ uint32_t bound_of_lanes(uint32_t key, uint32_t k, uin
         for (uint32_t q = 0; q < 4; q++) low = w + q < warps ? min(low, keys[q]) : low;
         high = max(max(high, max(tops.x, tops.y)), max(tops.z, tops.w));
     }
-    *largest = high;
-    return low;
+    return make_uint2(low, high);
 }
 
 // What a logit is worth (src/sampler.c:52-58).
@@ -642,8 +657,7 @@ __device__ __forceinline__ void list_all(const uint4 raw, uint32_t left, uint32_
                 if (((left >> j) & 1u) && !is_nonfinite(v[j]) && !seen_column(r, column + (uint32_t)j))
                     best = max(best, float_key(v[j]));
         }
-        uint32_t top;
-        const uint32_t key = bound_of_lanes(best, r.k, kWarps, true, &top);
+        const uint32_t key = tight_bound(best, r.k).x;
         if (threadIdx.x == 0 && key != 0) atomicMax(&sh.bound, (unsigned long long)key << 32);
         __syncthreads();
     }
@@ -667,16 +681,50 @@ __device__ __noinline__ void work_off() {
     if (__syncthreads_or(sh.count > kListLong)) tighten(false);
 }
 
+// Vectors of the turn at `base` (`pending`, a bit each) go into the queue if they are still worth a look; returns those
+// that found it full.
+template <typename T, int kHalf>
+__device__ __noinline__ uint32_t refill(const Vectors<T, kHalf> vectors, uint32_t base, uint32_t pending) {
+    constexpr int kPer = Lanes<T>::kPer;
+    constexpr int kBatch = 4;  // vectors on their way at a time
+    Shared &sh = shared();
+    const Sieve sieve = sieve_of(gate_of(peek64(&sh.bound)));
+    uint32_t left = 0;
+#pragma unroll 1
+    for (uint32_t rest = pending; rest != 0;) {
+        if (peek(&sh.queue_count) >= kQueueCap) return left | rest;
+        uint4 raw[kBatch];
+        uint32_t bit[kBatch];
+#pragma unroll
+        for (int q = 0; q < kBatch; q++) {
+            bit[q] = rest & (0u - rest);
+            raw[q] = vectors.fetch(vectors.number(base, (uint32_t)__ffs(rest != 0 ? rest : pending) - 1u));
+            rest &= rest - 1u;
+        }
+#pragma unroll
+        for (int q = 0; q < kBatch; q++) {
+            if (bit[q] == 0) continue;
+            const uint32_t column = vectors.column(vectors.number(base, (uint32_t)__ffs(bit[q]) - 1u));
+            float v[kPer];
+            Lanes<T>::unpack(raw[q], v);
+            if (!may_pass(v, column, sieve)) continue;
+            const uint32_t mask = passing(v, column, sieve);
+            if (mask != 0 && !enqueue(sh, raw[q], column, mask)) left |= bit[q];
+        }
+    }
+    return left;
+}
+
 // More than the queue holds is worth a look (`pending`: vectors of the turn at `base`, a bit each): the queue is worked
 // off, which lifts the bound, and filled with what still passes, until nothing is left.  After the first turn, whose
-// bound comes from all its lanes' largest logits, those of the pending vectors lift it before that.  All
-// threads call; ends synced.
+// bound comes from all its lanes' largest logits, and if far more than the queue holds was offered, those of the
+// pending vectors lift it before that.  All threads call; ends synced.
 template <typename T, int kHalf>
 __device__ __noinline__ void crowded(const Vectors<T, kHalf> vectors, uint32_t base, uint32_t pending) {
     constexpr int kPer = Lanes<T>::kPer;
     constexpr int kBatch = 4;  // vectors on their way at a time
     Shared &sh = shared();
-    if (base != 0 && __syncthreads_or(pending != 0)) {
+    if (base != 0 && peek(&sh.queue_count) > 2u * kQueueCap) {  // (what was offered; a few too many need no new bound)
         float best = __uint_as_float(0xff800000u);
 #pragma unroll 1
         for (uint32_t rest = pending; rest != 0;) {
@@ -696,40 +744,12 @@ __device__ __noinline__ void crowded(const Vectors<T, kHalf> vectors, uint32_t b
                 best = largest_unseen(v, column[q], best);
             }
         }
-        uint32_t top;
-        const uint32_t key = bound_of_lanes(is_nonfinite(best) ? 0u : float_key(best), sh.row.k, kWarps, true, &top);
+        const uint32_t key = tight_bound(is_nonfinite(best) ? 0u : float_key(best), sh.row.k).x;
         if (threadIdx.x == 0 && key != 0) atomicMax(&sh.bound, (unsigned long long)key << 32);
     }
     do {
         work_off<T>();
-        const Sieve sieve = sieve_of(gate_of(peek64(&sh.bound)));
-        uint32_t left = 0;
-#pragma unroll 1
-        for (uint32_t rest = pending; rest != 0;) {
-            if (peek(&sh.queue_count) >= kQueueCap) {
-                left |= rest;
-                break;
-            }
-            uint4 raw[kBatch];
-            uint32_t bit[kBatch];
-#pragma unroll
-            for (int q = 0; q < kBatch; q++) {
-                bit[q] = rest & (0u - rest);
-                raw[q] = vectors.fetch(vectors.number(base, (uint32_t)__ffs(rest != 0 ? rest : pending) - 1u));
-                rest &= rest - 1u;
-            }
-#pragma unroll
-            for (int q = 0; q < kBatch; q++) {
-                if (bit[q] == 0) continue;
-                const uint32_t column = vectors.column(vectors.number(base, (uint32_t)__ffs(bit[q]) - 1u));
-                float v[kPer];
-                Lanes<T>::unpack(raw[q], v);
-                if (!may_pass(v, column, sieve)) continue;
-                const uint32_t mask = passing(v, column, sieve);
-                if (mask != 0 && !enqueue(sh, raw[q], column, mask)) left |= bit[q];
-            }
-        }
-        pending = left;
+        if (pending != 0) pending = refill<T, kHalf>(vectors, base, pending);
     } while (__syncthreads_or(pending != 0));
 }
 
@@ -770,6 +790,7 @@ __device__ __forceinline__ void scan(const Params &p, Vectors<T, kHalf> &vectors
     for (;;) {
         uint32_t pending = 0;
         const Gate gate = gate_of(peek64(&sh.bound));
+        const VectorGate look_at = gate_of_vectors(gate);
         bool stopped = false;  // with a half looked at
         while (vectors.first_of(base, h) < vectors.count && !__any_sync(kFullMask, peek(&sh.queue_count) > kQueueLong)) {
             if (!vectors.wait(p, base, h, parity)) {
@@ -779,7 +800,7 @@ __device__ __forceinline__ void scan(const Params &p, Vectors<T, kHalf> &vectors
             const uint4 *stage = vectors.stage(p, h) + lane_id();
             const uint32_t first = vectors.number(base, h * kHalf);
             const int here = vectors.extent(base, h);
-            const float at_least = gate_of_vectors(gate, sh.row.id_base + vectors.column(vectors.first_of(base, h)));
+            const float at_least = vectors.column(vectors.first_of(base, h)) >= look_at.ties_lose ? look_at.above : look_at.at_least;
             uint32_t hot = 0;
 #pragma unroll
             for (int u = 0; u < kHalf; u++) {
@@ -791,7 +812,8 @@ __device__ __forceinline__ void scan(const Params &p, Vectors<T, kHalf> &vectors
             }
             const uint32_t finders = __ballot_sync(kFullMask, hot != 0);
             if (finders != 0) {
-                if (__popc(finders) > 16) {  // (not what a row as such has to offer)
+                if (__popc(finders) > 16 && __popc(__ballot_sync(kFullMask, (hot & (hot - 1u)) != 0)) > 16) {
+                    // (most lanes have found several: not what a row as such has to offer)
                     pending |= sift<T, kHalf>(stage, vectors.column(first), hot, gate) << (h * kHalf);
                 } else {
 #pragma unroll 1
@@ -1131,14 +1153,14 @@ __global__ void __launch_bounds__(kThreads, 2) team_select_kernel(const __grid_c
     }
     // (a last warp with less than half a warp's vectors has too few keys to bound the others)
     const uint32_t warps = max(1u, min((uint32_t)kWarps, (vectors.count + vectors.span) / (2u * vectors.span)));
-    uint32_t top;
     const bool tight = k > 1u && (!one_turn || (k > kLooseMost && warps == (uint32_t)kWarps));  // (fewer warps have too few keys)
-    uint32_t low = bound_of_lanes(key, k, warps, tight, &top);
+    const uint2 first_bound = tight ? tight_bound(key, k) : loose_bound(key, k, warps);
+    uint32_t low = first_bound.x;
     if (k == 1u) {
-        low = top;
-    } else if (!tight && !(key_to_float(top) - key_to_float(low) < kFarApart)) {
+        low = first_bound.y;
+    } else if (!tight && !(key_to_float(first_bound.y) - key_to_float(low) < kFarApart)) {
         __syncthreads();  // (everybody has read what the second bound is made over)
-        low = max(low, bound_of_lanes(key, k, warps, true, &top));
+        low = max(low, tight_bound(key, k).x);
     }
     const uint64_t bound = (uint64_t)low << 32;
     if (tid == 0) sh.bound = bound;
