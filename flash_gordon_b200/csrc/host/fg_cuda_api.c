@@ -684,7 +684,7 @@ static fg_status collect_status(fg_cuda_context *c, fg_error *err) {
     else if (status == FG_ERR_MISMATCH) why = "invalid output finalist";
     else if (status == FG_ERR_LIMIT && words[1] == 1u) why = "a device-side wait ran out (a tile never landed or a warp never came)";
     else if (status == FG_ERR_LIMIT) why = "history longer than history_max";
-    else if (status == FG_ERR_ARGUMENT) why = "a penalty that can raise a logit reached the kernel for lowering penalties";
+    else if (status == FG_ERR_ARGUMENT) why = "a penalty reached a kernel that does not take it";
     fg_error_set(err, status, "row %llu: %s", (unsigned long long)row, why);
     return status;
 }
@@ -797,8 +797,8 @@ static fg_status run_stream(fg_cuda_context *c, const fg_cuda_sample_args *a,
      * rows whose penalties can, and anything the caller pinned to it, through the register-prefetch kernel.
      * A large batch with few raising rows (`both`) is two launches, one per kind of row: of the team kernel
      * where it takes the rows, else of the ring and the register-prefetch kernel.  A small batch, or one
-     * with more raising rows, is faster through one launch.  Measured with the latter two kernels (both
-     * against one, us): one row in eight raising, bf16, 100,277 logits 148 rows 88 / 85, 200 rows 87 / 130, 400
+     * with more raising rows, is faster through one launch.  Measured with the latter two kernels, whose line
+     * the team kernel's batches follow too (both against one, us): one row in eight raising, bf16, 100,277 logits 148 rows 88 / 85, 200 rows 87 / 130, 400
      * rows 119 / 234; 39,552 logits 300 rows 85 / 76, 500 rows 94 / 116.  One in four, 152 rows of 100,277 91 / 112, 300
      * of 151,936 137 / 147, 900 of 39,552 147 / 174; every other one 118 / 111, 161 / 151, 166 / 196;
      * three in four 133 / 111, 179 / 144, 186 / 175. */
@@ -863,7 +863,7 @@ static fg_status run_stream(fg_cuda_context *c, const fg_cuda_sample_args *a,
     fill_output(&l.out, c, a);
     if (c->session_counts && !(all_ring && c->path != FG_CUDA_PATH_REGISTERS && vocab_offset == 0u)) {
         /* (the executor then falls back to token lists) */
-        fg_error_set(err, FG_ERR_UNAVAILABLE, "session tables are read by the ring kernel only");
+        fg_error_set(err, FG_ERR_UNAVAILABLE, "session tables are read by the team and the ring kernel, for penalties that only lower logits");
         return FG_ERR_UNAVAILABLE;
     }
     if (c->path == FG_CUDA_PATH_RING && !(all_ring && aligned)) {

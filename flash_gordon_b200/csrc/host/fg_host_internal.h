@@ -20,7 +20,7 @@ struct fg_cuda_context {
 
     /* Set by the stateful executor around a call: the batch's penalties come from session
      * tables (counts [slots][vocab], seen-bitmaps [slots][words], one session index per row)
-     * instead of token lists.  Only the ring kernel reads them. */
+     * instead of token lists.  Only the team and the ring kernel read them. */
     const uint32_t *session_counts;
     const uint32_t *session_bitmaps;
     const uint32_t *session_rows;

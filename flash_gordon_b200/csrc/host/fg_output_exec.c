@@ -6,14 +6,14 @@
  *
  * Per session the reference keeps one table of occurrence counts, vocabulary long
  * (src/output.c:525).  So does this executor, on the device, plus a bitmap of the ids that
- * occur at all; the ring kernel fetches the bitmap (19 KB for 151,936 ids) instead of
+ * occur at all; the sampling kernel fetches the bitmap (19 KB for 151,936 ids) instead of
  * rebuilding it from the token list on every step, and reads exact counts from the table.
  * After a step the tokens picked with penalties active are added to their sessions by a
  * small kernel on the same stream (src/output.c:742, 752).
  *
  * The token lists themselves are kept on the host as well: they are what
- * fg_output_history_reset is given, and what the register-prefetch kernel needs for the
- * batches the ring kernel does not take (penalties that can raise a logit).
+ * fg_output_history_reset is given, and what a
+ * batch with penalties that can raise a logit goes by: those are not read from the tables.
  */
 #include "fg_host_internal.h"
 
@@ -212,7 +212,7 @@ fg_status fg_cuda_output_sample_sessions(fg_cuda_output_executor *x, const fg_cu
     c->session_counts = c->session_bitmaps = c->session_rows = NULL;
     c->session_bitmap_words = 0;
     if (status == FG_ERR_UNAVAILABLE && any_active) {
-        /* the ring kernel cannot take this batch: token lists through the other kernel */
+        /* the tables do not serve this batch: token lists */
         uint64_t total = 0;
         for (uint32_t r = 0; r < rows; r++) total += x->length[slots[r]];
         const size_t offsets_at = (size_t)fg_align_up_u64(total * 4u, 256u);

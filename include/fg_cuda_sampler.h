@@ -68,9 +68,11 @@ fg_status fg_cuda_context_set_splits(fg_cuda_context *context, uint32_t splits, 
  * shared-memory ring fed by bulk copies (rows whose start, stride and length are
  * multiples of 16 bytes, penalties that cannot raise a logit), or the
  * register-prefetch kernel (anything).  AUTO is the library's choice: as a rule a third kernel, in which
- * up to eight CTAs share a row; for large fp32 batches the ring kernel, with the register-prefetch
- * kernel for raising penalties, and that one alone for what neither of the others takes (negative
- * frequency penalties, extreme repetition factors).  RING fails
+ * up to eight CTAs share a row, for raising penalties and unaligned rows too.  The ring kernel takes fp32 batches whose
+ * rows all only lower: aligned ones of more than 100 M logits, long rows whose last wave of CTAs would be half
+ * empty, and greedy rows with histories of an eighth of the vocabulary.  The register-prefetch kernel takes what neither
+ * does (negative frequency penalties, extreme repetition factors, raising penalties with histories of half
+ * the vocabulary).  Rows of more than a million logits are shared out between the latter two.  RING fails
  * with FG_ERR_ARGUMENT on a batch it cannot take or whose rows are not aligned,
  * RING_IF_POSSIBLE falls back to the register-prefetch kernel instead.
  * Results never depend on it. */
