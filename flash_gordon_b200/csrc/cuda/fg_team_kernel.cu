@@ -32,7 +32,7 @@
 // under the bound too (`raw_floor`).
 //
 // 256 threads with 128 registers: with 512 threads and 64 the same steps took half as long again (four warps
-// of a scheduler in step make every instruction cost four cycles), and spilled registers are read back from L2,
+// of a scheduler in step make every instruction cost four cycles), and what they spilled was read back from L2,
 // since shared memory leaves the L1 cache nothing.  For the same reason no function that is not inlined is
 // given the kernel's parameters: it would read them through memory.
 //
